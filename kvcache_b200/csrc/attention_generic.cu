@@ -1,7 +1,7 @@
 // Causal attention over cache pages for any mix of rows, any head size and either storage
-// type: the kernel of the float32 path and the fallback of the bfloat16 one.
+// type: the kernels of the float32 path and the fallback of the bfloat16 one.
 //
-// One block per (row, query head).  The row's keys lo..pos (lo = 0, pos - window + 1 for a
+// The first: one block per (row, query head).  The row's keys lo..pos (lo = 0, pos - window + 1 for a
 // windowed layer, the first of the row's chunk for a negative `window`: first_seen_key) are visited in chunks of the block's width: each thread scores
 // one key, the block takes the chunk's maximum and sum, and threads then own output
 // dimensions for the weighted sum of values.  The running (max, sum, acc) update is the
@@ -193,4 +193,287 @@ KVB_API int kvb_paged_attention_ext(int dtype, const void* q, const void* k_page
     if (cap < 0.f) return KVB_ERR_SHAPE;
     return launch_generic(dtype, q, k_pages, v_pages ? v_pages : k_pages, block_table, table_stride, positions, row_segment, out, T,
                           Hq, Hkv, D, Dv, page_size, window, scale, err, stream, keep_first, sink, cap, slopes);
+}
+
+// ---- float32, head sizes up to 128: tiles of query rows against tiles of keys ---------------------------------------------
+// A block takes 16 TM rows (token, query head) of one segment and key/value head - all of them read the same keys - and walks
+// the keys in tiles of 64 counted from position 0, so that a row meets the same tiles in the same order however the step was
+// cut and whatever TM is: a tile of which a row sees nothing leaves its sums as they are.  Thread (ty, tx) of 16 x 16 scores
+// rows ty + 16 i against keys tx + 16 j, four numbers along the head at a time, and then owns output columns 4 tx + 64 c.
+// K and V tiles come in by `cp.async`, the next pair while this one is worked on (rows of K start 4 numbers off a multiple of
+// 32: eight keys lie in different banks).  A row's maximum and sum run over the 16 lanes that share it.
+// Bound by the shared-memory loads beside the multiply-adds.  Measured against a block per (row, head), which reads every key
+// from L2 for each of them: 1,000 rows of 14 heads of 64: 2,008 -> 117 us; 512 rows of 16 heads of 128 behind 2,048 keys:
+// 9,935 -> 541 us; 16 decoded tokens with 4,000 keys, 14 heads of 64: 672 -> 268 us; 160 rows of 3 heads of 20 in chunks of 48
+// tokens, the least it was tried at: 12 -> 14 us.
+namespace rows32 {
+
+__device__ __forceinline__ void copy16(float* smem, const float* global, bool there) {
+    const int bytes = there ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(global), "r"(bytes)
+                 : "memory");
+}
+
+struct Params {
+    const float* q;
+    const float* k_pages;
+    const float* v_pages;
+    float* out;
+    const int* block_table;
+    const int* seg_q_start;
+    const int* seg_q_len;
+    const int* seg_kv_len;
+    const float* sink;
+    const float* slopes;
+    int* err;
+    int table_stride, segments, Hq, Hkv, D, Dv, page_size, reach, keep_first;
+    float scale, cap;
+};
+
+constexpr int BN = 64, PS = BN + 4;
+
+// acc += weights of BN keys . their values.  PARTIAL: a weight below zero marks a key that the row does not see, whose value is
+// left out whatever it holds (a later token's may be infinite).
+template <int TM, int CD, bool PARTIAL>
+__device__ __forceinline__ void weigh(const float* ps, const float* vt, float4 (&acc)[TM][CD]) {
+    constexpr int VS = CD * 64;
+#pragma unroll 2
+    for (int k = 0; k < BN; k += 4) {
+        float4 w[TM];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) w[i] = *(const float4*)(ps + 16 * i * PS + k);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int c = 0; c < CD; ++c) {
+                const float4 v = *(const float4*)(vt + (k + kk) * VS + 64 * c);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const float e = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
+                    if (PARTIAL && e < 0.f) continue;
+                    acc[i][c].x = fmaf(e, v.x, acc[i][c].x);
+                    acc[i][c].y = fmaf(e, v.y, acc[i][c].y);
+                    acc[i][c].z = fmaf(e, v.z, acc[i][c].z);
+                    acc[i][c].w = fmaf(e, v.w, acc[i][c].w);
+                }
+            }
+    }
+}
+
+template <int TM, int CD>      // CD: 64-column groups of a value row
+__global__ void __launch_bounds__(256) attention_rows_kernel(const Params p) {
+    constexpr int BM = 16 * TM, VS = CD * 64;
+    extern __shared__ __align__(16) float sm[];
+    const int KS = p.D + 4;
+    float* qs = sm;                        // [BM][KS]
+    float* ps = qs + BM * KS;              // [BM][PS]
+    float* ks = ps + BM * PS;              // [2][BN][KS]
+    float* vs = ks + 2 * BN * KS;          // [2][BN][VS]
+    __shared__ int where[3 * BN];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int group = p.Hq / p.Hkv, hk = blockIdx.y;
+    pdl_wait();
+    pdl_launch_dependents();
+
+    // Which segment and which of its tiles: segments take ceil(rows * group / BM) blocks each, the last tiles (most keys) first.
+    int seg = 0, tile = (int)gridDim.x - 1 - (int)blockIdx.x;
+    for (; seg < p.segments; ++seg) {
+        const int mine = (p.seg_q_len[seg] * group + BM - 1) / BM;
+        if (tile < mine) break;
+        tile -= mine;
+    }
+    if (seg == p.segments) return;
+    const int q_len = p.seg_q_len[seg], q_first = p.seg_q_start[seg], start = p.seg_kv_len[seg] - q_len;
+    const int m0 = tile * BM, rows = min(BM, q_len * group - m0);
+    const int* table = p.block_table + (size_t)seg * p.table_stride;
+
+    auto q_at = [&](int m) { return (size_t)(q_first + (m0 + m) / group) * p.Hq + hk * group + (m0 + m) % group; };
+    for (int c = tid; c < BM * (p.D / 4); c += 256) {
+        const int m = c / (p.D / 4), d = (c % (p.D / 4)) * 4;
+        *(float4*)(qs + m * KS + d) = m < rows ? *(const float4*)(p.q + q_at(m) * p.D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    int pos[TM], lo[TM];
+    float m_run[TM], l_run[TM], slope[TM];
+    float4 acc[TM][CD];
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int m = min(ty + 16 * i, rows - 1), h = hk * group + (m0 + m) % group;
+        pos[i] = start + (m0 + m) / group;
+        lo[i] = first_seen_key(pos[i], p.reach);
+        slope[i] = p.slopes ? p.slopes[h] : 0.f;
+        m_run[i] = p.sink ? p.sink[h] : -FLT_MAX;
+        l_run[i] = p.sink ? 1.f : 0.f;
+#pragma unroll
+        for (int c = 0; c < CD; ++c) acc[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const int end = start + (m0 + rows - 1) / group + 1;                       // keys any row of the tile sees end here ...
+    const int lo_first = first_seen_key(start + m0 / group, p.reach), lo_last = first_seen_key(end - 1, p.reach);
+    const int first = lo_first / BN;                                           // ... and start in this tile, kept ones apart
+    const int kept_tiles = min((min(p.keep_first, first * BN) + BN - 1) / BN, first);
+    const int tiles = kept_tiles + (end + BN - 1) / BN - first;
+
+    auto key_of = [&](int t) { return (t < kept_tiles ? t : first + t - kept_tiles) * BN; };
+    // Where the keys of tile t lie (a row of the pools, or -1), looked up two tiles ahead by one thread a key.
+    auto look_up = [&](int t) {
+        const int j = key_of(t) + tid;
+        if (t >= tiles || j >= end) return -1;
+        const int page = table[j / p.page_size];
+        if (page >= 0) return (page * p.Hkv + hk) * p.page_size + j % p.page_size;
+        // A page is wanted only if some row of the tile sees the key (a window's earlier pages have been given back).
+        if (j >= lo_first || j < p.keep_first) atomicOr(p.err, KVB_DEV_BAD_PAGE);
+        return -1;
+    };
+    auto fetch = [&](int t) {                          // a key row: 16 threads
+        float* kd = ks + (t & 1) * BN * KS;
+        float* vd = vs + (t & 1) * BN * VS;
+#pragma unroll
+        for (int r = ty; r < BN; r += 16) {
+            const int at = where[(t % 3) * BN + r];
+            const size_t row = at >= 0 ? at : 0;
+            for (int d = tx * 4; d < p.D; d += 64) copy16(kd + r * KS + d, p.k_pages + row * p.D + d, at >= 0);
+#pragma unroll
+            for (int c = 0; c < CD; ++c) {
+                const int d = tx * 4 + 64 * c;
+                copy16(vd + r * VS + d, p.v_pages + row * p.Dv + (d < p.Dv ? d : 0), at >= 0 && d < p.Dv);
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+
+    if (tid < BN) {
+        where[tid] = look_up(0);
+        where[BN + tid] = look_up(1);
+    }
+    __syncthreads();
+    fetch(0);
+    for (int t = 0; t < tiles; ++t) {
+        if (t + 1 < tiles) {
+            fetch(t + 1);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        const int later = tid < BN ? look_up(t + 2) : -1;
+        __syncthreads();
+        const int j0 = key_of(t);
+        const float* kt = ks + (t & 1) * BN * KS + tx * KS;
+        const float* vt = vs + (t & 1) * BN * VS + tx * 4;
+        const float* qt = qs + ty * KS;
+        float s[TM][4];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 4
+        for (int d = 0; d < p.D; d += 4) {
+            float4 a[TM];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) a[i] = *(const float4*)(qt + 16 * i * KS + d);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 b = *(const float4*)(kt + 16 * j * KS + d);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].x, b.x, s[i][j]);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].y, b.y, s[i][j]);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].z, b.z, s[i][j]);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].w, b.w, s[i][j]);
+            }
+        }
+        unsigned there = 0;                            // keys whose page is missing (flagged above) are seen by nobody
+#pragma unroll
+        for (int j = 0; j < 4; ++j) there |= where[(t % 3) * BN + tx + 16 * j] >= 0 ? 1u << j : 0u;
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            float top = -FLT_MAX;
+            unsigned seen = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int key = j0 + tx + 16 * j;
+                if ((there >> j & 1) && key <= pos[i] && (key >= lo[i] || key < p.keep_first)) {
+                    float v = __fmul_rn(s[i][j], p.scale);       // one rounding sequence in every instance of the kernel
+                    if (p.cap > 0.f) v = __fmul_rn(p.cap, tanhf(v / p.cap));
+                    if (p.slopes) v = fmaf(-slope[i], (float)(pos[i] - key), v);
+                    s[i][j] = v;
+                    seen |= 1u << j;
+                    top = fmaxf(top, v);
+                }
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            const float m_new = fmaxf(m_run[i], top), corr = expf(m_run[i] - m_new);
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float e = (seen >> j & 1) ? expf(s[i][j] - m_new) : 0.f;
+                ps[(ty + 16 * i) * PS + tx + 16 * j] = (seen >> j & 1) ? e : -1.f;
+                sum += e;
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            l_run[i] = fmaf(l_run[i], corr, sum);
+            m_run[i] = m_new;
+#pragma unroll
+            for (int c = 0; c < CD; ++c) {
+                acc[i][c].x *= corr; acc[i][c].y *= corr; acc[i][c].z *= corr; acc[i][c].w *= corr;
+            }
+        }
+        const bool whole = j0 + BN - 1 <= start + m0 / group && (j0 >= lo_last || j0 + BN <= p.keep_first);
+        const bool held = __syncthreads_and(there == 15u);   // (rows past the segment's last carry its last row's position)
+        if (whole && held) weigh<TM, CD, false>(ps + ty * PS, vt, acc);
+        else weigh<TM, CD, true>(ps + ty * PS, vt, acc);
+        if (tid < BN) where[((t + 2) % 3) * BN + tid] = later;
+        __syncthreads();                               // the tile's stage is free for the one after next
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int m = ty + 16 * i;
+        if (m >= rows) continue;
+        const float l = l_run[i];
+#pragma unroll
+        for (int c = 0; c < CD; ++c) {
+            const int d = tx * 4 + 64 * c;
+            if (d >= p.Dv) continue;
+            const float4 a = acc[i][c];
+            *(float4*)(p.out + q_at(m) * p.Dv + d) = l > 0.f ? make_float4(a.x / l, a.y / l, a.z / l, a.w / l) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+}
+
+template <int TM, int CD>
+static int launch(const Params& p, int T, cudaStream_t stream) {
+    const int smem = (int)sizeof(float) * (16 * TM * (p.D + 4) + 16 * TM * PS + 2 * BN * (p.D + 4) + 2 * BN * CD * 64);
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<TM, CD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    const long long blocks = ((long long)T * (p.Hq / p.Hkv) + 16 * TM - 1) / (16 * TM) + p.segments;
+    if (blocks > 0x7fffffffLL || p.Hkv > 65535) return KVB_ERR_LIMIT;
+    kvb_launch(attention_rows_kernel<TM, CD>, dim3((unsigned)blocks, p.Hkv), dim3(256), smem, stream, p);
+    return kvb_launch_status();
+}
+
+}  // namespace rows32
+
+// float32, D and Dv up to 128 in steps of 4, every option of `kvb_paged_attention_ext`; rows by segment: segment s is rows
+// seg_q_start[s] .. + seg_q_len[s], the last of its seg_kv_len[s] positions.  `seg_rows`: the longest segment's rows.
+KVB_API int kvb_paged_attention_rows32(const void* q, const void* k_pages, const void* v_pages, const int* block_table, int table_stride,
+                                       const int* seg_q_start, const int* seg_q_len, const int* seg_kv_len, void* out, int T,
+                                       int segments, int seg_rows, int Hq, int Hkv, int D, int Dv, int page_size, int reach,
+                                       int keep_first, const float* sink, float scale, float cap, const float* slopes, int* err,
+                                       cudaStream_t stream) {
+    if (T <= 0 || segments <= 0) return KVB_OK;
+    if (D < 4 || D > 128 || D % 4 || Dv < 4 || Dv > 128 || Dv % 4 || Hkv < 1 || Hq % Hkv != 0 || v_pages == k_pages || keep_first < 0 || cap < 0.f)
+        return KVB_ERR_SHAPE;
+    if (((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)out) % 16 != 0) return KVB_ERR_ALIGN;
+    rows32::Params p{(const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out, block_table, seg_q_start, seg_q_len,
+                     seg_kv_len, sink, slopes, err, table_stride, segments, Hq, Hkv, D, Dv, page_size, reach,
+                     reach > 0 ? keep_first : 0, scale, cap};
+    // The most rows a block that one segment fills and that leave every SM a block: fewer reads of the keys, more rows per load.
+    const long long all = (long long)T * (Hq / Hkv), one = (long long)seg_rows * (Hq / Hkv), sms = kvb_sm_count();
+    const int tm = one > 32 && (all + 63) / 64 * Hkv >= sms ? 4 : one > 16 && (all + 31) / 32 * Hkv >= sms ? 2 : 1;
+    if (Dv <= 64) return tm == 4 ? rows32::launch<4, 1>(p, T, stream) : tm == 2 ? rows32::launch<2, 1>(p, T, stream) : rows32::launch<1, 1>(p, T, stream);
+    return tm == 4 ? rows32::launch<4, 2>(p, T, stream) : tm == 2 ? rows32::launch<2, 2>(p, T, stream) : rows32::launch<1, 2>(p, T, stream);
 }

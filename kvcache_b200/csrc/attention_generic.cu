@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(256) attention_rows_kernel(const Params p) {
 template <int TM, int CD>
 static int launch(const Params& p, int T, cudaStream_t stream) {
     const int smem = (int)sizeof(float) * (16 * TM * (p.D + 4) + 16 * TM * PS + 2 * BN * (p.D + 4) + 2 * BN * CD * 64);
-    if (smem > 48 * 1024) {
+    if (smem > 44 * 1024) {                            // (the kernel has some shared memory of its own beside it)
         cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<TM, CD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
     }

@@ -45,6 +45,7 @@ ROWS32 = [
     ([(700, 70), (3, 90)], 3, 1, 20, 4, 16, dict(chunk=48)),
     ([(0, 130), (900, 300)], 16, 2, 128, 128, 32, dict(window=64)),
     ([(200, 700)], 2, 2, 128, 100, 64, {}),
+    ([(30, 1), (3, 2)], 2, 1, 16, 16, 16, {}),                                           # shared memory right below what needs no asking for
 ]
 
 

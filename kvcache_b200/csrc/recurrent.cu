@@ -402,6 +402,14 @@ __global__ void channel_decay_kernel(float* __restrict__ z, size_t total, float 
         z[i] = expf(log_sigmoid(z[i]) / tau);
 }
 
+// z = sigmoid(z)^(1 / tau), element by element: the decays of the channel-decay form.
+static void launch_channel_decay(float* z, size_t total, float tau, cudaStream_t stream) {
+    size_t blocks = (total + 255) / 256;
+    const size_t most = (size_t)kvb_sm_count() * 16;
+    if (blocks > most) blocks = most;
+    kvb_launch(channel_decay_kernel, dim3((int)blocks), dim3(256), 0, stream, z, total, tau);
+}
+
 // Launch (2) of the chunked form: a thread per element of a (segment, head)'s state walks the segment's chunks in order.
 template <int MODE>
 __global__ void scan_chunk_starts_kernel(const int* __restrict__ seg_q_len, const int* __restrict__ seg_slot,
@@ -658,11 +666,7 @@ static int scan_any(int mode, const float* proj, int P, int q_col, int k_col, in
     }
     if (mode == SCAN_CHANNEL_DECAY) {
         if (g0 != 0 || gate_stride != H * D) return KVB_ERR_SHAPE;       // the logits are rows of their own
-        const size_t total = (size_t)T * H * D;
-        size_t blocks = (total + 255) / 256;
-        const size_t most = (size_t)kvb_sm_count() * 16;
-        if (blocks > most) blocks = most;
-        if (!decays_ready) kvb_launch(channel_decay_kernel, dim3((int)blocks), dim3(256), 0, stream, const_cast<float*>(gate), total, p0);
+        if (!decays_ready) launch_channel_decay(const_cast<float*>(gate), (size_t)T * H * D, p0, stream);
     }
     // A column's key channels over KS lanes, so that a lane holds at most 64 of them (measured at 128 key channels: 64 a
     // lane took 312 us where 128 took 489 and 32 took 475; at 64 key channels one lane a column 129 us, four 160);
@@ -699,6 +703,12 @@ static int scan_any(int mode, const float* proj, int P, int q_col, int k_col, in
 #undef KVB_SCAN_KS
 #undef KVB_SCAN
     if (rc != KVB_OK) return rc;
+    return kvb_launch_status();
+}
+
+KVB_API int kvb_channel_decay(float* z, long long total, float tau, cudaStream_t stream) {
+    if (total <= 0) return KVB_OK;
+    launch_channel_decay(z, (size_t)total, tau, stream);
     return kvb_launch_status();
 }
 
@@ -775,15 +785,29 @@ __global__ void delta_rule_inputs_kernel(const float* __restrict__ proj, int P, 
 // S' = diag(w) S - (a u)(u^T S) + k v^T, out = S'^T r.  proj: float32 [T, P] with r, k, v and the removal logits at their
 // columns (H * D numbers each); z: float32 [T, H * D], the decay logits; aux: float32 [T, 3 * H * D] of scratch.
 // `max_chunks` > 0: the chunked form, as for the other scans, with `scratch` of max_chunks * H * (3 D D + 2 D + 3) floats.
+static int launch_delta_rule_inputs(const float* proj, int P, int k_col, int a_col, const float* z, float rate, float unit_eps, float* aux,
+                                    int T, int H, int D, cudaStream_t stream) {
+    const int pairs = T * H, warps = 4;
+    kvb_launch(delta_rule_inputs_kernel, dim3((pairs + warps - 1) / warps), dim3(32 * warps), 0, stream, proj, P, k_col, a_col, z, rate,
+               unit_eps, aux, pairs, H, D);
+    return kvb_launch_status();
+}
+// aux [T, 3 * H * D] = [decays | unit keys | removals], what the scan reads besides the projections.
+KVB_API int kvb_delta_rule_inputs(const float* proj, int P, int k_col, int a_col, const float* z, float rate, float unit_eps, float* aux,
+                                  int T, int H, int D, cudaStream_t stream) {
+    if (T <= 0) return KVB_OK;
+    if (H < 1 || D < 1 || aux == nullptr) return KVB_ERR_SHAPE;
+    return launch_delta_rule_inputs(proj, P, k_col, a_col, z, rate, unit_eps, aux, T, H, D, stream);
+}
+
 KVB_API int kvb_delta_rule_scan(const float* proj, int P, int r_col, int k_col, int v_col, int a_col, const float* z, float rate,
                                 float unit_eps, float* aux, const int* seg_q_start, const int* seg_q_len, const int* seg_slot,
                                 float* memory, float* out, int T, int S, int H, int D, int chunk_len, int max_chunks, float* scratch,
                                 cudaStream_t stream) {
     if (S <= 0 || T <= 0) return KVB_OK;
     if (H < 1 || D < 1 || aux == nullptr) return KVB_ERR_SHAPE;
-    const int pairs = T * H, warps = 4;
-    kvb_launch(delta_rule_inputs_kernel, dim3((pairs + warps - 1) / warps), dim3(32 * warps), 0, stream, proj, P, k_col, a_col, z, rate,
-               unit_eps, aux, pairs, H, D);
+    const int rc = launch_delta_rule_inputs(proj, P, k_col, a_col, z, rate, unit_eps, aux, T, H, D, stream);
+    if (rc != KVB_OK) return rc;
     return scan_any(SCAN_DELTA_RULE, proj, P, r_col, k_col, v_col, aux, 3 * H * D, 0, H * D, 0.f, 1.f, 0.f, seg_q_start, seg_q_len,
                     seg_slot, memory, nullptr, nullptr, out, T, S, H, D, D, chunk_len, max_chunks, scratch, stream);
 }

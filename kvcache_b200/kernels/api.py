@@ -114,6 +114,9 @@ _SIGNATURES = {
                                 _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p,
                                 _c_void_p],
         "kvb_delta_rule_set_lanes": [_c_int],
+        "kvb_channel_decay": [_c_void_p, _c_longlong, _c_float, _c_void_p],
+        "kvb_delta_rule_inputs": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_float, _c_void_p, _c_int, _c_int, _c_int,
+                                  _c_void_p],
         "kvb_head_norm_gate": [_c_int, _c_void_p, _c_void_p, _c_int, _c_float, _c_void_p, _c_int, _c_int, _c_int, _c_float, _c_void_p,
                                _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
         "kvb_head_gate": [_c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_float, _c_void_p, _c_int, _c_int, _c_int, _c_int,
@@ -133,6 +136,13 @@ _SIGNATURES = {
                                _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
         "kvb_bigram_embed": [_c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                              _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
+    },
+    "scan_chunk": {
+        "kvb_chunk_record_floats": [_c_int, _c_int],
+        "kvb_chunk_shared_floats": [_c_int, _c_int],
+        "kvb_chunk_scan": [_c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p,
+                           _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p,
+                           _c_void_p],
     },
     "scan_wide": {
         "kvb_gated_delta_scan_wide": [_c_void_p, _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int,
@@ -300,6 +310,7 @@ class CudaKernels(KernelSet):
         self._latent = _Library("latent")
         self._recurrent = _Library("recurrent")
         self._scan_wide = _Library("scan_wide")
+        self._scan_chunk = _Library("scan_chunk")
         self._moe = _Library("moe")
         self._latent_flash = _Library("latent_flash")
         self._gemm_grouped = _Library("gemm_grouped")
@@ -1315,12 +1326,15 @@ class CudaKernels(KernelSet):
     DELTA_LONG_ROWS = 1536           # the delta rule: steps whose longest portion has at least this many rows ...
     DELTA_LONG_CHUNK = 128           # ... are cut into chunks of this many tokens
 
-    def _scan(self, mode: int, proj, q_col, k_col, v_col, gate, g0, g1, p0, q_scale, floor, batch, memory, normalizer, maximum, out,
-              H, D, Dv, workspace=None) -> None:
+    def _scan_checks(self, proj, gate, out, memory, H, D, Dv) -> None:
         if proj.dtype != torch.float32 or gate.dtype != torch.float32 or out.dtype != torch.float32 or memory.dtype != torch.float32:
             raise KernelError("the matrix-state scan takes float32 rows and states")
         if tuple(memory.shape[1:]) != (H, D, Dv):
             raise KernelError(f"the matrix-state scan wants states [slots, {H}, {D}, {Dv}], got {tuple(memory.shape)}")
+
+    def _scan(self, mode: int, proj, q_col, k_col, v_col, gate, g0, g1, p0, q_scale, floor, batch, memory, normalizer, maximum, out,
+              H, D, Dv, workspace=None) -> None:
+        self._scan_checks(proj, gate, out, memory, H, D, Dv)
         max_chunks, scratch = 0, None
         if workspace is not None and self.SCAN_CHUNK and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS:
             # Sized by the step's rows and segments alone, so that a recorded step finds the same launches.
@@ -1334,12 +1348,39 @@ class CudaKernels(KernelSet):
             _ptr(maximum), _ptr(out), proj.shape[0], batch.num_segments, H, D, Dv, self.SCAN_CHUNK, max_chunks, _ptr(scratch),
             self._stream()), "matrix_state_scan")
 
+    def _gated_linear_chunks(self, batch: StepBatch, workspace, D: int) -> bool:
+        return (workspace is not None and self.SCAN_CHUNK and D <= self.CHUNK_SCAN_MAX_DIM and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS
+                and (D > 64 or batch.max_q_len <= 1024))
+
+    # Portions go sixteen tokens at a time over the tensor cores (csrc/scan_chunk.cu) where a head has at most CHUNK_SCAN_MAX_DIM key
+    # channels.
+    CHUNK_SCAN_MAX_DIM = 128
+    CHUNK_MODES = {"gated_delta": 0, "delta_rule": 1, "channel_decay": 2, "head_decay": 3}
+
+    def _chunk_scan(self, mode: str, rows, cols, qk_div: int, gates, q_scale: float, batch: StepBatch, memory, out, H: int, D: int, Dv: int,
+                    workspace) -> None:
+        code, lib = self.CHUNK_MODES[mode], self._scan_chunk
+        T, S = rows.shape[0], batch.num_segments
+        max_chunks = T // 16 + S             # by the step's rows and segments alone, so that a recorded step finds the same launches
+        size = H * lib.kvb_chunk_record_floats(code, D) + H // qk_div * lib.kvb_chunk_shared_floats(code, D)
+        records = workspace.buffer("recurrent.chunk_records", (max_chunks * size,), torch.float32)
+        self.launches += 1 if mode == "head_decay" else 2        # the records' sums and rows, beside the walk
+        _check(lib.kvb_chunk_scan(code, _ptr(rows), rows.shape[1], *cols, qk_div, _ptr(gates), gates.shape[1], float(q_scale),
+                                  _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), _ptr(memory), _ptr(out), T, S, H, D,
+                                  Dv, max_chunks, _ptr(records), _ptr(self.error_word), self._stream()), f"{mode} (chunks)")
+
     def gated_linear_scan(self, proj: torch.Tensor, cols, z: torch.Tensor, tau: float, q_scale: float, batch: StepBatch,
                           memory: torch.Tensor, out: torch.Tensor, H: int, D: int, Dv: int, workspace=None) -> None:
         """Per segment, from and into memory[slot] ([H, D, Dv], float32): S = diag(a_t) S + k_t v_t^T, out_t = S^T (q_t q_scale),
         a_t = sigmoid(z_t)^(1 / tau) per key channel; q, k, v at columns `cols` of the float32 rows `proj`.  `z` [T, H * D] is
         overwritten by the decays."""
         self.launches += 1
+        if self._gated_linear_chunks(batch, workspace, D):
+            self._scan_checks(proj, z, out, memory, H, D, Dv)
+            self._count("matrix_state_scan")
+            _check(self._recurrent.kvb_channel_decay(_ptr(z), z.numel(), float(tau), self._stream()), "channel_decay")
+            self._chunk_scan("channel_decay", proj, tuple(cols), 1, z, q_scale, batch, memory, out, H, D, Dv, workspace)
+            return
         self._scan(0, proj, cols[0], cols[1], cols[2], z, 0, 0, tau, q_scale, 0.0, batch, memory, None, None, out, H, D, Dv, workspace)
 
     def lightning_scan(self, proj: torch.Tensor, cols, decay: torch.Tensor, batch: StepBatch, memory: torch.Tensor,
@@ -1384,6 +1425,13 @@ class CudaKernels(KernelSet):
             raise KernelError(f"the delta-rule scan wants states [slots, {H}, {D}, {D}], got {tuple(memory.shape)}")
         T = proj.shape[0]
         aux = workspace.buffer("recurrent.delta_inputs", (T, 3 * H * D), torch.float32)
+        if self.SCAN_CHUNK and D <= self.CHUNK_SCAN_MAX_DIM and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS:
+            self.launches += 1
+            self._count("delta_rule_scan")
+            _check(self._recurrent.kvb_delta_rule_inputs(_ptr(proj), proj.shape[1], cols[1], cols[3], _ptr(z), float(rate), float(unit_eps),
+                                                         _ptr(aux), T, H, D, self._stream()), "delta_rule_inputs")
+            self._chunk_scan("delta_rule", proj, tuple(cols[:3]), 1, aux, 1.0, batch, memory, out, H, D, D, workspace)
+            return
         max_chunks, scratch = 0, None
         # Long portions take longer chunks: every chunk costs a product with its transition in the launch that walks the start
         # states (measured at 14 heads of 64 / 16 heads of 128 channels, chunks of 64 against 128 tokens: 143 / 328 us against
@@ -1443,6 +1491,11 @@ class CudaKernels(KernelSet):
             raise KernelError(f"the gated delta scan wants states [slots, {H}, {D}, {Dv}], got {tuple(memory.shape)}")
         segments = (_ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), _ptr(memory), _ptr(out))
         self._count("gated_delta_scan")
+        if batch.max_q_len >= self.SCAN_WIDE_MIN_ROWS and D <= self.CHUNK_SCAN_MAX_DIM:
+            if rows.shape[1] != 2 * G * D + H * Dv or gates.shape[1] < H * D + H:
+                raise KernelError("gated_delta_scan: the rows or gates do not fit the heads")
+            self._chunk_scan("gated_delta", rows, (0, G * D, 2 * G * D), H // G, gates, q_scale, batch, memory, out, H, D, Dv, workspace)
+            return
         chunked = self.SCAN_CHUNK and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS
         if batch.max_q_len >= self.SCAN_WIDE_MIN_ROWS and (D > self.DELTA_WIDE_ABOVE or not chunked):
             _check(self._scan_wide.kvb_gated_delta_scan_wide(_ptr(rows), _ptr(gates), gates.shape[1], float(q_scale), *segments,
@@ -1476,8 +1529,10 @@ class CudaKernels(KernelSet):
             _ptr(gates), _ptr(batch.row_segment), _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), T,
             batch.num_segments, H, self._stream()), "state_space_inputs")
 
+    STATE_SPACE_CHUNK_MIN_ROWS = 512
+
     def state_space_scan(self, rows: torch.Tensor, gates: torch.Tensor, batch: StepBatch, memory: torch.Tensor, out: torch.Tensor, H: int,
-                         G: int, N: int, Dv: int) -> None:
+                         G: int, N: int, Dv: int, workspace=None) -> None:
         """Per segment, from and into memory[slot] ([H, N, Dv], float32): S = decay S + d B x^T, out = S^T C; `rows` =
         [x: H Dv | B: G N | C: G N] and `gates` = [decay: H | d: H] as `state_space_inputs` makes them (head h: group h // (H / G))."""
         self._float32_only("state_space_scan", rows, gates, memory, out)
@@ -1485,6 +1540,9 @@ class CudaKernels(KernelSet):
             raise KernelError(f"the state-space scan wants states [slots, {H}, {N}, {Dv}], got {tuple(memory.shape)}")
         segments = (_ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), _ptr(memory), _ptr(out))
         self._count("state_space_scan")
+        if workspace is not None and batch.max_q_len >= self.STATE_SPACE_CHUNK_MIN_ROWS and N <= self.CHUNK_SCAN_MAX_DIM:
+            self._chunk_scan("head_decay", rows, (H * Dv + G * N, H * Dv, 0), H // G, gates, 1.0, batch, memory, out, H, N, Dv, workspace)
+            return
         if batch.max_q_len >= self.SCAN_WIDE_MIN_ROWS:
             _check(self._scan_wide.kvb_state_space_scan_wide(_ptr(rows), _ptr(gates), *segments, batch.num_segments, H, G, N, Dv,
                                                              self._stream()), "state_space_scan (wide)")

@@ -1530,6 +1530,7 @@ class CudaKernels(KernelSet):
             batch.num_segments, H, self._stream()), "state_space_inputs")
 
     STATE_SPACE_CHUNK_MIN_ROWS = 512
+    state_space_takes_workspace = True   # `state_space_scan` takes `workspace`
 
     def state_space_scan(self, rows: torch.Tensor, gates: torch.Tensor, batch: StepBatch, memory: torch.Tensor, out: torch.Tensor, H: int,
                          G: int, N: int, Dv: int, workspace=None) -> None:

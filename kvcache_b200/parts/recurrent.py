@@ -434,7 +434,9 @@ class StateSpaceMixer(Mixer):
         k.state_space_inputs(proj, W, W + self.channels, self.conv_w, self.conv_b, ctx.state["conv"], self.dt_bias, self.rate, ctx.batch,
                              rows, gates, H)
         y = ws.buffer("recurrent.o", (T, W), torch.float32)
-        k.state_space_scan(rows, gates, ctx.batch, ctx.state["memory"], y, H, self.groups, self.state, self.vdim, ws)
+        # A kernel set may want scratch for portions of prompts.
+        more = {"workspace": ws} if getattr(k, "state_space_takes_workspace", False) else {}
+        k.state_space_scan(rows, gates, ctx.batch, ctx.state["memory"], y, H, self.groups, self.state, self.vdim, **more)
         k.gate_part_norm(y, rows, self.skip, (proj, 0), self.norm, self.eps, scale, out, out_col, H, self.vdim, self.norm_parts)
 
     def forward(self, x: torch.Tensor, ctx: LayerContext) -> torch.Tensor:

@@ -758,8 +758,12 @@ KVB_API int kvb_lightning_scan(float* proj, int P, int q_col, int k_col, int v_c
 //   aux[t, 0 * HD + h D + d] = w  = exp(-rate * sigmoid(z[t, h D + d]))            decay of key channel d
 //   aux[t, 1 * HD + h D + d] = u  = k / sqrt(sum_d k^2 + unit_eps)                 the head's unit key
 //   aux[t, 2 * HD + h D + d] = a u, a = sigmoid(proj[t, a_col + h D + d])          what the state loses along u
+// `a_bias` and `z_bias` (H * D numbers, or null) are added to the removal and decay logits first.  Bound by memory: 1,811 rows of 16
+// heads of 128, 26 us with 4 bytes a lane at a time, 20 with 16; the biases as passes of their own over the projections took 56 more.
+template <bool WIDE>          // 16 bytes at a time: rows and columns start on them, and D is a multiple of 4
 __global__ void delta_rule_inputs_kernel(const float* __restrict__ proj, int P, int k_col, int a_col, const float* __restrict__ z,
-                                         float rate, float unit_eps, float* __restrict__ aux, int pairs, int H, int D) {
+                                         const float* __restrict__ a_bias, const float* __restrict__ z_bias, float rate, float unit_eps,
+                                         float* __restrict__ aux, int pairs, int H, int D) {
     pdl_wait();
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
@@ -770,43 +774,80 @@ __global__ void delta_rule_inputs_kernel(const float* __restrict__ proj, int P, 
     const float* a = proj + (size_t)t * P + a_col + (size_t)h * D;
     const float* zr = z + (size_t)t * H * D + (size_t)h * D;
     float* dst = aux + (size_t)t * 3 * H * D + (size_t)h * D;
+    const float* ab = a_bias ? a_bias + h * D : nullptr;
+    const float* zb = z_bias ? z_bias + h * D : nullptr;
+    constexpr int N = WIDE ? 4 : 1;
+    auto load = [](const float* p, float (&v)[N]) {
+        if constexpr (WIDE) {
+            const float4 x = *(const float4*)p;
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        } else {
+            v[0] = *p;
+        }
+    };
+    auto store = [](float* p, const float (&v)[N]) {
+        if constexpr (WIDE) *(float4*)p = make_float4(v[0], v[1], v[2], v[3]);
+        else *p = v[0];
+    };
     float ss = 0.f;
-    for (int d = lane; d < D; d += 32) ss += k[d] * k[d];
+    for (int d = N * lane; d < D; d += 32 * N) {
+        float kk[N];
+        load(k + d, kk);
+#pragma unroll
+        for (int i = 0; i < N; ++i) ss += kk[i] * kk[i];
+    }
     const float inv = 1.f / sqrtf(warp_sum(ss) + unit_eps);
-    for (int d = lane; d < D; d += 32) {
-        const float u = k[d] * inv;
-        dst[d] = expf(-rate / (1.f + expf(-zr[d])));
-        dst[(size_t)H * D + d] = u;
-        dst[(size_t)2 * H * D + d] = u / (1.f + expf(-a[d]));
+    for (int d = N * lane; d < D; d += 32 * N) {
+        float kk[N], zd[N], ad[N], bias[N], w[N];
+        load(k + d, kk);
+        load(zr + d, zd);
+        load(a + d, ad);
+        if (zb) {
+            load(zb + d, bias);
+#pragma unroll
+            for (int i = 0; i < N; ++i) zd[i] += bias[i];
+        }
+        if (ab) {
+            load(ab + d, bias);
+#pragma unroll
+            for (int i = 0; i < N; ++i) ad[i] += bias[i];
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            w[i] = expf(-rate / (1.f + expf(-zd[i])));
+            kk[i] *= inv;
+            ad[i] = kk[i] / (1.f + expf(-ad[i]));
+        }
+        store(dst + d, w);
+        store(dst + (size_t)H * D + d, kk);
+        store(dst + (size_t)2 * H * D + d, ad);
     }
 }
 
-// The generalized delta rule over the tokens of every segment, from and into memory[slot] ([H, D, D], float32):
-// S' = diag(w) S - (a u)(u^T S) + k v^T, out = S'^T r.  proj: float32 [T, P] with r, k, v and the removal logits at their
-// columns (H * D numbers each); z: float32 [T, H * D], the decay logits; aux: float32 [T, 3 * H * D] of scratch.
-// `max_chunks` > 0: the chunked form, as for the other scans, with `scratch` of max_chunks * H * (3 D D + 2 D + 3) floats.
-static int launch_delta_rule_inputs(const float* proj, int P, int k_col, int a_col, const float* z, float rate, float unit_eps, float* aux,
-                                    int T, int H, int D, cudaStream_t stream) {
+static int launch_delta_rule_inputs(const float* proj, int P, int k_col, int a_col, const float* z, const float* a_bias, const float* z_bias,
+                                    float rate, float unit_eps, float* aux, int T, int H, int D, cudaStream_t stream) {
     const int pairs = T * H, warps = 4;
-    kvb_launch(delta_rule_inputs_kernel, dim3((pairs + warps - 1) / warps), dim3(32 * warps), 0, stream, proj, P, k_col, a_col, z, rate,
-               unit_eps, aux, pairs, H, D);
+    const bool wide = ((D | P | k_col | a_col) & 3) == 0 &&
+                      (((uintptr_t)proj | (uintptr_t)z | (uintptr_t)a_bias | (uintptr_t)z_bias | (uintptr_t)aux) & 15) == 0;
+    kvb_launch(wide ? delta_rule_inputs_kernel<true> : delta_rule_inputs_kernel<false>, dim3((pairs + warps - 1) / warps), dim3(32 * warps), 0,
+               stream, proj, P, k_col, a_col, z, a_bias, z_bias, rate, unit_eps, aux, pairs, H, D);
     return kvb_launch_status();
 }
 // aux [T, 3 * H * D] = [decays | unit keys | removals], what the scan reads besides the projections.
-KVB_API int kvb_delta_rule_inputs(const float* proj, int P, int k_col, int a_col, const float* z, float rate, float unit_eps, float* aux,
-                                  int T, int H, int D, cudaStream_t stream) {
+KVB_API int kvb_delta_rule_inputs(const float* proj, int P, int k_col, int a_col, const float* z, const float* a_bias, const float* z_bias,
+                                  float rate, float unit_eps, float* aux, int T, int H, int D, cudaStream_t stream) {
     if (T <= 0) return KVB_OK;
     if (H < 1 || D < 1 || aux == nullptr) return KVB_ERR_SHAPE;
-    return launch_delta_rule_inputs(proj, P, k_col, a_col, z, rate, unit_eps, aux, T, H, D, stream);
+    return launch_delta_rule_inputs(proj, P, k_col, a_col, z, a_bias, z_bias, rate, unit_eps, aux, T, H, D, stream);
 }
 
-KVB_API int kvb_delta_rule_scan(const float* proj, int P, int r_col, int k_col, int v_col, int a_col, const float* z, float rate,
-                                float unit_eps, float* aux, const int* seg_q_start, const int* seg_q_len, const int* seg_slot,
+KVB_API int kvb_delta_rule_scan(const float* proj, int P, int r_col, int k_col, int v_col, int a_col, const float* z,
+                                const float* a_bias, const float* z_bias, float rate, float unit_eps, float* aux, const int* seg_q_start, const int* seg_q_len, const int* seg_slot,
                                 float* memory, float* out, int T, int S, int H, int D, int chunk_len, int max_chunks, float* scratch,
                                 cudaStream_t stream) {
     if (S <= 0 || T <= 0) return KVB_OK;
     if (H < 1 || D < 1 || aux == nullptr) return KVB_ERR_SHAPE;
-    const int rc = launch_delta_rule_inputs(proj, P, k_col, a_col, z, rate, unit_eps, aux, T, H, D, stream);
+    const int rc = launch_delta_rule_inputs(proj, P, k_col, a_col, z, a_bias, z_bias, rate, unit_eps, aux, T, H, D, stream);
     if (rc != KVB_OK) return rc;
     return scan_any(SCAN_DELTA_RULE, proj, P, r_col, k_col, v_col, aux, 3 * H * D, 0, H * D, 0.f, 1.f, 0.f, seg_q_start, seg_q_len,
                     seg_slot, memory, nullptr, nullptr, out, T, S, H, D, D, chunk_len, max_chunks, scratch, stream);

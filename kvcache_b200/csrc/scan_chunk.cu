@@ -14,7 +14,7 @@
 //   S_C = L_C S_0 + K1^T V + K2^T Z       K_s = r(C, s) key_s
 //
 // Launches (1), a block per (chunk, head) and all of them at once, make the matrices that do not know S_0 (the "record" of the
-// chunk: sums over the channels first, then its rows) on the CUDA cores: the decays between two tokens are multiplied up one after the other and never divided by, so that
+// chunk) on the CUDA cores: the decays between two tokens are multiplied up one after the other and never divided by, so that
 // any decay down to zero is exact.  Launch (2) walks a segment's chunks in order, a block per 16 value channels of a head:
 // S^T lives in the accumulators of its warps, each with 8 KT key channels, and is at the same time the A operand of Y S_0 and
 // Q S_0 - the two fragments of `mma.sync` hold the same numbers if neighbouring channels are taken as the halves of a step of
@@ -29,7 +29,7 @@
 // What bounds it: the chain of a chunk - its products, one exchange, one wait: 0.8 us with 64 key channels, 1.2 to 1.4 with 128 -
 // times the chunks of the longest segment; the tensor pipe is idle for most of it.  Measured beside the form each replaces (us;
 // records and walk): gated delta 777 x 14 x 64 x 64: 117 -> 64, 1,500 x 16 x 128 x 128: 326 -> 154; delta rule 543 + 905 + 363 x 16 x
-// 128: 662 -> 183 (records 63), 1,000 x 14 x 64: 199 -> 90; channel decays 600 + 400 x 8 x 128 x 256: 154 -> 56; head decays 2,048 x 64 x
+// 128: 662 -> 179 (records 45, systems 11, walk 123), 1,000 x 14 x 64: 199 -> 90; channel decays 600 + 400 x 8 x 128 x 256: 154 -> 56; head decays 2,048 x 64 x
 // 128 x 64: 279 -> 189.
 // A segment's result does not depend on what else the step holds.  An infinite or undefined value spreads within its chunk of
 // sixteen tokens, in its own value channel, also to tokens before it.
@@ -81,6 +81,20 @@ struct Segments {
     int count;
 };
 
+// Which rows the step's chunk `id` covers; false beyond the last.
+__device__ __forceinline__ bool find_chunk(int id, const Segments& seg, int& r0, int& count) {
+    for (int s = 0; s < seg.count; ++s) {
+        const int n = seg.q_len[s], mine = (n + C - 1) / C;
+        if (id < mine) {
+            r0 = seg.q_start[s] + id * C;
+            count = min(C, n - id * C);
+            return true;
+        }
+        id -= mine;
+    }
+    return false;
+}
+
 // v[i]: this lane's share of 16 sums over 16 neighbouring lanes; lane `part` returns the sum of number `part`.
 __device__ __forceinline__ float sum16(float (&v)[16], int part) {
 #pragma unroll
@@ -100,171 +114,197 @@ __device__ __forceinline__ float dot4(const float4& a, const float4& b, float c)
 __device__ __forceinline__ void scale4(float4& a, const float4& b) { a.x *= b.x; a.y *= b.y; a.z *= b.z; a.w *= b.w; }
 
 // ---- launches (1): the records ---------------------------------------------------------------------------------------------
-// Sums over the channels and the triangular system: grid (chunks, heads), 256 threads.  Thread (s, part): token s as a key, channels 4 part .. + 3 of every 64.
+// grid (chunks, heads), 256 threads.  Thread (s, part): token s as a key, channels 4 part .. + 3 of every 64.
 template <int MODE, int NI>          // NI: 64-channel groups of a row
-__global__ void __launch_bounds__(256, MODE == CHUNK_DELTA_RULE && NI == 2 ? 3 : 4) chunk_sums_kernel(const Rows in, const Segments seg, float* __restrict__ records, int H, int D) {
+__global__ void __launch_bounds__(256, MODE == CHUNK_DELTA_RULE && NI == 2 ? 3 : 4) chunk_records_kernel(const Rows in, const Segments seg,
+                                                                                                       float* __restrict__ records, int H,
+                                                                                                       int D, int wide) {
     constexpr int DP = 64 * NI, PARTS = MODE == CHUNK_DELTA_RULE ? 5 : 3;
     __shared__ __align__(16) float rows_s[PARTS][C][DP];       // q, k, a (, u, c)
-    __shared__ float low_s[2][C][C + 1], mat_s[C][C + 1], b_s[C];
+    __shared__ float low_s[C][C + 1], mat_s[C][C + 1], b_s[C];
     const int tid = threadIdx.x, s = tid >> 4, part = tid & 15, h = blockIdx.y;
     pdl_wait();
     pdl_launch_dependents();
-    int id = blockIdx.x, sg = 0, n = 0;
-    for (; sg < seg.count; ++sg) {
-        n = seg.q_len[sg];
-        const int mine = (n + C - 1) / C;
-        if (id < mine) break;
-        id -= mine;
-    }
-    if (sg == seg.count) return;
-    const int r0 = seg.q_start[sg] + id * C, count = min(C, n - id * C);
+    int r0, count;
+    if (!find_chunk(blockIdx.x, seg, r0, count)) return;
     constexpr Record R = record_of(MODE, DP);
     float* rec = records + ((size_t)blockIdx.x * H + h) * R.total;
-    const int qk = h / in.qk_div * D;
 
     // Tokens beyond the segment's end change nothing: a = 1, everything else 0.  So do channels beyond D.
+    {
+        const bool row_there = s < count;
+        const float* row = in.rows + (size_t)(r0 + (row_there ? s : 0)) * in.stride + h / in.qk_div * D;
+        const float* gate = in.gates + (size_t)(r0 + (row_there ? s : 0)) * in.gate_stride + (size_t)h * D;
+        const float* from[5] = {row + in.q_col, row + in.k_col, gate, gate + (size_t)H * D, gate + (size_t)2 * H * D};
 #pragma unroll
-    for (int i = 0; i < NI; ++i)
+        for (int i = 0; i < NI; ++i) {
+            const int d = 64 * i + 4 * part;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int d = 64 * i + 4 * part + e;
-            const bool there = s < count && d < D;
-            const float* row = in.rows + (size_t)(r0 + (there ? s : 0)) * in.stride;
-            const float* gate = in.gates + (size_t)(r0 + (there ? s : 0)) * in.gate_stride + (size_t)h * D;
-            const int dd = there ? d : 0;
-            rows_s[0][s][d] = there ? row[in.q_col + qk + dd] : 0.f;
-            rows_s[1][s][d] = there ? row[in.k_col + qk + dd] : 0.f;
-            rows_s[2][s][d] = there ? gate[dd] : 1.f;
-            if (MODE == CHUNK_DELTA_RULE) {
-                rows_s[3][s][d] = there ? gate[(size_t)H * D + dd] : 0.f;
-                rows_s[4][s][d] = there ? gate[(size_t)2 * H * D + dd] : 0.f;
+            for (int x = 0; x < PARTS; ++x) {
+                const float none = x == 2 ? 1.f : 0.f;
+                float4 v = make_float4(none, none, none, none);
+                if (row_there) {
+                    if (wide) {                                    // rows start on 16 bytes and D is a multiple of 4
+                        if (d < D) v = *(const float4*)(from[x] + d);
+                    } else {
+                        if (d < D) v.x = from[x][d];
+                        if (d + 1 < D) v.y = from[x][d + 1];
+                        if (d + 2 < D) v.z = from[x][d + 2];
+                        if (d + 3 < D) v.w = from[x][d + 3];
+                    }
+                }
+                *(float4*)&rows_s[x][s][d] = v;
             }
         }
+    }
     if (MODE == CHUNK_GATED_DELTA && tid < C) b_s[tid] = tid < count ? in.gates[(size_t)(r0 + tid) * in.gate_stride + (size_t)H * D + h] : 0.f;
     __syncthreads();
 
     auto at = [&](int which, int t, int i) { return *(const float4*)&rows_s[which][t][64 * i + 4 * part]; };
-    // Sums over the channels between token s and every later one, the key decayed on the way.
-    float4 key[NI], rem[NI];
-    float qs[C], us[C], qc[C], uc[C];
+    {
+        // Sums over the channels between token s and every later one, the key decayed on the way.
+        float4 key[NI], rem[NI];
+        float qs[C], us[C], qc[C], uc[C];
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-        key[i] = at(1, s, i);
-        if (MODE == CHUNK_DELTA_RULE) rem[i] = at(4, s, i);
-    }
+        for (int i = 0; i < NI; ++i) {
+            key[i] = at(1, s, i);
+            if (MODE == CHUNK_DELTA_RULE) rem[i] = at(4, s, i);
+        }
 #pragma unroll
-    for (int t = 0; t < C; ++t) {
-        qs[t] = us[t] = qc[t] = uc[t] = 0.f;
-        if (t >= s) {
+        for (int t = 0; t < C; ++t) {
+            qs[t] = us[t] = qc[t] = uc[t] = 0.f;
+            if (t >= s) {
 #pragma unroll
-            for (int i = 0; i < NI; ++i) {
-                const float4 q = at(0, t, i);
-                if (t > s) {
-                    const float4 a = at(2, t, i);
-                    if (MODE == CHUNK_DELTA_RULE) {                    // reads the state before the token's own decay
-                        const float4 u = at(3, t, i);
-                        us[t] = dot4(u, key[i], us[t]);
-                        uc[t] = dot4(u, rem[i], uc[t]);
-                        scale4(rem[i], a);
+                for (int i = 0; i < NI; ++i) {
+                    const float4 q = at(0, t, i);
+                    if (t > s) {
+                        const float4 a = at(2, t, i);
+                        if (MODE == CHUNK_DELTA_RULE) {            // reads the state before the token's own decay
+                            const float4 u = at(3, t, i);
+                            us[t] = dot4(u, key[i], us[t]);
+                            uc[t] = dot4(u, rem[i], uc[t]);
+                            scale4(rem[i], a);
+                        }
+                        scale4(key[i], a);
+                        if (MODE == CHUNK_GATED_DELTA) us[t] = dot4(at(1, t, i), key[i], us[t]);
                     }
-                    scale4(key[i], a);
-                    if (MODE == CHUNK_GATED_DELTA) us[t] = dot4(at(1, t, i), key[i], us[t]);
+                    qs[t] = dot4(q, key[i], qs[t]);
+                    if (MODE == CHUNK_DELTA_RULE) qc[t] = dot4(q, rem[i], qc[t]);
                 }
-                qs[t] = dot4(q, key[i], qs[t]);
-                if (MODE == CHUNK_DELTA_RULE) qc[t] = dot4(q, rem[i], qc[t]);
+            }
+        }
+        // Token `part` reads key s (zero before it).
+        rec[(MODE == CHUNK_GATED_DELTA ? R.a2 : R.a1) + part * 24 + s] = sum16(qs, part);
+        if (MODE == CHUNK_GATED_DELTA) low_s[part][s] = sum16(us, part);
+        if (MODE == CHUNK_DELTA_RULE) {                            // for the next launch: u . c below the diagonal, u . k mirrored above
+            rec[R.a2 + part * 24 + s] = -sum16(qc, part);
+            const float uk = sum16(us, part), ur = sum16(uc, part);
+            if (part > s) {
+                rec[R.w + part * 24 + s] = ur;
+                rec[R.w + s * 24 + part] = uk;
             }
         }
     }
-    rec[(MODE == CHUNK_GATED_DELTA ? R.a2 : R.a1) + part * 24 + s] = sum16(qs, part);     // token `part` reads key s (zero before it)
-    if (MODE == CHUNK_DELTA_RULE) rec[R.a2 + part * 24 + s] = -sum16(qc, part);
-    if (has_z(MODE)) low_s[0][part][s] = sum16(us, part);
-    if (MODE == CHUNK_DELTA_RULE) low_s[1][part][s] = sum16(uc, part);
-    if (!has_z(MODE)) return;
-    __syncthreads();
-    // The triangular system, a thread per column; its inverse goes where Y will lie, for the launch that makes Y.
-    if (tid < C) {
-        float x[C];
+    if (MODE == CHUNK_GATED_DELTA) {
+        __syncthreads();
+        if (tid < C) {                                             // the triangular system, a thread per column
+            float x[C];
 #pragma unroll
-        for (int t = 0; t < C; ++t) {
-            float v = t == tid ? 1.f : 0.f;
+            for (int t = 0; t < C; ++t) {
+                float v = t == tid ? 1.f : 0.f;
 #pragma unroll
-            for (int j = 0; j < C; ++j)
-                if (j < t) v = fmaf(-low_s[MODE == CHUNK_DELTA_RULE ? 1 : 0][t][j], x[j], v);
-            x[t] = MODE == CHUNK_GATED_DELTA ? b_s[t] * v : v;
-            mat_s[t][tid] = x[t];
+                for (int j = 0; j < C; ++j)
+                    if (j < t) v = fmaf(-low_s[t][j], x[j], v);
+                x[t] = b_s[t] * v;
+                mat_s[t][tid] = x[t];
+            }
         }
     }
-    __syncthreads();
-    const float m = part <= s ? mat_s[s][part] : 0.f;
-    rec[R.y + s * 24 + part] = m;
-    float w = m;
-    if (MODE == CHUNK_DELTA_RULE) {
-        w = 0.f;
+    // Rows decayed from the chunk's start (the lower threads) and to its end (the upper), a thread per channel.
+    if (MODE != CHUNK_GATED_DELTA) __syncthreads();                // all have read q
+    const int d = tid % DP;
+    if (tid < DP) {
+        float run = 1.f;
 #pragma unroll
-        for (int j = 0; j < C; ++j)
-            if (j <= s && j > part) w = fmaf(mat_s[s][j], low_s[0][j][part], w);
+        for (int t = 0; t < C; ++t) {
+            const float before = run;
+            run *= rows_s[2][t][d];
+            rec[R.q + t * (DP + 8) + d] = rows_s[0][t][d] * run;
+            if (MODE == CHUNK_GATED_DELTA) rows_s[0][t][d] = rows_s[1][t][d] * run;                    // the key as it meets S_0
+            if (MODE == CHUNK_DELTA_RULE) rec[R.y + t * (DP + 8) + d] = rows_s[3][t][d] * before;
+        }
+        rec[R.decay + d] = run;
+    } else if (tid < 2 * DP) {
+        float run = 1.f;
+#pragma unroll
+        for (int t = C - 1; t >= 0; --t) {
+            rec[(has_v(MODE) ? R.k1 : R.k2) + t * (DP + 4) + d] = rows_s[1][t][d] * run;
+            if (MODE == CHUNK_DELTA_RULE) rec[R.k2 + t * (DP + 4) + d] = -rows_s[4][t][d] * run;
+            run *= rows_s[2][t][d];
+        }
     }
-    rec[R.w + s * 24 + part] = w;
+    if (MODE != CHUNK_GATED_DELTA) return;
+    __syncthreads();
+    // Y = -W . (the keys that meet S_0): thread (t = s, part).
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+            if (j <= s) {
+                const float m = -mat_s[s][j];
+                const float4 v = at(0, j, i);
+                sum.x = fmaf(m, v.x, sum.x); sum.y = fmaf(m, v.y, sum.y); sum.z = fmaf(m, v.z, sum.z); sum.w = fmaf(m, v.w, sum.w);
+            }
+        }
+        *(float4*)(rec + R.y + s * (DP + 8) + 64 * i + 4 * part) = sum;
+    }
+    rec[R.w + s * 24 + part] = part <= s ? mat_s[s][part] : 0.f;
 }
 
-// The rows of the records, decayed from the chunk's start and to its end: grid (chunks, heads), a thread per channel.
-template <int MODE, int NI>
-__global__ void __launch_bounds__(64 * NI) chunk_rows_kernel(const Rows in, const Segments seg, float* __restrict__ records, int H, int D) {
+// Delta rule: T = (1 + u . c)^-1, Y = T . (the reads that meet S_0, where Y will lie), W = T (u . k).  grid (chunks, heads), a thread
+// per channel.  By itself, because half a block would wait for the system's sixteen threads in the launch before it.
+template <int NI>
+__global__ void __launch_bounds__(64 * NI) chunk_solve_kernel(const Segments seg, float* __restrict__ records, int H) {
     constexpr int DP = 64 * NI;
-    constexpr Record R = record_of(MODE, DP);
-    __shared__ float mat_s[C][C];
-    const int d = threadIdx.x, h = blockIdx.y;
+    constexpr Record R = record_of(CHUNK_DELTA_RULE, DP);
+    __shared__ float low_s[C][C + 1], mat_s[C][C + 1];
+    const int d = threadIdx.x;
     pdl_wait();
     pdl_launch_dependents();
-    int id = blockIdx.x, sg = 0, n = 0;
-    for (; sg < seg.count; ++sg) {
-        n = seg.q_len[sg];
-        const int mine = (n + C - 1) / C;
-        if (id < mine) break;
-        id -= mine;
-    }
-    if (sg == seg.count) return;
-    const int r0 = seg.q_start[sg] + id * C, count = min(C, n - id * C);
-    float* rec = records + ((size_t)blockIdx.x * H + h) * R.total;
-    if (has_z(MODE)) {
-        for (int i = d; i < C * C; i += DP) mat_s[i / C][i % C] = rec[R.y + i / C * 24 + i % C];
-        __syncthreads();                                           // read before Y is written over it
-    }
-    const float* row = in.rows + (size_t)r0 * in.stride + h / in.qk_div * D + d;
-    const float* gate = in.gates + (size_t)r0 * in.gate_stride + (size_t)h * D + d;
-    float a[C], key[C], rem[C], x[C];
-    float run = 1.f;
+    int r0, count;
+    if (!find_chunk(blockIdx.x, seg, r0, count)) return;
+    float* rec = records + ((size_t)blockIdx.x * H + blockIdx.y) * R.total;
+    for (int i = d; i < C * C; i += DP) low_s[i / C][i % C] = i / C == i % C ? 0.f : rec[R.w + i / C * 24 + i % C];
+    float x[C];
 #pragma unroll
-    for (int t = 0; t < C; ++t) {
-        const bool there = t < count && d < D;
-        a[t] = there ? gate[(size_t)t * in.gate_stride] : 1.f;
-        const float q = there ? row[(size_t)t * in.stride + in.q_col] : 0.f;
-        key[t] = there ? row[(size_t)t * in.stride + in.k_col] : 0.f;
-        if (MODE == CHUNK_DELTA_RULE) {
-            x[t] = (there ? gate[(size_t)t * in.gate_stride + (size_t)H * D] : 0.f) * run;          // reads before the token's decay
-            rem[t] = there ? gate[(size_t)t * in.gate_stride + (size_t)2 * H * D] : 0.f;
-        }
-        run *= a[t];
-        if (MODE == CHUNK_GATED_DELTA) x[t] = key[t] * run;
-        rec[R.q + t * (DP + 8) + d] = q * run;
-    }
-    rec[R.decay + d] = run;
-    run = 1.f;
-#pragma unroll
-    for (int t = C - 1; t >= 0; --t) {
-        rec[(has_v(MODE) ? R.k1 : R.k2) + t * (DP + 4) + d] = key[t] * run;
-        if (MODE == CHUNK_DELTA_RULE) rec[R.k2 + t * (DP + 4) + d] = -rem[t] * run;
-        run *= a[t];
-    }
-    if (has_z(MODE)) {
+    for (int t = 0; t < C; ++t) x[t] = rec[R.y + t * (DP + 8) + d];
+    __syncthreads();
+    if (d < C) {
+        float v[C];
 #pragma unroll
         for (int t = 0; t < C; ++t) {
-            float y = 0.f;
+            v[t] = t == d ? 1.f : 0.f;
 #pragma unroll
             for (int j = 0; j < C; ++j)
-                if (j <= t) y = fmaf(mat_s[t][j], x[j], y);
-            rec[R.y + t * (DP + 8) + d] = MODE == CHUNK_GATED_DELTA ? -y : y;
+                if (j < t) v[t] = fmaf(-low_s[t][j], v[j], v[t]);
+            mat_s[t][d] = v[t];
         }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < C; ++t) {
+        float y = 0.f;
+#pragma unroll
+        for (int j = 0; j < C; ++j)
+            if (j <= t) y = fmaf(mat_s[t][j], x[j], y);
+        rec[R.y + t * (DP + 8) + d] = y;
+    }
+    for (int i = d; i < C * C; i += DP) {
+        const int t = i / C, s = i % C;
+        float w = 0.f;
+        for (int j = s + 1; j <= t; ++j) w = fmaf(mat_s[t][j], low_s[s][j], w);       // u . k of (j, s) lies at (s, j)
+        rec[R.w + t * 24 + s] = w;
     }
 }
 
@@ -277,15 +317,8 @@ __global__ void __launch_bounds__(256) head_records_kernel(const Rows in, const 
     const int tid = threadIdx.x, s = tid >> 4, part = tid & 15, g = blockIdx.y;
     pdl_wait();
     pdl_launch_dependents();
-    int id = blockIdx.x, sg = 0, n = 0;
-    for (; sg < seg.count; ++sg) {
-        n = seg.q_len[sg];
-        const int mine = (n + C - 1) / C;
-        if (id < mine) break;
-        id -= mine;
-    }
-    if (sg == seg.count) return;
-    const int r0 = seg.q_start[sg] + id * C, count = min(C, n - id * C);
+    int r0, count;
+    if (!find_chunk(blockIdx.x, seg, r0, count)) return;
 #pragma unroll
     for (int i = 0; i < NI; ++i)
 #pragma unroll
@@ -684,8 +717,10 @@ static int run(const Rows& in, const Segments& seg, float* records, int max_chun
         kvb_launch(head_records_kernel<NI>, dim3(max_chunks, H / in.qk_div), dim3(256), 0, stream, in, seg, records, H, D);
     else
     {
-        kvb_launch(chunk_sums_kernel<MODE, NI>, dim3(max_chunks, H), dim3(256), 0, stream, in, seg, records, H, D);
-        kvb_launch(chunk_rows_kernel<MODE, NI>, dim3(max_chunks, H), dim3(64 * NI), 0, stream, in, seg, records, H, D);
+        const int wide = ((D | in.stride | in.gate_stride | in.q_col | in.k_col) & 3) == 0 && (((uintptr_t)in.rows | (uintptr_t)in.gates) & 15) == 0;
+        kvb_launch(chunk_records_kernel<MODE, NI>, dim3(max_chunks, H), dim3(256), 0, stream, in, seg, records, H, D, wide);
+        if constexpr (MODE == CHUNK_DELTA_RULE)
+            kvb_launch(chunk_solve_kernel<NI>, dim3(max_chunks, H), dim3(64 * NI), 0, stream, seg, records, H);
     }
     const int rc = kvb_launch_status();
     if (rc != KVB_OK) return rc;

@@ -110,13 +110,13 @@ _SIGNATURES = {
         "kvb_matrix_state_scan": [_c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_float,
                                   _c_float, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                                   _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
-        "kvb_delta_rule_scan": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_float, _c_void_p, _c_void_p,
+        "kvb_delta_rule_scan": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_float, _c_float, _c_void_p, _c_void_p,
                                 _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p,
                                 _c_void_p],
         "kvb_delta_rule_set_lanes": [_c_int],
         "kvb_channel_decay": [_c_void_p, _c_longlong, _c_float, _c_void_p],
-        "kvb_delta_rule_inputs": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_float, _c_void_p, _c_int, _c_int, _c_int,
-                                  _c_void_p],
+        "kvb_delta_rule_inputs": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_float, _c_float, _c_void_p, _c_int,
+                                  _c_int, _c_int, _c_void_p],
         "kvb_head_norm_gate": [_c_int, _c_void_p, _c_void_p, _c_int, _c_float, _c_void_p, _c_int, _c_int, _c_int, _c_float, _c_void_p,
                                _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
         "kvb_head_gate": [_c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_float, _c_void_p, _c_int, _c_int, _c_int, _c_int,
@@ -1364,7 +1364,7 @@ class CudaKernels(KernelSet):
         max_chunks = T // 16 + S             # by the step's rows and segments alone, so that a recorded step finds the same launches
         size = H * lib.kvb_chunk_record_floats(code, D) + H // qk_div * lib.kvb_chunk_shared_floats(code, D)
         records = workspace.buffer("recurrent.chunk_records", (max_chunks * size,), torch.float32)
-        self.launches += 1 if mode == "head_decay" else 2        # the records' sums and rows, beside the walk
+        self.launches += 2 if mode == "delta_rule" else 1        # the records (and their triangular systems), beside the walk
         _check(lib.kvb_chunk_scan(code, _ptr(rows), rows.shape[1], *cols, qk_div, _ptr(gates), gates.shape[1], float(q_scale),
                                   _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), _ptr(memory), _ptr(out), T, S, H, D,
                                   Dv, max_chunks, _ptr(records), _ptr(self.error_word), self._stream()), f"{mode} (chunks)")
@@ -1414,22 +1414,29 @@ class CudaKernels(KernelSet):
         self._scan(1, proj, cols[0], cols[1], cols[2], proj, cols[3], cols[4], cap, q_scale, floor, batch, memory, normalizer, maximum,
                    out, H, D, Dv, workspace)
 
+    delta_rule_adds_bias = True          # `delta_rule_scan` takes `bias`
+
     def delta_rule_scan(self, proj: torch.Tensor, cols, z: torch.Tensor, rate: float, unit_eps: float, batch: StepBatch,
-                        memory: torch.Tensor, out: torch.Tensor, H: int, D: int, workspace) -> None:
-        """Per segment, from and into memory[slot] ([H, D, D], float32): w = exp(-rate sigmoid(z)) per key channel,
+                        memory: torch.Tensor, out: torch.Tensor, H: int, D: int, workspace, bias=(None, None)) -> None:
+        """`bias` = (removal, decay), float32 [H * D] each or None: added to the removal logits and to `z` where they are read.
+        Per segment, from and into memory[slot] ([H, D, D], float32): w = exp(-rate sigmoid(z)) per key channel,
         u = k / sqrt(sum k^2 + unit_eps) per head, a = sigmoid(removal logits); S = diag(w) S - (a u)(u^T S) + k v^T (both
         terms read the old state), out = S^T r; r, k, v and the removal logits at columns `cols` of the float32 rows `proj`."""
         if proj.dtype != torch.float32 or z.dtype != torch.float32 or out.dtype != torch.float32 or memory.dtype != torch.float32:
             raise KernelError("the delta-rule scan takes float32 rows and states")
         if tuple(memory.shape[1:]) != (H, D, D) or z.shape[1] != H * D:
             raise KernelError(f"the delta-rule scan wants states [slots, {H}, {D}, {D}], got {tuple(memory.shape)}")
+        for b in bias:
+            if b is not None and (b.dtype != torch.float32 or b.numel() != H * D):
+                raise KernelError("the delta-rule scan's biases are one float32 number per head and key channel")
+        a_bias, z_bias = (_ptr(b) for b in bias)
         T = proj.shape[0]
         aux = workspace.buffer("recurrent.delta_inputs", (T, 3 * H * D), torch.float32)
         if self.SCAN_CHUNK and D <= self.CHUNK_SCAN_MAX_DIM and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS:
             self.launches += 1
             self._count("delta_rule_scan")
-            _check(self._recurrent.kvb_delta_rule_inputs(_ptr(proj), proj.shape[1], cols[1], cols[3], _ptr(z), float(rate), float(unit_eps),
-                                                         _ptr(aux), T, H, D, self._stream()), "delta_rule_inputs")
+            _check(self._recurrent.kvb_delta_rule_inputs(_ptr(proj), proj.shape[1], cols[1], cols[3], _ptr(z), a_bias, z_bias, float(rate),
+                                                         float(unit_eps), _ptr(aux), T, H, D, self._stream()), "delta_rule_inputs")
             self._chunk_scan("delta_rule", proj, tuple(cols[:3]), 1, aux, 1.0, batch, memory, out, H, D, D, workspace)
             return
         max_chunks, scratch = 0, None
@@ -1445,7 +1452,7 @@ class CudaKernels(KernelSet):
         self.launches += 1
         self._count("delta_rule_scan")
         _check(self._recurrent.kvb_delta_rule_scan(
-            _ptr(proj), proj.shape[1], cols[0], cols[1], cols[2], cols[3], _ptr(z), float(rate), float(unit_eps), _ptr(aux),
+            _ptr(proj), proj.shape[1], cols[0], cols[1], cols[2], cols[3], _ptr(z), a_bias, z_bias, float(rate), float(unit_eps), _ptr(aux),
             _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), _ptr(memory), _ptr(out), T, batch.num_segments,
             H, D, chunk, max_chunks, _ptr(scratch), self._stream()), "delta_rule_scan")
 

@@ -217,7 +217,7 @@ class DeltaRuleMixer(_MatrixStateMixer):
         super().__init__(hidden, num_heads, dim, dim, eps=eps, prefix=prefix, dtype=dtype)
         self.decay_rank = decay_rank          # None: whatever the checkpoint's Ww1 and Ww2 agree on
         self.a_col = self.g_col + self.heads_width
-        self.w_w1 = self.w_w2 = self.b_w2 = None
+        self.w_w1 = self.w_w2 = self.b_w2 = self.b_a = None
 
     def tensor_specs(self) -> Dict[str, TensorSpec]:
         p, n = self.prefix, self.qk_size
@@ -234,6 +234,7 @@ class DeltaRuleMixer(_MatrixStateMixer):
         bias = torch.zeros(self.w_in.shape[0], dtype=torch.float32)
         bias[self.a_col:self.a_col + self.qk_size] = tensors[p + "a.b"].to(torch.float32)
         self.b_in = bias.to(device).contiguous()
+        self.b_a = self.b_in[self.a_col:self.a_col + self.qk_size].contiguous()
         if tensors[p + "w1"].shape[0] != tensors[p + "w2"].shape[1]:
             raise WeightError(f"{p}w1 has {tensors[p + 'w1'].shape[0]} rows but {p}w2 has {tensors[p + 'w2'].shape[1]} columns")
         self.w_w1, self.w_w2 = self._place(tensors[p + "w1"], device), self._place(tensors[p + "w2"], device)
@@ -250,15 +251,18 @@ class DeltaRuleMixer(_MatrixStateMixer):
     def forward_heads(self, x: torch.Tensor, ctx: LayerContext, out: torch.Tensor, out_col: int = 0, scale: float = 1.0) -> None:
         T = x.shape[0]
         k, ws = ctx.kernels, ctx.workspace
-        proj = self._project(x, ctx)
+        # A kernel set may add the biases where the scan reads the logits, instead of passing over the projections for them.
+        adds = getattr(k, "delta_rule_adds_bias", False)
+        proj = ws.buffer("recurrent.proj", (T, self.w_in.shape[0]), torch.float32)
+        k.linear(x, self.w_in, proj, None if adds else self.b_in)
         low = ws.buffer("recurrent.low", (T, self.w_w1.shape[0]), self.dtype)
         k.linear(x, self.w_w1, low)
         k.activation_(low, "tanh")
         z = ws.buffer("recurrent.z", (T, self.qk_size), torch.float32)
-        k.linear(low, self.w_w2, z, self.b_w2)
+        k.linear(low, self.w_w2, z, None if adds else self.b_w2)
         o = ws.buffer("recurrent.o", (T, self.heads_width), torch.float32)
         k.delta_rule_scan(proj, (self.q_col, self.k_col, self.v_col, self.a_col), z, self.DECAY_RATE, self.UNIT_KEY_EPS, ctx.batch,
-                          ctx.state["memory"], o, self.num_heads, self.dim, ws)
+                          ctx.state["memory"], o, self.num_heads, self.dim, ws, **({"bias": (self.b_a, self.b_w2)} if adds else {}))
         k.head_norm_gate(o, self.norm, self.eps, (proj, self.g_col), "sigmoid", scale, out, out_col, self.num_heads, self.dim)
 
 

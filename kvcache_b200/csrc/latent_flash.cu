@@ -7,8 +7,10 @@
 //
 // A block of 8 warps owns BM = 16 * MT rows and a run of keys [kb, ke) (a work item made on the host, see
 // kernels/latent_plan.py).  Per tile of 64 keys, brought by cp.async into rows padded by 16 bytes:
-//   scores   warp w takes keys 8 w .. 8 w + 7 for all MT row tiles (mma.sync m16n8k16 over Dk), scaled to base 2,
-//            masked (causal by the row's own position, window) and written to shared memory as float32;
+//   scores   a warp takes one of the MT row tiles and an MT-th of the keys (mma.sync m16n8k16 over Dk), scaled to base 2,
+//            masked (causal by the row's own position, window) and written to shared memory as float32 (with a warp on eight
+//            keys of every row tile, Q was read from shared memory eight times a tile and bound it: 2,048 rows of 16 heads, keys
+//            of 576, 448 -> 404 us; 1,024 rows behind 1,024 of 14 heads, keys of 288, 200 -> 177; tiles of 48 keys in two stages: the same);
 //   softmax  float32: running maximum and sum per row, p = 2^(s - m) rounded to bfloat16 for the second product,
 //            the sum taken from the unrounded p;
 //   values   warp w owns output columns [8 NV w, 8 NV (w + 1)) for all row tiles: O = O * 2^(m_old - m_new) + P . V,
@@ -86,6 +88,7 @@ __global__ void __launch_bounds__(THREADS, (MT == 4 && NV <= 4) ? 2 : 1) latent_
     const int* __restrict__ seg_kv_len, float* __restrict__ part_o, float* __restrict__ part_ml, int H, int Dk, int Dv,
     int page_size, int window, float scale_log2, int nsplit, int nstage, const float* __restrict__ sink, int* __restrict__ err) {
     constexpr int BM = 16 * MT;
+    constexpr int SN = 8 / MT, NT = BN / (8 * SN);          // scores: warps along the keys, and tiles of eight keys a warp
     extern __shared__ __align__(16) unsigned char smem[];
     const Layout L = make_layout(MT, NV, Dk, nstage);
     bf16* Qs = reinterpret_cast<bf16*>(smem + L.q_off);
@@ -164,41 +167,44 @@ __global__ void __launch_bounds__(THREADS, (MT == 4 && NV <= 4) ? 2 : 1) latent_
         const bf16* Kt = Ks + (size_t)stage * BN * L.rs;
         const int key0 = kb + tile * BN;
 
-        // ---- scores of keys 8 warp .. 8 warp + 7 for every row tile ------------------------------------------------
-        float s[MT][4];
+        // ---- scores: a warp takes one row tile and NT tiles of eight keys, so that Q and the keys are read SN and MT times ----
+        const int mt = warp / SN, key_first = (warp % SN) * 8 * NT;
+        float s[NT][4];
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) s[mt][0] = s[mt][1] = s[mt][2] = s[mt][3] = 0.f;
-#pragma unroll 3
+        for (int nt = 0; nt < NT; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+        constexpr int AHEAD = MT == 4 ? 2 : 3;
+#pragma unroll AHEAD
         for (int k2 = 0; k2 < KS2; ++k2) {
-            uint32_t b[4];
-            ldmatrix_x4(b[0], b[1], b[2], b[3], Kt + (size_t)(8 * warp + (lane & 7)) * L.rs + k2 * 32 + (lane >> 3) * 8);
+            uint32_t a[2][4];
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
+            for (int half = 0; half < 2; ++half)
+                ldmatrix_x4(a[half][0], a[half][1], a[half][2], a[half][3],
+                            Qs + (size_t)(mt * 16 + (lane & 15)) * L.qs + k2 * 32 + half * 16 + (lane >> 4) * 8);
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    uint32_t a[4];
-                    ldmatrix_x4(a[0], a[1], a[2], a[3], Qs + (size_t)(mt * 16 + (lane & 15)) * L.qs + k2 * 32 + half * 16 + (lane >> 4) * 8);
-                    mma_bf16(s[mt], a, b[2 * half], b[2 * half + 1]);
-                }
+            for (int nt = 0; nt < NT; ++nt) {
+                uint32_t b[4];
+                ldmatrix_x4(b[0], b[1], b[2], b[3], Kt + (size_t)(key_first + 8 * nt + (lane & 7)) * L.rs + k2 * 32 + (lane >> 3) * 8);
+                mma_bf16(s[nt], a[0], b[0], b[1]);
+                mma_bf16(s[nt], a[1], b[2], b[3]);
             }
         }
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
+        for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
             for (int hi = 0; hi < 2; ++hi) {             // rows g and g + 8: two columns each, stored as one 8-byte word
                 const int r = mt * 16 + g + hi * 8;
-                const int c = 8 * warp + 2 * t4;
+                const int c = key_first + 8 * nt + 2 * t4;
                 const int pos = rowpos[r];
                 float2 v;
                 {
                     const int j = key0 + c;
                     const bool seen = j < ke && j <= pos && (window <= 0 || j > pos - window);
-                    v.x = seen ? s[mt][2 * hi] * scale_log2 : MASKED;
+                    v.x = seen ? s[nt][2 * hi] * scale_log2 : MASKED;
                 }
                 {
                     const int j = key0 + c + 1;
                     const bool seen = j < ke && j <= pos && (window <= 0 || j > pos - window);
-                    v.y = seen ? s[mt][2 * hi + 1] * scale_log2 : MASKED;
+                    v.y = seen ? s[nt][2 * hi + 1] * scale_log2 : MASKED;
                 }
                 *reinterpret_cast<float2*>(Ss + r * L.ss + c) = v;
             }

@@ -322,6 +322,179 @@ __global__ void __launch_bounds__(mt::THREADS) head_linear_mma_kernel(const bf16
     }
 }
 
+// The same for more than 16 rows: tiles of BM x 128 outputs, 64 of K at a time in a ring of stages, the rotated columns made while
+// the first are on their way, the gates asked for before the product, the result through shared memory to rows of 16 bytes.  K is
+// walked in the same order as above: the same bits.  WM x WN warps.  Bound by the writes (prompts) and by the latency of W and x.
+// Tiles of 64 x 64 with 32 of K in two stages, 4-byte stores and one of eight blocks on all of a tile's rotated columns took, for 16 heads
+// of 128 -> 512 (+ 64 rotated) and 512 -> 128 with gates: 28 and 25 us at 32 rows (now 9 and 15), 43 and 29 at 200 (12 and 16), 72 and 43 at 2,048 (40 and 43).
+namespace hl {
+constexpr int BN = 128, BK = 64, STRIDE = BK + 8, OUT_STRIDE = BN + 8;
+template <int BM, int STAGES> __host__ __device__ constexpr int smem_bytes() { return STAGES * (BM + BN) * STRIDE * 2; }     // the result fits in what the stages leave
+}
+template <int BM, int WM, int WN, int STAGES, bool CHANNEL_GATE>      // a gate for every number, or one a head (or none)
+__global__ void __launch_bounds__(32 * WM * WN) head_linear_wide_kernel(const bf16* __restrict__ x, int xs, int x_ld, const bf16* __restrict__ w,
+                                                                        bf16* __restrict__ out, int os, int M, int N, int K, int H,
+                                                                        const bf16* __restrict__ gate, int gs, int gc, int rot,
+                                                                        int rot_half, const float* __restrict__ cos_t,
+                                                                        const float* __restrict__ sin_t, int table_len,
+                                                                        const int* __restrict__ positions, int* __restrict__ err) {
+    constexpr int BN = hl::BN, BK = hl::BK, STRIDE = hl::STRIDE, THREADS = 32 * WM * WN, CH = BK / 8;
+    constexpr int MT = BM / WM / 16, NT = BN / WN / 8;
+    static_assert(NT % 2 == 0 && BM * hl::OUT_STRIDE * 2 <= hl::smem_bytes<BM, STAGES>(), "");
+    extern __shared__ __align__(16) unsigned char hl_smem[];
+    bf16* as = reinterpret_cast<bf16*>(hl_smem);                   // [STAGES][BM][STRIDE]
+    bf16* ws = as + STAGES * BM * STRIDE;                          // [STAGES][BN][STRIDE]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp / WN, wn = warp % WN;
+    const int h = blockIdx.z, m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const bf16* xh = x + (size_t)h * xs;
+    const bf16* wh = w + ((size_t)h * N + n0) * K;
+    const int steps = (K + BK - 1) / BK, n_valid = min(BN, N - n0);
+    auto load_w = [&](int step) {                                  // no kernel writes weights
+        bf16* dst = ws + (step % STAGES) * BN * STRIDE;
+        for (int e = tid; e < BN * CH; e += THREADS) {
+            const int r = e / CH, c = (e % CH) * 8, k = step * BK + c;
+            const bool valid = r < n_valid && k < K;
+            mt::cp_async16(dst + r * STRIDE + c, valid ? wh + (size_t)r * K + k : w, valid);
+        }
+    };
+    auto load_x = [&](int step) {
+        bf16* dst = as + (step % STAGES) * BM * STRIDE;
+        for (int e = tid; e < BM * CH; e += THREADS) {
+            const int r = e / CH, c = (e % CH) * 8, k = step * BK + c;
+            const bool valid = m0 + r < M && k < K;
+            mt::cp_async16(dst + r * STRIDE + c, valid ? xh + (size_t)(m0 + r) * x_ld + k : w, valid);
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s)
+        if (s < steps) load_w(s);
+    pdl_wait();
+    pdl_launch_dependents();
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < steps) load_x(s);
+        mt::cp_async_commit();
+    }
+    // The rotated columns, while the first steps are on their way: the blocks of a row tile share its rows, a thread takes both
+    // numbers of a pair (or one that is not rotated).
+    if (rot > 0) {
+        const int items = rot - rot_half, per = (BM + (int)gridDim.x - 1) / (int)gridDim.x, first = blockIdx.x * per;
+        const int rows = min(min(per, BM - first), M - m0 - first);
+        for (int e = tid; e < rows * items; e += THREADS) {
+            const int row = e / items, i = e - row * items, gm = m0 + first + row;
+            const int pos = positions[gm];
+            const bool pos_ok = pos >= 0 && pos < table_len;
+            if (!pos_ok) atomicOr(err, KVB_DEV_BAD_POS);
+            const bf16* src = xh + (size_t)gm * x_ld + K;
+            bf16* dst = out + (size_t)gm * H * os + (size_t)h * os + N;
+            if (i < rot_half) {
+                float v = __bfloat162float(src[i]), vp = __bfloat162float(src[i + rot_half]);
+                if (pos_ok) {
+                    const float c = cos_t[(size_t)pos * rot_half + i], s = sin_t[(size_t)pos * rot_half + i];
+                    const float low = v * c - vp * s;
+                    vp = vp * c + v * s;
+                    v = low;
+                }
+                dst[i] = __float2bfloat16_rn(v);
+                dst[i + rot_half] = __float2bfloat16_rn(vp);
+            } else {
+                dst[i + rot_half] = src[i + rot_half];
+            }
+        }
+    }
+    // The gates of this thread's results are asked for before the product.
+    const int g = lane >> 2, t4 = lane & 3;
+    float2 gates[MT][2][NT];
+    if (CHANNEL_GATE) {
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int hi = 0; hi < 2; ++hi)
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    const int gm = m0 + wm * MT * 16 + i * 16 + g + 8 * hi, gn = n0 + wn * NT * 8 + j * 8 + 2 * t4;
+                    const bool there = gm < M && gn < N;           // N is even
+                    const bf16* gp = gate + (there ? (size_t)gm * gs + gc + (size_t)h * os + gn : 0);
+                    gates[i][hi][j] = there ? make_float2(__bfloat162float(gp[0]), __bfloat162float(gp[1])) : make_float2(0.f, 0.f);
+                }
+    }
+    float acc[MT][NT][4];
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
+    for (int s = 0; s < steps; ++s) {
+        mt::cp_async_wait<STAGES - 2>();
+        __syncthreads();                                           // step s is there, and all are done with the stage refilled now
+        if (s + STAGES - 1 < steps) {
+            load_w(s + STAGES - 1);
+            load_x(s + STAGES - 1);
+        }
+        mt::cp_async_commit();
+        const bf16* at = as + (s % STAGES) * BM * STRIDE + (wm * MT * 16 + (lane & 15)) * STRIDE + (lane >> 4) * 8;
+        const bf16* wt = ws + (s % STAGES) * BN * STRIDE + (wn * NT * 8 + (lane & 7) + (lane >> 4) * 8) * STRIDE + ((lane >> 3) & 1) * 8;
+#pragma unroll
+        for (int ks = 0; ks < BK / 16; ++ks) {
+            uint32_t a[MT][4];
+#pragma unroll
+            for (int i = 0; i < MT; ++i) mt::ldmatrix_x4(a[i][0], a[i][1], a[i][2], a[i][3], at + i * 16 * STRIDE + ks * 16);
+#pragma unroll
+            for (int j = 0; j < NT; j += 2) {
+                uint32_t b[4];
+                mt::ldmatrix_x4(b[0], b[1], b[2], b[3], wt + j * 8 * STRIDE + ks * 16);
+#pragma unroll
+                for (int i = 0; i < MT; ++i) {
+                    mt::mma_bf16(acc[i][j], a[i], b[0], b[1]);
+                    mt::mma_bf16(acc[i][j + 1], a[i], b[2], b[3]);
+                }
+            }
+        }
+    }
+    mt::cp_async_wait<0>();
+    __syncthreads();                                               // the stages become the result's tile
+    bf16* tile = as;
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int hi = 0; hi < 2; ++hi) {
+            const int r = wm * MT * 16 + i * 16 + g + 8 * hi, gm = m0 + r;
+            float head_gate = 1.f;
+            if (!CHANNEL_GATE && gate && gm < M) head_gate = 1.f / (1.f + expf(-__bfloat162float(gate[(size_t)gm * gs + gc + h])));
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                const int c = wn * NT * 8 + j * 8 + 2 * t4;
+                float v0 = acc[i][j][2 * hi], v1 = acc[i][j][2 * hi + 1];
+                if (!CHANNEL_GATE) {
+                    v0 *= head_gate;
+                    v1 *= head_gate;
+                } else {
+                    v0 *= 1.f / (1.f + expf(-gates[i][hi][j].x));
+                    v1 *= 1.f / (1.f + expf(-gates[i][hi][j].y));
+                }
+                *reinterpret_cast<__nv_bfloat162*>(tile + r * hl::OUT_STRIDE + c) = __floats2bfloat162_rn(v0, v1);
+            }
+        }
+    __syncthreads();
+    for (int e = tid; e < BM * (BN / 8); e += THREADS) {
+        const int r = e / (BN / 8), c = (e % (BN / 8)) * 8;
+        if (m0 + r < M && n0 + c < N)
+            *reinterpret_cast<uint4*>(out + (size_t)(m0 + r) * H * os + (size_t)h * os + n0 + c) =
+                *reinterpret_cast<const uint4*>(tile + r * hl::OUT_STRIDE + c);
+    }
+}
+
+template <int BM, int WM, int WN, int STAGES>
+static int launch_head_linear_wide(const bf16* x, int xs, int x_ld, const bf16* w, bf16* out, int os, int M, int N, int K, int H,
+                                   const bf16* gate, int gs, int gc, int gate_heads, int rot, int rot_half, const float* cos_t,
+                                   const float* sin_t, int table_len, const int* positions, int* err, cudaStream_t stream) {
+    auto kernel = gate && !gate_heads ? head_linear_wide_kernel<BM, WM, WN, STAGES, true> : head_linear_wide_kernel<BM, WM, WN, STAGES, false>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hl::smem_bytes<BM, STAGES>());
+    if (e != cudaSuccess) return (int)e;
+    kvb_launch(kernel, dim3((N + hl::BN - 1) / hl::BN, (M + BM - 1) / BM, H), dim3(32 * WM * WN), hl::smem_bytes<BM, STAGES>(), stream, x, xs, x_ld, w,
+               out, os, M, N, K, H, gate, gs, gc, rot, rot_half, cos_t, sin_t, table_len, positions, err);
+    return kvb_launch_status();
+}
+
 template <typename T, int BM>
 static void launch_head_linear(const T* x, int xs, int x_ld, const T* w, T* out, int os, int M, int N, int K, int H, const T* gate, int gs,
                                int gc, int gate_heads, int rot, int rot_half, const float* cos_t, const float* sin_t, int table_len,
@@ -347,6 +520,16 @@ KVB_API int kvb_head_linear(int dtype, const void* x, int xs, int x_ld, const vo
                              (uintptr_t)out % 4 == 0;
         if (aligned && getenv("KVB_HEAD_LINEAR_SIMT") == nullptr) {
             const bf16 *xb = (const bf16*)x, *wb = (const bf16*)w, *gb = (const bf16*)gate;
+            // Rows of the result that start on 16 bytes; tiles of 32 rows with four stages while few of them fill the GPU, then of 64 rows with
+            // two, so that more blocks share an SM (2,048 rows of 16 heads, 128 -> 512: 41 us, 82 with tiles of 32, 49 with 128).
+            if (M > 16 && N % 8 == 0 && os % 8 == 0 && (uintptr_t)out % 16 == 0) {
+const long long small = (long long)((N + hl::BN - 1) / hl::BN) * ((M + 31) / 32) * H;
+                return small <= 2 * kvb_sm_count()
+                           ? launch_head_linear_wide<32, 1, 4, 4>(xb, xs, x_ld, wb, (bf16*)out, os, M, N, K, H, gb, gs, gc, gate_heads, rot,
+                                                                  rot_half, cos_t, sin_t, table_len, positions, err, stream)
+                           : launch_head_linear_wide<64, 2, 4, 2>(xb, xs, x_ld, wb, (bf16*)out, os, M, N, K, H, gb, gs, gc, gate_heads, rot,
+                                                                  rot_half, cos_t, sin_t, table_len, positions, err, stream);
+            }
             if (M <= 16)
                 kvb_launch(head_linear_mma_kernel<1>, dim3((N + 63) / 64, (M + 15) / 16, H), dim3(mt::THREADS), 0, stream, xb, xs, x_ld, wb,
                            (bf16*)out, os, M, N, K, H, gb, gs, gc, gate_heads, rot, rot_half, cos_t, sin_t, table_len, positions, err);

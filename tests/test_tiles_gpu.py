@@ -165,3 +165,41 @@ def test_scan_in_chunks(kernels, mode, lens, H, G, D, Dv):
         assert ((got.double() - ref).norm() / ref.norm()).item() <= 2e-6
     alone, memory_alone = run([0], 0)
     assert torch.equal(alone, out[:lens[0]]) and torch.equal(memory_alone[slots[0]], memory[slots[0]])
+
+
+@pytest.mark.parametrize("M", [17, 32, 33, 65, 300])
+@pytest.mark.parametrize("H,N,K,rot,gate", [(3, 512, 128, 64, None), (3, 128, 512, 0, "channel"), (5, 136, 72, 24, "head"), (20, 8, 8, 3, None)])
+def test_head_products_in_tiles(kernels, M, H, N, K, rot, gate):
+    """More than 16 rows: remainders of rows, outputs and K, rotated columns (an odd number of them not rotated), both kinds of gate;
+    and every row bit for bit what sixteen rows at a time give."""
+    g = torch.Generator().manual_seed(61)
+    rot_half = rot // 4
+    rot_pad = rot + -rot % 8 if rot else 0                                   # rows of x and of the result start on 16 bytes
+    if rot_pad != rot:
+        rot = rot_pad
+    x = torch.randn(M, H * (K + rot), generator=g).to(torch.bfloat16)
+    w = torch.randn(H, N, K, generator=g).to(torch.bfloat16)
+    gates = torch.randn(M, 8 + H * (N + rot), generator=g).to(torch.bfloat16)
+    positions = torch.randperm(400, generator=g)[:M].to(torch.int32)
+    cos, sin = torch.randn(400, max(rot_half, 1), generator=g), torch.randn(400, max(rot_half, 1), generator=g)
+
+    def run(rows):
+        out = torch.full((rows.stop - rows.start, H * (N + rot)), float("nan"), dtype=torch.bfloat16, device=DEV)
+        more = {}
+        if rot:
+            more["rotate"] = (cos.to(DEV), sin.to(DEV), positions[rows].contiguous().to(DEV))
+        if gate:
+            more.update(gate=(gates[rows].contiguous().to(DEV), 8), gate_per_head=gate == "head")
+        kernels.head_linear(x[rows].contiguous().to(DEV), w.to(DEV), out, **more)
+        kernels.check_errors()
+        return out.cpu()
+
+    out = run(slice(0, M))
+    assert torch.equal(out, torch.cat([run(slice(i, min(i + 16, M))) for i in range(0, M, 16)]))
+    xs = x.view(M, H, K + rot).double()
+    want = torch.einsum("mhk,hnk->mhn", xs[:, :, :K], w.double())
+    if gate:
+        logits = gates[:, 8:8 + H].double()[:, :, None] if gate == "head" else gates[:, 8:].double().view(M, H, N + rot)[:, :, :N]
+        want = want * torch.sigmoid(logits)
+    # float32 sums of K products, rounded to 8 bits of fraction once.
+    assert_close(out.view(M, H, N + rot)[:, :, :N], want, 2.0 ** -8 + K * 2.0 ** -22)

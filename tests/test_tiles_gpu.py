@@ -203,3 +203,26 @@ def test_head_products_in_tiles(kernels, M, H, N, K, rot, gate):
         want = want * torch.sigmoid(logits)
     # float32 sums of K products, rounded to 8 bits of fraction once.
     assert_close(out.view(M, H, N + rot)[:, :, :N], want, 2.0 ** -8 + K * 2.0 ** -22)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,H,Dv,parts", [(3, 5, 4, 1), (7, 3, 64, 3), (130, 2, 128, 2), (5, 64, 64, 1)])
+def test_gated_norms_in_fours(kernels, dtype, T, H, Dv, parts):
+    """Rows that start on 16 bytes go four numbers at a time; the same rows one column further go one at a time: the same results but
+    for the order of a sum of W squares (at most W 2^-24 of it) and one rounding to the result's type."""
+    W = H * Dv
+    rand = lambda *s: torch.randn(*s, generator=torch.Generator(device=DEV).manual_seed(len(s) * 7 + s[0]), device=DEV)
+    o, x, skip, w, head_w = rand(T, W), rand(T, W + 8), rand(H), rand(W), rand(Dv)
+    aligned, shifted = torch.zeros(T, W + 8, device=DEV), torch.zeros(T, W + 9, device=DEV)
+    aligned[:, 4:4 + W] = rand(T, W) * 3
+    shifted[:, 5:5 + W] = aligned[:, 4:4 + W]
+    results = []
+    for gate, col, width in ((aligned, 4, W + 12), (shifted, 5, W + 13)):
+        part, head = (torch.full((T, width), 7.0, dtype=dtype, device=DEV) for _ in range(2))
+        kernels.gate_part_norm(o, x, skip, (gate, col), w, 1e-6, 0.5, part, col + 4, H, Dv, parts)
+        kernels.head_norm_gate(o, head_w, 1e-6, (gate, col), "silu", 0.5, head, col + 4, H, Dv)
+        for r in (part, head):
+            assert (r[:, :col + 4] == 7.0).all() and (r[:, col + 4 + W:] == 7.0).all()
+        results.append((part[:, col + 4:col + 4 + W], head[:, col + 4:col + 4 + W]))
+    for a, b in zip(*results):
+        assert_close(a, b, 2.0 ** -7 if dtype == torch.bfloat16 else 1e-6 + W * 2.0 ** -24)

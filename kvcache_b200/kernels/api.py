@@ -1349,6 +1349,8 @@ class CudaKernels(KernelSet):
             self._stream()), "matrix_state_scan")
 
     def _gated_linear_chunks(self, batch: StepBatch, workspace, D: int) -> bool:
+        """Sixteen tokens at a time: 600 + 400 rows of 8 heads of 128 x 256 56 us against 154, 1,000 rows of 7 heads of 64 x 128 58
+        against 68; 2,048 rows of those 112 against 105, which chunks of 64 side by side take."""
         return (workspace is not None and self.SCAN_CHUNK and D <= self.CHUNK_SCAN_MAX_DIM and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS
                 and (D > 64 or batch.max_q_len <= 1024))
 
@@ -1482,10 +1484,11 @@ class CudaKernels(KernelSet):
             float(unit_eps), _ptr(rows), _ptr(gates), gates.shape[1], _ptr(batch.row_segment), _ptr(batch.seg_q_start), _ptr(batch.seg_q_len),
             _ptr(batch.seg_slot), T, batch.num_segments, H, G, D, Dv, self._stream()), "gated_delta_inputs")
 
-    # Portions of at least SCAN_WIDE_MIN_ROWS rows go through the scan that spreads a column over many lanes (csrc/scan_wide.cu):
-    # the state space always (28 heads of 128 x 64: 40 us at 64 rows in one piece, 15 us), the gated delta rule where a head has more
-    # key channels than DELTA_WIDE_ABOVE (2,048 rows, 16 heads of 128: 818 us in chunks, 454 us); with fewer, portions long enough
-    # for chunks that run side by side take those (14 heads of 64: 235 us at 2,048 rows, 527 us).
+    # Portions of at least SCAN_WIDE_MIN_ROWS rows leave the walk over tokens in one piece: the gated delta rule with up to
+    # CHUNK_SCAN_MAX_DIM key channels goes sixteen tokens at a time (64 rows of 14 heads of 64: 13 us, 25 with a column over many
+    # lanes, 58 in one piece), with more through the scan that spreads a column over many lanes (csrc/scan_wide.cu; where a head has
+    # no more than DELTA_WIDE_ABOVE, portions long enough for chunks of SCAN_CHUNK side by side take those).  The state space
+    # spreads its columns (28 heads of 128 x 64: 40 us at 64 rows in one piece, 15 us) up to STATE_SPACE_CHUNK_MIN_ROWS.
     SCAN_WIDE_MIN_ROWS = 48
     DELTA_WIDE_ABOVE = 64
 
@@ -1536,6 +1539,8 @@ class CudaKernels(KernelSet):
             _ptr(gates), _ptr(batch.row_segment), _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), T,
             batch.num_segments, H, self._stream()), "state_space_inputs")
 
+    # From here on sixteen tokens at a time: 45 us against 53 (a column over many lanes) at 512 rows of 28 heads of 128 x 64, 54 against
+    # 73 with 64 heads, 189 against 279 at 2,048 rows of 64; level at 256 rows.
     STATE_SPACE_CHUNK_MIN_ROWS = 512
     state_space_takes_workspace = True   # `state_space_scan` takes `workspace`
 

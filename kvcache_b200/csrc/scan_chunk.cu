@@ -729,13 +729,26 @@ static int run(const Rows& in, const Segments& seg, float* records, int max_chun
     return launch_walk<MODE, NI, 2 * NI, 2>(in, seg, records, max_chunks, q_scale, memory, out, H, D, Dv, err, stream);
 }
 
+// Whether the columns that the heads read lie within a row of `rows` and of `gates` (the decays of CHUNK_CHANNEL_DECAY are rows of
+// their own).
+static bool rows_fit(int mode, const Rows& in, int H, int G, int D, int Dv) {
+    const long long qk = (long long)G * D, a = (long long)H * D;
+    if (in.q_col < 0 || in.k_col < 0 || in.v_col < 0 || in.q_col + qk > in.stride || in.k_col + qk > in.stride ||
+        in.v_col + (long long)H * Dv > in.stride)
+        return false;
+    if (mode == CHUNK_CHANNEL_DECAY) return in.gate_stride == a;
+    return in.gate_stride >= (mode == CHUNK_GATED_DELTA ? a + H : mode == CHUNK_DELTA_RULE ? 3 * a : 2LL * H);
+}
+
 template <int MODE>
 static int run(const Rows& in, const Segments& seg, float* records, int max_chunks, float q_scale, float* memory, float* out, int T, int H,
-               int D, int Dv, int* err, cudaStream_t stream) {
+               int G, int D, int Dv, int* err, cudaStream_t stream) {
+    if (H < 1 || G < 1 || H % G || D < 1 || Dv < 1 || !rows_fit(MODE, in, H, G, D, Dv)) return KVB_ERR_SHAPE;
     if (seg.count <= 0 || T <= 0) return KVB_OK;
-    if (H < 1 || D < 1 || Dv < 1 || in.qk_div < 1 || H % in.qk_div || records == nullptr) return KVB_ERR_SHAPE;
+    if (records == nullptr) return KVB_ERR_SHAPE;
     if ((uintptr_t)records & 15) return KVB_ERR_ALIGN;
     if (D > 128 || H > 65535 || seg.count > 65535 || max_chunks < T / C + seg.count) return KVB_ERR_LIMIT;
+    if (MODE == CHUNK_CHANNEL_DECAY && Dv > 512) return KVB_ERR_LIMIT;      // as the other forms of this scan
     return D <= 64 ? run<MODE, 1>(in, seg, records, max_chunks, q_scale, memory, out, H, D, Dv, err, stream)
                    : run<MODE, 2>(in, seg, records, max_chunks, q_scale, memory, out, H, D, Dv, err, stream);
 }
@@ -749,17 +762,17 @@ KVB_API int kvb_chunk_record_floats(int mode, int D) {
 // ... and what a (chunk, group of heads that share q and k) takes besides.
 KVB_API int kvb_chunk_shared_floats(int mode, int D) { return mode < 0 || mode > 3 || D < 1 ? -1 : sc::record_of(mode, sc::padded(D)).shared; }
 
-// The scans over portions of prompts.  `rows` [T, stride] holds q, k and v at their columns (head h: number h / qk_div of D for q and k,
-// number h of Dv for v), `gates` [T, gate_stride] the mode's own numbers (sc::Rows); `records`: scratch of max_chunks (at least
-// T / 16 + S) times the floats above for all heads and groups, on 16 bytes.  D up to 128.
-KVB_API int kvb_chunk_scan(int mode, const float* rows, int stride, int q_col, int k_col, int v_col, int qk_div, const float* gates,
+// The scans over portions of prompts.  `rows` [T, stride] holds q, k and v at their columns (head h: number h / (H / G) of D for q and k,
+// number h of Dv for v; H a multiple of G), `gates` [T, gate_stride] the mode's own numbers (sc::Rows); `records`: scratch of max_chunks
+// (at least T / 16 + S) times the floats above for all H heads and G groups, on 16 bytes.  D up to 128.
+KVB_API int kvb_chunk_scan(int mode, const float* rows, int stride, int q_col, int k_col, int v_col, int G, const float* gates,
                            int gate_stride, float q_scale, const int* seg_q_start, const int* seg_q_len, const int* seg_slot, float* memory,
                            float* out, int T, int S, int H, int D, int Dv, int max_chunks, float* records, int* err, cudaStream_t stream) {
-    const sc::Rows in = {rows, gates, stride, gate_stride, q_col, k_col, v_col, qk_div};
+    const sc::Rows in = {rows, gates, stride, gate_stride, q_col, k_col, v_col, G > 0 ? H / G : 0};
     const sc::Segments seg = {seg_q_start, seg_q_len, seg_slot, S};
-    if (mode == sc::CHUNK_GATED_DELTA) return sc::run<sc::CHUNK_GATED_DELTA>(in, seg, records, max_chunks, q_scale, memory, out, T, H, D, Dv, err, stream);
-    if (mode == sc::CHUNK_DELTA_RULE) return sc::run<sc::CHUNK_DELTA_RULE>(in, seg, records, max_chunks, q_scale, memory, out, T, H, D, Dv, err, stream);
-    if (mode == sc::CHUNK_CHANNEL_DECAY) return sc::run<sc::CHUNK_CHANNEL_DECAY>(in, seg, records, max_chunks, q_scale, memory, out, T, H, D, Dv, err, stream);
-    if (mode == sc::CHUNK_HEAD_DECAY) return sc::run<sc::CHUNK_HEAD_DECAY>(in, seg, records, max_chunks, q_scale, memory, out, T, H, D, Dv, err, stream);
+    if (mode == sc::CHUNK_GATED_DELTA) return sc::run<sc::CHUNK_GATED_DELTA>(in, seg, records, max_chunks, q_scale, memory, out, T, H, G, D, Dv, err, stream);
+    if (mode == sc::CHUNK_DELTA_RULE) return sc::run<sc::CHUNK_DELTA_RULE>(in, seg, records, max_chunks, q_scale, memory, out, T, H, G, D, Dv, err, stream);
+    if (mode == sc::CHUNK_CHANNEL_DECAY) return sc::run<sc::CHUNK_CHANNEL_DECAY>(in, seg, records, max_chunks, q_scale, memory, out, T, H, G, D, Dv, err, stream);
+    if (mode == sc::CHUNK_HEAD_DECAY) return sc::run<sc::CHUNK_HEAD_DECAY>(in, seg, records, max_chunks, q_scale, memory, out, T, H, G, D, Dv, err, stream);
     return KVB_ERR_SHAPE;
 }

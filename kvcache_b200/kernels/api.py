@@ -1359,15 +1359,17 @@ class CudaKernels(KernelSet):
     CHUNK_SCAN_MAX_DIM = 128
     CHUNK_MODES = {"gated_delta": 0, "delta_rule": 1, "channel_decay": 2, "head_decay": 3}
 
-    def _chunk_scan(self, mode: str, rows, cols, qk_div: int, gates, q_scale: float, batch: StepBatch, memory, out, H: int, D: int, Dv: int,
+    def _chunk_scan(self, mode: str, rows, cols, G: int, gates, q_scale: float, batch: StepBatch, memory, out, H: int, D: int, Dv: int,
                     workspace) -> None:
+        if G < 1 or H % G:
+            raise KernelError(f"{mode}: {H} heads cannot share {G} queries and keys evenly")
         code, lib = self.CHUNK_MODES[mode], self._scan_chunk
         T, S = rows.shape[0], batch.num_segments
         max_chunks = T // 16 + S             # by the step's rows and segments alone, so that a recorded step finds the same launches
-        size = H * lib.kvb_chunk_record_floats(code, D) + H // qk_div * lib.kvb_chunk_shared_floats(code, D)
+        size = H * lib.kvb_chunk_record_floats(code, D) + G * lib.kvb_chunk_shared_floats(code, D)
         records = workspace.buffer("recurrent.chunk_records", (max_chunks * size,), torch.float32)
         self.launches += 2 if mode == "delta_rule" else 1        # the records (and their triangular systems), beside the walk
-        _check(lib.kvb_chunk_scan(code, _ptr(rows), rows.shape[1], *cols, qk_div, _ptr(gates), gates.shape[1], float(q_scale),
+        _check(lib.kvb_chunk_scan(code, _ptr(rows), rows.shape[1], *cols, G, _ptr(gates), gates.shape[1], float(q_scale),
                                   _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), _ptr(memory), _ptr(out), T, S, H, D,
                                   Dv, max_chunks, _ptr(records), _ptr(self.error_word), self._stream()), f"{mode} (chunks)")
 
@@ -1379,9 +1381,11 @@ class CudaKernels(KernelSet):
         self.launches += 1
         if self._gated_linear_chunks(batch, workspace, D):
             self._scan_checks(proj, z, out, memory, H, D, Dv)
+            if z.shape[1] != H * D or z.shape[0] < proj.shape[0]:
+                raise KernelError(f"gated_linear_scan wants decay logits [{proj.shape[0]}, {H * D}], got {tuple(z.shape)}")
             self._count("matrix_state_scan")
-            _check(self._recurrent.kvb_channel_decay(_ptr(z), z.numel(), float(tau), self._stream()), "channel_decay")
-            self._chunk_scan("channel_decay", proj, tuple(cols), 1, z, q_scale, batch, memory, out, H, D, Dv, workspace)
+            _check(self._recurrent.kvb_channel_decay(_ptr(z), proj.shape[0] * H * D, float(tau), self._stream()), "channel_decay")
+            self._chunk_scan("channel_decay", proj, tuple(cols), H, z, q_scale, batch, memory, out, H, D, Dv, workspace)
             return
         self._scan(0, proj, cols[0], cols[1], cols[2], z, 0, 0, tau, q_scale, 0.0, batch, memory, None, None, out, H, D, Dv, workspace)
 
@@ -1439,7 +1443,7 @@ class CudaKernels(KernelSet):
             self._count("delta_rule_scan")
             _check(self._recurrent.kvb_delta_rule_inputs(_ptr(proj), proj.shape[1], cols[1], cols[3], _ptr(z), a_bias, z_bias, float(rate),
                                                          float(unit_eps), _ptr(aux), T, H, D, self._stream()), "delta_rule_inputs")
-            self._chunk_scan("delta_rule", proj, tuple(cols[:3]), 1, aux, 1.0, batch, memory, out, H, D, D, workspace)
+            self._chunk_scan("delta_rule", proj, tuple(cols[:3]), H, aux, 1.0, batch, memory, out, H, D, D, workspace)
             return
         max_chunks, scratch = 0, None
         # Long portions take longer chunks: every chunk costs a product with its transition in the launch that walks the start
@@ -1504,7 +1508,7 @@ class CudaKernels(KernelSet):
         if batch.max_q_len >= self.SCAN_WIDE_MIN_ROWS and D <= self.CHUNK_SCAN_MAX_DIM:
             if rows.shape[1] != 2 * G * D + H * Dv or gates.shape[1] < H * D + H:
                 raise KernelError("gated_delta_scan: the rows or gates do not fit the heads")
-            self._chunk_scan("gated_delta", rows, (0, G * D, 2 * G * D), H // G, gates, q_scale, batch, memory, out, H, D, Dv, workspace)
+            self._chunk_scan("gated_delta", rows, (0, G * D, 2 * G * D), G, gates, q_scale, batch, memory, out, H, D, Dv, workspace)
             return
         chunked = self.SCAN_CHUNK and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS
         if batch.max_q_len >= self.SCAN_WIDE_MIN_ROWS and (D > self.DELTA_WIDE_ABOVE or not chunked):
@@ -1554,7 +1558,7 @@ class CudaKernels(KernelSet):
         segments = (_ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), _ptr(memory), _ptr(out))
         self._count("state_space_scan")
         if workspace is not None and batch.max_q_len >= self.STATE_SPACE_CHUNK_MIN_ROWS and N <= self.CHUNK_SCAN_MAX_DIM:
-            self._chunk_scan("head_decay", rows, (H * Dv + G * N, H * Dv, 0), H // G, gates, 1.0, batch, memory, out, H, N, Dv, workspace)
+            self._chunk_scan("head_decay", rows, (H * Dv + G * N, H * Dv, 0), G, gates, 1.0, batch, memory, out, H, N, Dv, workspace)
             return
         if batch.max_q_len >= self.SCAN_WIDE_MIN_ROWS:
             _check(self._scan_wide.kvb_state_space_scan_wide(_ptr(rows), _ptr(gates), *segments, batch.num_segments, H, G, N, Dv,

@@ -151,7 +151,7 @@ def test_scan_in_chunks(kernels, mode, lens, H, G, D, Dv):
         batch = StepBatch(sum(n), len(n), 0, None, None, None, i32([sum(n[:i]) for i in range(len(n))]), i32(n), None,
                           i32([slots[i] for i in which]), None, max_q_len=max(n))
         memory, out = state.to(DEV), torch.full((sum(n), H * Dv), float("nan"), device=DEV)
-        kernels._chunk_scan(mode, rows_.contiguous(), cols, H // G, gates_.contiguous(), 0.5, batch, memory, out, H, D, Dv, Workspace(DEV))
+        kernels._chunk_scan(mode, rows_.contiguous(), cols, G, gates_.contiguous(), 0.5, batch, memory, out, H, D, Dv, Workspace(DEV))
         kernels.check_errors()
         return out.view(-1, H, Dv).cpu(), memory.cpu()
 

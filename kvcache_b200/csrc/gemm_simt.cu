@@ -81,16 +81,15 @@ __global__ void __launch_bounds__(WARPS_M* WARPS_N * 32, 1)
 
     const Loader<TIn, BM, BK, THREADS, VEC> load_x(x, m0, M, K);
     const Loader<TIn, BN, BK, THREADS, VEC> load_w(w, n0, N, K);
-    // No kernel writes weights: the first tiles of W are on their way before the kernel before this one has ended.
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s)
-        if (s < tiles) load_w(ws + s * BN * STRIDE, s * BK);
-    pdl_wait();
+    pdl_wait();                                       // `linear` takes any W: the launch before this one may have made it
     pdl_launch_dependents();
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < tiles) load_x(xs + s * BM * STRIDE, s * BK);
-        copy_commit();                                // the first group holds all tiles of W asked for above
+        if (s < tiles) {
+            load_w(ws + s * BN * STRIDE, s * BK);
+            load_x(xs + s * BM * STRIDE, s * BK);
+        }
+        copy_commit();
     }
 
     float acc[TM][TN];

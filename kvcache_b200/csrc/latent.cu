@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(32 * WM * WN) head_linear_wide_kernel(const bf
     const bf16* xh = x + (size_t)h * xs;
     const bf16* wh = w + ((size_t)h * N + n0) * K;
     const int steps = (K + BK - 1) / BK, n_valid = min(BN, N - n0);
-    auto load_w = [&](int step) {                                  // no kernel writes weights
+    auto load_w = [&](int step) {
         bf16* dst = ws + (step % STAGES) * BN * STRIDE;
         for (int e = tid; e < BN * CH; e += THREADS) {
             const int r = e / CH, c = (e % CH) * 8, k = step * BK + c;
@@ -365,14 +365,14 @@ __global__ void __launch_bounds__(32 * WM * WN) head_linear_wide_kernel(const bf
             mt::cp_async16(dst + r * STRIDE + c, valid ? xh + (size_t)(m0 + r) * x_ld + k : w, valid);
         }
     };
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s)
-        if (s < steps) load_w(s);
-    pdl_wait();
+    pdl_wait();                                                    // the launch before this one may have made x, W or the gates
     pdl_launch_dependents();
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < steps) load_x(s);
+        if (s < steps) {
+            load_w(s);
+            load_x(s);
+        }
         mt::cp_async_commit();
     }
     // The rotated columns, while the first steps are on their way: the blocks of a row tile share its rows, a thread takes both

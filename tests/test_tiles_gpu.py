@@ -38,6 +38,34 @@ def test_float32_product_rows_do_not_depend_on_the_tile(kernels, N, K):
         assert torch.equal(part, full[:M]), M
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_products_with_a_matrix_made_by_the_launch_before(dtype):
+    """W may be the result of the launch before: nothing of it is read while that one still runs."""
+    from kvcache_b200.kernels.api import CudaKernels
+    kernels = CudaKernels(DEV, bf16_gemm="simt")             # a launch that lets the next one start before it has ended
+    g = torch.Generator(device=DEV).manual_seed(33)
+    H, N, K = 8, 512, 128
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV).to(dtype)
+    x, w = rand(40, K), torch.zeros(H * N, K, dtype=dtype, device=DEV)
+    heads_x, heads_out = rand(40, H * K), torch.empty(40, H * N, dtype=dtype, device=DEV)
+    out = torch.empty(40, H * N, dtype=dtype, device=DEV)
+    for _ in range(8):
+        a, b = rand(H * N, 320), rand(K, 320)
+        kernels.linear(a, b, w)
+        kernels.linear(x, w, out)
+        kernels.linear(a, b, w)
+        kernels.head_linear(heads_x, w.view(H, N, K), heads_out)
+        torch.cuda.synchronize()
+        after, heads_after = torch.empty_like(out), torch.empty_like(heads_out)
+        kernels.linear(x, w, after)
+        torch.cuda.synchronize()
+        kernels.head_linear(heads_x, w.view(H, N, K), heads_after)
+        torch.cuda.synchronize()
+        assert torch.equal(out, after) and torch.equal(heads_out, heads_after)
+        w.zero_()
+        torch.cuda.synchronize()
+
+
 ROWS32 = [
     ([(0, 1), (63, 1), (64, 1), (500, 1)], 14, 2, 64, 64, 16, {}),                       # decoded tokens at the edge of a key tile
     ([(0, 65), (64, 64), (127, 3), (5, 1)], 6, 2, 64, 64, 16, {}),                       # tiles of rows that end inside a segment

@@ -25,6 +25,11 @@ __device__ __forceinline__ void copy16(void* smem, const void* global, bool ther
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(global), "r"(bytes)
                  : "memory");
 }
+__device__ __forceinline__ void copy4(void* smem, const void* global, bool there) {
+    const int bytes = there ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(global), "r"(bytes)
+                 : "memory");
+}
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
@@ -60,6 +65,7 @@ struct Loader {
             const bool there = inside && i * STEP < left;
             const T* at = there ? from + (size_t)i * STEP * K + k0 + k : from;
             if (VEC) copy16(dst + i * STEP * STRIDE, at, there);
+            else if (sizeof(T) == 4) copy4(dst + i * STEP * STRIDE, at, there);
             else dst[i * STEP * STRIDE] = there ? *at : from_f32<T>(0.f);
         }
     }
@@ -163,6 +169,8 @@ static int launch(const void* x, const void* w, const float* bias, void* y, int 
 //   4 x 9,728 x 896: 23 | 27 | 25 | 37 | 63         16 x 896 x 4,864: 29 | 41 | 55 | 101 | 189   16 x 9,728 x 896: 47 | 29 | 25 | 37 | 64
 //   64 x 896 x 4,864: 76 | 49 | 57 | 100 | 186      128 x 896 x 4,864: 131 | 78 | 64 | 100 | 189  250 x 9,728 x 896: 496 | 215 | 155 | 127 | 134
 //   1,000 x 896 x 4,864: 879 | 410 | 301 | 287 | 328   1,000 x 9,728 x 896: 1,882 | 807 | 569 | 432 | 410
+// K that is no multiple of four numbers comes in 4 bytes at a time, also by cp.async (1,000 x 896 x 4,863: 340 us; with plain loads in the same
+// pipeline 470, before it 427), of eight in bfloat16 by plain loads (1,000 x 896 x 4,863: 428, before 458).
 // One tile of 64 x 64, transposed in registers and not fetched ahead, took 95 / 356 / 95 / 363 / 350 / 220 / 499 / 711 us; the
 // library's product takes 716 us at 2,048 x 9,728 x 896, this one 940.
 template <typename TIn, typename TOut, bool VEC>

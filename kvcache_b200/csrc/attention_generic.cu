@@ -202,10 +202,12 @@ KVB_API int kvb_paged_attention_ext(int dtype, const void* q, const void* k_page
 // rows ty + 16 i against keys tx + 16 j, four numbers along the head at a time, and then owns output columns 4 tx + 64 c.
 // K and V tiles come in by `cp.async`, the next pair while this one is worked on (rows of K start 4 numbers off a multiple of
 // 32: eight keys lie in different banks).  A row's maximum and sum run over the 16 lanes that share it.
-// Bound by the shared-memory loads beside the multiply-adds.  Measured against a block per (row, head), which reads every key
-// from L2 for each of them: 1,000 rows of 14 heads of 64: 2,008 -> 117 us; 512 rows of 16 heads of 128 behind 2,048 keys:
-// 9,935 -> 541 us; 16 decoded tokens with 4,000 keys, 14 heads of 64: 672 -> 268 us; 160 rows of 3 heads of 20 in chunks of 48
-// tokens, the least it was tried at: 12 -> 14 us.
+// Bound by the shared-memory loads beside the multiply-adds in prompts, by the latency of a tile of keys in single tokens.  Measured
+// against a block per (row, head), which reads every key from L2 for each of them: 1,000 rows of 14 heads of 64: 2,008 -> 117 us; 512 rows of
+// 16 heads of 128 behind 2,048 keys: 9,935 -> 541 us; one token with 1,000 keys, 14 heads of 64 (two of keys): 105 -> 53 us; 64 tokens with
+// 1,000 keys: 365 -> 69; eight rows of a new prompt: 5.2 -> 4.7.  The line in `CudaKernels.paged_attention`: heads of 48 and 32 numbers with
+// keys of their own are ahead in prompts (160 rows of 8: 29 -> 14 and 31 -> 13 us) but behind in 64 single tokens with 30 keys (16 heads of 48: 11 -> 14 us;
+// 8 of 32 level); 20 numbers: 160 rows of 3 heads in chunks of 48 tokens 7.0 -> 8.2.
 namespace rows32 {
 
 __device__ __forceinline__ void copy16(float* smem, const float* global, bool there) {
@@ -232,13 +234,13 @@ struct Params {
 
 constexpr int BN = 64, PS = BN + 4;
 
-// acc += weights of BN keys . their values.  PARTIAL: a weight below zero marks a key that the row does not see, whose value is
-// left out whatever it holds (a later token's may be infinite).
+// acc += weights of keys k0 .. k1 - 1 (multiples of 4) of a tile . their values.  PARTIAL: a weight below zero marks a key that the row
+// does not see, whose value is left out whatever it holds (a later token's may be infinite).
 template <int TM, int CD, bool PARTIAL>
-__device__ __forceinline__ void weigh(const float* ps, const float* vt, float4 (&acc)[TM][CD]) {
+__device__ __forceinline__ void weigh(const float* ps, const float* vt, float4 (&acc)[TM][CD], int k0, int k1) {
     constexpr int VS = CD * 64;
 #pragma unroll 2
-    for (int k = 0; k < BN; k += 4) {
+    for (int k = k0; k < k1; k += 4) {
         float4 w[TM];
 #pragma unroll
         for (int i = 0; i < TM; ++i) w[i] = *(const float4*)(ps + 16 * i * PS + k);
@@ -260,35 +262,74 @@ __device__ __forceinline__ void weigh(const float* ps, const float* vt, float4 (
     }
 }
 
-template <int TM, int CD>      // CD: 64-column groups of a value row
-__global__ void __launch_bounds__(256) attention_rows_kernel(const Params p) {
-    constexpr int BM = 16 * TM, VS = CD * 64;
+// s[i][j] = q row i . key 16 j, for the first NJ of the four.
+template <int TM, int NJ>
+__device__ __forceinline__ void score(const float* qt, const float* kt, int D, int KS, float (&s)[TM][4]) {
+#pragma unroll 4
+    for (int d = 0; d < D; d += 4) {
+        float4 a[TM];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) a[i] = *(const float4*)(qt + 16 * i * KS + d);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const float4 b = *(const float4*)(kt + 16 * j * KS + d);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].x, b.x, s[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].y, b.y, s[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].z, b.z, s[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].w, b.w, s[i][j]);
+        }
+    }
+}
+
+// CD: 64-column groups of a value row; STAGES: tiles of keys held at once; NY: rows side by side, 16 threads each (16, or 4 with TM = 1).
+template <int TM, int CD, int STAGES, int NY>
+__global__ void __launch_bounds__(16 * NY) attention_rows_kernel(const Params p) {
+    constexpr int BM = NY * TM, VS = CD * 64, THREADS = 16 * NY;
+    static_assert((NY == 16 || TM == 1) && THREADS >= BN, "a thread looks up one key of a tile");
     extern __shared__ __align__(16) float sm[];
     const int KS = p.D + 4;
     float* qs = sm;                        // [BM][KS]
     float* ps = qs + BM * KS;              // [BM][PS]
-    float* ks = ps + BM * PS;              // [2][BN][KS]
-    float* vs = ks + 2 * BN * KS;          // [2][BN][VS]
+    float* ks = ps + BM * PS;              // [STAGES][BN][KS]
+    float* vs = ks + STAGES * BN * KS;     // [STAGES][BN][VS]
     __shared__ int where[3 * BN];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int group = p.Hq / p.Hkv, hk = blockIdx.y;
     pdl_wait();
     pdl_launch_dependents();
 
-    // Which segment and which of its tiles: segments take ceil(rows * group / BM) blocks each, the last tiles (most keys) first.
-    int seg = 0, tile = (int)gridDim.x - 1 - (int)blockIdx.x;
-    for (; seg < p.segments; ++seg) {
-        const int mine = (p.seg_q_len[seg] * group + BM - 1) / BM;
-        if (tile < mine) break;
-        tile -= mine;
+    // Which segment and which of its tiles: segments take ceil(rows * group / BM) blocks each, the last tiles (most keys) first.  A
+    // warp counts 32 segments at a time.
+    int seg = -1, tile = (int)gridDim.x - 1 - (int)blockIdx.x;
+    for (int base = 0; base < p.segments; base += 32) {
+        const int lane = tid & 31, mine = base + lane < p.segments ? (p.seg_q_len[base + lane] * group + BM - 1) / BM : 0;
+        int upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int before = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += before;
+        }
+        const unsigned found = __ballot_sync(0xffffffffu, tile < upto);
+        if (found) {
+            const int at = __ffs(found) - 1;
+            seg = base + at;
+            tile -= __shfl_sync(0xffffffffu, upto - mine, at);
+            break;
+        }
+        tile -= __shfl_sync(0xffffffffu, upto, 31);
     }
-    if (seg == p.segments) return;
+    if (seg < 0) return;
     const int q_len = p.seg_q_len[seg], q_first = p.seg_q_start[seg], start = p.seg_kv_len[seg] - q_len;
     const int m0 = tile * BM, rows = min(BM, q_len * group - m0);
     const int* table = p.block_table + (size_t)seg * p.table_stride;
+    const bool working = TM > 1 || (tid >> 5) * 2 < rows;      // (one row tile) a warp whose two rows are past the end only fetches
 
     auto q_at = [&](int m) { return (size_t)(q_first + (m0 + m) / group) * p.Hq + hk * group + (m0 + m) % group; };
-    for (int c = tid; c < BM * (p.D / 4); c += 256) {
+    for (int c = tid; c < BM * (p.D / 4); c += THREADS) {
         const int m = c / (p.D / 4), d = (c % (p.D / 4)) * 4;
         *(float4*)(qs + m * KS + d) = m < rows ? *(const float4*)(p.q + q_at(m) * p.D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -323,18 +364,25 @@ __global__ void __launch_bounds__(256) attention_rows_kernel(const Params p) {
         if (j >= lo_first || j < p.keep_first) atomicOr(p.err, KVB_DEV_BAD_PAGE);
         return -1;
     };
+    // Steps of few rows (one row tile): of a tile's keys only those k0 .. k1 - 1 that some row sees, to the next four, are fetched (from
+    // the tile's first on), scored and weighed.
+    auto seen_from = [&](int t) { return TM > 1 || key_of(t) < p.keep_first ? 0 : max(lo_first - key_of(t), 0) & ~3; };
+    auto seen_to = [&](int t) { return TM > 1 ? BN : min(BN, ((t < kept_tiles ? p.keep_first : end) - key_of(t) + 3) & ~3); };
     auto fetch = [&](int t) {                          // a key row: 16 threads
-        float* kd = ks + (t & 1) * BN * KS;
-        float* vd = vs + (t & 1) * BN * VS;
+        float* kd = ks + t % STAGES * BN * KS;
+        float* vd = vs + t % STAGES * BN * VS;
+        const int rows_seen = seen_to(t);
 #pragma unroll
-        for (int r = ty; r < BN; r += 16) {
+        for (int r0 = 0; r0 < BN; r0 += NY) {
+            const int r = r0 + ty;
+            if (TM == 1 && r >= rows_seen) break;
             const int at = where[(t % 3) * BN + r];
             const size_t row = at >= 0 ? at : 0;
             for (int d = tx * 4; d < p.D; d += 64) copy16(kd + r * KS + d, p.k_pages + row * p.D + d, at >= 0);
 #pragma unroll
             for (int c = 0; c < CD; ++c) {
                 const int d = tx * 4 + 64 * c;
-                copy16(vd + r * VS + d, p.v_pages + row * p.Dv + (d < p.Dv ? d : 0), at >= 0 && d < p.Dv);
+                if (d < p.Dv) copy16(vd + r * VS + d, p.v_pages + row * p.Dv + d, at >= 0);      // (columns past a value row are never stored)
             }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -345,9 +393,10 @@ __global__ void __launch_bounds__(256) attention_rows_kernel(const Params p) {
         where[BN + tid] = look_up(1);
     }
     __syncthreads();
-    fetch(0);
+    if (STAGES == 2) fetch(0);
     for (int t = 0; t < tiles; ++t) {
-        if (t + 1 < tiles) {
+        if (STAGES == 1) fetch(t);
+        if (STAGES == 2 && t + 1 < tiles) {
             fetch(t + 1);
             asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         } else {
@@ -356,37 +405,25 @@ __global__ void __launch_bounds__(256) attention_rows_kernel(const Params p) {
         const int later = tid < BN ? look_up(t + 2) : -1;
         __syncthreads();
         const int j0 = key_of(t);
-        const float* kt = ks + (t & 1) * BN * KS + tx * KS;
-        const float* vt = vs + (t & 1) * BN * VS + tx * 4;
+        const float* kt = ks + t % STAGES * BN * KS + tx * KS;
+        const float* vt = vs + t % STAGES * BN * VS + tx * 4;
         const float* qt = qs + ty * KS;
         float s[TM][4];
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-#pragma unroll 4
-        for (int d = 0; d < p.D; d += 4) {
-            float4 a[TM];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = *(const float4*)(qt + 16 * i * KS + d);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float4 b = *(const float4*)(kt + 16 * j * KS + d);
-#pragma unroll
-                for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].x, b.x, s[i][j]);
-#pragma unroll
-                for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].y, b.y, s[i][j]);
-#pragma unroll
-                for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].z, b.z, s[i][j]);
-#pragma unroll
-                for (int i = 0; i < TM; ++i) s[i][j] = fmaf(a[i].w, b.w, s[i][j]);
-            }
+        const int k0 = seen_from(t), k1 = seen_to(t);
+        if (working) {
+            if (TM == 1 && k1 <= 16) score<TM, 1>(qt, kt, p.D, KS, s);
+            else score<TM, 4>(qt, kt, p.D, KS, s);
         }
         unsigned there = 0;                            // keys whose page is missing (flagged above) are seen by nobody
 #pragma unroll
         for (int j = 0; j < 4; ++j) there |= where[(t % 3) * BN + tx + 16 * j] >= 0 ? 1u << j : 0u;
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
+            if (!working) break;
             float top = -FLT_MAX;
             unsigned seen = 0;
 #pragma unroll
@@ -422,8 +459,11 @@ __global__ void __launch_bounds__(256) attention_rows_kernel(const Params p) {
         }
         const bool whole = j0 + BN - 1 <= start + m0 / group && (j0 >= lo_last || j0 + BN <= p.keep_first);
         const bool held = __syncthreads_and(there == 15u);   // (rows past the segment's last carry its last row's position)
-        if (whole && held) weigh<TM, CD, false>(ps + ty * PS, vt, acc);
-        else weigh<TM, CD, true>(ps + ty * PS, vt, acc);
+        if (working) {
+            if (whole && held) weigh<TM, CD, false>(ps + ty * PS, vt, acc, 0, BN);
+            else if (k1 - k0 == BN) weigh<TM, CD, true>(ps + ty * PS, vt, acc, 0, BN);
+            else weigh<TM, CD, true>(ps + ty * PS, vt, acc, k0, k1);
+        }
         if (tid < BN) where[((t + 2) % 3) * BN + tid] = later;
         __syncthreads();                               // the tile's stage is free for the one after next
     }
@@ -442,16 +482,16 @@ __global__ void __launch_bounds__(256) attention_rows_kernel(const Params p) {
     }
 }
 
-template <int TM, int CD>
+template <int TM, int CD, int STAGES = 2, int NY = 16>
 static int launch(const Params& p, int T, cudaStream_t stream) {
-    const int smem = (int)sizeof(float) * (16 * TM * (p.D + 4) + 16 * TM * PS + 2 * BN * (p.D + 4) + 2 * BN * CD * 64);
+    const int smem = (int)sizeof(float) * (NY * TM * (p.D + 4) + NY * TM * PS + STAGES * BN * (p.D + 4) + STAGES * BN * CD * 64);
     if (smem > 44 * 1024) {                            // (the kernel has some shared memory of its own beside it)
-        cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<TM, CD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<TM, CD, STAGES, NY>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
     }
-    const long long blocks = ((long long)T * (p.Hq / p.Hkv) + 16 * TM - 1) / (16 * TM) + p.segments;
+    const long long blocks = ((long long)T * (p.Hq / p.Hkv) + NY * TM - 1) / (NY * TM) + p.segments;
     if (blocks > 0x7fffffffLL || p.Hkv > 65535) return KVB_ERR_LIMIT;
-    kvb_launch(attention_rows_kernel<TM, CD>, dim3((unsigned)blocks, p.Hkv), dim3(256), smem, stream, p);
+    kvb_launch(attention_rows_kernel<TM, CD, STAGES, NY>, dim3((unsigned)blocks, p.Hkv), dim3(16 * NY), smem, stream, p);
     return kvb_launch_status();
 }
 
@@ -474,6 +514,12 @@ KVB_API int kvb_paged_attention_rows32(const void* q, const void* k_pages, const
     // The most rows a block that one segment fills and that leave every SM a block: fewer reads of the keys, more rows per load.
     const long long all = (long long)T * (Hq / Hkv), one = (long long)seg_rows * (Hq / Hkv), sms = kvb_sm_count();
     const int tm = one > 32 && (all + 63) / 64 * Hkv >= sms ? 4 : one > 16 && (all + 31) / 32 * Hkv >= sms ? 2 : 1;
+    // Many segments of few rows: one stage of keys a block, so that more blocks share an SM (and for values of up to 64 numbers eight rows
+    // a block).  64 single tokens behind 100 keys, 8 heads of 64 | 128, each with keys of its own: 13 | 24 us, in blocks of sixteen rows with
+    // two stages 23 | 50, a block per row and head 24 | 37.
+    const long long blocks = (long long)segments * Hkv;
+    if (Dv <= 64 && one <= 8 && blocks > 2 * sms) return rows32::launch<1, 1, 1, 8>(p, T, stream);
+    if (Dv > 64 && one <= 16 && blocks > sms) return rows32::launch<1, 2, 1>(p, T, stream);
     if (Dv <= 64) return tm == 4 ? rows32::launch<4, 1>(p, T, stream) : tm == 2 ? rows32::launch<2, 1>(p, T, stream) : rows32::launch<1, 1>(p, T, stream);
     return tm == 4 ? rows32::launch<4, 2>(p, T, stream) : tm == 2 ? rows32::launch<2, 2>(p, T, stream) : rows32::launch<1, 2>(p, T, stream);
 }

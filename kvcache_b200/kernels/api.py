@@ -848,6 +848,10 @@ class CudaKernels(KernelSet):
             self._stream()), "flash_decode_tma (rotation and append fused)")
         return True
 
+    # Narrowest float32 heads that go through tiles of query rows: with keys of their own, and where query heads share keys.  The
+    # figures on both sides of the lines: csrc/attention_generic.cu.
+    ROWS32_MIN, ROWS32_MIN_SHARED = 64, 32
+
     def paged_attention(self, q: torch.Tensor, batch: StepBatch, kv: PagedKVView, out: torch.Tensor,
                         num_heads: int, scale: float, workspace=None, sink: Optional[torch.Tensor] = None,
                         score_cap: Optional[float] = None, slopes: Optional[torch.Tensor] = None, reach: Optional[int] = None) -> None:
@@ -872,9 +876,11 @@ class CudaKernels(KernelSet):
             slopes = self._zero_slopes.get(num_heads)
             if slopes is None:
                 slopes = self._zero_slopes[num_heads] = torch.zeros(num_heads, dtype=torch.float32, device=self.device)
-        # float32, heads of up to 128 numbers in steps of four: tiles of query rows (1,000 rows of 14 heads of 64: 117 us, with a
-        # block per row and head 2,008 us).  Wider heads and those of odd sizes, and rows that do not start on 16 bytes, keep that.
-        if (q.dtype == torch.float32 and D % 4 == 0 and D <= 128 and spec.v_head_dim % 4 == 0 and 0 < spec.v_head_dim <= 128
+        # float32, heads of 64 to 128 numbers in steps of four (from 32 where several query heads share keys): tiles of query rows
+        # (1,000 rows of 14 heads of 64: 117 us, with a block per row and head 2,008 us).  Heads of other sizes, and rows that do not start on
+        # 16 bytes, keep that.  By the layer's sizes alone: a row's bits do not depend on the step it is in.
+        if (q.dtype == torch.float32 and D % 4 == 0 and (self.ROWS32_MIN_SHARED if num_heads > Hkv else self.ROWS32_MIN) <= D <= 128
+                and spec.v_head_dim % 4 == 0 and 0 < spec.v_head_dim <= 128
                 and (q.data_ptr() | out.data_ptr() | kv.k_pages.data_ptr() | kv.v_pages.data_ptr()) % 16 == 0):
             self._count("attention_generic")
             _check(self._attn_generic.kvb_paged_attention_rows32(

@@ -74,12 +74,16 @@ ROWS32 = [
     ([(0, 130), (900, 300)], 16, 2, 128, 128, 32, dict(window=64)),
     ([(200, 700)], 2, 2, 128, 100, 64, {}),
     ([(30, 1), (3, 2)], 2, 1, 16, 16, 16, {}),                                           # shared memory right below what needs no asking for
+    ([(7 * i % 130, 1 + i % 2) for i in range(90)], 8, 4, 64, 64, 16, {}),               # many segments of few rows: eight a block ...
+    ([(7 * i % 130, 1 + i % 3) for i in range(50)], 20, 4, 68, 128, 16, dict(window=40, keep_first=3)),      # ... and one stage of keys
 ]
 
 
 @pytest.mark.parametrize("scenario", ROWS32)
 @pytest.mark.parametrize("options", [False, True])
-def test_float32_attention_tiles(kernels, scenario, options):
+def test_float32_attention_tiles(kernels, scenario, options, monkeypatch):
+    monkeypatch.setattr(kernels, "ROWS32_MIN", 4)                                        # narrower heads than the dispatch gives it
+    monkeypatch.setattr(kernels, "ROWS32_MIN_SHARED", 4)
     segments, Hq, Hkv, D, Dv, page, spec = scenario
     batch, kv = paged_scenario(segments, num_kv_heads=Hkv, head_dim=D, page_size=page, dtype=torch.float32, device="cpu", seed=41)
     g = torch.Generator().manual_seed(42)

@@ -14,23 +14,21 @@
 //   S_C = L_C S_0 + K1^T V + K2^T Z       K_s = r(C, s) key_s
 //
 // Launches (1), a block per (chunk, head) and all of them at once, make the matrices that do not know S_0 (the "record" of the
-// chunk) on the CUDA cores: the decays between two tokens are multiplied up one after the other and never divided by, so that
-// any decay down to zero is exact.  Launch (2) walks a segment's chunks in order, a block per 16 value channels of a head:
-// S^T lives in the accumulators of its warps, each with 8 KT key channels, and is at the same time the A operand of Y S_0 and
-// Q S_0 - the two fragments of `mma.sync` hold the same numbers if neighbouring channels are taken as the halves of a step of
-// eight.  The warps' partial sums meet once a chunk through shared memory, added in one order by all of them.  A record lies in
-// scratch as it will lie in shared memory and comes in by one bulk copy, a chunk ahead.
+// chunk): the decays between two tokens are multiplied up one after the other and never divided by, so that any decay down to zero is
+// exact.  Launch (2) walks a segment's chunks in order, a block per 16 value channels of a head: S lives in registers, a thread's key
+// channels of two value channels; Y S_0 and Q S_0 are summed over a warp's key channels by shuffles and over the warps through shared
+// memory, in one order by all of them.  A record lies in scratch as it will lie in shared memory and comes in by one bulk copy, a chunk ahead.
 //
-// A number x is split into h = tf32(x) and l = x - h, and a product is h h + h l + l h (what is left out is 2^-22 of it); sums that
-// run on from step to step are added on the CUDA cores, because the tensor cores' own accumulation truncates.  Against 64 bits a
-// scan alone is off by 1.3e-7 to 1.6e-7 of its results and 1.1e-7 to 1.6e-7 of its state, the scans over tokens by 1.0e-7 and 0.6e-7;
-// a layer's state, whose inputs come from products with float32 sums of their own, by 7e-6 to 3e-5 either way.
+// All of it is float32 multiply-adds on the CUDA cores, in an order that rounds no worse than a walk over tokens: decays over the
+// chunk are products that are rounded once, and the chunk's last tokens are added to the state one by one.  Against 64 bits results and
+// states are off by 0.6 to 1.1 of what the scans over tokens are off by (states of models: 0.5e-7 to 1.1e-7; slow decays 1.6e-7 to 4.3e-7 where those
+// are at 1.9e-7 to 4.9e-7).
 //
-// What bounds it: the chain of a chunk - its products, one exchange, one wait: 0.8 us with 64 key channels, 1.2 to 1.4 with 128 -
-// times the chunks of the longest segment; the tensor pipe is idle for most of it.  Measured beside the form each replaces (us;
-// records and walk): gated delta 777 x 14 x 64 x 64: 117 -> 64, 1,500 x 16 x 128 x 128: 326 -> 154; delta rule 543 + 905 + 363 x 16 x
-// 128: 662 -> 179 (records 45, systems 11, walk 123), 1,000 x 14 x 64: 199 -> 90; channel decays 600 + 400 x 8 x 128 x 256: 154 -> 56; head decays 2,048 x 64 x
-// 128 x 64: 279 -> 189.
+// What bounds it: the latency of a chunk's steps - shared memory, shuffles, two or three barriers, 1.0 to 1.9 us - times the chunks of the longest
+// segment.  Measured beside the form each replaces (us; records and walk): gated delta 777 x 14 x 64 x 64: 115 -> 84, 1,500 x 16 x 128 x 128:
+// 325 -> 220; delta rule 543 + 905 + 363 x 16 x 128: 660 -> 250, 1,000 x 14 x 64: 196 -> 131; channel decays 600 + 400 x 8 x 128 x 256: 148 -> 64; head
+// decays 2,048 x 64 x 128 x 64: 278 -> 239.  Products of tf32 halves on the tensor cores in the walk took 61, 146, 188, 97, 54 and 187, with states
+// up to three times as far from 64 bits.
 // A segment's result does not depend on what else the step holds.  An infinite or undefined value spreads within its chunk of
 // sixteen tokens, in its own value channel, also to tokens before it.
 // State layout: [slot, head, key channel, value channel].
@@ -112,6 +110,17 @@ __device__ __forceinline__ float dot4(const float4& a, const float4& b, float c)
     return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c))));
 }
 __device__ __forceinline__ void scale4(float4& a, const float4& b) { a.x *= b.x; a.y *= b.y; a.z *= b.z; a.w *= b.w; }
+
+// A product of many decays and what its roundings lost: it counts once for all sixteen tokens, so it is rounded once.
+struct Decay {
+    float high = 1.f, low = 0.f;
+    __device__ __forceinline__ void times(float a) {
+        const float p = __fmul_rn(high, a);
+        low = fmaf(low, a, fmaf(high, a, -p));
+        high = p;
+    }
+    __device__ __forceinline__ float value() const { return __fadd_rn(high, low); }
+};
 
 // ---- launches (1): the records ---------------------------------------------------------------------------------------------
 // grid (chunks, heads), 256 threads.  Thread (s, part): token s as a key, channels 4 part .. + 3 of every 64.
@@ -224,23 +233,25 @@ __global__ void __launch_bounds__(256, MODE == CHUNK_DELTA_RULE && NI == 2 ? 3 :
     if (MODE != CHUNK_GATED_DELTA) __syncthreads();                // all have read q
     const int d = tid % DP;
     if (tid < DP) {
-        float run = 1.f;
+        Decay run;
 #pragma unroll
         for (int t = 0; t < C; ++t) {
-            const float before = run;
-            run *= rows_s[2][t][d];
-            rec[R.q + t * (DP + 8) + d] = rows_s[0][t][d] * run;
-            if (MODE == CHUNK_GATED_DELTA) rows_s[0][t][d] = rows_s[1][t][d] * run;                    // the key as it meets S_0
+            const float before = run.value();
+            run.times(rows_s[2][t][d]);
+            const float upto = run.value();
+            rec[R.q + t * (DP + 8) + d] = rows_s[0][t][d] * upto;
+            if (MODE == CHUNK_GATED_DELTA) rows_s[0][t][d] = rows_s[1][t][d] * upto;                   // the key as it meets S_0
             if (MODE == CHUNK_DELTA_RULE) rec[R.y + t * (DP + 8) + d] = rows_s[3][t][d] * before;
         }
-        rec[R.decay + d] = run;
+        rec[R.decay + d] = run.value();
     } else if (tid < 2 * DP) {
-        float run = 1.f;
+        Decay run;
 #pragma unroll
         for (int t = C - 1; t >= 0; --t) {
-            rec[(has_v(MODE) ? R.k1 : R.k2) + t * (DP + 4) + d] = rows_s[1][t][d] * run;
-            if (MODE == CHUNK_DELTA_RULE) rec[R.k2 + t * (DP + 4) + d] = -rows_s[4][t][d] * run;
-            run *= rows_s[2][t][d];
+            const float after = run.value();
+            rec[(has_v(MODE) ? R.k1 : R.k2) + t * (DP + 4) + d] = rows_s[1][t][d] * after;
+            if (MODE == CHUNK_DELTA_RULE) rec[R.k2 + t * (DP + 4) + d] = -rows_s[4][t][d] * after;
+            run.times(rows_s[2][t][d]);
         }
     }
     if (MODE != CHUNK_GATED_DELTA) return;
@@ -365,68 +376,53 @@ __global__ void __launch_bounds__(256) head_records_kernel(const Rows in, const 
         if (h < last) {
             float* rec = records + ((size_t)blockIdx.x * H + h) * (R.total - R.shared);
             const float gain = d_s[s][part];
-            float run = 1.f, all = 1.f;
+            Decay run, all;
 #pragma unroll
             for (int t = 0; t < C; ++t) {
                 const float a = a_s[s][t];
-                if (t > part) run *= a;
-                all *= t <= part ? a : 1.f;
-                rec[R.a1 - R.shared + t * 24 + part] = t >= part ? qk_s[t][part] * (gain * run) : 0.f;
+                if (t > part) run.times(a);
+                else all.times(a);
+                const float full = gain * run.high, rest = fmaf(gain, run.low, fmaf(gain, run.high, -full)), qk = qk_s[t][part];
+                rec[R.a1 - R.shared + t * 24 + part] = t >= part ? fmaf(qk, full, qk * rest) : 0.f;
             }
-            rec[part] = all;                                       // L_t, t = part
-            rec[C + part] = gain * run;
-            if (part == C - 1) rec[2 * C] = all;                   // L_C
+            rec[part] = all.value();                               // L_t, t = part
+            rec[C + part] = gain * run.value();
+            if (part == C - 1) rec[2 * C] = all.value();           // L_C
         }
     }
 }
 
 // ---- launch (2): the walk -------------------------------------------------------------------------------------------------
-struct Split { uint32_t h[4], l[4]; };
-__device__ __forceinline__ void split1(float x, uint32_t& h, uint32_t& l) {
-    h = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;         // ten bits of fraction, rounded to the nearest
-    l = __float_as_uint(x - __uint_as_float(h));
+// Two float32 multiply-adds in one instruction, each rounded as `fmaf` rounds.
+__device__ __forceinline__ float2 fma2(const float2& a, const float2& b, const float2& c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(*(const uint64_t*)&a), "l"(*(const uint64_t*)&b), "l"(*(const uint64_t*)&c));
+    return *(const float2*)&d;
 }
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+__device__ __forceinline__ float2 mul2(const float2& a, const float2& b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(*(const uint64_t*)&a), "l"(*(const uint64_t*)&b));
+    return *(const float2*)&d;
 }
-// An accumulator fragment (columns 2 t, 2 t + 1) as the A operand of a step of eight along those columns.
-__device__ __forceinline__ Split as_operand(const float (&c)[4]) {
-    Split s;
-    split1(c[0], s.h[0], s.l[0]);
-    split1(c[2], s.h[1], s.l[1]);
-    split1(c[1], s.h[2], s.l[2]);
-    split1(c[3], s.h[3], s.l[3]);
-    return s;
-}
-// p[i] = a(i) b[i], N of them side by side: a product waits about 70 clocks for the one before it on the same accumulator, so that
-// one after the other they would bound the walk.  The cross products come first: the large one is rounded last.
-template <int N, typename A>
-__device__ __forceinline__ void products(float (&p)[N][4], A a, const float (&b)[N][2]) {
-    uint32_t h[N][2], l[N][2];
+__device__ __forceinline__ float2 low2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 high2(const float4& v) { return make_float2(v.z, v.w); }
+
+// N neighbouring numbers in shared memory.
+template <int N> __device__ __forceinline__ void load(const float* at, float (&v)[N]) {
+    if constexpr (N == 2) {
+        const float2 x = *(const float2*)at;
+        v[0] = x.x; v[1] = x.y;
+    } else {
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        split1(b[i][0], h[i][0], l[i][0]);
-        split1(b[i][1], h[i][1], l[i][1]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) p[i][e] = 0.f;
+        for (int i = 0; i < N / 4; ++i) {
+            const float4 x = *(const float4*)(at + 4 * i);
+            v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+        }
     }
-#pragma unroll
-    for (int i = 0; i < N; ++i) mma_tf32(p[i], a(i).h, l[i][0], l[i][1]);
-#pragma unroll
-    for (int i = 0; i < N; ++i) mma_tf32(p[i], a(i).l, h[i][0], h[i][1]);
-#pragma unroll
-    for (int i = 0; i < N; ++i) mma_tf32(p[i], a(i).h, h[i][0], h[i][1]);
 }
-__device__ __forceinline__ void pair(float (&b)[2], const float* at) {
-    const float2 v = *(const float2*)at;
-    b[0] = v.x;
-    b[1] = v.y;
-}
-__device__ __forceinline__ void add4(float (&sum)[4], const float (&p)[4]) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) sum[e] += p[e];
+template <int N> __device__ __forceinline__ void keep(float* at, const float (&v)[N]) {
+    if constexpr (N == 2) *(float2*)at = make_float2(v[0], v[1]);
+    else *(float4*)at = make_float4(v[0], v[1], v[2], v[3]);
 }
 
 __device__ __forceinline__ void copy_bulk(float* smem, const float* gmem, uint32_t bytes, uint64_t* bar) {
@@ -434,37 +430,40 @@ __device__ __forceinline__ void copy_bulk(float* smem, const float* gmem, uint32
                  ::"r"(tc::smem_u32(smem)), "l"(gmem), "r"(bytes), "r"(tc::smem_u32(bar)) : "memory");
 }
 
-// grid (16 value channels, heads, segments), WD warps of 8 KT key channels.
-template <int MODE, int NI, int KT, int STAGES>
-__global__ void __launch_bounds__(64 * NI / (8 * KT) * 32) chunk_walk_kernel(const Rows in, const Segments seg, const float* __restrict__ records,
+// grid (16 value channels, heads, segments).  A thread holds TD neighbouring key channels of TC value channels of the state; a warp's lanes
+// are 2 TC groups of key channels by 16 / TC of value channels.  Beside that, every thread owns one token's OC value channels of Z and O.
+template <int MODE, int NI, int TD, int TC, int STAGES>
+__global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(const Rows in, const Segments seg, const float* __restrict__ records,
                                                                              int max_chunks, float q_scale, float* __restrict__ memory,
                                                                              float* __restrict__ out, int H, int D, int Dv, int* __restrict__ err) {
     constexpr bool Z = has_z(MODE), V = has_v(MODE);
-    constexpr int DP = 64 * NI, WD = DP / (8 * KT);
-    constexpr int NX = Z ? 4 : 2;                              // accumulator fragments a warp hands over: Q S_0 (, Y S_0)
+    constexpr int DP = 64 * NI, CG = 16 / TC, DG = 32 / CG, WARPS = DP / (TD * DG), OC = 16 * C / (32 * WARPS);
+    constexpr int NR = Z ? 2 * C : C;                          // rows that meet S_0: [Y | Q] or Q
     constexpr Record R = record_of(MODE, DP);
-    static_assert(WD >= 2, "the first two warps write the results of eight tokens each");
+    static_assert((OC == 2 || OC == 4) && (TC == 2 || TC == 4) && TD % 4 == 0, "");
+    static_assert(!Z || R.q == R.y + C * (DP + 8), "the rows of Y and Q follow one another");
     extern __shared__ __align__(128) float sm[];
-    __shared__ __align__(16) float4 meet[2][WD][NX][32];
+    __shared__ __align__(16) float meet[WARPS][NR][16];        // the warps' shares of Y S_0 and Q S_0
+    __shared__ __align__(16) float v_s[2][C][16], z_s[Z ? C : 1][16];
     __shared__ __align__(8) uint64_t full[STAGES];
-    const int tid = threadIdx.x, lane = tid & 31, wd = tid >> 5, g = lane >> 2, t4 = lane & 3;
+    const int tid = threadIdx.x, lane = tid & 31, wd = tid >> 5, cg = lane % CG, dg = lane / CG;
     const int h = blockIdx.y, sg = blockIdx.z;
     const int n = seg.q_len[sg], r0 = seg.q_start[sg], slot = seg.slot[sg];
     if (n <= 0) return;
     int chunk0 = 0;
     for (int i = 0; i < sg; ++i) chunk0 += (seg.q_len[i] + C - 1) / C;
-    const int chunks = (n + C - 1) / C, ch0 = 8 * KT * wd;
+    const int chunks = (n + C - 1) / C, d0 = (wd * DG + dg) * TD;
 
     float* mem = memory + ((size_t)slot * H + h) * D * Dv;
-    const int col = 16 * blockIdx.x + g;
-    const bool col0 = col < Dv, col1 = col + 8 < Dv;
-    float S[KT][4];                                            // S^T: rows are value channels col, col + 8; columns key channels
+    const int col0 = 16 * blockIdx.x + cg * TC;
+    float2 S[TD / 2][TC];                                      // key channels d0 + 2 i and the next
 #pragma unroll
-    for (int kt = 0; kt < KT; ++kt)
+    for (int i = 0; i < TD / 2; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int d = ch0 + 8 * kt + 2 * t4 + (e & 1);
-            S[kt][e] = d < D && (e < 2 ? col0 : col1) ? mem[(size_t)d * Dv + col + 8 * (e >> 1)] : 0.f;
+        for (int c = 0; c < TC; ++c) {
+            const int d = d0 + 2 * i;
+            const float* at = mem + (size_t)d * Dv + col0 + c;
+            S[i][c] = make_float2(d < D && col0 + c < Dv ? at[0] : 0.f, d + 1 < D && col0 + c < Dv ? at[Dv] : 0.f);
         }
     if (tid == 0) {
         for (int i = 0; i < STAGES; ++i) tc::mbar_init(&full[i], 1);
@@ -485,228 +484,226 @@ __global__ void __launch_bounds__(64 * NI / (8 * KT) * 32) chunk_walk_kernel(con
             copy_bulk(b, records + (id * H + h) * R.total, R.total * 4, bar);
         }
     };
-    // V^T as an operand: steps of eight tokens, tokens 2 t and 2 t + 1 its halves.
-    const float* v_at = in.rows + (size_t)(r0 + 2 * t4) * in.stride + in.v_col + (size_t)h * Dv + col;     // of the chunk asked for next
-    const size_t v_chunk = (size_t)C * in.stride;
-    auto values = [&](int left, float (&raw)[2][4]) {          // `left`: tokens from the chunk's first on
-        if (left >= C && 16 * (int)blockIdx.x + C <= Dv) {
+    // This thread's token of every chunk, and its value channels.
+    const int t = tid / (16 / OC), oc = OC * (tid % (16 / OC)), col = 16 * blockIdx.x + oc;
+    const float* v_at = in.rows + (size_t)(r0 + t) * in.stride + in.v_col + (size_t)h * Dv + col;
+    auto values = [&](int ci, float (&v)[OC]) {
+        const bool there = ci * C + t < n;
+        const float* at = v_at + (there ? (size_t)ci * C * in.stride : 0);
 #pragma unroll
-            for (int ks = 0; ks < 2; ++ks) {
-                const float* at = v_at + (size_t)(8 * ks) * in.stride;
-                raw[ks][0] = at[0]; raw[ks][2] = at[8];
-                at += in.stride;
-                raw[ks][1] = at[0]; raw[ks][3] = at[8];
-            }
-        } else {
-#pragma unroll
-            for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int t = 8 * ks + (e & 1);
-                    raw[ks][e] = 2 * t4 + t < left && (e < 2 ? col0 : col1) ? v_at[(size_t)t * in.stride + 8 * (e >> 1)] : 0.f;
-                }
-        }
-        v_at += v_chunk;
+        for (int c = 0; c < OC; ++c) v[c] = there && col + c < Dv ? at[c] : 0.f;
     };
+    float next[OC];
+    values(0, next);
+    keep<OC>(&v_s[0][t][oc], next);
     __syncthreads();
     if (tid == 0)
         for (int i = 0; i < STAGES - 1 && i < chunks; ++i) fetch(i);
-    float raw[2][4], next[2][4];
-    values(n, next);
 
-    // The results of a chunk: warps 0 and 1, eight tokens each.
-    float held[4], level[2];                                   // A V (+ A Z), and what Q S_0 is multiplied by (head decay)
-    const size_t o_row = (size_t)H * Dv;
-    float* o_at = out + (size_t)(r0 + 8 * wd + 2 * t4) * o_row + (size_t)h * Dv + col;
-    auto store = [&](int ci) {                                 // called for the chunks in order
-        float o[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int w = 0; w < WD; ++w) {
-            const float4 part = meet[ci & 1][w][wd][lane];
-            o[0] += part.x; o[1] += part.y; o[2] += part.z; o[3] += part.w;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            if (MODE == CHUNK_HEAD_DECAY) o[e] *= level[e & 1];
-            o[e] = (o[e] + held[e]) * q_scale;
-        }
-        const int left = n - ci * C - 8 * wd - 2 * t4;
-        if (left > 0) {
-            if (col0) o_at[0] = o[0];
-            if (col1) o_at[8] = o[2];
-        }
-        if (left > 1) {
-            if (col0) o_at[o_row] = o[1];
-            if (col1) o_at[o_row + 8] = o[3];
-        }
-        o_at += C * o_row;
-    };
-
-    bool bad = false;
+    bool bad = false, failed = false;
     int ci = 0;
-    for (; ci < chunks; ++ci) {
-        if (__syncthreads_or(bad)) break;                      // all are done with chunk ci - 1 (a wait that ran out ends the walk)
+    for (;; ++ci) {
+        failed = __syncthreads_or(bad);                        // all are done with chunk ci - 1 (a wait that ran out ends the walk)
+        if (failed || ci == chunks) break;
         if (tid == 0 && ci + STAGES - 1 < chunks) fetch(ci + STAGES - 1);
-        if (!Z && ci > 0 && wd < 2) store(ci - 1);
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) raw[ks][e] = next[ks][e];
-        if (ci + 1 < chunks) values(n - (ci + 1) * C, next);
+        values(ci + 1, next);
         if (!tc::mbar_wait(&full[ci % STAGES], (ci / STAGES) & 1)) {
             bad = true;
             atomicOr(err, tc::KVB_DEV_TIMEOUT);
         }
         const float* b = sm + (ci % STAGES) * R.total;
+        const float(*v_c)[16] = v_s[ci & 1];
 
-        // This warp's channels' share of Q S_0 and Y S_0.
-        float sum[NX][4];
+        // Y S_0 and Q S_0, eight rows at a time: this thread's key channels, then the warp's.
+        const float* rows = b + (Z ? R.y : R.q) + d0;
 #pragma unroll
-        for (int x = 0; x < NX; ++x)
+        for (int row0 = 0; row0 < NR; row0 += 8) {
+            float2 acc[8][TC];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) sum[x][e] = 0.f;
-        constexpr int KP = KT < 8 / NX ? KT : 8 / NX;          // steps of eight channels taken together
+            for (int r = 0; r < 8; ++r)
 #pragma unroll
-        for (int k0 = 0; k0 < KT; k0 += KP) {
-            Split a[KP];
-            float bb[KP * NX][2], p[KP * NX][4];
+                for (int q = 0; q < TD / 4; ++q) {
+                    const float4 y = *(const float4*)(rows + (row0 + r) * (DP + 8) + 4 * q);
 #pragma unroll
-            for (int k = 0; k < KP; ++k) {
-                a[k] = as_operand(S[k0 + k]);
-#pragma unroll
-                for (int x = 0; x < NX; ++x)
-                    pair(bb[k * NX + x], b + (x < 2 ? R.q : R.y) + (8 * (x & 1) + g) * (DP + 8) + ch0 + 8 * (k0 + k) + 2 * t4);
-            }
-            products<KP * NX>(p, [&](int i) -> const Split& { return a[i / NX]; }, bb);
-#pragma unroll
-            for (int i = 0; i < KP * NX; ++i) add4(sum[i % NX], p[i]);
-        }
-#pragma unroll
-        for (int x = 0; x < NX; ++x) meet[ci & 1][wd][x][lane] = make_float4(sum[x][0], sum[x][1], sum[x][2], sum[x][3]);
-
-        Split v[2], z[2];
-        v[0] = as_operand(raw[0]);
-        v[1] = as_operand(raw[1]);
-        float wv[2][4];
-        if (Z) {
-            float bb[3][2], p[3][4];                           // W is zero above its diagonal
-            pair(bb[0], b + R.w + g * 24 + 2 * t4);
-            pair(bb[1], b + R.w + (8 + g) * 24 + 2 * t4);
-            pair(bb[2], b + R.w + (8 + g) * 24 + 8 + 2 * t4);
-            products<3>(p, [&](int i) -> const Split& { return v[i / 2]; }, bb);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                wv[0][e] = p[0][e];
-                wv[1][e] = p[1][e] + p[2][e];
-            }
-            __syncthreads();
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                float total[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int w = 0; w < WD; ++w) {
-                    const float4 part = meet[ci & 1][w][2 + nt][lane];
-                    total[0] += part.x; total[1] += part.y; total[2] += part.z; total[3] += part.w;
+                    for (int c = 0; c < TC; ++c) {
+                        acc[r][c] = q ? fma2(low2(y), S[2 * q][c], acc[r][c]) : mul2(low2(y), S[0][c]);
+                        acc[r][c] = fma2(high2(y), S[2 * q + 1][c], acc[r][c]);
+                    }
                 }
+            float sum[8][TC];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) total[e] += wv[nt][e];
-                z[nt] = as_operand(total);
+            for (int r = 0; r < 8; ++r)
+#pragma unroll
+                for (int c = 0; c < TC; ++c) sum[r][c] = acc[r][c].x + acc[r][c].y;
+            // A lane ends with 8 / DG of the rows, summed over the warp's key channels.
+            int mine = 0;
+#pragma unroll
+            for (int off = 16, count = 4; off >= CG; off >>= 1, count >>= 1) {
+                const bool upper = lane & off;
+                mine += upper ? count : 0;
+#pragma unroll
+                for (int r = 0; r < count; ++r)
+#pragma unroll
+                    for (int c = 0; c < TC; ++c) {
+                        const float keep = upper ? sum[r + count][c] : sum[r][c], give = upper ? sum[r][c] : sum[r + count][c];
+                        sum[r][c] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+                    }
+            }
+#pragma unroll
+            for (int r = 0; r < 8 / DG; ++r)
+#pragma unroll
+                for (int c = 0; c < TC; ++c) meet[wd][row0 + mine + r][cg * TC + c] = sum[r][c];
+        }
+        float z_own[OC] = {}, o[OC] = {};
+        if (Z) {                                               // W V, while the others get here
+            float w[C];
+            load<C>(b + R.w + t * 24, w);
+#pragma unroll
+            for (int s = 0; s < C; ++s) {
+                float v[OC];
+                load<OC>(&v_c[s][oc], v);
+#pragma unroll
+                for (int c = 0; c < OC; ++c) z_own[c] = fmaf(w[s], v[c], z_own[c]);
             }
         }
-        if (wd < 2) {
-            constexpr int NA = (V ? 2 : 0) + (Z ? 2 : 0);      // (for the first eight tokens the second half of A is zero)
-            float bb[NA][2], p[NA][4];
+        __syncthreads();
+        {
+            float y_sum[OC] = {};
 #pragma unroll
-            for (int ks = 0; ks < 2; ++ks) {
-                if (V) pair(bb[ks], b + R.a1 + (8 * wd + g) * 24 + 8 * ks + 2 * t4);
-                if (Z) pair(bb[(V ? 2 : 0) + ks], b + R.a2 + (8 * wd + g) * 24 + 8 * ks + 2 * t4);
+            for (int w = 0; w < WARPS; ++w) {
+                float part[OC];
+                if (Z) {
+                    load<OC>(&meet[w][t][oc], part);
+#pragma unroll
+                    for (int c = 0; c < OC; ++c) y_sum[c] += part[c];
+                }
+                load<OC>(&meet[w][NR - C + t][oc], part);
+#pragma unroll
+                for (int c = 0; c < OC; ++c) o[c] += part[c];
             }
-            products<NA>(p, [&](int i) -> const Split& { return V && i < 2 ? v[i & 1] : z[i & 1]; }, bb);
+            if (Z) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) held[e] = p[0][e] + p[1][e] + (NA > 2 ? p[NA - 2][e] + p[NA - 1][e] : 0.f);
+                for (int c = 0; c < OC; ++c) y_sum[c] += z_own[c];
+                keep<OC>(&z_s[t][oc], y_sum);
+            }
             if (MODE == CHUNK_HEAD_DECAY) {
-                level[0] = b[R.decay + 8 * wd + 2 * t4];
-                level[1] = b[R.decay + 8 * wd + 2 * t4 + 1];
-            }
-            if (Z) store(ci);
-        }
-
-        // The state: the chunk's sum by itself, then added.
-        if (MODE == CHUNK_HEAD_DECAY) {
+                const float level = b[R.decay + t];
 #pragma unroll
-            for (int ks = 0; ks < 2; ++ks) {
-                const float2 gain = *(const float2*)(b + R.decay + C + 8 * ks + 2 * t4);
-                raw[ks][0] *= gain.x; raw[ks][2] *= gain.x;
-                raw[ks][1] *= gain.y; raw[ks][3] *= gain.y;
-                v[ks] = as_operand(raw[ks]);
+                for (int c = 0; c < OC; ++c) o[c] *= level;
             }
         }
-        constexpr int NU = (V ? 2 : 0) + (Z ? 2 : 0), KU = KT < 8 / NU ? KT : 8 / NU;
+        if (Z) __syncthreads();
+        // The results: tokens in order on top of Q S_0.
+        {
+            float a1[C], a2[C];
+            if (V) load<C>(b + R.a1 + t * 24, a1);
+            if (Z) load<C>(b + R.a2 + t * 24, a2);
 #pragma unroll
-        for (int k0 = 0; k0 < KT; k0 += KU) {
-            float bb[KU * NU][2], p[KU * NU][4];
+            for (int s = 0; s < C; ++s) {
+                float x[OC];
+                if (Z) {
+                    load<OC>(&z_s[s][oc], x);
 #pragma unroll
-            for (int k = 0; k < KU; ++k) {
-                const int d = ch0 + 8 * (k0 + k) + g;
+                    for (int c = 0; c < OC; ++c) o[c] = fmaf(a2[s], x[c], o[c]);
+                }
+                if (V) {
+                    load<OC>(&v_c[s][oc], x);
 #pragma unroll
-                for (int ks = 0; ks < 2; ++ks) {
-                    const int t = 8 * ks + 2 * t4;
-                    if (V) {
-                        bb[k * NU + ks][0] = b[R.k1 + t * (DP + 4) + d];
-                        bb[k * NU + ks][1] = b[R.k1 + (t + 1) * (DP + 4) + d];
-                    }
-                    if (Z) {
-                        bb[k * NU + NU - 2 + ks][0] = b[R.k2 + t * (DP + 4) + d];
-                        bb[k * NU + NU - 2 + ks][1] = b[R.k2 + (t + 1) * (DP + 4) + d];
+                    for (int c = 0; c < OC; ++c) o[c] = fmaf(a1[s], x[c], o[c]);
+                }
+            }
+            if (ci * C + t < n) {
+                float* at = out + (size_t)(r0 + ci * C + t) * H * Dv + (size_t)h * Dv + col;
+#pragma unroll
+                for (int c = 0; c < OC; ++c)
+                    if (col + c < Dv) at[c] = o[c] * q_scale;
+            }
+        }
+        // The state: earlier tokens by themselves, the decayed state, the chunk's last tokens (eight of sixteen, fewer of fewer) on top, in their
+        // order: fewer roundings of a state that decays slowly than a walk over tokens makes, and no others where the last tokens dominate.
+        const int left = n - ci * C, split = left > 12 ? 8 : left > 8 ? 4 : 0;
+        float2 N[TD / 2][TC];
+#pragma unroll
+        for (int i = 0; i < TD / 2; ++i)
+#pragma unroll
+            for (int c = 0; c < TC; ++c) N[i][c] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < C; ++s) {
+            if (s % 4 == 0 && s <= 8 && s == split) {
+#pragma unroll
+                for (int i = 0; i < TD / 4; ++i) {
+                    float4 decay;
+                    if (MODE == CHUNK_HEAD_DECAY) decay.x = decay.y = decay.z = decay.w = b[R.decay + 2 * C];
+                    else decay = *(const float4*)(b + R.decay + d0 + 4 * i);
+#pragma unroll
+                    for (int c = 0; c < TC; ++c) {
+                        N[2 * i][c] = fma2(low2(decay), S[2 * i][c], N[2 * i][c]);
+                        N[2 * i + 1][c] = fma2(high2(decay), S[2 * i + 1][c], N[2 * i + 1][c]);
                     }
                 }
             }
-            products<KU * NU>(p, [&](int i) -> const Split& { return V && i % NU < 2 ? v[i & 1] : z[i & 1]; }, bb);
+            float v[TC], z[TC];
+            if (Z) load<TC>(&z_s[s][cg * TC], z);
+            if (V) load<TC>(&v_c[s][cg * TC], v);
+            if (MODE == CHUNK_HEAD_DECAY) {
+                const float gain = b[R.decay + C + s];
 #pragma unroll
-            for (int k = 0; k < KU; ++k) {
-                const int kt = k0 + k;
+                for (int c = 0; c < TC; ++c) v[c] *= gain;
+            }
 #pragma unroll
-                for (int i = 1; i < NU; ++i) add4(p[k * NU], p[k * NU + i]);
-                const float2 keep = MODE == CHUNK_HEAD_DECAY ? make_float2(b[R.decay + 2 * C], b[R.decay + 2 * C])
-                                                             : *(const float2*)(b + R.decay + ch0 + 8 * kt + 2 * t4);
-                S[kt][0] = fmaf(keep.x, S[kt][0], p[k * NU][0]);
-                S[kt][1] = fmaf(keep.y, S[kt][1], p[k * NU][1]);
-                S[kt][2] = fmaf(keep.x, S[kt][2], p[k * NU][2]);
-                S[kt][3] = fmaf(keep.y, S[kt][3], p[k * NU][3]);
+            for (int i = 0; i < TD / 4; ++i) {
+                float4 k1, k2;
+                if (Z) k2 = *(const float4*)(b + R.k2 + s * (DP + 4) + d0 + 4 * i);
+                if (V) k1 = *(const float4*)(b + R.k1 + s * (DP + 4) + d0 + 4 * i);
+#pragma unroll
+                for (int c = 0; c < TC; ++c) {
+                    float2 &low = N[2 * i][c], &high = N[2 * i + 1][c];
+                    if (Z) {
+                        low = fma2(low2(k2), make_float2(z[c], z[c]), low);
+                        high = fma2(high2(k2), make_float2(z[c], z[c]), high);
+                    }
+                    if (V) {
+                        low = fma2(low2(k1), make_float2(v[c], v[c]), low);
+                        high = fma2(high2(k1), make_float2(v[c], v[c]), high);
+                    }
+                }
             }
         }
+#pragma unroll
+        for (int i = 0; i < TD / 2; ++i)
+#pragma unroll
+            for (int c = 0; c < TC; ++c) S[i][c] = N[i][c];
+        keep<OC>(&v_s[(ci + 1) & 1][t][oc], next);
     }
-    if (ci < chunks || bad) {                                  // a record did not come: the copies asked for are waited for (or given up)
-        if (tid == 0) {
-            for (int i = ci; i < chunks && i < ci + STAGES - 1; ++i) tc::mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
-        }
+    if (failed) {                                              // the copies asked for are waited for (or given up)
+        if (tid == 0)
+            for (int i = ci - 1; i < chunks && i < ci + STAGES - 1; ++i) tc::mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
         return;
     }
-    if (!Z) {
-        __syncthreads();
-        if (wd < 2) store(chunks - 1);
-    }
 #pragma unroll
-    for (int kt = 0; kt < KT; ++kt)
+    for (int i = 0; i < TD / 2; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int d = ch0 + 8 * kt + 2 * t4 + (e & 1);
-            if (d < D && (e < 2 ? col0 : col1)) mem[(size_t)d * Dv + col + 8 * (e >> 1)] = S[kt][e];
+        for (int c = 0; c < TC; ++c) {
+            const int d = d0 + 2 * i;
+            float* at = mem + (size_t)d * Dv + col0 + c;
+            if (d < D && col0 + c < Dv) at[0] = S[i][c].x;
+            if (d + 1 < D && col0 + c < Dv) at[Dv] = S[i][c].y;
         }
 }
 
-template <int MODE, int NI, int KT, int STAGES>
+template <int MODE, int NI, int TD, int TC, int STAGES>
 static int launch_walk(const Rows& in, const Segments& seg, const float* records, int max_chunks, float q_scale, float* memory, float* out,
                        int H, int D, int Dv, int* err, cudaStream_t stream) {
     constexpr int bytes = STAGES * record_of(MODE, 64 * NI).total * (int)sizeof(float);
-    if (bytes > 8 * 1024) {                                    // (the kernel has up to 32 KB of its own beside it)
-        const cudaError_t e = cudaFuncSetAttribute(chunk_walk_kernel<MODE, NI, KT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    auto kernel = chunk_walk_kernel<MODE, NI, TD, TC, STAGES>;
+    if (bytes > 16 * 1024) {                                   // (the kernel has shared memory of its own beside it)
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return (int)e;
     }
     // Not as a dependent launch: blocks placed while the records are still being made crowd onto the SMs that are free first, and
     // stay there (7 heads of 64 x 128, 2,048 tokens: 219 us against 112).
-    chunk_walk_kernel<MODE, NI, KT, STAGES><<<dim3((Dv + 15) / 16, H, seg.count), 64 * NI / (8 * KT) * 32, bytes, stream>>>(
-        in, seg, records, max_chunks, q_scale, memory, out, H, D, Dv, err);
+    kernel<<<dim3((Dv + 15) / 16, H, seg.count), 16 * 64 * NI / (TD * TC), bytes, stream>>>(in, seg, records, max_chunks, q_scale, memory, out, H,
+                                                                                           D, Dv, err);
     return kvb_launch_status();
 }
 
@@ -724,9 +721,9 @@ static int run(const Rows& in, const Segments& seg, float* records, int max_chun
     }
     const int rc = kvb_launch_status();
     if (rc != KVB_OK) return rc;
-    // Key channels a warp holds: 16 of 64 (four warps), 32 of 128 (four warps); with two warps (eight) a column the same calls take 6
-    // to 45 % (8 to 22 %) longer.  A third stage never pays: it costs blocks an SM.
-    return launch_walk<MODE, NI, 2 * NI, 2>(in, seg, records, max_chunks, q_scale, memory, out, H, D, Dv, err, stream);
+    // Key and value channels a thread holds: 4 x 2 of 64 (four warps), 8 x 2 of 128 (four warps).  Half of the warps with 4 x 4 or 8 x 2 of 64
+    // take 16 to 35 % longer, 4 x 4 and 8 x 4 of 128 8 to 40 %, 8 x 1 30 to 50 %.
+    return launch_walk<MODE, NI, 4 * NI, 2, 2>(in, seg, records, max_chunks, q_scale, memory, out, H, D, Dv, err, stream);
 }
 
 // Whether the columns that the heads read lie within a row of `rows` and of `gates` (the decays of CHUNK_CHANNEL_DECAY are rows of

@@ -29,8 +29,8 @@
 // 325 -> 220; delta rule 543 + 905 + 363 x 16 x 128: 660 -> 250, 1,000 x 14 x 64: 196 -> 131; channel decays 600 + 400 x 8 x 128 x 256: 148 -> 64; head
 // decays 2,048 x 64 x 128 x 64: 278 -> 239.  Products of tf32 halves on the tensor cores in the walk took 61, 146, 188, 97, 54 and 187, with states
 // up to three times as far from 64 bits.
-// A segment's result does not depend on what else the step holds.  An infinite or undefined value spreads within its chunk of
-// sixteen tokens, in its own value channel, also to tokens before it.
+// A segment's result does not depend on what else the step holds, and a token's not on later ones, whatever they hold (an infinite or undefined
+// number of one reaches those after it, as in a walk over tokens).
 // State layout: [slot, head, key channel, value channel].
 #include "common.cuh"
 #include "tc_common.cuh"
@@ -556,14 +556,18 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
         }
         float z_own[OC] = {}, o[OC] = {};
         if (Z) {                                               // W V, while the others get here
-            float w[C];
-            load<C>(b + R.w + t * 24, w);
 #pragma unroll
-            for (int s = 0; s < C; ++s) {
-                float v[OC];
-                load<OC>(&v_c[s][oc], v);
+            for (int s0 = 0; s0 < C; s0 += 4) {
+                if (s0 > t) break;                             // later tokens are left out whatever they hold
+                float w[4], v[OC];
+                load<4>(b + R.w + t * 24 + s0, w);
 #pragma unroll
-                for (int c = 0; c < OC; ++c) z_own[c] = fmaf(w[s], v[c], z_own[c]);
+                for (int s = 0; s < 4; ++s) {
+                    load<OC>(&v_c[s0 + s][oc], v);
+#pragma unroll
+                    for (int c = 0; c < OC; ++c)
+                        if (s0 + s <= t) z_own[c] = fmaf(w[s], v[c], z_own[c]);
+                }
             }
         }
         __syncthreads();
@@ -595,21 +599,26 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
         if (Z) __syncthreads();
         // The results: tokens in order on top of Q S_0.
         {
-            float a1[C], a2[C];
-            if (V) load<C>(b + R.a1 + t * 24, a1);
-            if (Z) load<C>(b + R.a2 + t * 24, a2);
 #pragma unroll
-            for (int s = 0; s < C; ++s) {
-                float x[OC];
-                if (Z) {
-                    load<OC>(&z_s[s][oc], x);
+            for (int s0 = 0; s0 < C; s0 += 4) {
+                if (s0 > t) break;
+                float a1[4], a2[4], x[OC];
+                if (V) load<4>(b + R.a1 + t * 24 + s0, a1);
+                if (Z) load<4>(b + R.a2 + t * 24 + s0, a2);
 #pragma unroll
-                    for (int c = 0; c < OC; ++c) o[c] = fmaf(a2[s], x[c], o[c]);
-                }
-                if (V) {
-                    load<OC>(&v_c[s][oc], x);
+                for (int s = 0; s < 4; ++s) {
+                    if (Z) {
+                        load<OC>(&z_s[s0 + s][oc], x);
 #pragma unroll
-                    for (int c = 0; c < OC; ++c) o[c] = fmaf(a1[s], x[c], o[c]);
+                        for (int c = 0; c < OC; ++c)
+                            if (s0 + s <= t) o[c] = fmaf(a2[s], x[c], o[c]);
+                    }
+                    if (V) {
+                        load<OC>(&v_c[s0 + s][oc], x);
+#pragma unroll
+                        for (int c = 0; c < OC; ++c)
+                            if (s0 + s <= t) o[c] = fmaf(a1[s], x[c], o[c]);
+                    }
                 }
             }
             if (ci * C + t < n) {

@@ -179,7 +179,7 @@ def _scan_chunks(kernels, mode, lens, q, k, v, a, b, u, c, state, slots):
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
     batch = StepBatch(T, len(lens), 0, None, None, None, i32([sum(lens[:i]) for i in range(len(lens))]), i32(lens), None, i32(slots), None,
                       max_q_len=max(lens))
-    memory, out = state.to(DEV), torch.full((T, H * Dv), float("nan"), device=DEV)
+    memory, out = state.clone().to(DEV), torch.full((T, H * Dv), float("nan"), device=DEV)
     kernels._chunk_scan(mode, rows.contiguous().to(DEV), cols, G, gates.contiguous().to(DEV), 0.5, batch, memory, out, H, D, Dv, Workspace(DEV))
     kernels.check_errors()
     return out.view(-1, H, Dv).cpu(), memory.cpu()
@@ -219,6 +219,31 @@ def test_scan_in_chunks_rounds_no_worse_than_a_walk_over_tokens(kernels, mode, r
     for got, over_tokens, ref in zip((out, memory[slots]), walk, exact):
         off = lambda x: ((x.double() - ref).norm() / ref.norm()).item()
         assert off(got) <= 1.1 * off(over_tokens)
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("what", range(7))
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_scan_in_chunks_keeps_a_token_from_those_before_it(kernels, mode, what, value):
+    """An infinite or undefined number in any of a token's inputs: the tokens before it give the bits they give without it, and an
+    infinite value leaves the other value channels' alone."""
+    lens, H, D, Dv, at = [40], 2, 64, 24, 29
+    *tokens, state = _scan_inputs(mode, lens, H, H, D, Dv, lambda r: torch.exp(-r))
+    used = {"gated_delta": (0, 1, 2, 3, 4), "delta_rule": (0, 1, 2, 3, 5, 6), "channel_decay": (0, 1, 2, 3), "head_decay": (0, 1, 2, 3, 4)}[mode]
+    if what not in used:
+        pytest.skip("not an input of this form")
+    out, memory = _scan_chunks(kernels, mode, lens, *tokens, state, [1])
+    tokens[what] = tokens[what].clone()
+    if mode == "head_decay" and what == 3:
+        tokens[what][at] = value                                         # one decay for all channels of a head
+    else:
+        tokens[what][at].view(-1)[5 if what != 4 else 0] = value
+    bad, bad_memory = _scan_chunks(kernels, mode, lens, *tokens, state, [1])
+    assert torch.equal(bad[:at], out[:at])
+    assert not torch.isfinite(bad[at:]).all()
+    if what == 2:
+        others = [c for c in range(Dv) if c != 5]
+        assert torch.equal(bad[..., others], out[..., others]) and torch.equal(bad_memory[..., others], memory[..., others])
 
 
 @pytest.mark.parametrize("M", [17, 32, 33, 65, 300])

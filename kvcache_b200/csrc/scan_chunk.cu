@@ -123,11 +123,11 @@ struct Decay {
 };
 
 // ---- launches (1): the records ---------------------------------------------------------------------------------------------
-// grid (chunks, heads), 256 threads.  Thread (s, part): token s as a key, channels 4 part .. + 3 of every 64.
+// grid (chunks from `first` on, heads), 256 threads.  Thread (s, part): token s as a key, channels 4 part .. + 3 of every 64.
 template <int MODE, int NI>          // NI: 64-channel groups of a row
 __global__ void __launch_bounds__(256, MODE == CHUNK_DELTA_RULE && NI == 2 ? 3 : 4) chunk_records_kernel(const Rows in, const Segments seg,
-                                                                                                       float* __restrict__ records, int H,
-                                                                                                       int D, int wide) {
+                                                                                                       float* __restrict__ records, int first,
+                                                                                                       int H, int D, int wide) {
     constexpr int DP = 64 * NI, PARTS = MODE == CHUNK_DELTA_RULE ? 5 : 3;
     __shared__ __align__(16) float rows_s[PARTS][C][DP];       // q, k, a (, u, c)
     __shared__ float low_s[C][C + 1], mat_s[C][C + 1], b_s[C];
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256, MODE == CHUNK_DELTA_RULE && NI == 2 ? 3 :
     pdl_wait();
     pdl_launch_dependents();
     int r0, count;
-    if (!find_chunk(blockIdx.x, seg, r0, count)) return;
+    if (!find_chunk(first + blockIdx.x, seg, r0, count)) return;
     constexpr Record R = record_of(MODE, DP);
     float* rec = records + ((size_t)blockIdx.x * H + h) * R.total;
 
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256, MODE == CHUNK_DELTA_RULE && NI == 2 ? 3 :
 // Delta rule: T = (1 + u . c)^-1, Y = T . (the reads that meet S_0, where Y will lie), W = T (u . k).  grid (chunks, heads), a thread
 // per channel.  By itself, because half a block would wait for the system's sixteen threads in the launch before it.
 template <int NI>
-__global__ void __launch_bounds__(64 * NI) chunk_solve_kernel(const Segments seg, float* __restrict__ records, int H) {
+__global__ void __launch_bounds__(64 * NI) chunk_solve_kernel(const Segments seg, float* __restrict__ records, int first, int H) {
     constexpr int DP = 64 * NI;
     constexpr Record R = record_of(CHUNK_DELTA_RULE, DP);
     __shared__ float low_s[C][C + 1], mat_s[C][C + 1];
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(64 * NI) chunk_solve_kernel(const Segments seg
     pdl_wait();
     pdl_launch_dependents();
     int r0, count;
-    if (!find_chunk(blockIdx.x, seg, r0, count)) return;
+    if (!find_chunk(first + blockIdx.x, seg, r0, count)) return;
     float* rec = records + ((size_t)blockIdx.x * H + blockIdx.y) * R.total;
     for (int i = d; i < C * C; i += DP) low_s[i / C][i % C] = i / C == i % C ? 0.f : rec[R.w + i / C * 24 + i % C];
     float x[C];
@@ -319,9 +319,10 @@ __global__ void __launch_bounds__(64 * NI) chunk_solve_kernel(const Segments seg
     }
 }
 
-// Head decay: grid (chunks, groups of heads with one q and k).
+// Head decay: grid (chunks from `first` on, groups of heads with one q and k); `held`: the chunks that `records` has room for.
 template <int NI>
-__global__ void __launch_bounds__(256) head_records_kernel(const Rows in, const Segments seg, float* __restrict__ records, int H, int D) {
+__global__ void __launch_bounds__(256) head_records_kernel(const Rows in, const Segments seg, float* __restrict__ records, int first, int held, int H,
+                                                           int D) {
     constexpr int DP = 64 * NI, HEADS = 16;
     __shared__ __align__(16) float q_s[C][DP], k_s[C][DP];
     __shared__ float qk_s[C][C + 1], a_s[HEADS][C], d_s[HEADS][C];
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(256) head_records_kernel(const Rows in, const 
     pdl_wait();
     pdl_launch_dependents();
     int r0, count;
-    if (!find_chunk(blockIdx.x, seg, r0, count)) return;
+    if (!find_chunk(first + blockIdx.x, seg, r0, count)) return;
 #pragma unroll
     for (int i = 0; i < NI; ++i)
 #pragma unroll
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(256) head_records_kernel(const Rows in, const 
     }
     qk_s[part][s] = sum16(sums, part);
     constexpr Record R = record_of(CHUNK_HEAD_DECAY, DP);
-    const int groups = H / in.qk_div, first = g * in.qk_div, last = first + in.qk_div;
+    const int groups = H / in.qk_div, head0 = g * in.qk_div, head1 = head0 + in.qk_div;
     {
         float* rec = records + ((size_t)blockIdx.x * groups + g) * R.shared;
 #pragma unroll
@@ -360,12 +361,12 @@ __global__ void __launch_bounds__(256) head_records_kernel(const Rows in, const 
             *(float4*)(rec + R.q + s * (DP + 8) + d) = *(const float4*)&q_s[s][d];
             *(float4*)(rec + R.k1 + s * (DP + 4) + d) = *(const float4*)&k_s[s][d];
         }
-        records += (size_t)gridDim.x * groups * R.shared;
+        records += (size_t)held * groups * R.shared;
     }
-    for (int h0 = first; h0 < last; h0 += HEADS) {
+    for (int h0 = head0; h0 < head1; h0 += HEADS) {
         __syncthreads();
         {                                                          // head h0 + part, token s
-            const bool there = h0 + part < last && s < count;
+            const bool there = h0 + part < head1 && s < count;
             const float* gate = in.gates + (size_t)(r0 + (there ? s : 0)) * in.gate_stride + (there ? h0 + part : 0);
             a_s[part][s] = there ? gate[0] : 1.f;
             d_s[part][s] = there ? gate[H] : 0.f;
@@ -373,7 +374,7 @@ __global__ void __launch_bounds__(256) head_records_kernel(const Rows in, const 
         __syncthreads();
         // Thread (head h0 + s, token `part` as a key).
         const int h = h0 + s;
-        if (h < last) {
+        if (h < head1) {
             float* rec = records + ((size_t)blockIdx.x * H + h) * (R.total - R.shared);
             const float gain = d_s[s][part];
             Decay run, all;
@@ -430,11 +431,11 @@ __device__ __forceinline__ void copy_bulk(float* smem, const float* gmem, uint32
                  ::"r"(tc::smem_u32(smem)), "l"(gmem), "r"(bytes), "r"(tc::smem_u32(bar)) : "memory");
 }
 
-// grid (16 value channels, heads, segments).  A thread holds TD neighbouring key channels of TC value channels of the state; a warp's lanes
+// grid (16 value channels, heads, segments), over the chunks first .. first + held - 1 of the step.  A thread holds TD neighbouring key channels of TC value channels of the state; a warp's lanes
 // are 2 TC groups of key channels by 16 / TC of value channels.  Beside that, every thread owns one token's OC value channels of Z and O.
 template <int MODE, int NI, int TD, int TC, int STAGES>
 __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(const Rows in, const Segments seg, const float* __restrict__ records,
-                                                                             int max_chunks, float q_scale, float* __restrict__ memory,
+                                                                             int first, int held, float q_scale, float* __restrict__ memory,
                                                                              float* __restrict__ out, int H, int D, int Dv, int* __restrict__ err) {
     constexpr bool Z = has_z(MODE), V = has_v(MODE);
     constexpr int DP = 64 * NI, CG = 16 / TC, DG = 32 / CG, WARPS = DP / (TD * DG), OC = 16 * C / (32 * WARPS);
@@ -448,11 +449,16 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
     __shared__ __align__(8) uint64_t full[STAGES];
     const int tid = threadIdx.x, lane = tid & 31, wd = tid >> 5, cg = lane % CG, dg = lane / CG;
     const int h = blockIdx.y, sg = blockIdx.z;
-    const int n = seg.q_len[sg], r0 = seg.q_start[sg], slot = seg.slot[sg];
+    int n = seg.q_len[sg], r0 = seg.q_start[sg], chunk0 = 0;
+    const int slot = seg.slot[sg];
     if (n <= 0) return;
-    int chunk0 = 0;
     for (int i = 0; i < sg; ++i) chunk0 += (seg.q_len[i] + C - 1) / C;
-    const int chunks = (n + C - 1) / C, d0 = (wd * DG + dg) * TD;
+    // The segment's chunks from `begin` on that are among the `held` whose records are there.
+    const int begin = max(0, first - chunk0), chunks = min((n + C - 1) / C, first + held - chunk0) - begin, d0 = (wd * DG + dg) * TD;
+    if (chunks <= 0) return;
+    n -= begin * C;
+    r0 += begin * C;
+    chunk0 += begin - first;
 
     float* mem = memory + ((size_t)slot * H + h) * D * Dv;
     const int col0 = 16 * blockIdx.x + cg * TC;
@@ -479,7 +485,7 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
         tc::mbar_expect_tx(bar, R.total * 4);
         if (R.shared) {
             copy_bulk(b, records + (id * groups + h / in.qk_div) * R.shared, R.shared * 4, bar);
-            copy_bulk(b + R.shared, records + (size_t)max_chunks * groups * R.shared + (id * H + h) * (R.total - R.shared), (R.total - R.shared) * 4, bar);
+            copy_bulk(b + R.shared, records + (size_t)held * groups * R.shared + (id * H + h) * (R.total - R.shared), (R.total - R.shared) * 4, bar);
         } else {
             copy_bulk(b, records + (id * H + h) * R.total, R.total * 4, bar);
         }
@@ -701,7 +707,7 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
 }
 
 template <int MODE, int NI, int TD, int TC, int STAGES>
-static int launch_walk(const Rows& in, const Segments& seg, const float* records, int max_chunks, float q_scale, float* memory, float* out,
+static int launch_walk(const Rows& in, const Segments& seg, const float* records, int first, int held, float q_scale, float* memory, float* out,
                        int H, int D, int Dv, int* err, cudaStream_t stream) {
     constexpr int bytes = STAGES * record_of(MODE, 64 * NI).total * (int)sizeof(float);
     auto kernel = chunk_walk_kernel<MODE, NI, TD, TC, STAGES>;
@@ -711,28 +717,33 @@ static int launch_walk(const Rows& in, const Segments& seg, const float* records
     }
     // Not as a dependent launch: blocks placed while the records are still being made crowd onto the SMs that are free first, and
     // stay there (7 heads of 64 x 128, 2,048 tokens: 219 us against 112).
-    kernel<<<dim3((Dv + 15) / 16, H, seg.count), 16 * 64 * NI / (TD * TC), bytes, stream>>>(in, seg, records, max_chunks, q_scale, memory, out, H,
+    kernel<<<dim3((Dv + 15) / 16, H, seg.count), 16 * 64 * NI / (TD * TC), bytes, stream>>>(in, seg, records, first, held, q_scale, memory, out, H,
                                                                                            D, Dv, err);
     return kvb_launch_status();
 }
 
+// `held` chunks at a time, as many as `records` has room for; the states pass from one run of them to the next through `memory`.
 template <int MODE, int NI>
-static int run(const Rows& in, const Segments& seg, float* records, int max_chunks, float q_scale, float* memory, float* out, int H, int D,
+static int run(const Rows& in, const Segments& seg, float* records, int total, int held, float q_scale, float* memory, float* out, int H, int D,
                int Dv, int* err, cudaStream_t stream) {
-    if constexpr (MODE == CHUNK_HEAD_DECAY)
-        kvb_launch(head_records_kernel<NI>, dim3(max_chunks, H / in.qk_div), dim3(256), 0, stream, in, seg, records, H, D);
-    else
-    {
-        const int wide = ((D | in.stride | in.gate_stride | in.q_col | in.k_col) & 3) == 0 && (((uintptr_t)in.rows | (uintptr_t)in.gates) & 15) == 0;
-        kvb_launch(chunk_records_kernel<MODE, NI>, dim3(max_chunks, H), dim3(256), 0, stream, in, seg, records, H, D, wide);
-        if constexpr (MODE == CHUNK_DELTA_RULE)
-            kvb_launch(chunk_solve_kernel<NI>, dim3(max_chunks, H), dim3(64 * NI), 0, stream, seg, records, H);
+    for (int first = 0; first < total; first += held) {
+        const int count = min(held, total - first);
+        if constexpr (MODE == CHUNK_HEAD_DECAY) {
+            kvb_launch(head_records_kernel<NI>, dim3(count, H / in.qk_div), dim3(256), 0, stream, in, seg, records, first, held, H, D);
+        } else {
+            const int wide = ((D | in.stride | in.gate_stride | in.q_col | in.k_col) & 3) == 0 && (((uintptr_t)in.rows | (uintptr_t)in.gates) & 15) == 0;
+            kvb_launch(chunk_records_kernel<MODE, NI>, dim3(count, H), dim3(256), 0, stream, in, seg, records, first, H, D, wide);
+            if constexpr (MODE == CHUNK_DELTA_RULE)
+                kvb_launch(chunk_solve_kernel<NI>, dim3(count, H), dim3(64 * NI), 0, stream, seg, records, first, H);
+        }
+        int rc = kvb_launch_status();
+        if (rc != KVB_OK) return rc;
+        // Key and value channels a thread holds: 4 x 2 of 64 (four warps), 8 x 2 of 128 (four warps).  Half of the warps with 4 x 4 or 8 x 2 of 64
+        // take 16 to 35 % longer, 4 x 4 and 8 x 4 of 128 8 to 40 %, 8 x 1 30 to 50 %.
+        rc = launch_walk<MODE, NI, 4 * NI, 2, 2>(in, seg, records, first, held, q_scale, memory, out, H, D, Dv, err, stream);
+        if (rc != KVB_OK) return rc;
     }
-    const int rc = kvb_launch_status();
-    if (rc != KVB_OK) return rc;
-    // Key and value channels a thread holds: 4 x 2 of 64 (four warps), 8 x 2 of 128 (four warps).  Half of the warps with 4 x 4 or 8 x 2 of 64
-    // take 16 to 35 % longer, 4 x 4 and 8 x 4 of 128 8 to 40 %, 8 x 1 30 to 50 %.
-    return launch_walk<MODE, NI, 4 * NI, 2, 2>(in, seg, records, max_chunks, q_scale, memory, out, H, D, Dv, err, stream);
+    return KVB_OK;
 }
 
 // Whether the columns that the heads read lie within a row of `rows` and of `gates` (the decays of CHUNK_CHANNEL_DECAY are rows of
@@ -747,16 +758,18 @@ static bool rows_fit(int mode, const Rows& in, int H, int G, int D, int Dv) {
 }
 
 template <int MODE>
-static int run(const Rows& in, const Segments& seg, float* records, int max_chunks, float q_scale, float* memory, float* out, int T, int H,
+static int run(const Rows& in, const Segments& seg, float* records, int held, float q_scale, float* memory, float* out, int T, int H,
                int G, int D, int Dv, int* err, cudaStream_t stream) {
     if (H < 1 || G < 1 || H % G || D < 1 || Dv < 1 || !rows_fit(MODE, in, H, G, D, Dv)) return KVB_ERR_SHAPE;
     if (seg.count <= 0 || T <= 0) return KVB_OK;
     if (records == nullptr) return KVB_ERR_SHAPE;
     if ((uintptr_t)records & 15) return KVB_ERR_ALIGN;
-    if (D > 128 || H > 65535 || seg.count > 65535 || max_chunks < T / C + seg.count) return KVB_ERR_LIMIT;
+    if (D > 128 || H > 65535 || seg.count > 65535 || held < 1) return KVB_ERR_LIMIT;
     if (MODE == CHUNK_CHANNEL_DECAY && Dv > 512) return KVB_ERR_LIMIT;      // as the other forms of this scan
-    return D <= 64 ? run<MODE, 1>(in, seg, records, max_chunks, q_scale, memory, out, H, D, Dv, err, stream)
-                   : run<MODE, 2>(in, seg, records, max_chunks, q_scale, memory, out, H, D, Dv, err, stream);
+    const int total = T / C + seg.count;                       // no step has more chunks than this
+    held = min(held, total);
+    return D <= 64 ? run<MODE, 1>(in, seg, records, total, held, q_scale, memory, out, H, D, Dv, err, stream)
+                   : run<MODE, 2>(in, seg, records, total, held, q_scale, memory, out, H, D, Dv, err, stream);
 }
 
 }  // namespace sc
@@ -769,16 +782,17 @@ KVB_API int kvb_chunk_record_floats(int mode, int D) {
 KVB_API int kvb_chunk_shared_floats(int mode, int D) { return mode < 0 || mode > 3 || D < 1 ? -1 : sc::record_of(mode, sc::padded(D)).shared; }
 
 // The scans over portions of prompts.  `rows` [T, stride] holds q, k and v at their columns (head h: number h / (H / G) of D for q and k,
-// number h of Dv for v; H a multiple of G), `gates` [T, gate_stride] the mode's own numbers (sc::Rows); `records`: scratch of max_chunks
-// (at least T / 16 + S) times the floats above for all H heads and G groups, on 16 bytes.  D up to 128.
+// number h of Dv for v; H a multiple of G), `gates` [T, gate_stride] the mode's own numbers (sc::Rows); `records`: scratch of `held` times
+// the floats above for all H heads and G groups, on 16 bytes: a step of more chunks (at most T / 16 + S) goes through it `held` chunks at a
+// time, with the same results.  D up to 128.
 KVB_API int kvb_chunk_scan(int mode, const float* rows, int stride, int q_col, int k_col, int v_col, int G, const float* gates,
                            int gate_stride, float q_scale, const int* seg_q_start, const int* seg_q_len, const int* seg_slot, float* memory,
-                           float* out, int T, int S, int H, int D, int Dv, int max_chunks, float* records, int* err, cudaStream_t stream) {
+                           float* out, int T, int S, int H, int D, int Dv, int held, float* records, int* err, cudaStream_t stream) {
     const sc::Rows in = {rows, gates, stride, gate_stride, q_col, k_col, v_col, G > 0 ? H / G : 0};
     const sc::Segments seg = {seg_q_start, seg_q_len, seg_slot, S};
-    if (mode == sc::CHUNK_GATED_DELTA) return sc::run<sc::CHUNK_GATED_DELTA>(in, seg, records, max_chunks, q_scale, memory, out, T, H, G, D, Dv, err, stream);
-    if (mode == sc::CHUNK_DELTA_RULE) return sc::run<sc::CHUNK_DELTA_RULE>(in, seg, records, max_chunks, q_scale, memory, out, T, H, G, D, Dv, err, stream);
-    if (mode == sc::CHUNK_CHANNEL_DECAY) return sc::run<sc::CHUNK_CHANNEL_DECAY>(in, seg, records, max_chunks, q_scale, memory, out, T, H, G, D, Dv, err, stream);
-    if (mode == sc::CHUNK_HEAD_DECAY) return sc::run<sc::CHUNK_HEAD_DECAY>(in, seg, records, max_chunks, q_scale, memory, out, T, H, G, D, Dv, err, stream);
+    if (mode == sc::CHUNK_GATED_DELTA) return sc::run<sc::CHUNK_GATED_DELTA>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, err, stream);
+    if (mode == sc::CHUNK_DELTA_RULE) return sc::run<sc::CHUNK_DELTA_RULE>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, err, stream);
+    if (mode == sc::CHUNK_CHANNEL_DECAY) return sc::run<sc::CHUNK_CHANNEL_DECAY>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, err, stream);
+    if (mode == sc::CHUNK_HEAD_DECAY) return sc::run<sc::CHUNK_HEAD_DECAY>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, err, stream);
     return KVB_ERR_SHAPE;
 }

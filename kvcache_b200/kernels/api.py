@@ -1363,6 +1363,9 @@ class CudaKernels(KernelSet):
     # Portions go sixteen tokens at a time over the tensor cores (csrc/scan_chunk.cu) where a head has at most CHUNK_SCAN_MAX_DIM key
     # channels.
     CHUNK_SCAN_MAX_DIM = 128
+    # Scratch of a scan for portions: longer steps go through it in runs of as many chunks as it holds (16 heads of 128 channels under the delta
+    # rule: 39 KB a head and chunk, 6,800 tokens a run; the whole of a step of 30,000 would take 1.2 GB).
+    CHUNK_SCRATCH_BYTES = 256 << 20
     CHUNK_MODES = {"gated_delta": 0, "delta_rule": 1, "channel_decay": 2, "head_decay": 3}
 
     def _chunk_scan(self, mode: str, rows, cols, G: int, gates, q_scale: float, batch: StepBatch, memory, out, H: int, D: int, Dv: int,
@@ -1371,13 +1374,16 @@ class CudaKernels(KernelSet):
             raise KernelError(f"{mode}: {H} heads cannot share {G} queries and keys evenly")
         code, lib = self.CHUNK_MODES[mode], self._scan_chunk
         T, S = rows.shape[0], batch.num_segments
-        max_chunks = T // 16 + S             # by the step's rows and segments alone, so that a recorded step finds the same launches
         size = H * lib.kvb_chunk_record_floats(code, D) + G * lib.kvb_chunk_shared_floats(code, D)
-        records = workspace.buffer("recurrent.chunk_records", (max_chunks * size,), torch.float32)
-        self.launches += 2 if mode == "delta_rule" else 1        # the records (and their triangular systems), beside the walk
+        # By the step's rows and segments alone, so that a recorded step finds the same launches.
+        chunks = T // 16 + S
+        held = min(chunks, max(1, self.CHUNK_SCRATCH_BYTES // (4 * size)))
+        records = workspace.buffer("recurrent.chunk_records", (held * size,), torch.float32)
+        # Per run: the records (and their triangular systems) and the walk, one of which has been counted.
+        self.launches += -(-chunks // held) * (3 if mode == "delta_rule" else 2) - 1
         _check(lib.kvb_chunk_scan(code, _ptr(rows), rows.shape[1], *cols, G, _ptr(gates), gates.shape[1], float(q_scale),
                                   _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), _ptr(memory), _ptr(out), T, S, H, D,
-                                  Dv, max_chunks, _ptr(records), _ptr(self.error_word), self._stream()), f"{mode} (chunks)")
+                                  Dv, held, _ptr(records), _ptr(self.error_word), self._stream()), f"{mode} (chunks)")
 
     def gated_linear_scan(self, proj: torch.Tensor, cols, z: torch.Tensor, tau: float, q_scale: float, batch: StepBatch,
                           memory: torch.Tensor, out: torch.Tensor, H: int, D: int, Dv: int, workspace=None) -> None:

@@ -222,6 +222,25 @@ def test_scan_in_chunks_rounds_no_worse_than_a_walk_over_tokens(kernels, mode, r
 
 
 @pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("D", [64, 128])
+def test_scan_in_chunks_within_bounded_scratch(kernels, mode, D, monkeypatch):
+    """Scratch for one chunk, for two and for three at a time: the same bits as for all of them, through segments that end inside a run,
+    with one and that take several; and no more of it than the bound."""
+    lens, H, Dv = [40, 1, 16, 100, 33], 2, 24
+    *tokens, state = _scan_inputs(mode, lens, H, H, D, Dv, lambda r: torch.exp(-0.5 * r))
+    slots = [4, 2, 0, 1, 6]
+    out, memory = _scan_chunks(kernels, mode, lens, *tokens, state, slots)
+    code, lib = kernels.CHUNK_MODES[mode], kernels._scan_chunk
+    size = 4 * H * (lib.kvb_chunk_record_floats(code, D) + lib.kvb_chunk_shared_floats(code, D))
+    for held in (1, 2, 3):
+        monkeypatch.setattr(kernels, "CHUNK_SCRATCH_BYTES", held * size)
+        before = kernels.launches
+        got = _scan_chunks(kernels, mode, lens, *tokens, state, slots)
+        assert torch.equal(got[0], out) and torch.equal(got[1], memory)
+        assert kernels.launches - before == -(-(sum(lens) // 16 + len(lens)) // held) * (3 if mode == "delta_rule" else 2) - 1
+
+
+@pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("what", range(7))
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 def test_scan_in_chunks_keeps_a_token_from_those_before_it(kernels, mode, what, value):

@@ -611,9 +611,9 @@ static int launch_scan(const float* proj, int P, int q_col, int k_col, int v_col
         KVB_SCAN_PASS(SCAN_FROM_START, S);
         return KVB_OK;
     }
-    if constexpr (MODE == SCAN_HEAD_DECAY) {
+    if constexpr (MODE == SCAN_HEAD_DECAY || MODE == SCAN_GATED_DELTA) {
         return KVB_ERR_LIMIT;                                  // in one piece only
-    } else if constexpr (scan_mixes_keys(MODE)) {
+    } else if constexpr (MODE == SCAN_DELTA_RULE) {
         const int state_blocks = col_blocks;
         col_blocks = ((Dv + D + COLS - 1) / COLS + warps - 1) / warps;     // the transition's columns beside the state's
         KVB_SCAN_PASS(SCAN_LOCAL, max_chunks);
@@ -1107,16 +1107,14 @@ KVB_API int kvb_gated_delta_inputs(const float* proj, int P, int col, int b_col,
     return launch_conv_tail(cv, T, S, stream);
 }
 
-// The gated delta rule over the tokens of every segment, from and into memory[slot] ([H, D, Dv], float32); rows and gates as made
-// by kvb_gated_delta_inputs.  out = q_scale S'^T q.  `max_chunks` > 0: the chunked form, as for the other scans, with `scratch`
-// of max_chunks * H * (2 D Dv + D D + 2 D + 3) floats.
+// The gated delta rule over the tokens of every segment, from and into memory[slot] ([H, D, Dv], float32), in one piece; rows and gates
+// as made by kvb_gated_delta_inputs.  out = q_scale S'^T q.
 KVB_API int kvb_gated_delta_scan(const float* rows, const float* gates, int gate_stride, float q_scale, const int* seg_q_start, const int* seg_q_len,
-                                 const int* seg_slot, float* memory, float* out, int T, int S, int H, int G, int D, int Dv, int chunk_len,
-                                 int max_chunks, float* scratch, cudaStream_t stream) {
+                                 const int* seg_slot, float* memory, float* out, int T, int S, int H, int G, int D, int Dv, cudaStream_t stream) {
     if (S <= 0 || T <= 0) return KVB_OK;
     if (G < 1 || H % G || gate_stride < H * D + H) return KVB_ERR_SHAPE;
     return scan_any(SCAN_GATED_DELTA, rows, 2 * G * D + H * Dv, 0, G * D, 2 * G * D, gates, gate_stride, 0, H * D, 0.f, q_scale, 0.f, seg_q_start,
-                    seg_q_len, seg_slot, memory, nullptr, nullptr, out, T, S, H, D, Dv, chunk_len, max_chunks, scratch, stream, true, G);
+                    seg_q_len, seg_slot, memory, nullptr, nullptr, out, T, S, H, D, Dv, 0, 0, nullptr, stream, true, G);
 }
 
 // What the state-space recurrence reads, a warp per (row, job): a run of 128 convolved, activated channels each, then (the last

@@ -1,5 +1,6 @@
 // Scans of mixers that carry a matrix S [D, Dv] per request and head from token to token, a column of S spread over many lanes:
-// the form for portions of many tokens (single tokens and short portions, and delta-rule heads of few key channels: recurrent.cu).
+// the form for portions of many tokens of a gated delta rule with more than 128 key channels, and of a state space up to where sixteen tokens
+// at a time are ahead (scan_chunk.cu; single tokens and short portions: recurrent.cu).
 //
 //   WIDE_GATED_DELTA   S~ = diag(a) S, S' = S~ + k (b (v - S~^T k))^T, o = scale S'^T q   (a: a decay per key channel, b: a number)
 //   WIDE_HEAD_DECAY    S' = c S + d k v^T, o = scale S'^T q                               (c, d: numbers per head)
@@ -386,22 +387,18 @@ static int launch_wide(const WideRows& in, float q_scale, const int* seg_q_start
 }
 
 // rows: float32 [T, C] = [q: G heads of D | k: G heads of D | v: H heads of Dv], unit vectors and values as the delta rule wants them;
-// gates: float32 [T, gate_stride] = [decays: H of D | b: H | ...].  Head h reads query and key h / (H / G).
+// gates: float32 [T, gate_stride] = [decays: H of D | b: H | ...].  Head h reads query and key h / (H / G).  129 to 256 key channels (fewer:
+// scan_chunk.cu).
 KVB_API int kvb_gated_delta_scan_wide(const float* rows, const float* gates, int gate_stride, float q_scale, const int* seg_q_start,
                                  const int* seg_q_len, const int* seg_slot, float* memory, float* out, int S, int H, int G, int D, int Dv,
                                  cudaStream_t stream) {
     if (S <= 0) return KVB_OK;
     if (H < 1 || G < 1 || H % G || D < 1 || Dv < 1 || gate_stride < H * D + H) return KVB_ERR_SHAPE;
-    if (D > 256 || H > 65535 || S > 65535) return KVB_ERR_LIMIT;
+    if (D <= 128 || D > 256 || H > 65535 || S > 65535) return KVB_ERR_LIMIT;
     const int C = 2 * G * D + H * Dv;
     const bool wide = ((D | C | gate_stride) & 3) == 0 && (((uintptr_t)rows | (uintptr_t)gates) & 15) == 0;
     const WideRows in = {rows, gates, C, gate_stride, 0, G * D, 2 * G * D, 0, H * D, 0, H / G, wide ? 1 : 0};
-#define KVB_WIDE(NI, KS) launch_wide<WIDE_GATED_DELTA, NI, KS, DELTA_NC>(in, q_scale, seg_q_start, seg_q_len, seg_slot, memory, out, S, H, D, Dv, stream)
-    if (D <= 32) return KVB_WIDE(2, 4);
-    if (D <= 64) return KVB_WIDE(2, 8);
-    if (D <= 128) return KVB_WIDE(2, 16);
-    return KVB_WIDE(2, 32);
-#undef KVB_WIDE
+    return launch_wide<WIDE_GATED_DELTA, 2, 32, DELTA_NC>(in, q_scale, seg_q_start, seg_q_len, seg_slot, memory, out, S, H, D, Dv, stream);
 }
 
 // rows: float32 [T, C] = [x: H heads of Dv | B: G of N | C: G of N]; gates: float32 [T, 2 H] = [decay: H | d: H].  Head h reads B and C

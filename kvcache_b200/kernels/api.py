@@ -125,7 +125,7 @@ _SIGNATURES = {
                                    _c_float, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
                                    _c_int, _c_int, _c_int, _c_int, _c_void_p],
         "kvb_gated_delta_scan": [_c_void_p, _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int,
-                                 _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
+                                 _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
         "kvb_state_space_scan": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
                                  _c_int, _c_int, _c_int, _c_void_p],
         "kvb_state_space_inputs": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p,
@@ -1501,12 +1501,10 @@ class CudaKernels(KernelSet):
             _ptr(batch.seg_slot), T, batch.num_segments, H, G, D, Dv, self._stream()), "gated_delta_inputs")
 
     # Portions of at least SCAN_WIDE_MIN_ROWS rows leave the walk over tokens in one piece: the gated delta rule with up to
-    # CHUNK_SCAN_MAX_DIM key channels goes sixteen tokens at a time (64 rows of 14 heads of 64: 13 us, 25 with a column over many
-    # lanes, 58 in one piece), with more through the scan that spreads a column over many lanes (csrc/scan_wide.cu; where a head has
-    # no more than DELTA_WIDE_ABOVE, portions long enough for chunks of SCAN_CHUNK side by side take those).  The state space
+    # CHUNK_SCAN_MAX_DIM key channels goes sixteen tokens at a time (48 rows of 14 heads of 64: 11 us, 18 with a column over many lanes,
+    # 44 in one piece), with more through the scan that spreads a column over many lanes (csrc/scan_wide.cu).  The state space
     # spreads its columns (28 heads of 128 x 64: 40 us at 64 rows in one piece, 15 us) up to STATE_SPACE_CHUNK_MIN_ROWS.
     SCAN_WIDE_MIN_ROWS = 48
-    DELTA_WIDE_ABOVE = 64
 
     def gated_delta_scan(self, rows: torch.Tensor, gates: torch.Tensor, q_scale: float, batch: StepBatch, memory: torch.Tensor,
                          out: torch.Tensor, H: int, G: int, D: int, Dv: int, workspace) -> None:
@@ -1522,21 +1520,12 @@ class CudaKernels(KernelSet):
                 raise KernelError("gated_delta_scan: the rows or gates do not fit the heads")
             self._chunk_scan("gated_delta", rows, (0, G * D, 2 * G * D), G, gates, q_scale, batch, memory, out, H, D, Dv, workspace)
             return
-        chunked = self.SCAN_CHUNK and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS
-        if batch.max_q_len >= self.SCAN_WIDE_MIN_ROWS and (D > self.DELTA_WIDE_ABOVE or not chunked):
+        if batch.max_q_len >= self.SCAN_WIDE_MIN_ROWS:
             _check(self._scan_wide.kvb_gated_delta_scan_wide(_ptr(rows), _ptr(gates), gates.shape[1], float(q_scale), *segments,
                                                              batch.num_segments, H, G, D, Dv, self._stream()), "gated_delta_scan (wide)")
             return
-        max_chunks, scratch, chunk = 0, None, self.SCAN_CHUNK
-        if chunked:
-            if batch.max_q_len >= self.DELTA_LONG_ROWS:
-                chunk = max(chunk, self.DELTA_LONG_CHUNK)
-            max_chunks = -(-batch.num_tokens // chunk) + batch.num_segments          # as in `delta_rule_scan`
-            scratch = workspace.buffer("recurrent.delta_chunks", (max_chunks * H * (2 * D * Dv + D * D + 2 * D + 3),), torch.float32)
-            self.launches += 2
         _check(self._recurrent.kvb_gated_delta_scan(_ptr(rows), _ptr(gates), gates.shape[1], float(q_scale), *segments, rows.shape[0],
-                                                    batch.num_segments, H, G, D, Dv, chunk, max_chunks, _ptr(scratch), self._stream()),
-               "gated_delta_scan")
+                                                    batch.num_segments, H, G, D, Dv, self._stream()), "gated_delta_scan")
 
     def state_space_inputs(self, proj: torch.Tensor, col: int, dt_col: int, conv_w: torch.Tensor, conv_b: torch.Tensor, tail: torch.Tensor,
                            dt_bias: torch.Tensor, rate: torch.Tensor, batch: StepBatch, rows: torch.Tensor, gates: torch.Tensor,

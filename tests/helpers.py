@@ -118,3 +118,32 @@ def reference_attention_case():
         assert hashlib.sha256(arr.tobytes()).hexdigest() == meta["inputs_sha256"][name], f"{name} is not what the reference drew"
     out = np.fromfile(os.path.join(golden, "ref_attn_out.f32"), dtype="<f4").reshape(H, D)
     return torch.from_numpy(q), torch.from_numpy(K), torch.from_numpy(V), torch.from_numpy(out.copy())
+
+
+class ScanForms:
+    """Which scan entry points a kernel set calls, in order: a test of one form fails when a changed rule sends its sizes through another."""
+
+    class _Spy:
+        def __init__(self, library, calls):
+            self._library, self._calls = library, calls
+
+        def __getattr__(self, name):
+            fn = getattr(self._library, name)
+            if "scan" not in name:
+                return fn
+
+            def call(*args):
+                self._calls.append((name, args))
+                return fn(*args)
+            return call
+
+    def __init__(self, kernels, monkeypatch):
+        self.calls = []
+        for library in ("_recurrent", "_scan_wide", "_scan_chunk"):
+            monkeypatch.setattr(kernels, library, self._Spy(getattr(kernels, library), self.calls))
+
+    def taken(self):
+        """The entry points called since the last look."""
+        names = [name for name, _ in self.calls]
+        self.calls.clear()
+        return names

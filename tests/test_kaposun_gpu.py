@@ -12,7 +12,7 @@ import torch
 
 import plain_kaposun as plain
 import replay_modes
-from helpers import assert_close, batch_to, clone_kv, make_runner, paged_scenario, random_tokens
+from helpers import ScanForms, assert_close, batch_to, clone_kv, make_runner, paged_scenario, random_tokens
 from kaposun_configs import CONFIGS, PAGE_SIZE, make_kaposun_folder
 from torch_kernels import TorchKernels
 
@@ -243,31 +243,50 @@ def test_scans_of_long_portions(kernels, kind, H, G, D, Dv, shorter):
     assert_close(got, want, 1e-4, "read-out")
     assert_close(got_mem, ref_mem, 1e-4, "states")
     assert torch.equal(got_mem[6].cpu(), memory[6])
-    if kind == "space" or D > kernels.DELTA_WIDE_ABOVE or shorter:
-        at, alone_mem = 0, memory.clone().to(DEV)
-        for (start, n), slot in zip(segments, slots):
-            if n >= kernels.SCAN_WIDE_MIN_ROWS:
-                alone = batch_to(_segments_batch([(start, n)], [slot]), DEV)
-                assert torch.equal(_run_scan(kernels, kind, rows[at:at + n].to(DEV), gates[at:at + n].to(DEV), alone, alone_mem, sizes), got[at:at + n])
-                assert torch.equal(alone_mem[slot], got_mem[slot])
-            at += n
+    at, alone_mem = 0, memory.clone().to(DEV)
+    for (start, n), slot in zip(segments, slots):
+        if n >= kernels.SCAN_WIDE_MIN_ROWS:
+            alone = batch_to(_segments_batch([(start, n)], [slot]), DEV)
+            assert torch.equal(_run_scan(kernels, kind, rows[at:at + n].to(DEV), gates[at:at + n].to(DEV), alone, alone_mem, sizes), got[at:at + n])
+            assert torch.equal(alone_mem[slot], got_mem[slot])
+        at += n
 
 
-@pytest.mark.parametrize("D", [64, 96])
-def test_forms_of_the_delta_scan_agree(kernels, D):
-    """In one piece, in chunks, spread over lanes: the same read-outs and states up to rounding."""
+@pytest.mark.parametrize("D,form", [(64, "kvb_chunk_scan"), (96, "kvb_chunk_scan"), (128, "kvb_chunk_scan"), (129, "kvb_gated_delta_scan_wide"),
+                                    (200, "kvb_gated_delta_scan_wide")])
+def test_forms_of_the_delta_scan_agree(kernels, D, form, monkeypatch):
+    """Sixteen tokens at a time or spread over lanes, and in one piece: the same read-outs and states up to rounding."""
     H, G, Dv = 2, 1, 40
     segments = [(0, 300), (4, 70)]
     rows, gates = (t.to(DEV) for t in _delta_rows(370, H, G, D, Dv))
     batch = batch_to(_segments_batch(segments, [1, 0]), DEV)
-    saved, results = (kernels.DELTA_WIDE_ABOVE, kernels.SCAN_CHUNK, kernels.SCAN_WIDE_MIN_ROWS), []
-    try:
-        for above, chunk, rows_wide in ((0, 64, 48), (256, 64, 48), (256, 0, 1 << 30)):
-            kernels.DELTA_WIDE_ABOVE, kernels.SCAN_CHUNK, kernels.SCAN_WIDE_MIN_ROWS = above, chunk, rows_wide
-            memory = _rand(2, H, D, Dv, seed=3).to(DEV)
-            results.append((_run_scan(kernels, "delta", rows, gates, batch, memory, (H, G, D, Dv)), memory))
-    finally:
-        kernels.DELTA_WIDE_ABOVE, kernels.SCAN_CHUNK, kernels.SCAN_WIDE_MIN_ROWS = saved
+    forms, results = ScanForms(kernels, monkeypatch), []
+    for rows_wide, taken in ((kernels.SCAN_WIDE_MIN_ROWS, form), (1 << 30, "kvb_gated_delta_scan")):
+        monkeypatch.setattr(kernels, "SCAN_WIDE_MIN_ROWS", rows_wide)
+        memory = _rand(2, H, D, Dv, seed=3).to(DEV)
+        results.append((_run_scan(kernels, "delta", rows, gates, batch, memory, (H, G, D, Dv)), memory))
+        assert forms.taken() == [taken]
+    assert_close(results[0][0], results[1][0], 1e-5)
+    assert_close(results[0][1], results[1][1], 1e-5)
+
+
+@pytest.mark.parametrize("N", [64, 128, 130])
+def test_forms_of_the_state_space_scan_agree(kernels, N, monkeypatch):
+    """Sixteen tokens at a time (up to 128 channels), spread over lanes, and in one piece."""
+    from kvcache_b200.engine.workspace import Workspace
+    H, G, Dv = 4, 2, 24
+    segments = [(0, 530), (4, 70)]
+    rows, gates = (t.to(DEV) for t in _space_rows(600, H, G, N, Dv))
+    batch = batch_to(_segments_batch(segments, [1, 0]), DEV)
+    forms, results = ScanForms(kernels, monkeypatch), []
+    wide = "kvb_state_space_scan_wide"
+    for chunks, rows_wide, taken in ((512, 48, "kvb_chunk_scan" if N <= 128 else wide), (531, 48, wide), (531, 531, "kvb_state_space_scan")):
+        monkeypatch.setattr(kernels, "STATE_SPACE_CHUNK_MIN_ROWS", chunks)
+        monkeypatch.setattr(kernels, "SCAN_WIDE_MIN_ROWS", rows_wide)
+        memory, out = _rand(2, H, N, Dv, seed=3).to(DEV), torch.zeros(600, H * Dv, device=DEV)
+        kernels.state_space_scan(rows, gates, batch, memory, out, H, G, N, Dv, workspace=Workspace(DEV))
+        results.append((out, memory))
+        assert forms.taken() == [taken]
     for out, memory in results[1:]:
         assert_close(out, results[0][0], 1e-5)
         assert_close(memory, results[0][1], 1e-5)

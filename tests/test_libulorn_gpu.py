@@ -12,7 +12,7 @@ import torch
 
 import plain_libulorn as plain
 import replay_modes
-from helpers import assert_close, batch_to, clone_kv, make_runner, paged_scenario, random_tokens
+from helpers import ScanForms, assert_close, batch_to, clone_kv, make_runner, paged_scenario, random_tokens
 from libulorn_configs import CONFIGS, PAGE_SIZE, make_libulorn_folder
 from torch_kernels import TorchKernels
 
@@ -128,11 +128,13 @@ def test_matrix_memory_scan(kernels, H, D, Dv):
 
 @pytest.mark.parametrize("mode", ["channel decay", "exponential gates"])
 @pytest.mark.parametrize("H,D,Dv", [(3, 24, 16), (2, 64, 128), (1, 130, 40)])
-def test_scans_in_chunks_side_by_side(kernels, mode, H, D, Dv):
+def test_scans_in_chunks_side_by_side(kernels, mode, H, D, Dv, monkeypatch):
     """A step with a long segment is scanned in chunks of 64 tokens that run side by side: segments that end inside a
     chunk, at a chunk's edge, one token after it, a single token and a segment that continues a state, against the
     plain statement; the states left in the slots too."""
     from kvcache_b200.engine.workspace import Workspace
+    monkeypatch.setattr(kernels, "CHUNK_SCAN_MAX_DIM", 0)                      # (up to 1,024 rows these sizes go sixteen tokens at a time)
+    forms = ScanForms(kernels, monkeypatch)
     segments, slots = [(0, 300), (40, 1), (7, 128), (0, 65), (3, 63)], [1, 4, 0, 2, 5]
     batch = _segments_batch(segments, slots)
     assert batch.max_q_len >= kernels.SCAN_CHUNK_MIN_ROWS
@@ -153,9 +155,29 @@ def test_scans_in_chunks_side_by_side(kernels, mode, H, D, Dv):
     else:
         TorchKernels(wide=True).matrix_memory_scan(proj, cols, 6.0, 0.25, 1e-6, batch, ref[0], ref[1], ref[2], ref[3], H, D, Dv)
         kernels.matrix_memory_scan(proj.to(DEV), cols, 6.0, 0.25, 1e-6, batch_to(batch, DEV), got[0], got[1], got[2], got[3], H, D, Dv, Workspace(DEV))
+    form, args = forms.calls[-1]
+    assert form == "kvb_matrix_state_scan" and args[-4] == kernels.SCAN_CHUNK and args[-3] > 0
     for g, r, what in zip(got, ref, ("memory", "normalizer", "maximum", "read-out")):
         assert_close(g, r, 5e-5, what)
     assert torch.equal(got[0][3].cpu(), memory[3])
+
+
+@pytest.mark.parametrize("rows,D,form", [(255, 64, "kvb_matrix_state_scan"), (256, 64, "kvb_chunk_scan"), (1024, 64, "kvb_chunk_scan"),
+                                         (1025, 64, "kvb_matrix_state_scan"), (1025, 65, "kvb_chunk_scan"), (256, 129, "kvb_matrix_state_scan")])
+def test_which_form_the_gated_linear_scan_takes(kernels, rows, D, form, monkeypatch):
+    """On both sides of every line of the rule: the form it names, against the plain statement."""
+    from kvcache_b200.engine.workspace import Workspace
+    H, Dv = 2, 40
+    batch = _segments_batch([(0, rows), (3, 20)], [1, 0])
+    T, cols = batch.num_tokens, (0, H * D, 2 * H * D)
+    proj, z, memory = _rand(T, 2 * H * D + H * Dv, seed=4), _rand(T, H * D, seed=2, scale=2.0) + 3.0, _rand(2, H, D, Dv, seed=5)
+    ref, got = (memory.clone(), torch.zeros(T, H * Dv)), (memory.clone().to(DEV), torch.zeros(T, H * Dv, device=DEV))
+    TorchKernels(wide=True).gated_linear_scan(proj, cols, z, 5.0, 0.3, batch, *ref, H, D, Dv)
+    forms = ScanForms(kernels, monkeypatch)
+    kernels.gated_linear_scan(proj.to(DEV), cols, z.to(DEV), 5.0, 0.3, batch_to(batch, DEV), *got, H, D, Dv, Workspace(DEV))
+    assert forms.taken() == [form]
+    for g, r, what in zip(got, ref, ("memory", "read-out")):
+        assert_close(g, r, 5e-5, what)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

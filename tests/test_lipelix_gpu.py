@@ -14,7 +14,7 @@ import torch
 
 import plain_lipelix as plain
 import replay_modes
-from helpers import assert_close, batch_to, clone_kv, make_runner, paged_scenario, random_tokens
+from helpers import ScanForms, assert_close, batch_to, clone_kv, make_runner, paged_scenario, random_tokens
 from lipelix_configs import CONFIGS, PAGE_SIZE, config_dict, make_lipelix_folder
 from torch_kernels import TorchKernels
 
@@ -356,9 +356,9 @@ def test_delta_rule_scan(kernels, H, D):
 
 
 @pytest.mark.parametrize("H,D", [(2, 64), (1, 33), (2, 128), (3, 8), (1, 200)])
-def test_delta_rule_scan_of_long_portions_in_chunks(kernels, H, D):
-    """Portions long enough to be cut into chunks that run side by side (each leaves its end state and the product of its
-    tokens' transitions; the start states follow from those): from an empty state and from a filled one, lengths that are
+def test_delta_rule_scan_of_long_portions_in_chunks(kernels, H, D, monkeypatch):
+    """Portions long enough to be cut into chunks - up to 128 key channels sixteen tokens at a time, above chunks that run side by side
+    (each leaves its end state and the product of its tokens' transitions; the start states follow from those): from an empty state and from a filled one, lengths that are
     no multiple of the chunk, beside single tokens and a short portion; against the plain recurrence and against the
     same kernel in one piece."""
     from kvcache_b200.engine.workspace import Workspace
@@ -372,12 +372,17 @@ def test_delta_rule_scan_of_long_portions_in_chunks(kernels, H, D):
     memory[2].zero_()
     ref_mem, ref_out = memory.clone(), torch.zeros(T, H * D)
     TorchKernels(wide=True).delta_rule_scan(proj, cols, z, 0.6, 1e-6, batch, ref_mem, ref_out, H, D)
-    ws = Workspace(DEV)
+    ws, forms = Workspace(DEV), ScanForms(kernels, monkeypatch)
     got_mem, got_out = memory.clone().to(DEV), torch.zeros(T, H * D, device=DEV)
     before = kernels.launches
     kernels.delta_rule_scan(proj.to(DEV), cols, z.to(DEV), 0.6, 1e-6, batch_to(batch, DEV), got_mem, got_out, H, D, ws)
     kernels.check_errors()
-    assert kernels.launches - before == 4, "inputs, local scan, chunk starts, scan from the starts"
+    assert kernels.launches - before == 4, "inputs; records, systems and walk, or local scan, chunk starts and scan from the starts"
+    form, args = forms.calls[-1]
+    if D <= 128:
+        assert form == "kvb_chunk_scan"
+    else:
+        assert form == "kvb_delta_rule_scan" and args[-4] == kernels.SCAN_CHUNK and args[-3] > 0
     assert_close(got_out, ref_out, 1e-4, "read-out")
     assert_close(got_mem, ref_mem, 1e-4, "states")
     assert torch.equal(got_mem[4].cpu(), memory[4])
@@ -387,14 +392,18 @@ def test_delta_rule_scan_of_long_portions_in_chunks(kernels, H, D):
         kernels.delta_rule_scan(proj.to(DEV), cols, z.to(DEV), 0.6, 1e-6, batch_to(batch, DEV), whole_mem, whole_out, H, D, ws)
     finally:
         kernels.SCAN_CHUNK = chunk
+    form, args = forms.calls[-1]
+    assert form == "kvb_delta_rule_scan" and args[-3] == 0
     assert_close(got_out, whole_out, 1e-4, "read-out, chunks against one piece")
     assert_close(got_mem, whole_mem, 1e-4, "states, chunks against one piece")
 
 
-def test_delta_rule_scan_of_a_very_long_portion_takes_longer_chunks(kernels):
-    """A portion long enough for the longer chunks, beside a shorter one and a single token, against the plain recurrence."""
+def test_delta_rule_scan_of_a_very_long_portion_takes_longer_chunks(kernels, monkeypatch):
+    """A portion long enough for the longer chunks, beside a shorter one and a single token, against the plain recurrence: heads of more
+    than 128 key channels."""
     from kvcache_b200.engine.workspace import Workspace
-    H, D = 2, 64
+    H, D = 1, 132
+    forms = ScanForms(kernels, monkeypatch)
     segments, slots = [(10, kernels.DELTA_LONG_ROWS + 77), (0, 130), (5, 1)], [1, 0, 2]
     batch = _segments_batch(segments, slots)
     T = batch.num_tokens
@@ -406,6 +415,8 @@ def test_delta_rule_scan_of_a_very_long_portion_takes_longer_chunks(kernels):
     got_mem, got_out = memory.clone().to(DEV), torch.zeros(T, H * D, device=DEV)
     kernels.delta_rule_scan(proj.to(DEV), cols, z.to(DEV), 0.6, 1e-6, batch_to(batch, DEV), got_mem, got_out, H, D, Workspace(DEV))
     kernels.check_errors()
+    form, args = forms.calls[-1]
+    assert form == "kvb_delta_rule_scan" and args[-4] == kernels.DELTA_LONG_CHUNK and args[-3] > 0
     assert_close(got_out, ref_out, 1e-4, "read-out")
     assert_close(got_mem, ref_mem, 1e-4, "states")
 

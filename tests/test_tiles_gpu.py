@@ -20,22 +20,35 @@ def kernels():
     return CudaKernels(DEV)
 
 
-@pytest.mark.parametrize("N,K", [(1153, 132), (896, 4864), (9728, 100), (40, 77)])
-def test_float32_product_rows_do_not_depend_on_the_tile(kernels, N, K):
-    """Every number of rows at the edges of the tiles and of the rule that picks one: close to 64 bits, and each row bit for
-    bit what it is in the largest step (one chain over k, whatever the tile)."""
+@pytest.mark.parametrize("dtype,out_dtype,N,K", [
+    (torch.float32, torch.float32, 1153, 132), (torch.float32, torch.float32, 896, 4864), (torch.float32, torch.float32, 9728, 100),
+    (torch.float32, torch.float32, 40, 77), (torch.float32, torch.float32, 1153, 333), (torch.float32, torch.float32, 9728, 77),
+    (torch.bfloat16, torch.bfloat16, 1153, 136), (torch.bfloat16, torch.float32, 9728, 104), (torch.bfloat16, torch.bfloat16, 9728, 100),
+    (torch.bfloat16, torch.float32, 1153, 333)])
+def test_float32_product_rows_do_not_depend_on_the_tile(kernels, dtype, out_dtype, N, K):
+    """Every number of rows at the edges of the tiles and of the rule that picks one (1,153 and 9,728 outputs meet all five), K that
+    comes in 16 bytes at a time and K that does not: close to 64 bits, and each row bit for bit what it is in the largest step (one
+    chain over k, whatever the tile)."""
+    from kvcache_b200.kernels.api import _dtype_code, _ptr
     g = torch.Generator().manual_seed(31)
-    x, w, bias = torch.randn(1001, K, generator=g), torch.randn(N, K, generator=g), torch.randn(N, generator=g)
+    x, w, bias = torch.randn(1001, K, generator=g).to(dtype), torch.randn(N, K, generator=g).to(dtype), torch.randn(N, generator=g)
     xd, wd, bd = x.to(DEV), w.to(DEV), bias.to(DEV)
-    full = torch.empty(1001, N, device=DEV)
-    kernels.linear(xd, wd, full, bd)
-    # A chain of K rounded multiply-adds: at most K 2^-24 times the sum of magnitudes, which for normal numbers is 0.64 K.
+
+    def product(M):
+        out = torch.full((M, N), float("nan"), dtype=out_dtype, device=DEV)
+        with kernels.on_current_stream():
+            assert kernels._gemm_simt.kvb_gemm_simt(_dtype_code(dtype), _dtype_code(out_dtype), _ptr(xd), _ptr(wd), _ptr(bd), _ptr(out), M, N, K,
+                                                    kernels._stream()) == 0
+        return out
+
+    full, want = product(1001), x.double() @ w.double().t() + bias.double()
+    # A chain of K rounded multiply-adds: at most K 2^-24 times the sum of magnitudes, which for normal numbers is 0.64 K; then a rounding
+    # to 8 bits in bfloat16.
     bound = K * 2.0 ** -24 * ((x.abs().double() @ w.abs().double().t()).max().item() + 5.0)
-    assert (full.double().cpu() - (x.double() @ w.double().t() + bias.double())).abs().max().item() <= bound
+    bound += want.abs().max().item() * 2.0 ** -9 if out_dtype == torch.bfloat16 else 0.0
+    assert (full.double().cpu() - want).abs().max().item() <= bound
     for M in (1, 4, 5, 16, 17, 48, 49, 64, 65, 129, 513):
-        part = torch.full((M, N), float("nan"), device=DEV)
-        kernels.linear(xd[:M], wd, part, bd)
-        assert torch.equal(part, full[:M]), M
+        assert torch.equal(product(M), full[:M]), M
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

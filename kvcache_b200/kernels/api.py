@@ -1378,7 +1378,8 @@ class CudaKernels(KernelSet):
         # By the step's rows and segments alone, so that a recorded step finds the same launches.
         chunks = T // 16 + S
         held = min(chunks, max(1, self.CHUNK_SCRATCH_BYTES // (4 * size)))
-        records = workspace.buffer("recurrent.chunk_records", (held * size,), torch.float32)
+        records = (torch.empty(held * size, dtype=torch.float32, device=rows.device) if workspace is None else
+                   workspace.buffer("recurrent.chunk_records", (held * size,), torch.float32))
         # Per run: the records (and their triangular systems) and the walk, one of which has been counted.
         self.launches += -(-chunks // held) * (3 if mode == "delta_rule" else 2) - 1
         _check(lib.kvb_chunk_scan(code, _ptr(rows), rows.shape[1], *cols, G, _ptr(gates), gates.shape[1], float(q_scale),

@@ -268,6 +268,10 @@ def test_forms_of_the_delta_scan_agree(kernels, D, form, monkeypatch):
         assert forms.taken() == [taken]
     assert_close(results[0][0], results[1][0], 1e-5)
     assert_close(results[0][1], results[1][1], 1e-5)
+    monkeypatch.undo()
+    memory, out = _rand(2, H, D, Dv, seed=3).to(DEV), torch.zeros(370, H * Dv, device=DEV)
+    kernels.gated_delta_scan(rows, gates, 0.3, batch, memory, out, H, G, D, Dv, None)            # no workspace: scratch of its own
+    assert torch.equal(out, results[0][0]) and torch.equal(memory, results[0][1])
 
 
 @pytest.mark.parametrize("N", [64, 128, 130])

@@ -523,7 +523,7 @@ KVB_API int kvb_head_linear(int dtype, const void* x, int xs, int x_ld, const vo
             // Rows of the result that start on 16 bytes; tiles of 32 rows with four stages while few of them fill the GPU, then of 64 rows with
             // two, so that more blocks share an SM (2,048 rows of 16 heads, 128 -> 512: 41 us, 82 with tiles of 32, 49 with 128).
             if (M > 16 && N % 8 == 0 && os % 8 == 0 && (uintptr_t)out % 16 == 0) {
-const long long small = (long long)((N + hl::BN - 1) / hl::BN) * ((M + 31) / 32) * H;
+                const long long small = (long long)((N + hl::BN - 1) / hl::BN) * ((M + 31) / 32) * H;
                 return small <= 2 * kvb_sm_count()
                            ? launch_head_linear_wide<32, 1, 4, 4>(xb, xs, x_ld, wb, (bf16*)out, os, M, N, K, H, gb, gs, gc, gate_heads, rot,
                                                                   rot_half, cos_t, sin_t, table_len, positions, err, stream)

@@ -1204,10 +1204,8 @@ KVB_API int kvb_state_space_scan(const float* rows, const float* gates, const in
                     seg_q_len, seg_slot, memory, nullptr, nullptr, out, T, S, H, N, Dv, 0, 0, nullptr, stream, true, G);
 }
 
-// out[t, out_col + i] = y_i / sqrt(mean over i's part of y^2 + eps) * w_i * scale with y_i = (o[t, i] + skip[i / Dv] x[t, i]) silu(g[t, i]);
-// a row's W = H Dv numbers form `parts` equal parts, a block each.  o, x, g float32 (x and g columns of wider rows).
-// Rows of whole fours (`kvb_gate_part_norm` says when): 16 bytes a load, 8 or 16 a store.  Bound by memory; 2,048 rows of 4,096 numbers:
-// 27 us, 4 bytes at a time 41.
+// `gate_part_norm_kernel` for rows of whole fours (`kvb_gate_part_norm` says when): 16 bytes a load, 8 or 16 a store.  Bound by memory; 2,048
+// rows of 4,096 numbers: 27 us, 4 bytes at a time 41.
 template <typename T>
 __global__ void gate_part_norm4_kernel(const float* __restrict__ o, const float* __restrict__ x, int x_stride, const float* __restrict__ skip,
                                        const float* __restrict__ gate, int gate_stride, int gate_col, const float* __restrict__ w, float eps,
@@ -1243,6 +1241,8 @@ __global__ void gate_part_norm4_kernel(const float* __restrict__ o, const float*
     }
 }
 
+// out[t, out_col + i] = y_i / sqrt(mean over i's part of y^2 + eps) * w_i * scale with y_i = (o[t, i] + skip[i / Dv] x[t, i]) silu(g[t, i]);
+// a row's W = H Dv numbers form `parts` equal parts, a block each.  o, x, g float32 (x and g columns of wider rows).
 template <typename T>
 __global__ void gate_part_norm_kernel(const float* __restrict__ o, const float* __restrict__ x, int x_stride, const float* __restrict__ skip,
                                       const float* __restrict__ gate, int gate_stride, int gate_col, const float* __restrict__ w, float eps,

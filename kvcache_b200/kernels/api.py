@@ -1324,12 +1324,13 @@ class CudaKernels(KernelSet):
             col, {"silu": 0, "sigmoid": 1}[activation], float(scale), _ptr(out), out.shape[1], out_col, T, num_heads, value_dim,
             self._stream()), "head_norm_gate")
 
-    # A step whose longest segment has at least SCAN_CHUNK_MIN_ROWS tokens scans its segments in chunks of SCAN_CHUNK tokens
-    # that run side by side (three launches, see csrc/recurrent.cu); below that a segment is one piece, and a token's
-    # result is bit for bit the same however the request was cut.
+    # A step whose longest segment has at least SCAN_CHUNK_MIN_ROWS tokens does not walk them in one piece (in which a token's result is
+    # bit for bit the same however the request was cut).  Decays per channel and the delta rule, heads of up to CHUNK_SCAN_MAX_DIM key
+    # channels, take sixteen tokens at a time (below; `_gated_linear_chunks` has the exception); all others, and the matrix memory, chunks
+    # of SCAN_CHUNK tokens that run side by side (three launches, see csrc/recurrent.cu).
     SCAN_CHUNK = 64
     SCAN_CHUNK_MIN_ROWS = 256
-    DELTA_LONG_ROWS = 1536           # the delta rule: steps whose longest portion has at least this many rows ...
+    DELTA_LONG_ROWS = 1536           # the delta rule side by side: steps whose longest portion has at least this many rows ...
     DELTA_LONG_CHUNK = 128           # ... are cut into chunks of this many tokens
 
     def _scan_checks(self, proj, gate, out, memory, H, D, Dv) -> None:
@@ -1355,13 +1356,13 @@ class CudaKernels(KernelSet):
             self._stream()), "matrix_state_scan")
 
     def _gated_linear_chunks(self, batch: StepBatch, workspace, D: int) -> bool:
-        """Sixteen tokens at a time: 600 + 400 rows of 8 heads of 128 x 256 56 us against 154, 1,000 rows of 7 heads of 64 x 128 58
-        against 68; 2,048 rows of those 112 against 105, which chunks of 64 side by side take."""
+        """Sixteen tokens at a time: 600 + 400 rows of 8 heads of 128 x 256 64 us against 148, 256 rows of 7 heads of 64 x 128 23 against 85,
+        1,000 rows of those 76 against 83; longer portions of heads that narrow keep chunks of 64 side by side, whose time hardly
+        grows with the rows (2,048: 100)."""
         return (workspace is not None and self.SCAN_CHUNK and D <= self.CHUNK_SCAN_MAX_DIM and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS
                 and (D > 64 or batch.max_q_len <= 1024))
 
-    # Portions go sixteen tokens at a time over the tensor cores (csrc/scan_chunk.cu) where a head has at most CHUNK_SCAN_MAX_DIM key
-    # channels.
+    # Portions go sixteen tokens at a time (csrc/scan_chunk.cu) where a head has at most CHUNK_SCAN_MAX_DIM key channels.
     CHUNK_SCAN_MAX_DIM = 128
     # Scratch of a scan for portions: longer steps go through it in runs of as many chunks as it holds (16 heads of 128 channels under the delta
     # rule: 39 KB a head and chunk, 6,800 tokens a run; the whole of a step of 30,000 would take 1.2 GB).
@@ -1459,9 +1460,9 @@ class CudaKernels(KernelSet):
             self._chunk_scan("delta_rule", proj, tuple(cols[:3]), H, aux, 1.0, batch, memory, out, H, D, D, workspace)
             return
         max_chunks, scratch = 0, None
-        # Long portions take longer chunks: every chunk costs a product with its transition in the launch that walks the start
-        # states (measured at 14 heads of 64 / 16 heads of 128 channels, chunks of 64 against 128 tokens: 143 / 328 us against
-        # 223 / 349 us at 512 rows, 389 / 1,020 us against 279 / 731 us at 2,048 rows).
+        # Heads of more than CHUNK_SCAN_MAX_DIM key channels.  Long portions take longer chunks: every chunk costs a product with its
+        # transition in the launch that walks the start states (the line was drawn with heads of 64 and 128, which no
+        # longer come here: chunks of 64 against 128 tokens 143 / 328 us against 223 / 349 at 512 rows, 389 / 1,020 against 279 / 731 at 2,048).
         chunk = self.SCAN_CHUNK if batch.max_q_len < self.DELTA_LONG_ROWS else max(self.SCAN_CHUNK, self.DELTA_LONG_CHUNK)
         if self.SCAN_CHUNK and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS:
             # As in `_scan`; a chunk also leaves its transition, a matrix over the key channels.
@@ -1502,8 +1503,8 @@ class CudaKernels(KernelSet):
             _ptr(batch.seg_slot), T, batch.num_segments, H, G, D, Dv, self._stream()), "gated_delta_inputs")
 
     # Portions of at least SCAN_WIDE_MIN_ROWS rows leave the walk over tokens in one piece: the gated delta rule with up to
-    # CHUNK_SCAN_MAX_DIM key channels goes sixteen tokens at a time (48 rows of 14 heads of 64: 11 us, 18 with a column over many lanes,
-    # 44 in one piece), with more through the scan that spreads a column over many lanes (csrc/scan_wide.cu).  The state space
+    # CHUNK_SCAN_MAX_DIM key channels goes sixteen tokens at a time (64 rows of 14 heads of 64: 13 us, 23 with a column over many lanes,
+    # 58 in one piece), with more through the scan that spreads a column over many lanes (csrc/scan_wide.cu).  The state space
     # spreads its columns (28 heads of 128 x 64: 40 us at 64 rows in one piece, 15 us) up to STATE_SPACE_CHUNK_MIN_ROWS.
     SCAN_WIDE_MIN_ROWS = 48
 
@@ -1545,8 +1546,8 @@ class CudaKernels(KernelSet):
             _ptr(gates), _ptr(batch.row_segment), _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), T,
             batch.num_segments, H, self._stream()), "state_space_inputs")
 
-    # From here on sixteen tokens at a time: 45 us against 53 (a column over many lanes) at 512 rows of 28 heads of 128 x 64, 54 against
-    # 73 with 64 heads, 189 against 279 at 2,048 rows of 64; level at 256 rows.
+    # From here on sixteen tokens at a time: 49 us against 53 (a column over many lanes) at 512 rows of 28 heads of 128 x 64, 64 against
+    # 72 with 64 heads, 239 against 278 at 2,048 rows of 64.
     STATE_SPACE_CHUNK_MIN_ROWS = 512
     state_space_takes_workspace = True   # `state_space_scan` takes `workspace`
 

@@ -253,29 +253,29 @@ def test_scan_in_chunks_within_bounded_scratch(kernels, mode, D, monkeypatch):
         assert kernels.launches - before == -(-(sum(lens) // 16 + len(lens)) // held) * (3 if mode == "delta_rule" else 2) - 1
 
 
-@pytest.mark.parametrize("mode", MODES)
-@pytest.mark.parametrize("what", range(7))
-@pytest.mark.parametrize("value", [float("inf"), float("nan")])
-def test_scan_in_chunks_keeps_a_token_from_those_before_it(kernels, mode, what, value):
-    """An infinite or undefined number in any of a token's inputs: the tokens before it give the bits they give without it, and an
-    infinite value leaves the other value channels' alone."""
-    lens, H, D, Dv, at = [40], 2, 64, 24, 29
+INPUTS = {"gated_delta": "qkvab", "delta_rule": "qkvauc", "channel_decay": "qkva", "head_decay": "qkvab"}
+
+
+@pytest.mark.parametrize("mode,what", [(mode, what) for mode in MODES for what in INPUTS[mode]])
+def test_scan_in_chunks_keeps_a_token_from_those_before_it(kernels, mode, what):
+    """An infinite or undefined number in any of a token's inputs: the tokens before it give the bits they give without it, and such a
+    value leaves the other value channels' alone."""
+    lens, H, D, Dv, at, i = [40], 2, 64, 24, 29, "qkvabuc".index(what)
     *tokens, state = _scan_inputs(mode, lens, H, H, D, Dv, lambda r: torch.exp(-r))
-    used = {"gated_delta": (0, 1, 2, 3, 4), "delta_rule": (0, 1, 2, 3, 5, 6), "channel_decay": (0, 1, 2, 3), "head_decay": (0, 1, 2, 3, 4)}[mode]
-    if what not in used:
-        pytest.skip("not an input of this form")
     out, memory = _scan_chunks(kernels, mode, lens, *tokens, state, [1])
-    tokens[what] = tokens[what].clone()
-    if mode == "head_decay" and what == 3:
-        tokens[what][at] = value                                         # one decay for all channels of a head
-    else:
-        tokens[what][at].view(-1)[5 if what != 4 else 0] = value
-    bad, bad_memory = _scan_chunks(kernels, mode, lens, *tokens, state, [1])
-    assert torch.equal(bad[:at], out[:at])
-    assert not torch.isfinite(bad[at:]).all()
-    if what == 2:
-        others = [c for c in range(Dv) if c != 5]
-        assert torch.equal(bad[..., others], out[..., others]) and torch.equal(bad_memory[..., others], memory[..., others])
+    sound = tokens[i]
+    for number in (float("inf"), float("nan")):
+        tokens[i] = sound.clone()
+        if mode == "head_decay" and what == "a":
+            tokens[i][at] = number                                       # one decay for all channels of a head
+        else:
+            tokens[i][at].view(-1)[0 if what == "b" else 5] = number
+        bad, bad_memory = _scan_chunks(kernels, mode, lens, *tokens, state, [1])
+        assert torch.equal(bad[:at], out[:at])
+        assert not torch.isfinite(bad[at:]).all()
+        if what == "v":
+            others = [c for c in range(Dv) if c != 5]
+            assert torch.equal(bad[..., others], out[..., others]) and torch.equal(bad_memory[..., others], memory[..., others])
 
 
 @pytest.mark.parametrize("M", [17, 32, 33, 65, 300])

@@ -43,9 +43,9 @@ def test_float32_product_rows_do_not_depend_on_the_tile(kernels, dtype, out_dtyp
 
     full, want = product(1001), x.double() @ w.double().t() + bias.double()
     # A chain of K rounded multiply-adds: at most K 2^-24 times the sum of magnitudes, which for normal numbers is 0.64 K; then a rounding
-    # to 8 bits in bfloat16.
+    # to 8 significant bits in bfloat16, at most half of the last of them: 2^-8 of the result.
     bound = K * 2.0 ** -24 * ((x.abs().double() @ w.abs().double().t()).max().item() + 5.0)
-    bound += want.abs().max().item() * 2.0 ** -9 if out_dtype == torch.bfloat16 else 0.0
+    bound += want.abs().max().item() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0.0
     assert (full.double().cpu() - want).abs().max().item() <= bound
     for M in (1, 4, 5, 16, 17, 48, 49, 64, 65, 129, 513):
         assert torch.equal(product(M), full[:M]), M

@@ -24,11 +24,14 @@
 // states are off by 0.6 to 1.1 of what the scans over tokens are off by (states of models: 0.5e-7 to 1.1e-7; slow decays 1.6e-7 to 4.3e-7 where those
 // are at 1.9e-7 to 4.9e-7).
 //
-// What bounds it: the latency of a chunk's steps - shared memory, shuffles, two or three barriers, 1.0 to 1.9 us - times the chunks of the longest
-// segment.  Measured beside the form each replaces (us; records and walk): gated delta 777 x 14 x 64 x 64: 115 -> 84, 1,500 x 16 x 128 x 128:
-// 325 -> 220; delta rule 543 + 905 + 363 x 16 x 128: 660 -> 250, 1,000 x 14 x 64: 196 -> 131; channel decays 600 + 400 x 8 x 128 x 256: 148 -> 64; head
-// decays 2,048 x 64 x 128 x 64: 278 -> 239.  Products of tf32 halves on the tensor cores in the walk took 61, 146, 188, 97, 54 and 187, with states
-// up to three times as far from 64 bits.
+// What bounds it: the latency of a chunk's steps - shared memory, shuffles, two or three barriers, 1.2 to 2.6 us - times the chunks of the longest
+// segment.  Measured beside the form each replaces (us; records and walk): gated delta 777 x 14 x 64 x 64: 115 -> 85, 1,500 x 16 x 128 x 128:
+// 325 -> 235; delta rule 543 + 905 + 363 x 16 x 128: 660 -> 252, 1,000 x 14 x 64: 196 -> 143; channel decays 600 + 400 x 8 x 128 x 256: 148 -> 68; head
+// decays 2,048 x 64 x 128 x 64: 278 -> 262.  Level or up to 5 % behind: 2,048 x 14 x 64 under the delta rule (297 -> 311), 48 tokens beside 63
+// single ones under the gated one (46 -> 48), 512 x 28 x 128 x 64 head decays (53 -> 54).  Registers for four blocks an SM: with more, steps of
+// several segments take up to 40 % longer, with the compiler's own choice single ones 5 %.
+// A weight above a diagonal is zero and is multiplied like any other; only in a chunk whose values are not all finite (a vote) are
+// later tokens left out one by one, which takes 15 to 35 % longer where it is done always.
 // A segment's result does not depend on what else the step holds, and a token's not on later ones, whatever they hold (an infinite or undefined
 // number of one reaches those after it, as in a walk over tokens).
 // State layout: [slot, head, key channel, value channel].
@@ -426,6 +429,48 @@ template <int N> __device__ __forceinline__ void keep(float* at, const float (&v
     else *(float4*)at = make_float4(v[0], v[1], v[2], v[3]);
 }
 
+// Each number twice, for `fma2`.
+template <int N> __device__ __forceinline__ void pairs(const float* at, float2 (&v)[N]) {
+    float x[N];
+    load<N>(at, x);
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = make_float2(x[i], x[i]);
+}
+template <int N> __device__ __forceinline__ bool finite(const float (&v)[N]) {
+    bool all = true;
+#pragma unroll
+    for (int i = 0; i < N; ++i) all &= fabsf(v[i]) <= FLT_MAX;
+    return all;
+}
+// sum += tokens 0 .. t of x [C][16] with the weights of a row of a lower triangular matrix (of two, token by token), in order.  The zeros
+// above its diagonal are multiplied too, unless MASKED: zero times an infinite or undefined number of a later token is not zero.
+template <int N, bool MASKED>
+__device__ __forceinline__ void add_tokens(const float* row, const float* x, int t, float (&sum)[N]) {
+    float a[C], v[N];
+    load<C>(row, a);
+#pragma unroll
+    for (int s = 0; s < C; ++s) {
+        load<N>(x + 16 * s, v);
+#pragma unroll
+        for (int c = 0; c < N; ++c) sum[c] = MASKED && s > t ? sum[c] : fmaf(a[s], v[c], sum[c]);
+    }
+}
+template <int N, bool MASKED>
+__device__ __forceinline__ void add_tokens(const float* row1, const float* x1, const float* row2, const float* x2, int t, float (&sum)[N]) {
+    float a1[C], a2[C], v[N];
+    load<C>(row1, a1);
+    load<C>(row2, a2);
+#pragma unroll
+    for (int s = 0; s < C; ++s) {
+        load<N>(x1 + 16 * s, v);
+#pragma unroll
+        for (int c = 0; c < N; ++c) sum[c] = MASKED && s > t ? sum[c] : fmaf(a1[s], v[c], sum[c]);
+        load<N>(x2 + 16 * s, v);
+#pragma unroll
+        for (int c = 0; c < N; ++c) sum[c] = MASKED && s > t ? sum[c] : fmaf(a2[s], v[c], sum[c]);
+    }
+}
+
 __device__ __forceinline__ void copy_bulk(float* smem, const float* gmem, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
                  ::"r"(tc::smem_u32(smem)), "l"(gmem), "r"(bytes), "r"(tc::smem_u32(bar)) : "memory");
@@ -434,7 +479,7 @@ __device__ __forceinline__ void copy_bulk(float* smem, const float* gmem, uint32
 // grid (16 value channels, heads, segments), over the chunks first .. first + held - 1 of the step.  A thread holds TD neighbouring key channels of TC value channels of the state; a warp's lanes
 // are 2 TC groups of key channels by 16 / TC of value channels.  Beside that, every thread owns one token's OC value channels of Z and O.
 template <int MODE, int NI, int TD, int TC, int STAGES>
-__global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(const Rows in, const Segments seg, const float* __restrict__ records,
+__global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_walk_kernel(const Rows in, const Segments seg, const float* __restrict__ records,
                                                                              int first, int held, float q_scale, float* __restrict__ memory,
                                                                              float* __restrict__ out, int H, int D, int Dv, int* __restrict__ err) {
     constexpr bool Z = has_z(MODE), V = has_v(MODE);
@@ -509,7 +554,9 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
     bool bad = false, failed = false;
     int ci = 0;
     for (;; ++ci) {
-        failed = __syncthreads_or(bad);                        // all are done with chunk ci - 1 (a wait that ran out ends the walk)
+        // All are done with chunk ci - 1.  A wait that ran out ends the walk; values that are not all finite leave later tokens out one by one.
+        bool wild = __syncthreads_or(bad || !finite(next));
+        if (wild) failed = __syncthreads_or(bad);
         if (failed || ci == chunks) break;
         if (tid == 0 && ci + STAGES - 1 < chunks) fetch(ci + STAGES - 1);
         values(ci + 1, next);
@@ -519,6 +566,7 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
         }
         const float* b = sm + (ci % STAGES) * R.total;
         const float(*v_c)[16] = v_s[ci & 1];
+        const int left = n - ci * C;                           // tokens from the chunk's first on: those after them change nothing
 
         // Y S_0 and Q S_0, eight rows at a time: this thread's key channels, then the warp's.
         const float* rows = b + (Z ? R.y : R.q) + d0;
@@ -562,19 +610,8 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
         }
         float z_own[OC] = {}, o[OC] = {};
         if (Z) {                                               // W V, while the others get here
-#pragma unroll
-            for (int s0 = 0; s0 < C; s0 += 4) {
-                if (s0 > t) break;                             // later tokens are left out whatever they hold
-                float w[4], v[OC];
-                load<4>(b + R.w + t * 24 + s0, w);
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    load<OC>(&v_c[s0 + s][oc], v);
-#pragma unroll
-                    for (int c = 0; c < OC; ++c)
-                        if (s0 + s <= t) z_own[c] = fmaf(w[s], v[c], z_own[c]);
-                }
-            }
+            if (!wild) add_tokens<OC, false>(b + R.w + t * 24, &v_c[0][oc], t, z_own);
+            else add_tokens<OC, true>(b + R.w + t * 24, &v_c[0][oc], t, z_own);
         }
         __syncthreads();
         {
@@ -593,8 +630,8 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
             }
             if (Z) {
 #pragma unroll
-                for (int c = 0; c < OC; ++c) y_sum[c] += z_own[c];
-                keep<OC>(&z_s[t][oc], y_sum);
+                for (int c = 0; c < OC; ++c) z_own[c] = t < left ? y_sum[c] + z_own[c] : 0.f;
+                keep<OC>(&z_s[t][oc], z_own);
             }
             if (MODE == CHUNK_HEAD_DECAY) {
                 const float level = b[R.decay + t];
@@ -602,30 +639,17 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
                 for (int c = 0; c < OC; ++c) o[c] *= level;
             }
         }
-        if (Z) __syncthreads();
+        if (Z) wild |= (bool)__syncthreads_or(!finite(z_own));
         // The results: tokens in order on top of Q S_0.
         {
-#pragma unroll
-            for (int s0 = 0; s0 < C; s0 += 4) {
-                if (s0 > t) break;
-                float a1[4], a2[4], x[OC];
-                if (V) load<4>(b + R.a1 + t * 24 + s0, a1);
-                if (Z) load<4>(b + R.a2 + t * 24 + s0, a2);
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    if (Z) {
-                        load<OC>(&z_s[s0 + s][oc], x);
-#pragma unroll
-                        for (int c = 0; c < OC; ++c)
-                            if (s0 + s <= t) o[c] = fmaf(a2[s], x[c], o[c]);
-                    }
-                    if (V) {
-                        load<OC>(&v_c[s0 + s][oc], x);
-#pragma unroll
-                        for (int c = 0; c < OC; ++c)
-                            if (s0 + s <= t) o[c] = fmaf(a1[s], x[c], o[c]);
-                    }
-                }
+            const float *a1 = b + R.a1 + t * 24, *a2 = b + R.a2 + t * 24;
+            if constexpr (Z && V) {
+                if (!wild) add_tokens<OC, false>(a2, &z_s[0][oc], a1, &v_c[0][oc], t, o);
+                else add_tokens<OC, true>(a2, &z_s[0][oc], a1, &v_c[0][oc], t, o);
+            } else {
+                const float *a = Z ? a2 : a1, *x = Z ? &z_s[0][oc] : &v_c[0][oc];
+                if (!wild) add_tokens<OC, false>(a, x, t, o);
+                else add_tokens<OC, true>(a, x, t, o);
             }
             if (ci * C + t < n) {
                 float* at = out + (size_t)(r0 + ci * C + t) * H * Dv + (size_t)h * Dv + col;
@@ -636,7 +660,7 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
         }
         // The state: earlier tokens by themselves, the decayed state, the chunk's last tokens (eight of sixteen, fewer of fewer) on top, in their
         // order: fewer roundings of a state that decays slowly than a walk over tokens makes, and no others where the last tokens dominate.
-        const int left = n - ci * C, split = left > 12 ? 8 : left > 8 ? 4 : 0;
+        const int split = left > 12 ? 8 : left > 8 ? 4 : 0;
         float2 N[TD / 2][TC];
 #pragma unroll
         for (int i = 0; i < TD / 2; ++i)
@@ -657,13 +681,13 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
                     }
                 }
             }
-            float v[TC], z[TC];
-            if (Z) load<TC>(&z_s[s][cg * TC], z);
-            if (V) load<TC>(&v_c[s][cg * TC], v);
+            float2 v[TC], z[TC];
+            if (Z) pairs(&z_s[s][cg * TC], z);
+            if (V) pairs(&v_c[s][cg * TC], v);
             if (MODE == CHUNK_HEAD_DECAY) {
                 const float gain = b[R.decay + C + s];
 #pragma unroll
-                for (int c = 0; c < TC; ++c) v[c] *= gain;
+                for (int c = 0; c < TC; ++c) v[c] = mul2(v[c], make_float2(gain, gain));
             }
 #pragma unroll
             for (int i = 0; i < TD / 4; ++i) {
@@ -674,12 +698,12 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC)) chunk_walk_kernel(co
                 for (int c = 0; c < TC; ++c) {
                     float2 &low = N[2 * i][c], &high = N[2 * i + 1][c];
                     if (Z) {
-                        low = fma2(low2(k2), make_float2(z[c], z[c]), low);
-                        high = fma2(high2(k2), make_float2(z[c], z[c]), high);
+                        low = fma2(low2(k2), z[c], low);
+                        high = fma2(high2(k2), z[c], high);
                     }
                     if (V) {
-                        low = fma2(low2(k1), make_float2(v[c], v[c]), low);
-                        high = fma2(high2(k1), make_float2(v[c], v[c]), high);
+                        low = fma2(low2(k1), v[c], low);
+                        high = fma2(high2(k1), v[c], high);
                     }
                 }
             }

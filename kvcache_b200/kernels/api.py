@@ -1356,9 +1356,9 @@ class CudaKernels(KernelSet):
             self._stream()), "matrix_state_scan")
 
     def _gated_linear_chunks(self, batch: StepBatch, workspace, D: int) -> bool:
-        """Sixteen tokens at a time: 600 + 400 rows of 8 heads of 128 x 256 64 us against 148, 256 rows of 7 heads of 64 x 128 23 against 85,
+        """Sixteen tokens at a time: 600 + 400 rows of 8 heads of 128 x 256 68 us against 148, 256 rows of 7 heads of 64 x 128 24 against 85,
         1,000 rows of those 76 against 83; longer portions of heads that narrow keep chunks of 64 side by side, whose time hardly
-        grows with the rows (2,048: 100)."""
+        grows with the rows (2,048: 100; but it grows with heads and requests, and 28 heads or four requests are behind by up to half)."""
         return (workspace is not None and self.SCAN_CHUNK and D <= self.CHUNK_SCAN_MAX_DIM and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS
                 and (D > 64 or batch.max_q_len <= 1024))
 
@@ -1461,8 +1461,9 @@ class CudaKernels(KernelSet):
             return
         max_chunks, scratch = 0, None
         # Heads of more than CHUNK_SCAN_MAX_DIM key channels.  Long portions take longer chunks: every chunk costs a product with its
-        # transition in the launch that walks the start states (the line was drawn with heads of 64 and 128, which no
-        # longer come here: chunks of 64 against 128 tokens 143 / 328 us against 223 / 349 at 512 rows, 389 / 1,020 against 279 / 731 at 2,048).
+        # transition in the launch that walks the start states (4 heads of 160 / 8 heads of 256 channels, chunks of 64 against 128
+        # tokens: 437 / 697 us against 706 / 764 at 512 rows, 982 / 2,001 against 815 / 1,958 at 1,536, 1,241 / 2,710 against
+        # 1,160 / 2,373 at 2,048).
         chunk = self.SCAN_CHUNK if batch.max_q_len < self.DELTA_LONG_ROWS else max(self.SCAN_CHUNK, self.DELTA_LONG_CHUNK)
         if self.SCAN_CHUNK and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS:
             # As in `_scan`; a chunk also leaves its transition, a matrix over the key channels.
@@ -1504,7 +1505,7 @@ class CudaKernels(KernelSet):
 
     # Portions of at least SCAN_WIDE_MIN_ROWS rows leave the walk over tokens in one piece: the gated delta rule with up to
     # CHUNK_SCAN_MAX_DIM key channels goes sixteen tokens at a time (64 rows of 14 heads of 64: 13 us, 23 with a column over many lanes,
-    # 58 in one piece), with more through the scan that spreads a column over many lanes (csrc/scan_wide.cu).  The state space
+    # 27 in one piece), with more through the scan that spreads a column over many lanes (csrc/scan_wide.cu).  The state space
     # spreads its columns (28 heads of 128 x 64: 40 us at 64 rows in one piece, 15 us) up to STATE_SPACE_CHUNK_MIN_ROWS.
     SCAN_WIDE_MIN_ROWS = 48
 
@@ -1546,8 +1547,8 @@ class CudaKernels(KernelSet):
             _ptr(gates), _ptr(batch.row_segment), _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), T,
             batch.num_segments, H, self._stream()), "state_space_inputs")
 
-    # From here on sixteen tokens at a time: 49 us against 53 (a column over many lanes) at 512 rows of 28 heads of 128 x 64, 64 against
-    # 72 with 64 heads, 239 against 278 at 2,048 rows of 64.
+    # From here on sixteen tokens at a time: 54 us against 53 (a column over many lanes) at 512 rows of 28 heads of 128 x 64, 69 against
+    # 72 with 64 heads, 262 against 278 at 2,048 rows of 64, 105 against 123 for four requests of 512.
     STATE_SPACE_CHUNK_MIN_ROWS = 512
     state_space_takes_workspace = True   # `state_space_scan` takes `workspace`
 

@@ -17,7 +17,7 @@ import torch
 
 from ..parts.base import PagedKVView, StepBatch
 from . import build
-from .attention_plan import PREFILL_MIN_KEY_TILES, TC_MIN_KEY_TILES, PagedAttentionPlanner
+from .attention_plan import PREFILL_MIN_KEY_TILES, TC_MAX_PAIRS, TC_MIN_KEY_TILES, TC_PAIR_MIN_KEY_TILES, PagedAttentionPlanner
 from .latent_plan import LatentAttentionPlanner
 
 _c_int, _c_float, _c_void_p, _c_longlong = ctypes.c_int, ctypes.c_float, ctypes.c_void_p, ctypes.c_longlong
@@ -246,6 +246,11 @@ _SIGNATURES = {
                              _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,
                              _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_void_p, _c_void_p],
     },
+    "attention_pairs": {
+        "kvb_attention_pairs": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p,
+                                _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,
+                                _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_void_p, _c_void_p],
+    },
     "primitive_costs": {
         "kvb_primitive_costs_count": [],
         "kvb_primitive_costs": [_c_void_p, _c_void_p, _c_void_p, _c_void_p],
@@ -328,11 +333,24 @@ class CudaKernels(KernelSet):
         self.skinny_gemm = True              # bfloat16, M <= 64, K % 32 == 0: weight-streaming kernel
         self._flash: Dict[int, _Library] = {}
         self._attn_tc: Dict[int, _Library] = {}
+        self._attn_pairs: Dict[int, _Library] = {}
         # Portions of prompts with at least this many rows go through the tensor-memory attention kernel
         # (bfloat16, head size 64 or 128, pages of 8..64 tokens); None turns it off.  Measured on 24 layers of the
         # 0.5B shape: the mma.sync kernel is ahead at 128 and 256 rows (1.09 / 1.24 ms a step against 1.14 / 1.28),
         # the tensor-memory kernel from 512 rows on (1.56 against 1.69 ms).
+        # Behind a longer history (the plan cuts the portion's tiles into this many units) it is ahead from 128 rows on: 128 rows
+        # behind 2,000 tokens 29.7 against 39.9 us (16 heads of 128), 25.6 and 25.6 (14 heads of 64); 200 behind 8,000 60 against 137, 40 and 69.
         self.tc_attention_min_rows: Optional[int] = 384
+        self.tc_history_min_rows, self.tc_history_min_units = 128, 3
+        # Steps that the plan cuts into at least this many units - heads of 64: also two a tile, which they are behind some history -
+        # go through the kernel for pairs of row tiles (csrc/attention_pairs.cu), whose set-up and merge cost more and whose tiles
+        # cost less.  On both sides of the lines, in us, this kernel and that, 16 heads of 128 and 14 of 64: 800 rows (7 units in 7
+        # tiles) 25.5 and 29.7, 23.6 and 23.6; 1,024 rows (8 in 8) 29.5 and 29.7, 23.5 and 21.5; 800 behind 500 (10 in 7) 37.8 and
+        # 35.8, 25.5 and 27.5; 512 behind 2,000 (12 in 4) 48 and 37.9, 29.7 and 27.6; 2,048 (24 in 16) 61 and 43, 32.8 and 33.6 (24
+        # layers of a step of the latter: 2,490 and 2,565); 2,048 behind 2,048 150 and 76, 71 and 53.
+        self.tc_pairs_min_units: Optional[int] = 8
+        self.tc_pairs_units_a_tile = {64: 2, 128: 1}
+        self.tc_pairs_min_tiles = TC_PAIR_MIN_KEY_TILES
         # A window or chunks may leave a tile of a portion fewer key tiles than its units were planned for: a unit keeps at
         # least this many (what kernels/attention_plan.py plans with).
         self.tc_unit_min_tiles, self.prefill_unit_min_tiles = TC_MIN_KEY_TILES, PREFILL_MIN_KEY_TILES
@@ -919,8 +937,28 @@ class CudaKernels(KernelSet):
         if fast:
             lib = self._flash_library(D)
             counts, lists = plan.counts, plan.arrays
-            if (counts["tc_units"] and self.tc_attention_min_rows is not None and D in (64, 128)
-                    and 8 <= kv.page_size <= 64 and batch.max_q_len >= self.tc_attention_min_rows):
+            long_portion = (self.tc_attention_min_rows is not None and D in (64, 128) and 8 <= kv.page_size <= 64
+                            and (batch.max_q_len >= self.tc_attention_min_rows or (batch.max_q_len >= self.tc_history_min_rows
+                                                                                   and counts["tc_units"] >= self.tc_history_min_units)))
+            if (long_portion and self.tc_pairs_min_units is not None and 0 < counts["tc_pairs"] <= TC_MAX_PAIRS
+                    and counts["tc_units"] >= max(self.tc_pairs_min_units, self.tc_pairs_units_a_tile[D] * counts["tc_tiles"])):
+                pairs_lib = self._attn_pairs.get(D)
+                if pairs_lib is None:
+                    pairs_lib = self._attn_pairs[D] = _Library("attention_pairs", f"d{D}", [f"-DKVB_HEAD_DIM={D}"])
+                pairs = counts["tc_pairs"]
+                # Two places a block for the sums of a divided stream of keys; a ticket per (pair of row tiles, head, tile), which
+                # the kernel leaves zero.
+                scratch = workspace.buffer("attn.pairs_scratch", (4 * self.sm_count * 128 * (D + 2),), torch.float32)
+                tickets = workspace.zeros("attn.pairs_tickets", (2 * pairs * num_heads,), torch.int32)
+                self._count("attention_tc")                   # both tensor-memory kernels go by this name
+                _check(pairs_lib.kvb_attention_pairs(
+                    _ptr(q), _ptr(out), _ptr(kv.k_pages), _ptr(kv.v_pages), kv.k_pages.shape[0], _ptr(kv.block_table),
+                    kv.block_table.shape[1], _ptr(lists["tc_pairs"]), pairs, _ptr(scratch), _ptr(tickets), self.sm_count,
+                    _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_kv_len), T, num_heads, Hkv, kv.page_size,
+                    reach, float(scale), _ptr(sink), keep, _ptr(slopes), cap, self.tc_pairs_min_tiles, _ptr(self.error_word),
+                    self._stream()),
+                    "attention_pairs")
+            elif counts["tc_units"] and long_portion:
                 tc = self._attn_tc.get(D)
                 if tc is None:
                     tc = self._attn_tc[D] = _Library("attention_tc", f"d{D}", [f"-DKVB_HEAD_DIM={D}"])

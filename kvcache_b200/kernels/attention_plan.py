@@ -1,14 +1,16 @@
 """Work lists of the paged-attention kernels: which block of a launch does what.
 
-The tiling belongs to the kernels (csrc/attention_flash.cu, csrc/attention_tc.cu), so the
+The tiling belongs to the kernels (csrc/attention_flash.cu, csrc/attention_tc.cu, csrc/attention_pairs.cu), so the
 lists that follow from it are made here, beside the launchers, and not in the step function:
 the runner packs whatever a `StepPlanner` hands it.
 
 * `decode_items`: the segments that bring one token (each is one item of the decode kernels).
 * `prefill_units`: the segments that bring more, as tiles of 64 query rows cut into units of
-  about equal numbers of 64-key tiles (the `mma.sync` prefill kernel), and
+  about equal numbers of 64-key tiles (the `mma.sync` prefill kernel),
 * `tc_units`: the same segments as tiles of 128 rows with units of at least 16 key tiles
-  (the tensor-memory prefill kernel).
+  (the tensor-memory prefill kernel), and
+* `tc_pairs`: the same segments in pairs of tiles of 128 rows (the tensor-memory kernel for more work, which shares the
+  keys they see out among its blocks by itself).
 
 The reference has one block per (query row, head) and no such lists (src/qwen_kernels.cu:146-185).
 """
@@ -27,6 +29,9 @@ PREFILL_MIN_KEY_TILES = 4       # a unit has at least this many key tiles, unles
 PREFILL_MAX_UNITS = 16          # most units one tile may be cut into (csrc/attention_flash.cu)
 PREFILL_UNITS_WANTED = 256      # about this many units beyond one per tile, however long the prompts
 TC_TILE_ROWS = 128              # query rows of a tile of the tensor-memory attention kernel
+TC_PAIR_ROWS = 256              # query rows of a pair of row tiles of the kernel for more work
+TC_MAX_PAIRS = 256              # pairs a launch of that kernel takes
+TC_PAIR_MIN_KEY_TILES = 2       # a block of it takes at least this many tiles of 128 keys, unless there are fewer
 TC_MIN_KEY_TILES = 16           # a unit of that kernel has at least this many key tiles, unless its tile has fewer
 
 
@@ -71,19 +76,21 @@ class PagedAttentionPlanner(StepPlanner):
         T, S = num_tokens, num_segments
         return {"decode_items": S,
                 "prefill_units": 8 * (2 * (T // PREFILL_TILE_ROWS + S) + PREFILL_UNITS_WANTED),
-                "tc_units": 8 * (2 * (T // TC_TILE_ROWS + S) + PREFILL_UNITS_WANTED)}
+                "tc_units": 8 * (2 * (T // TC_TILE_ROWS + S) + PREFILL_UNITS_WANTED),
+                "tc_pairs": 2 * (T // TC_PAIR_ROWS + S)}
 
     def plan(self, starts, counts) -> Tuple[Dict[str, np.ndarray], Dict[str, int]]:
         counts = np.asarray(counts)
         S = len(counts)
         if int(counts.sum()) == S:                       # one token per request: every segment is an item, in order
             return ({"decode_items": np.arange(S, dtype=np.int32)},
-                    {"decode_items": S, "prefill_units": 0, "prefill_tiles": 0, "tc_units": 0, "tc_tiles": 0})
+                    {"decode_items": S, "prefill_units": 0, "prefill_tiles": 0, "tc_units": 0, "tc_tiles": 0, "tc_pairs": 0})
         single = counts == 1
         items = np.nonzero(single)[0].astype(np.int32)
         longer = [(int(i), int(starts[i]), int(counts[i])) for i in np.nonzero(~single)[0]]
         units, tiles = plan_prefill_units(longer)
         tc_units, tc_tiles = plan_prefill_units(longer, TC_TILE_ROWS, TC_MIN_KEY_TILES)
-        return ({"decode_items": items, "prefill_units": units.reshape(-1), "tc_units": tc_units.reshape(-1)},
+        pairs = np.asarray([(seg, row0) for seg, _, count in longer for row0 in range(0, count, TC_PAIR_ROWS)], dtype=np.int32)
+        return ({"decode_items": items, "prefill_units": units.reshape(-1), "tc_units": tc_units.reshape(-1), "tc_pairs": pairs.reshape(-1)},
                 {"decode_items": len(items), "prefill_units": len(units), "prefill_tiles": tiles,
-                 "tc_units": len(tc_units), "tc_tiles": tc_tiles})
+                 "tc_units": len(tc_units), "tc_tiles": tc_tiles, "tc_pairs": len(pairs)})

@@ -43,6 +43,7 @@ MODULES: Dict[str, dict] = {
     # Compiled per head size: variant "d<head_dim>" with -DKVB_HEAD_DIM=<head_dim>.
     "attention_flash": {"src": "attention_flash.cu", "deps": ["common.cuh", "flash_core.cuh", "no_alloc.h", "tc_common.cuh"]},
     "attention_tc": {"src": "attention_tc.cu", "deps": ["common.cuh", "tc_common.cuh"]},
+    "attention_pairs": {"src": "attention_pairs.cu", "deps": ["common.cuh", "tc_common.cuh"]},
     "gemm_wstream": {"src": "gemm_wstream.cu", "deps": ["common.cuh", "tc_common.cuh"]},
     # What barrier waits, votes, MMA issue and page copies cost on this GPU (python -m kvcache_b200.kernels.primitive_costs).
     "primitive_costs": {"src": "primitive_costs.cu", "deps": ["common.cuh", "tc_common.cuh"]},
@@ -51,7 +52,8 @@ MODULES: Dict[str, dict] = {
 }
 # Variants that `build_all` makes for modules compiled per size.
 DEFAULT_VARIANTS = {"attention_flash": [("d64", ["-DKVB_HEAD_DIM=64"]), ("d128", ["-DKVB_HEAD_DIM=128"])],
-                    "attention_tc": [("d64", ["-DKVB_HEAD_DIM=64"]), ("d128", ["-DKVB_HEAD_DIM=128"])]}
+                    "attention_tc": [("d64", ["-DKVB_HEAD_DIM=64"]), ("d128", ["-DKVB_HEAD_DIM=128"])],
+                    "attention_pairs": [("d64", ["-DKVB_HEAD_DIM=64"]), ("d128", ["-DKVB_HEAD_DIM=128"])]}
 
 _loaded: Dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()

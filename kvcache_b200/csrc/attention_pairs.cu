@@ -85,7 +85,9 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// Two float32 numbers in one 64-bit register, and the multiply-add and sum of such pairs (one instruction for two results).
+// 1 / (1 + e^-x), to about 2^-21 of itself.
+__device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.f, 1.f + ex2(-1.4426950408889634f * x)); }
+// Two float32 numbers in one 64-bit register, and the multiply-add of such pairs (one instruction for two results).
 __device__ __forceinline__ uint64_t pair(float x, float y) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
@@ -119,12 +121,10 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
+// lo += v's lower bfloat16, hi += its upper one, in float32.
+__device__ __forceinline__ void add_bf16x2(float& lo, float& hi, uint32_t v) {
+    asm("{.reg .b16 x, y; mov.b32 {x, y}, %2; add.rn.f32.bf16 %0, x, %0; add.rn.f32.bf16 %1, y, %1;}" : "+f"(lo), "+f"(hi) : "r"(v));
 }
-
 // The lowest `count` bits (none below 0, all from 32).
 __device__ __forceinline__ uint32_t below(int count) { return count >= 32 ? 0xffffffffu : count <= 0 ? 0u : (1u << count) - 1u; }
 
@@ -587,10 +587,11 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sh.top_known[wg]);
                 // P = 2^(s * scale - m) as bfloat16: keys 2c and 2c + 1 of the row in column c.  A masked score is -inf and gives
-                // 0.  The sum is taken from the unrounded numbers, in two chains of pairs.
+                // 0.  The sum is taken of the rounded numbers, in float32 over four chains: the weights that V gets then add up to 1 (from the
+                // unrounded ones errors against 64 bits were up to 1 % larger, where few keys take most of the weight).
                 const float base_m = m == NEG_INF ? 0.f : m;
                 const uint64_t scale2 = pair(scale_log2, scale_log2), minus2 = pair(-base_m, -base_m);
-                uint64_t l2[2] = {0, 0};
+                float l4[4] = {0.f, 0.f, 0.f, 0.f};
                 // The groups take turns at the exponentials: side by side each would take twice as long, and both would then want
                 // the tensor core at once and leave the exponentials idle meanwhile.
                 // From the block's first turn to its last, across pieces: a group that ran ahead of the other by a piece of one tile
@@ -606,9 +607,9 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     for (int e = 0; e < 16; ++e) {
                         const float2 y = unpair(fma2(pair(__uint_as_float(sv[e0 + 2 * e]), __uint_as_float(sv[e0 + 2 * e + 1])), scale2, minus2));
                         const float p0 = ex2(y.x), p1 = ex2(y.y);
-                        l2[e & 1] = add2(l2[e & 1], pair(p0, p1));
                         __nv_bfloat162 v = __floats2bfloat162_rn(p0, p1);
                         packed[e] = *reinterpret_cast<uint32_t*>(&v);
+                        add_bf16x2(l4[(2 * e) & 3], l4[(2 * e + 1) & 3], packed[e]);
                     }
                     tmem_st16(my_p + e0 / 2, packed);
                     if (e0 == TURN_AT) {
@@ -616,8 +617,7 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         if (lane == 0 && i < both) mbar_arrive(&sh.turn[wg ^ 1]);
                     }
                 }
-                const float2 la = unpair(add2(l2[0], l2[1]));
-                l += la.x + la.y;
+                l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
                 tmem_st_wait();
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 __syncwarp();
@@ -628,6 +628,10 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // The blocks whose runs hold a part of what these rows see of the stream.
             const int block0 = x.first / share, block1 = (x.first + hf.limit - 1) / share;
             int* ticket = p.tickets + ((size_t)t * p.Hq + x.index) * 2 + wg;
+            if (EXPANDED && pos >= 0) {                               // the row's gates, while the last product runs
+                const bf16* g = p.gate + (size_t)(p.seg_q_start[c.seg] + hf.row0 + row) * p.gate_stride + p.gate_col + (p.gate_per_head ? h : h * D);
+                for (int d = 0; d < (p.gate_per_head ? 1 : D); d += 64) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(g + d));
+            }
             ok = mbar_wait(&sh.o_full[wg], (OWN_P ? s_count - 1 : pieces) & 1);
             if (!ok) break;
             ++pieces;
@@ -640,10 +644,22 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // 32 results of the row from column d.  The warp's rows go into its stage, 16 bytes at a time, in an order that spreads
             // the banks, and out of it with four lanes a row.
             auto store32 = [&](int d, float* f) {
-                if (EXPANDED && p.gate && pos >= 0) {
+                if (EXPANDED && pos >= 0) {
                     const bf16* g = p.gate + (size_t)q_row * p.gate_stride + p.gate_col + (p.gate_per_head ? h : h * D + d);
+                    if (p.gate_per_head) {
+                        const float s = sigmoid(__bfloat162float(g[0]));
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) f[e] *= 1.f / (1.f + __expf(-__bfloat162float(g[p.gate_per_head ? 0 : e])));
+                        for (int e = 0; e < 32; ++e) f[e] *= s;
+                    } else {                                          // rows that start on 16 bytes
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const uint4 v = *reinterpret_cast<const uint4*>(g + 8 * q);
+                            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                            for (int e = 0; e < 8; ++e)
+                                f[8 * q + e] *= sigmoid(__uint_as_float(e & 1 ? u[e / 2] & 0xffff0000u : u[e / 2] << 16));
+                        }
+                    }
                 }
                 __syncwarp();
 #pragma unroll
@@ -828,5 +844,37 @@ KVB_API int kvb_attention_pairs(const void* q, void* out, const void* k_pages, c
     p.slopes = slopes; p.cap = cap; p.scale = scale;
     p.err = err;
     return launch(mq, mk, mv, p, scratch, blocks, stream);
+}
+#else
+// The same attention over keys and values that a latent was expanded to (csrc/latent.cu, kvb_latent_expand_prepare): kv [key_rows,
+// 2 * H * D] - the heads' keys, then the heads' values - and rot [key_rows, 64], the keys' rotated part that all heads share (`rot`
+// numbers of it).  q: rows of `q_ld` numbers, head h's D + rot at column h (D + rot).  seg_key_row: the row of kv that a segment's key 0
+// has, or would have.  gate: out *= sigmoid(gate[t, gate_col + h D + d]), or, with `gate_per_head`, sigmoid(gate[t, gate_col + h]).
+KVB_API int kvb_attention_pairs_expanded(const void* q, int q_ld, void* out, const void* kv, const void* rot_rows, int key_rows, const int* tiles,
+                                         int n_tiles, float* scratch, int* tickets, int blocks, const int* seg_key_row,
+                                         const int* seg_q_start, const int* seg_q_len, const int* seg_kv_len, int T, int H, int rot, int window,
+                                         float scale, const float* sink, const void* gate, int gate_stride, int gate_col, int gate_per_head,
+                                         int min_tiles, int* err, cudaStream_t stream) {
+    using namespace apr;
+    if (n_tiles <= 0) return KVB_OK;
+    if (H < 1 || H > 65535 || rot < 16 || rot > 64 || rot % 16 != 0 || q_ld % 8 != 0 || H * (D + rot) > q_ld || key_rows < 1 || !gate) return KVB_ERR_SHAPE;
+    if (((uintptr_t)q | (uintptr_t)out | (uintptr_t)kv | (uintptr_t)rot_rows) & 15) return KVB_ERR_ALIGN;
+    if (!gate_per_head && (((uintptr_t)gate & 15) || gate_stride % 8 != 0 || gate_col % 8 != 0)) return KVB_ERR_ALIGN;
+    CUtensorMap mq, mk, mr;
+    int rc = make_bf16_map(&mq, q, T, q_ld, q_ld, BQ);
+    if (rc != KVB_OK) return rc;
+    rc = make_bf16_map(&mk, kv, key_rows, 2 * H * D, 2LL * H * D, BK);
+    if (rc != KVB_OK) return rc;
+    rc = make_bf16_map(&mr, rot_rows, key_rows, 64, 64, BK);
+    if (rc != KVB_OK) return rc;
+    Params p = {};
+    p.out = (bf16*)out; p.tiles = tiles; p.n_tiles = n_tiles;
+    p.seg_q_start = seg_q_start; p.seg_q_len = seg_q_len; p.seg_kv_len = seg_kv_len; p.seg_key_row = seg_key_row;
+    p.tickets = tickets;
+    p.Hq = p.Hkv = H; p.q_head = D + rot; p.rot_steps = rot / 16;
+    p.window = window; p.min_tiles = min_tiles; p.sink = sink; p.scale = scale;
+    p.gate = (const bf16*)gate; p.gate_stride = gate_stride; p.gate_col = gate_col; p.gate_per_head = gate_per_head;
+    p.err = err;
+    return launch(mq, mk, mr, p, scratch, blocks, stream);
 }
 #endif

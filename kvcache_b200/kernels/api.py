@@ -18,7 +18,7 @@ import torch
 from ..parts.base import PagedKVView, StepBatch
 from . import build
 from .attention_plan import PREFILL_MIN_KEY_TILES, TC_MAX_PAIRS, TC_MIN_KEY_TILES, TC_PAIR_MIN_KEY_TILES, PagedAttentionPlanner
-from .latent_plan import LatentAttentionPlanner
+from .latent_plan import LatentAttentionPlanner, LatentExpandPlanner
 
 _c_int, _c_float, _c_void_p, _c_longlong = ctypes.c_int, ctypes.c_float, ctypes.c_void_p, ctypes.c_longlong
 
@@ -170,6 +170,9 @@ _SIGNATURES = {
     "latent": {
         "kvb_norm_add_rmsnorm": [_c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_float, _c_void_p, _c_float, _c_void_p, _c_void_p,
                                  _c_void_p, _c_int, _c_int, _c_void_p],
+        "kvb_latent_expand_prepare": [_c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p,
+                                      _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p,
+                                      _c_void_p],
         "kvb_latent_norm_rope_append": [_c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_float,
                                         _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int,
                                         _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p],
@@ -250,6 +253,9 @@ _SIGNATURES = {
         "kvb_attention_pairs": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p,
                                 _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,
                                 _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_void_p, _c_void_p],
+        "kvb_attention_pairs_expanded": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p,
+                                         _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_float, _c_void_p,
+                                         _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     },
     "primitive_costs": {
         "kvb_primitive_costs_count": [],
@@ -265,7 +271,8 @@ _SIGNATURES = {
 }
 
 
-_OPTIONAL = {"kvb_flash_decode_tma", "kvb_flash_decode_tma_max_clusters"}      # only in attention_flash variants for head sizes 64 and 128
+# Only in some variants of a module: attention_flash for head sizes 64 and 128, attention_pairs over pages or over expanded rows.
+_OPTIONAL = {"kvb_flash_decode_tma", "kvb_flash_decode_tma_max_clusters", "kvb_attention_pairs", "kvb_attention_pairs_expanded"}
 
 
 class _Library:
@@ -324,6 +331,9 @@ class CudaKernels(KernelSet):
         self.routed_tcgen05_min_pairs: Optional[int] = 1024
         self.latent_flash = True             # bfloat16, key rows in steps of 8 numbers: the tensor-core kernel over shared key rows
         self._latent_planners: Dict[tuple, "LatentAttentionPlanner"] = {}
+        self._expand_planners: Dict[int, "LatentExpandPlanner"] = {}
+        self._attn_expanded: Dict[int, _Library] = {}
+        self.latent_expand = True            # portions of enough rows: keys and values of all heads expanded before attention
         self._zero_slopes: Dict[int, torch.Tensor] = {}
         self._sampling = _Library("sampling")
         self._gemm_skinny = _Library("gemm_skinny")
@@ -494,6 +504,15 @@ class CudaKernels(KernelSet):
         return found
 
     # ---- operators ---------------------------------------------------------
+    # Bytes of a step's expanded keys and values, with the latents they come from; steps that need more are not expanded.
+    LATENT_EXPAND_MAX_BYTES = 256 << 20
+
+    def latent_expand_planner(self, dim: int, vdim: int, rot_dim: int, kv_rank: int, window: Optional[int] = None) -> Optional[LatentExpandPlanner]:
+        """The lists `latent_expanded_attention` reads from `StepBatch.plans`, or None for sizes that it does not take."""
+        if dim != vdim or dim not in (64, 128) or rot_dim % 16 or not 16 <= rot_dim <= 64 or kv_rank % 8:
+            return None
+        return self._expand_planners.setdefault(int(window or 0), LatentExpandPlanner(int(window or 0)))
+
     def embed(self, table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, src: Optional[torch.Tensor] = None,
               last: Optional[torch.Tensor] = None, out16: Optional[torch.Tensor] = None, scale: float = 1.0) -> None:
         """out[r] = table[ids[r]] * scale, or table[last[src[r]]] * scale where src[r] >= 0 (a token still on the device);
@@ -1117,6 +1136,56 @@ class CudaKernels(KernelSet):
             _dtype_code(x.dtype), x_first, xs, x.shape[1], _ptr(w), _ptr(out), os_, T, N, K, H, _ptr(g), 0 if g is None else g.shape[1],
             col, 1 if gate_per_head else 0, rot, 0 if cos is None else cos.shape[1], _ptr(cos), _ptr(sin),
             0 if cos is None else cos.shape[0], _ptr(positions), _ptr(self.error_word), self._stream()), "head_linear")
+
+    def latent_expanded_attention(self, q: torch.Tensor, w_ukv: torch.Tensor, batch: StepBatch, kv: PagedKVView, out: torch.Tensor, num_heads: int,
+                                  dim: int, scale: float, workspace, cos: torch.Tensor, sin: torch.Tensor, gate, gate_per_head: bool,
+                                  window: Optional[int], sink: Optional[torch.Tensor]) -> bool:
+        """A latent-attention layer's way from its queries to its gated heads, for portions of prompts: the cached rows that the step
+        sees are gathered, w_ukv [2 * H * dim, kv_rank] expands them to keys and values of every head (csrc/gemm_tcgen05.cu), and
+        attention runs over those.  q: the first H * (dim + rot_dim) columns of its rows are the heads' queries; their rotated
+        parts are turned in place.  out [T, H * dim] = attention * sigmoid(gate), `gate` and `gate_per_head` as in `head_linear`.
+        Returns False (and does nothing) where the step's plan or the sizes say otherwise."""
+        H, C = num_heads, w_ukv.shape[1]
+        rot_dim = kv.spec.head_dim - C
+        plan = batch.plans.get(LatentExpandPlanner.plan_name(int(window or 0)))
+        g, col = gate
+        if not (self.latent_expand and plan is not None and plan.counts["blocks"] and workspace is not None and q.dtype == torch.bfloat16
+                and self.bf16_gemm != "simt" and kv.spec.num_kv_heads == 1 and q.shape[1] % 8 == 0 and (q.data_ptr() | kv.k_pages.data_ptr()) % 16 == 0
+                and (gate_per_head or (g.data_ptr() % 16 == 0 and g.shape[1] % 8 == 0 and col % 8 == 0))):
+            return False
+        if kv.spec.window and (not window or window > kv.spec.window):
+            raise KernelError(f"latent_attention: a window of {window} over a cache entry that keeps {kv.spec.window} keys")
+        blocks, rows = plan.counts["blocks"], 128 * plan.counts["blocks"]
+        if 2 * rows * (2 * H * dim + C + 64) > self.LATENT_EXPAND_MAX_BYTES:
+            return False
+        T = q.shape[0]
+        if (tuple(w_ukv.shape) != (2 * H * dim, C) or tuple(out.shape) != (T, H * dim) or q.shape[1] < H * (dim + rot_dim)
+                or g.shape[0] != T or col + (H if gate_per_head else H * dim) > g.shape[1] or g.dtype != q.dtype):
+            raise KernelError("latent_expanded_attention: shapes do not fit one another")
+        lat = workspace.buffer("latent.expand_lat", (rows, C), torch.bfloat16)
+        rot = workspace.buffer("latent.expand_rot", (rows, 64), torch.bfloat16)
+        both = workspace.buffer("latent.expand_kv", (rows, 2 * H * dim), torch.bfloat16)
+        self._count("latent_expand_prepare")
+        _check(self._latent.kvb_latent_expand_prepare(
+            _ptr(kv.k_pages), _ptr(kv.block_table), kv.block_table.shape[1], kv.page_size, _ptr(plan.arrays["blocks"]), blocks,
+            _ptr(batch.seg_kv_len), C, rot_dim, _ptr(lat), _ptr(rot), _ptr(q), q.shape[1], H, dim, _ptr(cos), _ptr(sin), cos.shape[1],
+            cos.shape[0], _ptr(batch.positions), T, _ptr(self.error_word), self._stream()), "latent_expand_prepare")
+        self._count("gemm_tcgen05")
+        _check(self._gemm_tc.kvb_gemm_tcgen05(_dtype_code(both.dtype), 0, _ptr(lat), _ptr(w_ukv), None, _ptr(both), rows, 2 * H * dim, C,
+                                              0.0, _ptr(self.error_word), self._stream()), "latent_expanded_attention (keys and values)")
+        lib = self._attn_expanded.get(dim)
+        if lib is None:
+            lib = self._attn_expanded[dim] = _Library("attention_pairs", f"x{dim}", [f"-DKVB_HEAD_DIM={dim}", "-DKVB_EXPANDED=1"])
+        pairs = plan.counts["pairs"]
+        scratch = workspace.buffer("attn.pairs_scratch", (4 * self.sm_count * 128 * (dim + 2),), torch.float32)
+        tickets = workspace.zeros("attn.pairs_tickets", (2 * pairs * H,), torch.int32)
+        self._count("attention_pairs_expanded")
+        _check(lib.kvb_attention_pairs_expanded(
+            _ptr(q), q.shape[1], _ptr(out), _ptr(both), _ptr(rot), rows, _ptr(plan.arrays["pairs"]), pairs, _ptr(scratch), _ptr(tickets),
+            self.sm_count, _ptr(plan.arrays["key_row"]), _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_kv_len), T, H, rot_dim,
+            int(window or 0), float(scale), _ptr(sink), _ptr(g), g.shape[1], col, 1 if gate_per_head else 0, self.tc_pairs_min_tiles,
+            _ptr(self.error_word), self._stream()), "attention_pairs_expanded")
+        return True
 
     def latent_attention(self, q: torch.Tensor, batch: StepBatch, kv: PagedKVView, out: torch.Tensor, num_heads: int,
                          value_dim: int, scale: float, workspace=None, window: Optional[int] = -1,

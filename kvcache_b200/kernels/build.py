@@ -40,7 +40,7 @@ MODULES: Dict[str, dict] = {
     "sampling": {"src": "sampling.cu", "deps": ["common.cuh"]},
     "gemm_skinny": {"src": "gemm_skinny.cu", "deps": ["common.cuh"]},
     "gemm_tcgen05": {"src": "gemm_tcgen05.cu", "deps": ["common.cuh", "tc_common.cuh"]},
-    # Compiled per head size: variant "d<head_dim>" with -DKVB_HEAD_DIM=<head_dim>.
+    # Compiled per head size: variant "d<head_dim>" with -DKVB_HEAD_DIM=<head_dim>; "x<head_dim>": keys and values expanded from a latent.
     "attention_flash": {"src": "attention_flash.cu", "deps": ["common.cuh", "flash_core.cuh", "no_alloc.h", "tc_common.cuh"]},
     "attention_tc": {"src": "attention_tc.cu", "deps": ["common.cuh", "tc_common.cuh"]},
     "attention_pairs": {"src": "attention_pairs.cu", "deps": ["common.cuh", "tc_common.cuh"]},
@@ -53,7 +53,8 @@ MODULES: Dict[str, dict] = {
 # Variants that `build_all` makes for modules compiled per size.
 DEFAULT_VARIANTS = {"attention_flash": [("d64", ["-DKVB_HEAD_DIM=64"]), ("d128", ["-DKVB_HEAD_DIM=128"])],
                     "attention_tc": [("d64", ["-DKVB_HEAD_DIM=64"]), ("d128", ["-DKVB_HEAD_DIM=128"])],
-                    "attention_pairs": [("d64", ["-DKVB_HEAD_DIM=64"]), ("d128", ["-DKVB_HEAD_DIM=128"])]}
+                    "attention_pairs": [("d64", ["-DKVB_HEAD_DIM=64"]), ("d128", ["-DKVB_HEAD_DIM=128"]),
+                                        ("x64", ["-DKVB_HEAD_DIM=64", "-DKVB_EXPANDED=1"]), ("x128", ["-DKVB_HEAD_DIM=128", "-DKVB_EXPANDED=1"])]}
 
 _loaded: Dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()

@@ -1,4 +1,5 @@
-"""Work list of the attention kernel over shared key rows (csrc/latent_flash.cu).
+"""Work lists of latent attention: of the kernel over shared key rows (csrc/latent_flash.cu), and of portions whose keys and values
+are expanded first (csrc/attention_pairs.cu, at the end).
 
 All heads of a token read the same cached rows, so the kernel's rows are (token, head) pairs: a request that brings
 `count` tokens has count * H rows, cut into tiles of BM rows; a tile sees the keys up to its last token's position.
@@ -17,6 +18,7 @@ from typing import Dict, Tuple
 import numpy as np
 
 from ..parts.base import StepPlanner
+from .attention_plan import TC_PAIR_ROWS
 
 KEY_TILE = 64
 SMALL_TILE, LARGE_TILE = 16, 64      # rows of a tile: 16 while every request's rows fit one such tile, else 64
@@ -67,3 +69,48 @@ class LatentAttentionPlanner(StepPlanner):
         segments = tuple((i, int(s), int(c)) for i, (s, c) in enumerate(zip(starts, counts)))
         items, tiles, nsplit, bm = _plan(segments, self.heads, self.blocks_wanted, self.large_tile, self.window)
         return {"items": items.reshape(-1)}, {"items": len(items), "tiles": tiles, "nsplit": nsplit, "bm": bm}
+
+
+EXPAND_BLOCK = 128               # keys of a block of expanded rows: the key tile of csrc/attention_pairs.cu
+EXPAND_MAX_BLOCKS = 256          # blocks a step may bring
+EXPAND_MAX_PAIRS = 128           # pairs of row tiles (csrc/attention_pairs.cu, MAX_TILES)
+# Rows that every request of the step brings: an expanded key has to serve many.  A whole layer on both sides, in us, keys as they are
+# and expanded, 16 heads of 128 (rank 512) and 14 of 64 (rank 256): 64 rows 73 and 61, 52 and 45; 64 behind 2,000 93 and 89, 62.5 and 63;
+# four requests of 50 behind 2,000 208 and 206, 97 and 98; 128 behind 2,000 140 and 93, 80 and 63; 2,048 536 and 168, 269 and 90.
+EXPAND_MIN_ROWS = 64
+
+
+class LatentExpandPlanner(StepPlanner):
+    """Lists for steps of portions whose keys and values are expanded once per token and head before attention.
+
+    `blocks`: (segment, first key) of every 128 keys that any row of the step sees; `key_row`: the row that a segment's key 0 has
+    among the expanded rows, or would have; `pairs`: (segment, first row) of pairs of row tiles.  The count `blocks` is 0 where
+    the step is not expanded: a request brings fewer than EXPAND_MIN_ROWS rows, or the step sees more than the lists hold."""
+
+    def __init__(self, window: int = 0):
+        self.window = int(window or 0)
+        self.name = self.plan_name(self.window)
+
+    @staticmethod
+    def plan_name(window: int = 0) -> str:
+        return "latent_expand" + (f".w{window}" if window else "")
+
+    def sections(self, num_tokens: int, num_segments: int) -> Dict[str, int]:
+        return {"blocks": 2 * EXPAND_MAX_BLOCKS, "key_row": num_segments, "pairs": 2 * (num_tokens // TC_PAIR_ROWS + num_segments)}
+
+    def plan(self, starts, counts) -> Tuple[Dict[str, np.ndarray], Dict[str, int]]:
+        none = np.zeros(0, dtype=np.int32)
+        off = {"blocks": none, "key_row": none, "pairs": none}, {"blocks": 0, "pairs": 0}
+        if int(min(counts)) < EXPAND_MIN_ROWS:
+            return off
+        blocks, key_row, pairs = [], [], []
+        for i, (start, count) in enumerate(zip(starts, counts)):
+            start, count = int(start), int(count)
+            first = max(0, start - self.window + 1) // EXPAND_BLOCK * EXPAND_BLOCK if self.window else 0
+            key_row.append(EXPAND_BLOCK * len(blocks) - first)
+            blocks.extend((i, key) for key in range(first, start + count, EXPAND_BLOCK))
+            pairs.extend((i, row) for row in range(0, count, TC_PAIR_ROWS))
+        if len(blocks) > EXPAND_MAX_BLOCKS or len(pairs) > EXPAND_MAX_PAIRS:
+            return off
+        flat = lambda rows: np.asarray(rows, dtype=np.int32).reshape(-1)
+        return {"blocks": flat(blocks), "key_row": flat(key_row), "pairs": flat(pairs)}, {"blocks": len(blocks), "pairs": len(pairs)}

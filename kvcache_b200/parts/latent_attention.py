@@ -8,12 +8,14 @@ With h the mixer's input, per token:
     score(i, j) = scale * (q_i[:dim] . k_j + R_i(q_i[dim:]) . R_j(kr_j)),  j <= i;  softmax over j
     out = Wo (concat_heads(sum_j p_ij v_j) * sigmoid(Wg h))
 
-This part never expands a cached token.  Since k_j = Wuk c_j, the unrotated score is (Wuk^T q_i[:dim]) . c_j: the
+Two orders of the products, both here.  Steps of few rows never expand a cached token.  Since k_j = Wuk c_j, the unrotated score is (Wuk^T q_i[:dim]) . c_j: the
 query is taken into the latent's space once (a product per head with Wuk^T), attention then runs with one shared
 "key" row [c_j | R_j(kr_j)] of kv_rank + rot_dim numbers per token, whose first kv_rank numbers are also the "value",
 and the head's result sum_j p_ij c_j goes through Wuv afterwards.  The cache entry is one key head of that width and
 no value pool (`PagedKVSpec.value_dim == 0`); a step reads kv_rank + rot_dim numbers per cached token, whatever the
-number of heads.
+number of heads.  Portions of prompts, whose rows are many for each key, expand the keys and values that they see once per head
+(`latent_expanded_attention` of the kernel set, where it has one and the step's plan says so) and attend over heads of dim + rot_dim
+and vdim numbers: a quarter of the multiply-adds.
 
 Options.  `q_rank` None: the query comes straight from the input, q = Wq h (tensor `q`; no `dq`, `dq.norm`, `uq`).
 `window`: a query sees its own key and the window - 1 before it.  `sink` "learned": the softmax's denominator also holds
@@ -65,7 +67,7 @@ class LatentAttention(Mixer):
         self.kv_col = self.q_width
         self.gate_col = self.q_width + (self.key_dim if self.own_latent else 0)
         self.w_in: Optional[torch.Tensor] = None
-        self.w_uq = self.w_uk_t = self.w_uv = self.w_o = None
+        self.w_uq = self.w_uk_t = self.w_uv = self.w_ukv = self.w_o = None
         self.q_norm = self.kv_norm = self.sink_logits = None
 
     def keep_for_window(self, window: Optional[int]) -> None:
@@ -131,7 +133,12 @@ class LatentAttention(Mixer):
             self.sink_logits = tensors[f"{p}sink"].to(torch.float32).to(device).contiguous()
         # [H, kv_rank, dim]: the transposed key expansion, which takes a head's unrotated query to the latent's space.
         self.w_uk_t = place(tensors[f"{p}uk"].view(H, self.dim, self.kv_rank).transpose(1, 2))
-        self.w_uv = place(tensors[f"{p}uv"].view(H, self.vdim, self.kv_rank))
+        if self.dtype == torch.bfloat16 and self.dim == self.vdim:
+            # Both expansions as they are, one product for portions of prompts; the values' half also serves the other order.
+            self.w_ukv = place(torch.cat([tensors[f"{p}uk"], tensors[f"{p}uv"]], dim=0))
+            self.w_uv = self.w_ukv[H * self.dim:].view(H, self.vdim, self.kv_rank)
+        else:
+            self.w_uv = place(tensors[f"{p}uv"].view(H, self.vdim, self.kv_rank))
         self.w_o = place(tensors[f"{p}o"])
 
     def weight_bytes(self) -> int:
@@ -145,8 +152,11 @@ class LatentAttention(Mixer):
         planner = getattr(kernels, "latent_attention_planner", None)
         if planner is None:
             return ()
-        return (planner(self.num_heads, self.key_dim, self.kv_rank, self.window) if self.window else
-                planner(self.num_heads, self.key_dim, self.kv_rank),)
+        plans = (planner(self.num_heads, self.key_dim, self.kv_rank, self.window) if self.window else
+                 planner(self.num_heads, self.key_dim, self.kv_rank),)
+        expand = getattr(kernels, "latent_expand_planner", None)
+        more = expand(self.dim, self.vdim, self.rot_dim, self.kv_rank, self.window) if expand and self.dtype == torch.bfloat16 else None
+        return plans + (more,) if more is not None else plans
 
     def forward(self, x: torch.Tensor, ctx: LayerContext) -> torch.Tensor:
         T, H = x.shape[0], self.num_heads
@@ -157,18 +167,32 @@ class LatentAttention(Mixer):
         proj = ws.buffer("latent.proj", (T, self.w_in.shape[0]), self.dtype)
         k.linear(x, self.w_in, proj)
         rotate = (rotation.cos, rotation.sin, ctx.batch.positions)
-        q_lat = ws.buffer("latent.q_lat", (T, H * self.key_dim), self.dtype)
         if self.q_rank is not None:
             cq = ws.buffer("latent.cq", (T, self.q_rank), self.dtype)
             k.latent_norm_rope_append(proj, self.q_rank, self.kv_rank, self.rot_dim, self.q_norm, self.kv_norm, self.eps,
                                       rotation.cos, rotation.sin, ctx.batch, ctx.kv, cq)
             q = ws.buffer("latent.q", (T, H * self.q_head), self.dtype)
             k.linear(cq, self.w_uq, q)
-            k.head_linear(q, self.w_uk_t, q_lat, rotate=rotate)
         else:
+            q = proj
             if self.own_latent:
                 k.latent_norm_rope_append(proj, 0, self.kv_rank, self.rot_dim, None, self.kv_norm, self.eps, rotation.cos,
                                           rotation.sin, ctx.batch, ctx.kv, None, kv_col=self.kv_col)
+        o = ws.buffer("latent.o", (T, H * self.vdim), self.dtype)
+        expanded = getattr(k, "latent_expanded_attention", None) if self.w_ukv is not None else None
+        if expanded is None or not expanded(q, self.w_ukv, ctx.batch, ctx.kv, o, H, self.dim, self.scale, ws, rotation.cos, rotation.sin,
+                                            (proj, self.gate_col), self.gate == "head", self.window, self.sink_logits):
+            self._attend_in_latent_space(q, o, proj, rotate, ctx)
+        delta = ws.buffer("attn.delta", (T, self.hidden), self.dtype)
+        k.linear(o, self.w_o, delta)
+        return delta
+
+    def _attend_in_latent_space(self, q: torch.Tensor, o: torch.Tensor, proj: torch.Tensor, rotate, ctx: LayerContext) -> None:
+        T, H, k, ws = q.shape[0], self.num_heads, ctx.kernels, ctx.workspace
+        q_lat = ws.buffer("latent.q_lat", (T, H * self.key_dim), self.dtype)
+        if self.q_rank is not None:
+            k.head_linear(q, self.w_uk_t, q_lat, rotate=rotate)
+        else:
             k.head_linear(proj, self.w_uk_t, q_lat, rotate=rotate, x_col=0)
         o_lat = ws.buffer("latent.o_lat", (T, H * self.kv_rank), self.dtype)
         if self.sink_logits is None and self.window == ctx.kv.spec.window:
@@ -176,11 +200,7 @@ class LatentAttention(Mixer):
         else:
             k.latent_attention(q_lat, ctx.batch, ctx.kv, o_lat, H, self.kv_rank, self.scale, ws, window=self.window,
                                sink=self.sink_logits)
-        o = ws.buffer("latent.o", (T, H * self.vdim), self.dtype)
         if self.gate == "channel":
             k.head_linear(o_lat, self.w_uv, o, gate=(proj, self.gate_col))
         else:
             k.head_linear(o_lat, self.w_uv, o, gate=(proj, self.gate_col), gate_per_head=True)
-        delta = ws.buffer("attn.delta", (T, self.hidden), self.dtype)
-        k.linear(o, self.w_o, delta)
-        return delta

@@ -332,7 +332,8 @@ __global__ void __launch_bounds__(THREADS, (MT == 4 && NV <= 4) ? 2 : 1) latent_
 // out[row] = sum_s 2^(m_s - M) O_s[row] / sum_s 2^(m_s - M) l_s over the `nsplit` items of the row's tile.
 // Grid (tiles, BM); the items of tile i are i * nsplit .. (i + 1) * nsplit - 1.  A block is MERGE_GROUPS x Dv / 4 threads:
 // thread (g, c) adds four columns of the splits g, g + MERGE_GROUPS, ... (independent loads, all in flight at once), and the
-// groups' sums are added in the order of the groups - a fixed order, whichever block runs first.
+// groups' sums are added in the order of the groups - a fixed order, whichever block runs first.  At least a warp of threads, which
+// the splits' weights take, however few the columns are.
 constexpr int MAX_SPLITS = 32, MERGE_GROUPS = 8;
 __global__ void latent_flash_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                           const int* __restrict__ items, const int* __restrict__ seg_q_start,
@@ -354,7 +355,7 @@ __global__ void latent_flash_merge_kernel(const float* __restrict__ part_o, cons
 #pragma unroll
     for (int i = 0; i < MAX_SPLITS / MERGE_GROUPS; ++i) {
         const int s = g + i * MERGE_GROUPS;
-        v[i] = s < nsplit ? base[(size_t)s * step] : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[i] = g < MERGE_GROUPS && s < nsplit ? base[(size_t)s * step] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (threadIdx.x < 32) {
         const int s = threadIdx.x;
@@ -372,10 +373,10 @@ __global__ void latent_flash_merge_kernel(const float* __restrict__ part_o, cons
 #pragma unroll
     for (int i = 0; i < MAX_SPLITS / MERGE_GROUPS; ++i) {
         const int s = g + i * MERGE_GROUPS;
-        const float w = s < nsplit ? weight[s] : 0.f;
+        const float w = g < MERGE_GROUPS && s < nsplit ? weight[s] : 0.f;
         acc.x += w * v[i].x; acc.y += w * v[i].y; acc.z += w * v[i].z; acc.w += w * v[i].w;
     }
-    sums[g * cols + c] = acc;
+    if (g < MERGE_GROUPS) sums[g * cols + c] = acc;
     __syncthreads();
     if (g == 0) {
         float4 t = sums[c];
@@ -451,7 +452,7 @@ KVB_API int kvb_latent_flash(const void* q, void* out, const void* k_pages, cons
     }
 #undef KVB_LF
     if (code != KVB_OK || nsplit == 1) return code;
-    kvb_launch(lf::latent_flash_merge_kernel, dim3(n_tiles, BM), dim3(lf::MERGE_GROUPS * (Dv / 4)), (size_t)lf::MERGE_GROUPS * Dv * 4, stream, (const float*)part_o, (const float*)part_ml,
+    kvb_launch(lf::latent_flash_merge_kernel, dim3(n_tiles, BM), dim3(lf::MERGE_GROUPS * (Dv / 4) < 32 ? 32 : lf::MERGE_GROUPS * (Dv / 4)), (size_t)lf::MERGE_GROUPS * Dv * 4, stream, (const float*)part_o, (const float*)part_ml,
                items, seg_q_start, seg_q_len, (bf16*)out, H, Dv, BM, nsplit);
     return kvb_launch_status();
 }

@@ -22,7 +22,7 @@
 // that holds the first key its first row sees, and keys before that key are not fetched (a windowed cache entry may have
 // given their pages back) but zero-filled and masked.  `sink` (one logit per head, or null): the softmax's denominator
 // also holds exp(sink[h]); the rows of a tile's first split start from (m, l) = (sink, 1) instead of (-inf, 0).
-#include "common.cuh"
+#include "tc_common.cuh"
 
 namespace lf {
 
@@ -329,6 +329,218 @@ __global__ void __launch_bounds__(THREADS, (MT == 4 && NV <= 4) ? 2 : 1) latent_
         }
 }
 
+// ---- tiles of 16 rows: decoded tokens ------------------------------------------------------------------------------------
+// The same sums for one tile of rows, with what bounded it there taken out: the rows' Q is held in registers (every warp read it from
+// shared memory for every tile of keys), a warp's scores run in four chains of products, they stay in registers (row maxima meet in
+// shared memory, P alone is written), and keys come as one bulk copy a row, STAGES - 1 tiles ahead, their pages looked up a tile before.  Two
+// barriers a tile instead of four.  KS: sixteens of Q a thread holds.
+// What bounds it: the stream of keys, 3.4 TB/s of it (32 tokens of 16 heads with 4,096 keys of 576: 66 us with tiles of 16 rows of the kernel
+// above, 44 here; a layer of 64 of them 173 -> 128 us, of 14 heads with keys of 288 93 -> 82, of one 31 -> 29).  With pages looked up
+// where they are wanted, by one warp for all rows, it took 72: everything waited for that warp at the next barrier.
+template <int NV, int KS, int STAGES, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS) latent_rows16_kernel(
+    const bf16* __restrict__ q, bf16* __restrict__ out, const bf16* __restrict__ k_pages, const int* __restrict__ block_table,
+    int table_stride, const int* __restrict__ items, const int* __restrict__ seg_q_start, const int* __restrict__ seg_q_len,
+    const int* __restrict__ seg_kv_len, float* __restrict__ part_o, float* __restrict__ part_ml, int H, int Dk, int Dv, int rs,
+    int page_size, int window, float scale_log2, int nsplit, const float* __restrict__ sink, int* __restrict__ err) {
+    constexpr int BM = 16, WARPS = THREADS / 32;
+    constexpr bool OWN_Q = KS <= 20;                        // Q has a place of its own, else it is read by way of the last stage
+    constexpr int LEAD = OWN_Q ? STAGES : STAGES - 1;       // tiles asked for at once
+    extern __shared__ __align__(128) unsigned char smem[];
+    bf16* Ks = reinterpret_cast<bf16*>(smem);               // stage s at s * BN * rs; rows of rs numbers, 16 bytes beyond a multiple of 128
+    __shared__ __align__(16) bf16 Ps[2][BM][BN + 8];
+    __shared__ __align__(16) float tops[2][BM][WARPS];
+    __shared__ __align__(8) uint64_t full[STAGES];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+    const int* item = items + 4 * blockIdx.x;
+    const int seg = item[0], m0 = item[1], kb = item[2], ke = item[3];
+    const int q_len = seg_q_len[seg], kv_len = seg_kv_len[seg], start = kv_len - q_len, M_total = q_len * H;
+    const size_t row_base = (size_t)seg_q_start[seg] * H + m0;
+    const int* table = block_table + (size_t)seg * table_stride;
+    const int key_lo = window > 0 ? max(0, start + m0 / H - window + 1) : 0;
+    const bool first_split = blockIdx.x % nsplit == 0;
+    const int ntiles = (ke - kb + BN - 1) / BN, row_bytes = Dk * 2;
+    if (tid == 0) {
+        for (int i = 0; i < STAGES; ++i) tc::mbar_init(&full[i], WARPS);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    // Columns beyond Dk, up to what products read, are zeros for good.
+    const int pad = (max(KS * 16, 64 * NV) - Dk) / 8;
+    for (int i = tid; i < STAGES * BN * pad; i += THREADS)
+        *reinterpret_cast<uint4*>(Ks + (size_t)(i / pad) * rs + Dk + i % pad * 8) = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+
+    // Every warp brings in eight rows of a tile, its first lanes one each; rows that no query sees, or beyond the run, are zeros.  The
+    // page a lane wants is looked up a tile before it is wanted: the way to it is what all would wait for at the next barrier.
+    const int my_row = 8 * warp + (lane & 7);
+    auto lookup = [&](int tile) -> int {
+        const int j = kb + tile * BN + my_row;
+        if (lane >= 8 || j >= ke || j < key_lo) return -1;
+        const int page = table[j / page_size];
+        if (page < 0) atomicOr(err, KVB_DEV_BAD_PAGE);
+        return max(page, 0);
+    };
+    auto fetch = [&](int tile, int page) {
+        bf16* dst = Ks + ((size_t)(tile % STAGES) * BN + my_row) * rs;
+        uint64_t* bar = &full[tile % STAGES];
+        const int there = __popc(__ballot_sync(0xffffffffu, page >= 0));
+        if (lane < 8 && page < 0)
+            for (int c = 0; c < Dk / 8; ++c) *reinterpret_cast<uint4*>(dst + c * 8) = make_uint4(0, 0, 0, 0);
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");       // copies may come to the same place later
+        __syncwarp();                                       // the zeros before the barrier's word
+        if (lane == 0) tc::mbar_expect_tx(bar, there * row_bytes);
+        __syncwarp();
+        if (page >= 0)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                         ::"r"(smem_addr(dst)), "l"(k_pages + ((size_t)page * page_size + (kb + tile * BN + my_row) % page_size) * Dk), "r"(row_bytes),
+                           "r"(smem_addr(bar)) : "memory");
+    };
+    // Keys of earlier steps are asked for while the kernel before is still running; its own are among a request's last.
+    int asked = 0;
+    for (; asked < LEAD && asked < ntiles && min(ke, kb + (asked + 1) * BN) <= start; ++asked) fetch(asked, lookup(asked));
+    int page_next = lookup(asked);
+    pdl_wait();
+    pdl_launch_dependents();
+    for (; asked < LEAD && asked < ntiles; ++asked) {
+        fetch(asked, page_next);
+        page_next = lookup(asked + 1);
+    }
+
+    // Rows g and g + 8 of Q, by way of shared memory (straight from memory, four bytes a load and all of it for every
+    // warp, they cost a step of short histories 3 us).
+    uint32_t a[KS][4];
+    {
+        bf16* Qs = Ks + (size_t)(OWN_Q ? STAGES : STAGES - 1) * BN * rs;
+        for (int e = tid; e < BM * KS * 2; e += THREADS) {
+            const int r = e / (KS * 2), c = e % (KS * 2) * 8;
+            *reinterpret_cast<uint4*>(Qs + (size_t)r * rs + c) =
+                m0 + r < M_total && c < Dk ? *reinterpret_cast<const uint4*>(q + (row_base + r) * Dk + c) : make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < KS; ++k) ldmatrix_x4(a[k][0], a[k][1], a[k][2], a[k][3], Qs + (size_t)(lane & 15) * rs + k * 16 + (lane >> 4) * 8);
+        if (!OWN_Q) __syncthreads();
+        for (int e = tid; !OWN_Q && e < BM * pad; e += THREADS) *reinterpret_cast<uint4*>(Qs + (size_t)(e / pad) * rs + Dk + e % pad * 8) = make_uint4(0, 0, 0, 0);
+    }
+    float m[2], l[2];
+    int pos[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int row = m0 + g + 8 * i;
+        pos[i] = row < M_total ? start + row / H : -1;
+        const bool from_sink = sink != nullptr && first_split && row < M_total;
+        m[i] = from_sink ? sink[row % H] * 1.4426950408889634f : MASKED;
+        l[i] = from_sink && warp == 0 && t4 == 0 ? 1.f : 0.f;
+    }
+    float o[NV][4];
+#pragma unroll
+    for (int nv = 0; nv < NV; ++nv) o[nv][0] = o[nv][1] = o[nv][2] = o[nv][3] = 0.f;
+
+    bool ok = true;
+    for (int tile = 0; tile < ntiles; ++tile) {
+        const int par = tile & 1;
+        const bf16* Kt = Ks + (size_t)(tile % STAGES) * BN * rs;
+        ok = ok && tc::mbar_wait(&full[tile % STAGES], (tile / STAGES) & 1);
+        float s[4][4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s[c][0] = s[c][1] = s[c][2] = s[c][3] = 0.f;
+        const bf16* at = Kt + (size_t)(8 * warp + (lane & 7)) * rs + (lane >> 3) * 8;
+#pragma unroll
+        for (int k2 = 0; k2 < KS / 2; ++k2) {
+            uint32_t b[4];
+            ldmatrix_x4(b[0], b[1], b[2], b[3], at + k2 * 32);
+            mma_bf16(s[(2 * k2) & 3], a[2 * k2], b[0], b[1]);
+            mma_bf16(s[(2 * k2 + 1) & 3], a[2 * k2 + 1], b[2], b[3]);
+        }
+        float v[2][2], top[2];
+        const int j0 = kb + tile * BN + 8 * warp + 2 * t4;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int j = j0 + e, x = 2 * i + e;
+                const bool seen = j < ke && j <= pos[i] && (window <= 0 || j > pos[i] - window);
+                v[i][e] = seen ? ((s[0][x] + s[1][x]) + (s[2][x] + s[3][x])) * scale_log2 : MASKED;
+            }
+            top[i] = fmaxf(v[i][0], v[i][1]);
+            top[i] = fmaxf(top[i], __shfl_xor_sync(0xffffffffu, top[i], 1));
+            top[i] = fmaxf(top[i], __shfl_xor_sync(0xffffffffu, top[i], 2));
+            if (t4 == 0) tops[par][g + 8 * i][warp] = top[i];
+        }
+        __syncthreads();                                    // ... and all are done with the tile before: its stage may be filled
+        const int next = tile + STAGES - 1;
+        if (next >= LEAD && next < ntiles) {
+            fetch(next, page_next);
+            page_next = lookup(next + 1);
+        }
+        float corr[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float4* f = reinterpret_cast<const float4*>(tops[par][g + 8 * i]);
+            const float4 x = f[0], y = f[1];
+            const float m_new = fmaxf(m[i], fmaxf(fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)), fmaxf(fmaxf(y.x, y.y), fmaxf(y.z, y.w))));
+            corr[i] = exp2f(m[i] - m_new);
+            m[i] = m_new;
+            const float p0 = v[i][0] > 0.5f * MASKED ? exp2f(v[i][0] - m_new) : 0.f, p1 = v[i][1] > 0.5f * MASKED ? exp2f(v[i][1] - m_new) : 0.f;
+            l[i] = l[i] * corr[i] + (p0 + p1);
+            *reinterpret_cast<__nv_bfloat162*>(&Ps[par][g + 8 * i][8 * warp + 2 * t4]) = __floats2bfloat162_rn(p0, p1);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int nv = 0; nv < NV; ++nv) { o[nv][0] *= corr[0]; o[nv][1] *= corr[0]; o[nv][2] *= corr[1]; o[nv][3] *= corr[1]; }
+#pragma unroll
+        for (int kk = 0; kk < BN / 16; ++kk) {
+            uint32_t p[4], b[NV][2];
+            ldmatrix_x4(p[0], p[1], p[2], p[3], &Ps[par][lane & 15][kk * 16 + (lane >> 4) * 8]);
+            const int krow = kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
+            if constexpr (NV == 1) {
+                ldmatrix_x2_trans(b[0][0], b[0][1], Kt + (size_t)krow * rs + warp * 8);
+            } else {
+#pragma unroll
+                for (int n2 = 0; n2 < NV / 2; ++n2)
+                    ldmatrix_x4_trans(b[2 * n2][0], b[2 * n2][1], b[2 * n2 + 1][0], b[2 * n2 + 1][1],
+                                      Kt + (size_t)krow * rs + warp * 8 * NV + n2 * 16 + (lane >> 4) * 8);
+            }
+#pragma unroll
+            for (int nv = 0; nv < NV; ++nv) mma_bf16(o[nv], p, b[nv][0], b[nv][1]);
+        }
+    }
+    if (!ok) atomicOr(err, tc::KVB_DEV_TIMEOUT);            // copies that are still asked for have been waited for as long as that
+
+    // The rows' sums: over the four lanes of a row, then over the warps in their order.
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
+        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
+        if (t4 == 0) tops[0][g + 8 * i][warp] = l[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int r = g + 8 * i;
+        if (m0 + r >= M_total) continue;
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) sum += tops[0][r][w];
+        const float inv = sum > 0.f ? 1.f / sum : 0.f;
+        bf16* orow = out + (row_base + r) * Dv;
+        float* prow = nsplit > 1 ? part_o + ((size_t)blockIdx.x * BM + r) * Dv : nullptr;
+#pragma unroll
+        for (int nv = 0; nv < NV; ++nv) {
+            const int d = warp * 8 * NV + nv * 8 + 2 * t4;   // Dv is a multiple of four
+            if (d >= Dv) continue;
+            if (nsplit == 1) *reinterpret_cast<__nv_bfloat162*>(orow + d) = __floats2bfloat162_rn(o[nv][2 * i] * inv, o[nv][2 * i + 1] * inv);
+            else *reinterpret_cast<float2*>(prow + d) = make_float2(o[nv][2 * i], o[nv][2 * i + 1]);
+        }
+        if (nsplit > 1 && warp == 0 && t4 == 0) {
+            part_ml[((size_t)blockIdx.x * BM + r) * 2] = m[i];
+            part_ml[((size_t)blockIdx.x * BM + r) * 2 + 1] = sum;
+        }
+    }
+}
+
 // out[row] = sum_s 2^(m_s - M) O_s[row] / sum_s 2^(m_s - M) l_s over the `nsplit` items of the row's tile.
 // Grid (tiles, BM); the items of tile i are i * nsplit .. (i + 1) * nsplit - 1.  A block is MERGE_GROUPS x Dv / 4 threads:
 // thread (g, c) adds four columns of the splits g, g + MERGE_GROUPS, ... (independent loads, all in flight at once), and the
@@ -418,6 +630,29 @@ static int launch(const bf16* q, bf16* out, const bf16* k_pages, const int* bloc
     return kvb_launch_status();
 }
 
+// Whether the kernel for tiles of 16 rows takes these sizes: every row on 16 bytes, Q's sixteens in registers.
+static bool rows16_fits(int Dk, int Dv, const void* k_pages) { return Dk <= 576 && Dv <= Dk && !((uintptr_t)k_pages & 15); }
+
+template <int NV, int KS, int STAGES, int BLOCKS>
+static int launch_rows16(const bf16* q, bf16* out, const bf16* k_pages, const int* block_table, int table_stride, const int* items,
+                         int n_items, const int* seg_q_start, const int* seg_q_len, const int* seg_kv_len, float* part_o, float* part_ml,
+                         int H, int Dk, int Dv, int page_size, int window, float scale, int nsplit, const float* sink, int* err,
+                         cudaStream_t stream) {
+    constexpr int columns = KS * 16 > 64 * NV ? KS * 16 : 64 * NV;
+    const int rs = (columns + 63) / 64 * 64 + 8;
+    constexpr int bytes = (STAGES * BN + (KS <= 20 ? 16 : 0)) * ((columns + 63) / 64 * 64 + 8) * 2;
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(latent_rows16_kernel<NV, KS, STAGES, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+            return (int)cudaGetLastError();
+        configured = true;
+    }
+    kvb_launch(latent_rows16_kernel<NV, KS, STAGES, BLOCKS>, dim3(n_items), dim3(THREADS), (size_t)bytes, stream, q, out, k_pages, block_table,
+               table_stride, items, seg_q_start, seg_q_len, seg_kv_len, part_o, part_ml, H, Dk, Dv, rs, page_size, window,
+               scale * 1.4426950408889634f, nsplit, sink, err);
+    return kvb_launch_status();
+}
+
 }  // namespace lf
 
 // Whether the kernel takes these sizes (else the caller uses the generic kernel): 0 yes, negative no.
@@ -443,7 +678,16 @@ KVB_API int kvb_latent_flash(const void* q, void* out, const void* k_pages, cons
     code = lf::launch<MT, NV_>((const bf16*)q, (bf16*)out, (const bf16*)k_pages, block_table, table_stride, items, n_items,  \
                                seg_q_start, seg_q_len, seg_kv_len, part_o, part_ml, H, Dk, Dv, page_size, window, scale,    \
                                nsplit, sink, err, stream)
-    if (BM == 16) {
+#define KVB_ROWS16(NV_, KS, STAGES, BLOCKS)                                                                                    \
+    code = lf::launch_rows16<NV_, KS, STAGES, BLOCKS>((const bf16*)q, (bf16*)out, (const bf16*)k_pages, block_table, table_stride, items,  \
+                                                      n_items, seg_q_start, seg_q_len, seg_kv_len, part_o, part_ml, H, Dk, Dv, page_size,  \
+                                                      window, scale, nsplit, sink, err, stream)
+    if (BM == 16 && lf::rows16_fits(Dk, Dv, k_pages)) {
+        if (Dk <= 160) { if (NV == 1) KVB_ROWS16(1, 10, 2, 2); else KVB_ROWS16(2, 10, 2, 2); }
+        else if (Dk <= 320) { if (NV == 1) KVB_ROWS16(1, 20, 2, 2); else if (NV == 2) KVB_ROWS16(2, 20, 2, 2); else KVB_ROWS16(4, 20, 2, 2); }
+        else if (NV == 1) KVB_ROWS16(1, 36, 3, 1); else if (NV == 2) KVB_ROWS16(2, 36, 3, 1); else if (NV == 4) KVB_ROWS16(4, 36, 3, 1);
+        else KVB_ROWS16(8, 36, 3, 1);
+    } else if (BM == 16) {
         if (NV == 1) KVB_LF(1, 1); else if (NV == 2) KVB_LF(1, 2); else if (NV == 4) KVB_LF(1, 4); else KVB_LF(1, 8);
     } else if (BM == 32) {
         if (NV == 1) KVB_LF(2, 1); else if (NV == 2) KVB_LF(2, 2); else if (NV == 4) KVB_LF(2, 4); else KVB_LF(2, 8);
@@ -451,6 +695,7 @@ KVB_API int kvb_latent_flash(const void* q, void* out, const void* k_pages, cons
         if (NV == 1) KVB_LF(4, 1); else if (NV == 2) KVB_LF(4, 2); else if (NV == 4) KVB_LF(4, 4); else KVB_LF(4, 8);
     }
 #undef KVB_LF
+#undef KVB_ROWS16
     if (code != KVB_OK || nsplit == 1) return code;
     kvb_launch(lf::latent_flash_merge_kernel, dim3(n_tiles, BM), dim3(lf::MERGE_GROUPS * (Dv / 4) < 32 ? 32 : lf::MERGE_GROUPS * (Dv / 4)), (size_t)lf::MERGE_GROUPS * Dv * 4, stream, (const float*)part_o, (const float*)part_ml,
                items, seg_q_start, seg_q_len, (bf16*)out, H, Dv, BM, nsplit);

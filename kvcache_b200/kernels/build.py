@@ -35,7 +35,7 @@ MODULES: Dict[str, dict] = {
     "scan_chunk": {"src": "scan_chunk.cu", "deps": ["common.cuh", "tc_common.cuh"]},
     "scan_wide": {"src": "scan_wide.cu", "deps": ["common.cuh"]},
     "moe": {"src": "moe.cu", "deps": ["common.cuh", "mma_tile.cuh"]},
-    "latent_flash": {"src": "latent_flash.cu", "deps": ["common.cuh"]},
+    "latent_flash": {"src": "latent_flash.cu", "deps": ["common.cuh", "tc_common.cuh"]},
     "gemm_grouped": {"src": "gemm_grouped.cu", "deps": ["common.cuh", "tc_common.cuh"]},
     "sampling": {"src": "sampling.cu", "deps": ["common.cuh"]},
     "gemm_skinny": {"src": "gemm_skinny.cu", "deps": ["common.cuh"]},

@@ -21,7 +21,7 @@ def kernels():
 
 
 @pytest.mark.parametrize("window", [None, 70])
-@pytest.mark.parametrize("H,Dk,Dv", [(16, 8, 8), (2, 16, 4), (5, 168, 64)])
+@pytest.mark.parametrize("H,Dk,Dv", [(16, 8, 8), (2, 16, 4), (1, 160, 128), (5, 168, 64), (14, 320, 256), (16, 328, 300), (16, 576, 512), (3, 576, 60), (2, 584, 512)])
 def test_single_tokens_over_shared_key_rows(kernels, H, Dk, Dv, window):
     from kvcache_b200.engine.workspace import Workspace
     from kvcache_b200.parts.base import StepPlan

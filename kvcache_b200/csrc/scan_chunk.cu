@@ -30,6 +30,8 @@
 // decays 2,048 x 64 x 128 x 64: 278 -> 262.  Level or up to 5 % behind: 2,048 x 14 x 64 under the delta rule (297 -> 311), 48 tokens beside 63
 // single ones under the gated one (46 -> 48), 512 x 28 x 128 x 64 head decays (53 -> 54).  Registers for four blocks an SM: with more, steps of
 // several segments take up to 40 % longer, with the compiler's own choice single ones 5 %.
+// Where heads are few, runs of a segment's chunks are walked at once (modes without Z, further down): 2,048 rows of 7 heads of 64 x 128, records
+// and walk 135 -> 56 us; a layer of 28 heads of 128 x 64 under head decays 277 -> 205 us.  From 256 blocks on the walk has warps enough (64 heads: 431 -> 455).
 // A weight above a diagonal is zero and is multiplied like any other; only in a chunk whose values are not all finite (a vote) are
 // later tokens left out one by one, which takes 15 to 35 % longer where it is done always.
 // A segment's result does not depend on what else the step holds, and a token's not on later ones, whatever they hold (an infinite or undefined
@@ -476,12 +478,29 @@ __device__ __forceinline__ void copy_bulk(float* smem, const float* gmem, uint32
                  ::"r"(tc::smem_u32(smem)), "l"(gmem), "r"(bytes), "r"(tc::smem_u32(bar)) : "memory");
 }
 
-// grid (16 value channels, heads, segments), over the chunks first .. first + held - 1 of the step.  A thread holds TD neighbouring key channels of TC value channels of the state; a warp's lanes
+// What a segment's chunks are cut into where several runs of them are walked at once (`chunks` of them each, see launches (2) below).
+struct Runs {
+    int chunks;                  // 0: a segment is one run
+    float* starts;               // [runs, H, D, Dv]: the states that runs start from
+    float* decays;               // [runs, H, 64 NI or 1]: the product of a run's decays
+};
+// Run `id` of the step: its segment, its number within it and the segment's count of runs; false beyond the last.
+__device__ __forceinline__ bool find_run(int id, const Segments& seg, const Runs& runs, int& sg, int& k, int& count) {
+    for (sg = 0; sg < seg.count; ++sg) {
+        count = ((seg.q_len[sg] + C - 1) / C + runs.chunks - 1) / runs.chunks;
+        if (id < count) { k = id; return true; }
+        id -= count;
+    }
+    return false;
+}
+
+// grid (16 value channels, heads, segments or runs), over the chunks first .. first + held - 1 of the step.  A thread holds TD neighbouring key channels of TC value channels of the state; a warp's lanes
 // are 2 TC groups of key channels by 16 / TC of value channels.  Beside that, every thread owns one token's OC value channels of Z and O.
 template <int MODE, int NI, int TD, int TC, int STAGES>
 __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_walk_kernel(const Rows in, const Segments seg, const float* __restrict__ records,
                                                                              int first, int held, float q_scale, float* __restrict__ memory,
-                                                                             float* __restrict__ out, int H, int D, int Dv, int* __restrict__ err) {
+                                                                             float* __restrict__ out, int H, int D, int Dv, const Runs runs,
+                                                                             int* __restrict__ err) {
     constexpr bool Z = has_z(MODE), V = has_v(MODE);
     constexpr int DP = 64 * NI, CG = 16 / TC, DG = 32 / CG, WARPS = DP / (TD * DG), OC = 16 * C / (32 * WARPS);
     constexpr int NR = Z ? 2 * C : C;                          // rows that meet S_0: [Y | Q] or Q
@@ -493,19 +512,24 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_walk_kernel
     __shared__ __align__(16) float v_s[2][C][16], z_s[Z ? C : 1][16];
     __shared__ __align__(8) uint64_t full[STAGES];
     const int tid = threadIdx.x, lane = tid & 31, wd = tid >> 5, cg = lane % CG, dg = lane / CG;
-    const int h = blockIdx.y, sg = blockIdx.z;
+    const int h = blockIdx.y;
+    int sg = blockIdx.z, run = 0, run_count = 1;
+    if (runs.chunks > 0 && !find_run(blockIdx.z, seg, runs, sg, run, run_count)) return;
     int n = seg.q_len[sg], r0 = seg.q_start[sg], chunk0 = 0;
     const int slot = seg.slot[sg];
     if (n <= 0) return;
     for (int i = 0; i < sg; ++i) chunk0 += (seg.q_len[i] + C - 1) / C;
     // The segment's chunks from `begin` on that are among the `held` whose records are there.
-    const int begin = max(0, first - chunk0), chunks = min((n + C - 1) / C, first + held - chunk0) - begin, d0 = (wd * DG + dg) * TD;
+    const int begin = max(run * runs.chunks, first - chunk0), d0 = (wd * DG + dg) * TD;
+    int chunks = min((n + C - 1) / C, first + held - chunk0) - begin;
+    if (runs.chunks > 0) chunks = min(chunks, runs.chunks);
     if (chunks <= 0) return;
     n -= begin * C;
     r0 += begin * C;
     chunk0 += begin - first;
 
     float* mem = memory + ((size_t)slot * H + h) * D * Dv;
+    const float* start = runs.chunks > 0 ? runs.starts + ((size_t)blockIdx.z * H + h) * D * Dv : mem;
     const int col0 = 16 * blockIdx.x + cg * TC;
     float2 S[TD / 2][TC];                                      // key channels d0 + 2 i and the next
 #pragma unroll
@@ -513,7 +537,7 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_walk_kernel
 #pragma unroll
         for (int c = 0; c < TC; ++c) {
             const int d = d0 + 2 * i;
-            const float* at = mem + (size_t)d * Dv + col0 + c;
+            const float* at = start + (size_t)d * Dv + col0 + c;
             S[i][c] = make_float2(d < D && col0 + c < Dv ? at[0] : 0.f, d + 1 < D && col0 + c < Dv ? at[Dv] : 0.f);
         }
     if (tid == 0) {
@@ -719,6 +743,7 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_walk_kernel
             for (int i = ci - 1; i < chunks && i < ci + STAGES - 1; ++i) tc::mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
         return;
     }
+    if (run + 1 < run_count) return;                           // the next run has started from this state already
 #pragma unroll
     for (int i = 0; i < TD / 2; ++i)
 #pragma unroll
@@ -730,9 +755,181 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_walk_kernel
         }
 }
 
+// ---- launches (2) of the modes without Z, where the heads are too few to fill the GPU: several runs of a segment's chunks at once -----
+// A run's end is P S_0 + U, with P the product of its decays and U what its tokens leave of a state of zero.  First U and P of every run but a
+// segment's last (a thread's share of the state as in the walk, no barrier but the one that hands a stage back), then the states that
+// runs start from, one after the other element by element, then the walk with a block for every run.
+// grid (16 value channels, heads, runs).  U of run r goes to place r + 1.
+template <int MODE, int NI, int TD, int TC, int STAGES>
+__global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_ends_kernel(const Rows in, const Segments seg, const float* __restrict__ records,
+                                                                             int held, int H, int D, int Dv, const Runs runs,
+                                                                             int* __restrict__ err) {
+    static_assert(!has_z(MODE), "");
+    constexpr int DP = 64 * NI, CG = 16 / TC, DG = 32 / CG, THREADS = 16 * DP / (TD * TC);
+    constexpr Record R = record_of(MODE, DP);
+    constexpr bool HEAD = MODE == CHUNK_HEAD_DECAY;
+    constexpr int KEYS = C * (DP + 4), PART = KEYS + (HEAD ? 3 * C : DP);      // what is wanted of a record: K1 and the decays
+    static_assert(HEAD || R.decay == R.k1 + KEYS, "K1 and the decays follow one another");
+    extern __shared__ __align__(128) float sm[];
+    __shared__ __align__(16) float v_s[2][C][16];
+    __shared__ __align__(8) uint64_t full[STAGES];
+    const int tid = threadIdx.x, lane = tid & 31, wd = tid >> 5, cg = lane % CG, dg = lane / CG, h = blockIdx.y;
+    int sg, run, run_count;
+    if (!find_run(blockIdx.z, seg, runs, sg, run, run_count) || run + 1 == run_count) return;
+    int r0 = seg.q_start[sg], chunk0 = run * runs.chunks;
+    for (int i = 0; i < sg; ++i) chunk0 += (seg.q_len[i] + C - 1) / C;
+    r0 += run * runs.chunks * C;
+    const int chunks = runs.chunks, d0 = (wd * DG + dg) * TD, col0 = 16 * blockIdx.x + cg * TC, groups = H / in.qk_div;
+    if (tid == 0) {
+        for (int i = 0; i < STAGES; ++i) tc::mbar_init(&full[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    auto fetch = [&](int ci) {
+        float* b = sm + (ci % STAGES) * PART;
+        uint64_t* bar = &full[ci % STAGES];
+        const size_t id = chunk0 + ci;
+        tc::mbar_expect_tx(bar, PART * 4);
+        if (HEAD) {
+            copy_bulk(b, records + (id * groups + h / in.qk_div) * R.shared + R.k1, KEYS * 4, bar);
+            copy_bulk(b + KEYS, records + (size_t)held * groups * R.shared + (id * H + h) * (R.total - R.shared), 3 * C * 4, bar);
+        } else {
+            copy_bulk(b, records + (id * H + h) * R.total + R.k1, PART * 4, bar);
+        }
+    };
+    // 16 x 16 values of a chunk, shared out over the threads.
+    auto values = [&](int ci, float (&v)[16 * C / THREADS]) {
+#pragma unroll
+        for (int e = 0; e < 16 * C / THREADS; ++e) {
+            const int at = tid + e * THREADS, t = at >> 4, col = 16 * blockIdx.x + (at & 15);
+            v[e] = ci < chunks && col < Dv ? in.rows[(size_t)(r0 + ci * C + t) * in.stride + in.v_col + (size_t)h * Dv + col] : 0.f;
+        }
+    };
+    auto keep_values = [&](int ci, const float (&v)[16 * C / THREADS]) {
+#pragma unroll
+        for (int e = 0; e < 16 * C / THREADS; ++e) v_s[ci & 1][(tid + e * THREADS) >> 4][(tid + e * THREADS) & 15] = v[e];
+    };
+    float next[16 * C / THREADS];
+    values(0, next);
+    keep_values(0, next);
+    float2 S[TD / 2][TC];
+#pragma unroll
+    for (int i = 0; i < TD / 2; ++i)
+#pragma unroll
+        for (int c = 0; c < TC; ++c) S[i][c] = make_float2(0.f, 0.f);
+    Decay product[HEAD ? 1 : TD];
+    bool zero[HEAD ? 1 : TD] = {};
+    __syncthreads();
+    if (tid == 0)
+        for (int i = 0; i < STAGES - 1 && i < chunks; ++i) fetch(i);
+    bool ok = true, failed = false;
+    int ci = 0;
+    for (; ci < chunks; ++ci) {
+        failed = ci > 0 && __syncthreads_or(!ok);              // all are done with chunk ci - 1, and its values are there
+        if (failed) break;
+        if (tid == 0 && ci + STAGES - 1 < chunks) fetch(ci + STAGES - 1);
+        values(ci + 1, next);
+        ok = tc::mbar_wait(&full[ci % STAGES], (ci / STAGES) & 1);
+        const float* b = sm + (ci % STAGES) * PART;
+        // As in the walk: earlier tokens by themselves, the decayed state, the last eight tokens on top.  A run's chunks are full.
+        float2 N[TD / 2][TC];
+#pragma unroll
+        for (int i = 0; i < TD / 2; ++i)
+#pragma unroll
+            for (int c = 0; c < TC; ++c) N[i][c] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < C; ++s) {
+            if (s == C / 2) {
+#pragma unroll
+                for (int i = 0; i < TD / 4; ++i) {
+                    float4 decay;
+                    if (HEAD) decay.x = decay.y = decay.z = decay.w = b[KEYS + 2 * C];
+                    else decay = *(const float4*)(b + KEYS + d0 + 4 * i);
+                    if (!HEAD || i == 0) {
+                        const float a[4] = {decay.x, decay.y, decay.z, decay.w};
+#pragma unroll
+                        for (int e = 0; e < (HEAD ? 1 : 4); ++e) {
+                            product[4 * i + e].times(a[e]);
+                            zero[4 * i + e] |= a[e] == 0.f;
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < TC; ++c) {
+                        N[2 * i][c] = fma2(low2(decay), S[2 * i][c], N[2 * i][c]);
+                        N[2 * i + 1][c] = fma2(high2(decay), S[2 * i + 1][c], N[2 * i + 1][c]);
+                    }
+                }
+            }
+            float2 v[TC];
+            pairs(&v_s[ci & 1][s][cg * TC], v);
+            if (HEAD) {
+                const float gain = b[KEYS + C + s];
+#pragma unroll
+                for (int c = 0; c < TC; ++c) v[c] = mul2(v[c], make_float2(gain, gain));
+            }
+#pragma unroll
+            for (int i = 0; i < TD / 4; ++i) {
+                const float4 k1 = *(const float4*)(b + s * (DP + 4) + d0 + 4 * i);
+#pragma unroll
+                for (int c = 0; c < TC; ++c) {
+                    N[2 * i][c] = fma2(low2(k1), v[c], N[2 * i][c]);
+                    N[2 * i + 1][c] = fma2(high2(k1), v[c], N[2 * i + 1][c]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < TD / 2; ++i)
+#pragma unroll
+            for (int c = 0; c < TC; ++c) S[i][c] = N[i][c];
+        keep_values(ci + 1, next);
+    }
+    if (!ok || failed) {                                       // the copies asked for are waited for (or given up)
+        atomicOr(err, tc::KVB_DEV_TIMEOUT);
+        if (failed && tid == 0)
+            for (int i = ci - 1; i < chunks && i < ci + STAGES - 1; ++i) tc::mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
+        return;
+    }
+    const size_t place = (size_t)blockIdx.z * H + h;
+    float* end = runs.starts + (place + H) * D * Dv;
+#pragma unroll
+    for (int i = 0; i < TD / 2; ++i)
+#pragma unroll
+        for (int c = 0; c < TC; ++c) {
+            const int d = d0 + 2 * i;
+            float* at = end + (size_t)d * Dv + col0 + c;
+            if (d < D && col0 + c < Dv) at[0] = S[i][c].x;
+            if (d + 1 < D && col0 + c < Dv) at[Dv] = S[i][c].y;
+        }
+    // A product that runs out of exponents is the smallest number there is, not zero, so that an infinite state stays infinite as in a
+    // walk; zero only where a chunk's decay is zero.
+    auto value = [&](int e) { return zero[e] ? product[e].value() : fmaxf(product[e].value(), 1.4e-45f); };
+    if (HEAD) {
+        if (blockIdx.x == 0 && tid == 0) runs.decays[place] = value(0);
+    } else if (blockIdx.x == 0 && cg == 0) {
+#pragma unroll
+        for (int e = 0; e < TD; ++e) runs.decays[place * DP + d0 + e] = value(HEAD ? 0 : e);
+    }
+}
+
+// grid (elements of a state in 256s, heads, segments): the states that a segment's runs start from.
+template <bool HEAD, int DP>
+__global__ void __launch_bounds__(256) run_starts_kernel(const Segments seg, const float* __restrict__ memory, int H, int D, int Dv, const Runs runs) {
+    const int e = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y, sg = blockIdx.z;
+    if (e >= D * Dv || seg.q_len[sg] <= 0) return;
+    auto count_of = [&](int s) { return ((seg.q_len[s] + C - 1) / C + runs.chunks - 1) / runs.chunks; };
+    int first = 0;
+    for (int s = 0; s < sg; ++s) first += count_of(s);
+    const int count = count_of(sg), d = e / Dv;
+    float S = memory[((size_t)seg.slot[sg] * H + h) * D * Dv + e];
+    for (int k = 0; k < count; ++k) {
+        const size_t place = (size_t)(first + k) * H + h;
+        runs.starts[place * D * Dv + e] = S;
+        if (k + 1 < count) S = fmaf(runs.decays[HEAD ? place : place * DP + d], S, runs.starts[(place + H) * D * Dv + e]);
+    }
+}
+
 template <int MODE, int NI, int TD, int TC, int STAGES>
 static int launch_walk(const Rows& in, const Segments& seg, const float* records, int first, int held, float q_scale, float* memory, float* out,
-                       int H, int D, int Dv, int* err, cudaStream_t stream) {
+                       int H, int D, int Dv, const Runs& runs, int blocks_z, int* err, cudaStream_t stream) {
     constexpr int bytes = STAGES * record_of(MODE, 64 * NI).total * (int)sizeof(float);
     auto kernel = chunk_walk_kernel<MODE, NI, TD, TC, STAGES>;
     if (bytes > 16 * 1024) {                                   // (the kernel has shared memory of its own beside it)
@@ -741,15 +938,30 @@ static int launch_walk(const Rows& in, const Segments& seg, const float* records
     }
     // Not as a dependent launch: blocks placed while the records are still being made crowd onto the SMs that are free first, and
     // stay there (7 heads of 64 x 128, 2,048 tokens: 219 us against 112).
-    kernel<<<dim3((Dv + 15) / 16, H, seg.count), 16 * 64 * NI / (TD * TC), bytes, stream>>>(in, seg, records, first, held, q_scale, memory, out, H,
-                                                                                           D, Dv, err);
+    kernel<<<dim3((Dv + 15) / 16, H, blocks_z), 16 * 64 * NI / (TD * TC), bytes, stream>>>(in, seg, records, first, held, q_scale, memory, out, H,
+                                                                                          D, Dv, runs, err);
+    return kvb_launch_status();
+}
+
+// The runs' starts: `count` runs at most.
+template <int MODE, int NI, int TD, int TC, int STAGES>
+static int launch_starts(const Rows& in, const Segments& seg, const float* records, int held, const float* memory, int H, int D, int Dv,
+                         const Runs& runs, int count, int* err, cudaStream_t stream) {
+    constexpr int bytes = STAGES * (C * (64 * NI + 4) + (MODE == CHUNK_HEAD_DECAY ? 3 * C : 64 * NI)) * (int)sizeof(float);
+    auto kernel = chunk_ends_kernel<MODE, NI, TD, TC, STAGES>;
+    if (bytes > 16 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return (int)e;
+    }
+    kernel<<<dim3((Dv + 15) / 16, H, count), 16 * 64 * NI / (TD * TC), bytes, stream>>>(in, seg, records, held, H, D, Dv, runs, err);
+    run_starts_kernel<MODE == CHUNK_HEAD_DECAY, 64 * NI><<<dim3((D * Dv + 255) / 256, H, seg.count), 256, 0, stream>>>(seg, memory, H, D, Dv, runs);
     return kvb_launch_status();
 }
 
 // `held` chunks at a time, as many as `records` has room for; the states pass from one run of them to the next through `memory`.
 template <int MODE, int NI>
 static int run(const Rows& in, const Segments& seg, float* records, int total, int held, float q_scale, float* memory, float* out, int H, int D,
-               int Dv, int* err, cudaStream_t stream) {
+               int Dv, const Runs& runs, int run_count, int* err, cudaStream_t stream) {
     for (int first = 0; first < total; first += held) {
         const int count = min(held, total - first);
         if constexpr (MODE == CHUNK_HEAD_DECAY) {
@@ -764,7 +976,13 @@ static int run(const Rows& in, const Segments& seg, float* records, int total, i
         if (rc != KVB_OK) return rc;
         // Key and value channels a thread holds: 4 x 2 of 64 (four warps), 8 x 2 of 128 (four warps).  Half of the warps with 4 x 4 or 8 x 2 of 64
         // take 16 to 35 % longer, 4 x 4 and 8 x 4 of 128 8 to 40 %, 8 x 1 30 to 50 %.
-        rc = launch_walk<MODE, NI, 4 * NI, 2, 2>(in, seg, records, first, held, q_scale, memory, out, H, D, Dv, err, stream);
+        if constexpr (!has_z(MODE))
+            if (runs.chunks > 0) {                             // one run of all chunks then (kvb_chunk_scan)
+                rc = launch_starts<MODE, NI, 4 * NI, 2, 2>(in, seg, records, held, memory, H, D, Dv, runs, run_count, err, stream);
+                if (rc != KVB_OK) return rc;
+            }
+        rc = launch_walk<MODE, NI, 4 * NI, 2, 2>(in, seg, records, first, held, q_scale, memory, out, H, D, Dv, runs,
+                                                 runs.chunks > 0 ? run_count : seg.count, err, stream);
         if (rc != KVB_OK) return rc;
     }
     return KVB_OK;
@@ -783,7 +1001,7 @@ static bool rows_fit(int mode, const Rows& in, int H, int G, int D, int Dv) {
 
 template <int MODE>
 static int run(const Rows& in, const Segments& seg, float* records, int held, float q_scale, float* memory, float* out, int T, int H,
-               int G, int D, int Dv, int* err, cudaStream_t stream) {
+               int G, int D, int Dv, int run_chunks, float* starts, int* err, cudaStream_t stream) {
     if (H < 1 || G < 1 || H % G || D < 1 || Dv < 1 || !rows_fit(MODE, in, H, G, D, Dv)) return KVB_ERR_SHAPE;
     if (seg.count <= 0 || T <= 0) return KVB_OK;
     if (records == nullptr) return KVB_ERR_SHAPE;
@@ -792,8 +1010,12 @@ static int run(const Rows& in, const Segments& seg, float* records, int held, fl
     if (MODE == CHUNK_CHANNEL_DECAY && Dv > 512) return KVB_ERR_LIMIT;      // as the other forms of this scan
     const int total = T / C + seg.count;                       // no step has more chunks than this
     held = min(held, total);
-    return D <= 64 ? run<MODE, 1>(in, seg, records, total, held, q_scale, memory, out, H, D, Dv, err, stream)
-                   : run<MODE, 2>(in, seg, records, total, held, q_scale, memory, out, H, D, Dv, err, stream);
+    if (run_chunks < 0 || (run_chunks > 0 && (has_z(MODE) || held < total || !starts))) return KVB_ERR_SHAPE;
+    const int count = run_chunks > 0 ? T / (C * run_chunks) + seg.count : 0;   // no step has more runs than this
+    if (count > 65535) return KVB_ERR_LIMIT;
+    const Runs runs = {run_chunks, starts, starts + (size_t)count * H * D * Dv};
+    return D <= 64 ? run<MODE, 1>(in, seg, records, total, held, q_scale, memory, out, H, D, Dv, runs, count, err, stream)
+                   : run<MODE, 2>(in, seg, records, total, held, q_scale, memory, out, H, D, Dv, runs, count, err, stream);
 }
 
 }  // namespace sc
@@ -809,14 +1031,21 @@ KVB_API int kvb_chunk_shared_floats(int mode, int D) { return mode < 0 || mode >
 // number h of Dv for v; H a multiple of G), `gates` [T, gate_stride] the mode's own numbers (sc::Rows); `records`: scratch of `held` times
 // the floats above for all H heads and G groups, on 16 bytes: a step of more chunks (at most T / 16 + S) goes through it `held` chunks at a
 // time, with the same results.  D up to 128.
+// `held` + (r << 20) (modes 2 and 3, all chunks held): a segment's chunks are walked in runs of r of them at once; behind the records
+// `records` then has (T / (16 r) + S) H (D Dv + D rounded up to 64) floats more.
 KVB_API int kvb_chunk_scan(int mode, const float* rows, int stride, int q_col, int k_col, int v_col, int G, const float* gates,
                            int gate_stride, float q_scale, const int* seg_q_start, const int* seg_q_len, const int* seg_slot, float* memory,
                            float* out, int T, int S, int H, int D, int Dv, int held, float* records, int* err, cudaStream_t stream) {
+    const int run_chunks = held < 0 ? 0 : held >> 20;
+    if (held > 0) held &= (1 << 20) - 1;
+    float* starts = nullptr;
+    if (run_chunks > 0 && records && D >= 1 && H >= 1 && G >= 1)
+        starts = records + (size_t)held * ((size_t)H * kvb_chunk_record_floats(mode, D) + (size_t)G * kvb_chunk_shared_floats(mode, D));
     const sc::Rows in = {rows, gates, stride, gate_stride, q_col, k_col, v_col, G > 0 ? H / G : 0};
     const sc::Segments seg = {seg_q_start, seg_q_len, seg_slot, S};
-    if (mode == sc::CHUNK_GATED_DELTA) return sc::run<sc::CHUNK_GATED_DELTA>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, err, stream);
-    if (mode == sc::CHUNK_DELTA_RULE) return sc::run<sc::CHUNK_DELTA_RULE>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, err, stream);
-    if (mode == sc::CHUNK_CHANNEL_DECAY) return sc::run<sc::CHUNK_CHANNEL_DECAY>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, err, stream);
-    if (mode == sc::CHUNK_HEAD_DECAY) return sc::run<sc::CHUNK_HEAD_DECAY>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, err, stream);
+    if (mode == sc::CHUNK_GATED_DELTA) return sc::run<sc::CHUNK_GATED_DELTA>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, run_chunks, starts, err, stream);
+    if (mode == sc::CHUNK_DELTA_RULE) return sc::run<sc::CHUNK_DELTA_RULE>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, run_chunks, starts, err, stream);
+    if (mode == sc::CHUNK_CHANNEL_DECAY) return sc::run<sc::CHUNK_CHANNEL_DECAY>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, run_chunks, starts, err, stream);
+    if (mode == sc::CHUNK_HEAD_DECAY) return sc::run<sc::CHUNK_HEAD_DECAY>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, run_chunks, starts, err, stream);
     return KVB_ERR_SHAPE;
 }

@@ -1462,19 +1462,35 @@ class CudaKernels(KernelSet):
             _ptr(maximum), _ptr(out), proj.shape[0], batch.num_segments, H, D, Dv, self.SCAN_CHUNK, max_chunks, _ptr(scratch),
             self._stream()), "matrix_state_scan")
 
-    def _gated_linear_chunks(self, batch: StepBatch, workspace, D: int) -> bool:
+    def _gated_linear_chunks(self, batch: StepBatch, workspace, H: int, D: int, Dv: int) -> bool:
         """Sixteen tokens at a time: 600 + 400 rows of 8 heads of 128 x 256 68 us against 148, 256 rows of 7 heads of 64 x 128 24 against 85,
-        1,000 rows of those 76 against 83; longer portions of heads that narrow keep chunks of 64 side by side, whose time hardly
-        grows with the rows (2,048: 100; but it grows with heads and requests, and 28 heads or four requests are behind by up to half)."""
-        return (workspace is not None and self.SCAN_CHUNK and D <= self.CHUNK_SCAN_MAX_DIM and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS
-                and (D > 64 or batch.max_q_len <= 1024))
+        1,000 rows of those 76 against 83.  Longer portions of heads that narrow only where `_chunk_scan` walks runs of chunks at once
+        (2,048 rows of 7 such heads, a whole layer: 117 us against 154 in chunks of 64 side by side, and 220 in one run)."""
+        if not (workspace is not None and self.SCAN_CHUNK and D <= self.CHUNK_SCAN_MAX_DIM and batch.max_q_len >= self.SCAN_CHUNK_MIN_ROWS):
+            return False
+        if D > 64 or batch.max_q_len <= 1024:
+            return True
+        walkers = H * -(-Dv // 16)
+        return walkers >= self.CHUNK_RUN_MIN_WALKERS and self._chunk_runs("channel_decay", batch.num_tokens, batch.num_segments, walkers) > 1
 
     # Portions go sixteen tokens at a time (csrc/scan_chunk.cu) where a head has at most CHUNK_SCAN_MAX_DIM key channels.
     CHUNK_SCAN_MAX_DIM = 128
     # Scratch of a scan for portions: longer steps go through it in runs of as many chunks as it holds (16 heads of 128 channels under the delta
     # rule: 39 KB a head and chunk, 6,800 tokens a run; the whole of a step of 30,000 would take 1.2 GB).
     CHUNK_SCRATCH_BYTES = 256 << 20
+    # Where a walk of the decays alone has at most so many blocks and its segments on average so many chunks, they are walked in runs of at
+    # least CHUNK_RUN_MIN, as many as bring it to about CHUNK_RUN_BLOCKS blocks (four an SM).  Whole layers, in us, without and with: decays per
+    # channel, 7 heads of 64 x 128, 2,048 rows 220 and 117, 512 81 and 68, 300 (not taken) 62 and 60; 8 heads of 128 x 256, 2,048 rows 339 and
+    # 280, two requests (256 blocks) 312 and 277, three (384; not taken) 255 and 256, 300 rows (not taken) 85 and 91; decays per head, 28 heads of 128 x
+    # 64, 2,048 rows 277 and 205, two requests (224) 262 and 212, four (448; not taken) 175 and 214; 64 heads (256; not taken) 431 and 455.
+    CHUNK_RUN_BLOCKS, CHUNK_RUN_MIN, CHUNK_RUN_MIN_CHUNKS, CHUNK_RUN_MIN_WALKERS = 592, 4, 24, 16
+    CHUNK_RUN_MAX_BLOCKS = {"channel_decay": 256, "head_decay": 224}
     CHUNK_MODES = {"gated_delta": 0, "delta_rule": 1, "channel_decay": 2, "head_decay": 3}
+
+    def _chunk_runs(self, mode: str, T: int, S: int, walkers: int) -> int:
+        """Runs to cut a step's chunks into, where a walk has `walkers` blocks a segment (0: none)."""
+        few = walkers * S <= self.CHUNK_RUN_MAX_BLOCKS.get(mode, 0) and T >= 16 * self.CHUNK_RUN_MIN_CHUNKS * S
+        return self.CHUNK_RUN_BLOCKS // walkers if few else 0
 
     def _chunk_scan(self, mode: str, rows, cols, G: int, gates, q_scale: float, batch: StepBatch, memory, out, H: int, D: int, Dv: int,
                     workspace) -> None:
@@ -1486,13 +1502,21 @@ class CudaKernels(KernelSet):
         # By the step's rows and segments alone, so that a recorded step finds the same launches.
         chunks = T // 16 + S
         held = min(chunks, max(1, self.CHUNK_SCRATCH_BYTES // (4 * size)))
-        records = (torch.empty(held * size, dtype=torch.float32, device=rows.device) if workspace is None else
-                   workspace.buffer("recurrent.chunk_records", (held * size,), torch.float32))
         # Per run: the records (and their triangular systems) and the walk, one of which has been counted.
         self.launches += -(-chunks // held) * (3 if mode == "delta_rule" else 2) - 1
+        # Decays alone: a run's end is its decays times its start, plus what its tokens leave, so that runs of chunks can be walked at once.
+        run_chunks, floats, walkers = 0, held * size, H * -(-Dv // 16)
+        if held == chunks < 1 << 20 and workspace is not None:
+            runs = self._chunk_runs(mode, T, S, walkers)
+            if runs > S:
+                run_chunks = max(self.CHUNK_RUN_MIN, -(-(T // 16) // runs))
+                floats += (T // (16 * run_chunks) + S) * H * (D * Dv + -(-D // 64) * 64)
+                self.launches += 2
+        records = (torch.empty(floats, dtype=torch.float32, device=rows.device) if workspace is None else
+                   workspace.buffer("recurrent.chunk_records", (floats,), torch.float32))
         _check(lib.kvb_chunk_scan(code, _ptr(rows), rows.shape[1], *cols, G, _ptr(gates), gates.shape[1], float(q_scale),
                                   _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), _ptr(memory), _ptr(out), T, S, H, D,
-                                  Dv, held, _ptr(records), _ptr(self.error_word), self._stream()), f"{mode} (chunks)")
+                                  Dv, held + (run_chunks << 20), _ptr(records), _ptr(self.error_word), self._stream()), f"{mode} (chunks)")
 
     def gated_linear_scan(self, proj: torch.Tensor, cols, z: torch.Tensor, tau: float, q_scale: float, batch: StepBatch,
                           memory: torch.Tensor, out: torch.Tensor, H: int, D: int, Dv: int, workspace=None) -> None:
@@ -1500,7 +1524,7 @@ class CudaKernels(KernelSet):
         a_t = sigmoid(z_t)^(1 / tau) per key channel; q, k, v at columns `cols` of the float32 rows `proj`.  `z` [T, H * D] is
         overwritten by the decays."""
         self.launches += 1
-        if self._gated_linear_chunks(batch, workspace, D):
+        if self._gated_linear_chunks(batch, workspace, H, D, Dv):
             self._scan_checks(proj, z, out, memory, H, D, Dv)
             if z.shape[1] != H * D or z.shape[0] < proj.shape[0]:
                 raise KernelError(f"gated_linear_scan wants decay logits [{proj.shape[0]}, {H * D}], got {tuple(z.shape)}")

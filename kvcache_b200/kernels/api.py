@@ -64,14 +64,22 @@ def _dtype_code(t: torch.dtype) -> int:
     raise KernelError(f"kernels take float32 or bfloat16 tensors, got {t}")
 
 
-def _ptr(t: Optional[torch.Tensor]) -> _c_void_p:
-    if t is None:
-        return _c_void_p(0)
-    if not t.is_contiguous():
-        raise KernelError("kernels take contiguous tensors")
-    if not t.is_cuda:
-        raise KernelError("kernels take tensors on the device; a host tensor's address means nothing there")
-    return _c_void_p(t.data_ptr())
+# Launchers are called through csrc/host_call.cpp: `_ptr` asks a tensor for its address (it has to be contiguous and on the device), and a
+# pointer parameter takes such an address.  With ctypes in that place a layer of 48 single tokens took 66 us, now 54, a routed feed-forward
+# over one token 59, now 37.
+def _ptr(t: Optional[torch.Tensor]) -> int:
+    global _ptr
+    _ptr = _host_calls().ptr                                   # from now on the extension's own function
+    return _ptr(t)
+
+
+def _host_calls():
+    extension = build.host_call()
+    extension.set_error(KernelError)
+    return extension
+
+
+_TYPE_LETTERS = {_c_int: "i", _c_float: "f", _c_void_p: "p", _c_longlong: "l"}
 
 
 _RETURN_CODES = {-1: "unsupported dtype", -2: "unsupported shape", -3: "misaligned operand", -4: "size beyond the kernel's limit"}
@@ -284,7 +292,7 @@ class _Library:
 
     def __getattr__(self, name: str):
         if self._lib is None:
-            lib = build.load_module(self.module, self.variant, self.flags)
+            lib, calls = build.load_module(self.module, self.variant, self.flags), _host_calls()
             for fname, argtypes in _SIGNATURES[self.module].items():
                 try:
                     fn = getattr(lib, fname)
@@ -292,10 +300,11 @@ class _Library:
                     if fname in _OPTIONAL:
                         continue              # a variant compiled for a size that has no such entry point
                     raise
-                fn.argtypes = argtypes
-                fn.restype = _c_int
+                address = ctypes.cast(fn, _c_void_p).value
+                setattr(self, fname, calls.Call(address, "".join(_TYPE_LETTERS[t] for t in argtypes), fname))
             self._lib = lib
-        return getattr(self._lib, name)
+            return getattr(self, name)
+        raise AttributeError(f"module '{self.module}' has no entry point '{name}'")
 
 
 class CudaKernels(KernelSet):
@@ -389,7 +398,7 @@ class CudaKernels(KernelSet):
         self.error_word = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.launches = 0
         self.launch_counts: Counter = Counter()      # launches by kernel, as issued from the host (a replayed graph adds none)
-        self._pinned_stream: Optional[_c_void_p] = None
+        self._pinned_stream: Optional[int] = None
         self._tma_cluster_capacity: Dict[tuple, int] = {}
         self._timing = None
         self._attention_planner: Optional[PagedAttentionPlanner] = None
@@ -400,16 +409,16 @@ class CudaKernels(KernelSet):
         self.launches += 1
         self.launch_counts[kernel] += 1
 
-    def _stream(self) -> _c_void_p:
+    def _stream(self) -> int:
         if self._pinned_stream is not None:
             return self._pinned_stream
-        return _c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return torch.cuda.current_stream(self.device).cuda_stream
 
     @contextlib.contextmanager
     def on_current_stream(self):
         """Within the block every launch goes to the stream that is current now (asked for once, not per launch)."""
         saved = self._pinned_stream
-        self._pinned_stream = _c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        self._pinned_stream = torch.cuda.current_stream(self.device).cuda_stream
         try:
             yield
         finally:
@@ -768,7 +777,7 @@ class CudaKernels(KernelSet):
         if out.dtype == torch.bfloat16 and M <= 16 and self._skinny(x.dtype, M, K, N):
             self._count("gemm_skinny")
             _ptr(out)                                        # a contiguous tensor on the device, as for every operand
-            _check(self._gemm_skinny.kvb_gemm_skinny_unary(self.ACTIVATIONS[kind], _ptr(x), _ptr(w), _c_void_p(out.data_ptr() + 2 * out_col),
+            _check(self._gemm_skinny.kvb_gemm_skinny_unary(self.ACTIVATIONS[kind], _ptr(x), _ptr(w), out.data_ptr() + 2 * out_col,
                                                            out.shape[1], M, N, K, self._stream()), "linear_act (skinny)")
             return
         if out_col == 0 and out.shape[1] == N:
@@ -1130,7 +1139,7 @@ class CudaKernels(KernelSet):
         if g is not None and (g.shape[0] != T or col + (H if gate_per_head else H * os_) > g.shape[1] or g.dtype != x.dtype):
             raise KernelError("head_linear: the gate does not fit")
         self._count("head_linear")
-        x_first = _c_void_p(x.data_ptr() + x_col * x.element_size()) if x_col else _ptr(x)
+        x_first = x.data_ptr() + x_col * x.element_size() if x_col else _ptr(x)
         _ptr(x)                                                    # the checks of a device tensor
         _check(self._latent.kvb_head_linear(
             _dtype_code(x.dtype), x_first, xs, x.shape[1], _ptr(w), _ptr(out), os_, T, N, K, H, _ptr(g), 0 if g is None else g.shape[1],
@@ -1326,7 +1335,7 @@ class CudaKernels(KernelSet):
         if base is None or g.dtype != torch.float32 or g.shape[0] != T or not 0 <= col < g.shape[1]:
             raise KernelError("routed_experts: the base's gate is one float32 logit per row of a base")
         _ptr(g)                                                    # the checks of a device tensor
-        _check(self._moe.kvb_routed_combine_gated(code, _ptr(y), _ptr(place), _ptr(share), _ptr(base), _c_void_p(g.data_ptr() + 4 * col),
+        _check(self._moe.kvb_routed_combine_gated(code, _ptr(y), _ptr(place), _ptr(share), _ptr(base), g.data_ptr() + 4 * col,
                                                   g.shape[1], _ptr(out), T, top, H, stream), "routed_combine")
 
     def _routed_general(self, x, w_up, w_down, chosen, share, out, act: int, limit: float, base, ws, base_gate=None) -> None:
@@ -1509,7 +1518,7 @@ class CudaKernels(KernelSet):
         if held == chunks < 1 << 20 and workspace is not None:
             runs = self._chunk_runs(mode, T, S, walkers)
             if runs > S:
-                run_chunks = max(self.CHUNK_RUN_MIN, -(-(T // 16) // runs))
+                run_chunks = min(2047, max(self.CHUNK_RUN_MIN, -(-(T // 16) // runs)))      # what the bits above `held` hold
                 floats += (T // (16 * run_chunks) + S) * H * (D * Dv + -(-D // 64) * 64)
                 self.launches += 2
         records = (torch.empty(floats, dtype=torch.float32, device=rows.device) if workspace is None else

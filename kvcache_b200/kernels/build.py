@@ -10,21 +10,33 @@ compiler or a failed build raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
 import tempfile
 import threading
 import time
-from typing import Dict, Iterable, List, Optional, Sequence
+from typing import Any, Dict, Iterable, List, Optional, Sequence
 
 CSRC_DIR = os.path.normpath(os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "csrc"))
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 BASE_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-shared"]
 
-# module name -> (source file, headers it includes, extra flags, extra link libraries)
+def _host_flags() -> List[str]:
+    """What a source that speaks to Python and torch is compiled with; torch's version is part of its digest."""
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    return [f"-DKVB_TORCH_{re.sub('[^0-9A-Za-z]', '_', torch.__version__)}", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-I" + sysconfig.get_paths()["include"], f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-L{root}/lib",
+            "-ltorch_python", "-ltorch_cpu", "-lc10"]
+
+
+# module name -> (source file, headers it includes, extra flags or a function that returns them, extra link libraries)
 MODULES: Dict[str, dict] = {
     "elementwise": {"src": "elementwise.cu", "deps": ["common.cuh"]},
     "rope_append": {"src": "rope_append.cu", "deps": ["common.cuh"]},
@@ -47,6 +59,8 @@ MODULES: Dict[str, dict] = {
     "gemm_wstream": {"src": "gemm_wstream.cu", "deps": ["common.cuh", "tc_common.cuh"]},
     # What barrier waits, votes, MMA issue and page copies cost on this GPU (python -m kvcache_b200.kernels.primitive_costs).
     "primitive_costs": {"src": "primitive_costs.cu", "deps": ["common.cuh", "tc_common.cuh"]},
+    # Calls of all these from Python (a CPython extension; see `host_call`).
+    "host_call": {"src": "host_call.cpp", "flags": _host_flags},
     # One wait that cannot end, with a short poll limit: shows that a stalled wait reaches the host as an error bit.
     "wait_probe": {"src": "wait_probe.cu", "deps": ["common.cuh", "tc_common.cuh"], "flags": ["-DKVB_SPIN_LIMIT=4096"]},
 }
@@ -57,6 +71,7 @@ DEFAULT_VARIANTS = {"attention_flash": [("d64", ["-DKVB_HEAD_DIM=64"]), ("d128",
                                         ("x64", ["-DKVB_HEAD_DIM=64", "-DKVB_EXPANDED=1"]), ("x128", ["-DKVB_HEAD_DIM=128", "-DKVB_EXPANDED=1"])]}
 
 _loaded: Dict[str, ctypes.CDLL] = {}
+_extensions: Dict[str, Any] = {}
 _lock = threading.Lock()
 _dir_lock = threading.Lock()
 
@@ -113,6 +128,16 @@ def _choose_build_dir() -> str:
     raise BuildError(f"no writable folder for compiled kernels (tried {in_tree} and {fallback})")
 
 
+def _flags(module: str) -> List[str]:
+    flags = MODULES[module].get("flags", [])
+    return list(flags() if callable(flags) else flags)
+
+
+@functools.lru_cache(maxsize=None)
+def _own_flags(module: str) -> Sequence[str]:
+    return tuple(_flags(module))
+
+
 def _digest(module: str, extra_flags: Sequence[str]) -> str:
     info = MODULES[module]
     h = hashlib.sha256()
@@ -120,7 +145,7 @@ def _digest(module: str, extra_flags: Sequence[str]) -> str:
         with open(os.path.join(CSRC_DIR, name), "rb") as fh:
             h.update(name.encode())
             h.update(fh.read())
-    h.update(" ".join([*ARCH_FLAGS, *BASE_FLAGS, *info.get("flags", []), *extra_flags]).encode())
+    h.update(" ".join([*ARCH_FLAGS, *BASE_FLAGS, *_own_flags(module), *extra_flags]).encode())
     return h.hexdigest()[:16]
 
 
@@ -151,8 +176,8 @@ def compile_module(module: str, variant: str = "", extra_flags: Sequence[str] = 
     info = MODULES[module]
     out = library_path(module, variant, extra_flags)
     tmp = f"{out}.{os.getpid()}.tmp"
-    cmd = [find_nvcc(), *ARCH_FLAGS, *BASE_FLAGS, *info.get("flags", []), *extra_flags,
-           "-I", CSRC_DIR, "-o", tmp, os.path.join(CSRC_DIR, info["src"]), *info.get("libs", [])]
+    cmd = [find_nvcc(), *ARCH_FLAGS, *BASE_FLAGS, *extra_flags,
+           "-I", CSRC_DIR, "-o", tmp, os.path.join(CSRC_DIR, info["src"]), *_own_flags(module), *info.get("libs", [])]
     _log(f"compiling {info['src']}{(' [' + variant + ']') if variant else ''} for sm_100a ...")
     start = time.time()
     proc = subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
@@ -191,6 +216,21 @@ def load_module(module: str, variant: str = "", extra_flags: Sequence[str] = ())
             lib = ctypes.CDLL(compile_module(module, variant, extra_flags))
             _loaded[key] = lib
         return lib
+
+
+def host_call():
+    """The extension that calls the launchers (csrc/host_call.cpp)."""
+    with _lock:
+        if "host_call" not in _extensions:
+            import importlib.machinery
+            import importlib.util
+            import torch  # noqa: F401  (the libraries the extension is linked with)
+            loader = importlib.machinery.ExtensionFileLoader("kvb200_host_call", compile_module("host_call"))
+            spec = importlib.util.spec_from_loader("kvb200_host_call", loader)
+            module = importlib.util.module_from_spec(spec)
+            loader.exec_module(module)
+            _extensions["host_call"] = module
+        return _extensions["host_call"]
 
 
 def build_all(modules: Optional[Iterable[str]] = None, jobs: int = 0) -> List[str]:

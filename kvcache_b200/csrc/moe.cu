@@ -20,6 +20,9 @@
 
 // One warp per row.  Ties go to the lower expert index.
 // `over_all`: weights are exp(z - max) / sum over ALL experts (not renormalised over the chosen).
+// PER: experts a lane looks at, 1 (up to 32 experts), 4 or 32: with 32 for any number the step took 6.5 us (2,048 rows of 16
+// experts) and 12.4 us (32 experts), most of it over numbers that were not there; it takes 4.1 and 9.2 us.
+template <int PER>
 __global__ void route_top_kernel(const float* __restrict__ logits, int* __restrict__ chosen, float* __restrict__ share, int T,
                                  int E, int top, int over_all) {
     pdl_wait();
@@ -27,7 +30,6 @@ __global__ void route_top_kernel(const float* __restrict__ logits, int* __restri
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= T) return;
-    constexpr int PER = MOE_MAX_EXPERTS / 32;
     float z[PER];
 #pragma unroll
     for (int c = 0; c < PER; ++c) {
@@ -80,7 +82,8 @@ static int launch_route_top(const float* logits, int* chosen, float* share, int 
     if (T <= 0) return KVB_OK;
     if (E < 1 || E > MOE_MAX_EXPERTS || top < 1 || top > E) return KVB_ERR_SHAPE;
     const int warps = 4;
-    kvb_launch(route_top_kernel, dim3((T + warps - 1) / warps), dim3(32 * warps), 0, stream, logits, chosen, share, T, E, top, over_all);
+    auto kernel = E <= 32 ? route_top_kernel<1> : E <= 128 ? route_top_kernel<4> : route_top_kernel<MOE_MAX_EXPERTS / 32>;
+    kvb_launch(kernel, dim3((T + warps - 1) / warps), dim3(32 * warps), 0, stream, logits, chosen, share, T, E, top, over_all);
     return kvb_launch_status();
 }
 

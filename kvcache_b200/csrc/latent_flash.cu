@@ -630,8 +630,12 @@ static int launch(const bf16* q, bf16* out, const bf16* k_pages, const int* bloc
     return kvb_launch_status();
 }
 
-// Whether the kernel for tiles of 16 rows takes these sizes: every row on 16 bytes, Q's sixteens in registers.
-static bool rows16_fits(int Dk, int Dv, const void* k_pages) { return Dk <= 576 && Dv <= Dk && !((uintptr_t)k_pages & 15); }
+// Whether an instance of the kernel for tiles of 16 rows takes these sizes: every row on 16 bytes, Q's sixteens in registers, and as many
+// value columns as the instance of that key size has accumulators for.  Other sizes go to the kernel above.
+static bool rows16_fits(int Dk, int Dv, const void* k_pages) {
+    const int most = Dk <= 160 ? 128 : Dk <= 320 ? 256 : 512;
+    return Dk <= 576 && Dv <= Dk && Dv <= most && !((uintptr_t)k_pages & 15);
+}
 
 template <int NV, int KS, int STAGES, int BLOCKS>
 static int launch_rows16(const bf16* q, bf16* out, const bf16* k_pages, const int* block_table, int table_stride, const int* items,

@@ -20,12 +20,13 @@ def kernels():
     return CudaKernels(DEV)
 
 
-@pytest.mark.parametrize("window", [None, 70])
-@pytest.mark.parametrize("H,Dk,Dv", [(16, 8, 8), (2, 16, 4), (1, 160, 128), (5, 168, 64), (14, 320, 256), (16, 328, 300), (16, 576, 512), (3, 576, 60), (2, 584, 512)])
-def test_single_tokens_over_shared_key_rows(kernels, H, Dk, Dv, window):
+STEPS = ([(63, 1), (64, 1), (0, 1), (191, 1), (700, 1)], [(2000, 1)])
+
+
+def _compare(kernels, H, Dk, Dv, window, steps=STEPS):
     from kvcache_b200.engine.workspace import Workspace
     from kvcache_b200.parts.base import StepPlan
-    for segments in ([(63, 1), (64, 1), (0, 1), (191, 1), (700, 1)], [(2000, 1)]):
+    for segments in steps:
         batch, kv = paged_scenario(segments, num_kv_heads=1, head_dim=Dk, page_size=16, dtype=torch.bfloat16, device="cpu", seed=8, window=window)
         planner = kernels.latent_attention_planner(H, Dk, Dv, window)
         arrays, counts = planner.plan(np.asarray([s for s, _ in segments]), np.asarray([n for _, n in segments]))
@@ -43,3 +44,16 @@ def test_single_tokens_over_shared_key_rows(kernels, H, Dk, Dv, window):
             kernels.latent_attention(q.to(DEV), batch_to(batch, DEV), held, got, H, Dv, Dk ** -0.5, Workspace(DEV), sink=None if sink is None else sink.to(DEV))
             kernels.check_errors()
             assert_close(got, ref, TOL)
+
+
+@pytest.mark.parametrize("window", [None, 70])
+@pytest.mark.parametrize("H,Dk,Dv", [(16, 8, 8), (2, 16, 4), (1, 160, 128), (5, 168, 64), (14, 320, 256), (16, 328, 300), (16, 576, 512), (3, 576, 60), (2, 584, 512)])
+def test_single_tokens_over_shared_key_rows(kernels, H, Dk, Dv, window):
+    _compare(kernels, H, Dk, Dv, window)
+
+
+@pytest.mark.parametrize("H,Dk,Dv", [(14, 152, 132), (16, 160, 144), (3, 160, 160), (16, 264, 260), (5, 304, 272), (16, 320, 288), (2, 320, 320)])
+def test_values_wider_than_an_instance_of_their_key_size(kernels, H, Dk, Dv):
+    """More value columns than the instance that their key size leads to adds up: 128 for keys of up to 160 numbers, 256 up to 320.  Cut into
+    several splits, and more requests than the plan wants blocks, a single one."""
+    _compare(kernels, H, Dk, Dv, None, (*STEPS, [(17 * i % 90, 1) for i in range(2 * 148 + 4)]))

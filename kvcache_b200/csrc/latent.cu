@@ -172,14 +172,15 @@ KVB_API int kvb_latent_norm_rope_append(int dtype, const void* proj, int P, int 
 // ---------------------------------------------------------------------------------------------------------------
 // What attention over an expanded latent starts from, in one launch.  The first 32 * n_blocks blocks copy four cached rows each:
 // the keys of a list of blocks of 128 (segment, first key) out of the pages, the latent into lat [128 n_blocks, C], the rotated part
-// into rot [128 n_blocks, 64]; rows beyond the segment's keys and columns beyond the rotated part are zeros.  The others rotate
+// into rot [128 n_blocks, 64]; rows beyond the segment's keys, rows before the first key that a window of `window` keys leaves its first
+// row (their pages may have been given back) and columns beyond the rotated part are zeros.  The others rotate
 // the queries where they lie: the last `rot_dim` numbers of each head of q (rows of `q_ld`, heads of dim + rot_dim), by the row's position.
 // Bound by launch and latency: 2,048 keys of 576 numbers and 16 heads of 64 rotated numbers are 13 MB, 2 us of them.  VEC pairs a
 // thread: eight, 16 bytes a load, where the halves of the rotated part are steps of eight (2,048 rows of 16 heads: 10.8 us with one a thread, 4.4 with eight).
 template <int VEC>
 __global__ void __launch_bounds__(128) latent_expand_prepare_kernel(
     const bf16* __restrict__ k_pages, const int* __restrict__ block_table, int table_stride, int page_size, const int* __restrict__ blocks,
-    int n_blocks, const int* __restrict__ seg_kv_len, int C, int rot_dim, bf16* __restrict__ lat, bf16* __restrict__ rot, bf16* __restrict__ q,
+    int n_blocks, const int* __restrict__ seg_q_len, const int* __restrict__ seg_kv_len, int window, int C, int rot_dim, bf16* __restrict__ lat, bf16* __restrict__ rot, bf16* __restrict__ q,
     int q_ld, int H, int dim, const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot_half, int table_len,
     const int* __restrict__ positions, int T, int* __restrict__ err) {
     const int copies = 32 * n_blocks, tid = threadIdx.x;
@@ -187,7 +188,8 @@ __global__ void __launch_bounds__(128) latent_expand_prepare_kernel(
         const int row = 4 * blockIdx.x + (tid >> 5), lane = tid & 31;      // a warp a row
         const int seg = blocks[2 * (row >> 7)], key = blocks[2 * (row >> 7) + 1] + (row & 127);
         const bf16* src = nullptr;
-        if (key < seg_kv_len[seg]) {
+        const int kv_len = seg_kv_len[seg];
+        if (key < kv_len && key >= first_seen_key(kv_len - seg_q_len[seg], window)) {
             const int page = block_table[(size_t)seg * table_stride + key / page_size];
             if (page < 0) {
                 if (lane == 0) atomicOr(err, KVB_DEV_BAD_PAGE);
@@ -237,20 +239,20 @@ __global__ void __launch_bounds__(128) latent_expand_prepare_kernel(
     }
 }
 
-// blocks: int32 [n_blocks, 2] (segment, first key of 128).  Latents and rotated parts in steps of eight numbers, rows on 16 bytes.
+// blocks: int32 [n_blocks, 2] (segment, first key of 128); window: keys that a row sees (0: all).  Latents and rotated parts in steps of eight numbers, rows on 16 bytes.
 KVB_API int kvb_latent_expand_prepare(const void* k_pages, const int* block_table, int table_stride, int page_size, const int* blocks, int n_blocks,
-                                      const int* seg_kv_len, int C, int rot_dim, void* lat, void* rot, void* q, int q_ld, int H, int dim,
+                                      const int* seg_q_len, const int* seg_kv_len, int window, int C, int rot_dim, void* lat, void* rot, void* q, int q_ld, int H, int dim,
                                       const float* cos_t, const float* sin_t, int rot_half, int table_len, const int* positions, int T,
                                       int* err, cudaStream_t stream) {
     if (T <= 0 || n_blocks <= 0) return KVB_OK;
     if (C < 8 || C % 8 != 0 || rot_dim < 8 || rot_dim > 64 || rot_dim % 8 != 0 || rot_half < 0 || 2 * rot_half > rot_dim || page_size < 1 ||
-        H < 1 || H * (dim + rot_dim) > q_ld || (long long)T * H * rot_half > 0x7fffff00LL)
+        window < 0 || H < 1 || H * (dim + rot_dim) > q_ld || (long long)T * H * rot_half > 0x7fffff00LL)
         return KVB_ERR_SHAPE;
     if (((uintptr_t)k_pages | (uintptr_t)lat | (uintptr_t)rot) & 15) return KVB_ERR_ALIGN;
     const bool eights = rot_half % 8 == 0 && dim % 8 == 0 && q_ld % 8 == 0 && !((uintptr_t)q & 15);
     const int turns = (T * H * rot_half / (eights ? 8 : 1) + 127) / 128;
     kvb_launch(eights ? latent_expand_prepare_kernel<8> : latent_expand_prepare_kernel<1>, dim3(32 * n_blocks + turns), dim3(128), 0, stream, (const bf16*)k_pages, block_table, table_stride,
-               page_size, blocks, n_blocks, seg_kv_len, C, rot_dim, (bf16*)lat, (bf16*)rot, (bf16*)q, q_ld, H, dim, cos_t, sin_t, rot_half,
+               page_size, blocks, n_blocks, seg_q_len, seg_kv_len, window, C, rot_dim, (bf16*)lat, (bf16*)rot, (bf16*)q, q_ld, H, dim, cos_t, sin_t, rot_half,
                table_len, positions, T, err);
     return kvb_launch_status();
 }

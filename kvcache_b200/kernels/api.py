@@ -178,9 +178,9 @@ _SIGNATURES = {
     "latent": {
         "kvb_norm_add_rmsnorm": [_c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_float, _c_void_p, _c_float, _c_void_p, _c_void_p,
                                  _c_void_p, _c_int, _c_int, _c_void_p],
-        "kvb_latent_expand_prepare": [_c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p,
-                                      _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p,
-                                      _c_void_p],
+        "kvb_latent_expand_prepare": [_c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
+                                      _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p,
+                                      _c_int, _c_void_p, _c_void_p],
         "kvb_latent_norm_rope_append": [_c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_float,
                                         _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int,
                                         _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p],
@@ -1177,7 +1177,7 @@ class CudaKernels(KernelSet):
         self._count("latent_expand_prepare")
         _check(self._latent.kvb_latent_expand_prepare(
             _ptr(kv.k_pages), _ptr(kv.block_table), kv.block_table.shape[1], kv.page_size, _ptr(plan.arrays["blocks"]), blocks,
-            _ptr(batch.seg_kv_len), C, rot_dim, _ptr(lat), _ptr(rot), _ptr(q), q.shape[1], H, dim, _ptr(cos), _ptr(sin), cos.shape[1],
+            _ptr(batch.seg_q_len), _ptr(batch.seg_kv_len), int(window or 0), C, rot_dim, _ptr(lat), _ptr(rot), _ptr(q), q.shape[1], H, dim, _ptr(cos), _ptr(sin), cos.shape[1],
             cos.shape[0], _ptr(batch.positions), T, _ptr(self.error_word), self._stream()), "latent_expand_prepare")
         self._count("gemm_tcgen05")
         _check(self._gemm_tc.kvb_gemm_tcgen05(_dtype_code(both.dtype), 0, _ptr(lat), _ptr(w_ukv), None, _ptr(both), rows, 2 * H * dim, C,

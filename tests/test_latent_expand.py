@@ -40,6 +40,9 @@ CASES = [
     ([(130, 700)], 4, 128, 48, 64, 64, 24, None, False, False),
     ([(900, 500), (5, 90)], 2, 64, 64, 72, 16, 0, 200, True, False),
     ([(300, 257)], 3, 128, 32, 128, 16, 8, 1, False, True),
+    # the first key that is seen lies within a block of 128, and the pages before it have been given back
+    ([(1000, 300), (900, 64)], 2, 64, 32, 64, 16, 0, 200, False, False),
+    ([(2048, 100), (77, 130)], 3, 128, 16, 64, 8, 0, 1000, True, False),
     ([(0, 2000)], 14, 64, 32, 256, 16, 0, None, False, False),        # many pieces: streams divided and added up
 ]
 
@@ -76,7 +79,8 @@ def test_expanded_latent_attention(case):
         L = start + n
         pages = kv.block_table[i, :-(-L // page)].long()
         rows = kv.k_pages[pages, 0].reshape(-1, C + R)[:L].double()
-        held[pages, 0] |= (torch.arange(len(pages) * page) < L).view(-1, page)
+        at_key = torch.arange(len(pages) * page)
+        held[pages, 0] |= ((at_key < L) & (at_key >= (max(0, start - window + 1) if window else 0))).view(-1, page)
         keys = torch.cat([(rows[:, :C] @ w[:H * dim].double().t()).view(L, H, dim), rows[:, None, C:].expand(L, H, R)], dim=-1)
         values = (rows[:, :C] @ w[H * dim:].double().t()).view(L, H, dim)
         pos, j = start + torch.arange(n)[:, None], torch.arange(L)[None]
@@ -90,10 +94,10 @@ def test_expanded_latent_attention(case):
     sig = torch.sigmoid(gate[:, 8:8 + (H if per_head else H * dim)].double())
     want = (want * (sig[:, :, None] if per_head else sig.view(T, H, dim))).reshape(T, H * dim)
 
-    kv.k_pages[~held] = float("nan")                                   # rows that no request holds must not be used
+    kv.k_pages[~held] = float("nan")                                   # rows that no request holds, or sees any more, must not be used
     if window:
         for i, (start, _) in enumerate(segments):
-            kv.block_table[i, :max(0, start - window + 1) // 128 * 128 // page] = -1
+            kv.block_table[i, :max(0, start - window + 1) // page] = -1        # as the cache gives pages back
     planner = kernels.latent_expand_planner(dim, dim, R, C, window)
     arrays, counts = planner.plan(np.asarray([a for a, _ in segments]), np.asarray([n for _, n in segments]))
     place = lambda t: None if t is None else t.to(DEV)

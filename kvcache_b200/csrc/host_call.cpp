@@ -13,6 +13,7 @@
 // leaves every parameter where the launcher looks for it.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <climits>
@@ -40,8 +41,10 @@ struct Call {
     PyObject* name;
 };
 
-// The address of a contiguous tensor on the device; false with an exception set.
+// The address of a contiguous tensor on the device; false with an exception set.  Every question to the tensor may throw (a layout
+// without strides, a subclass that answers in Python, a tensor without storage).
 bool address_of(PyObject* obj, W& out) {
+    HANDLE_TH_ERRORS
     const at::Tensor& t = THPVariable_Unpack(obj);
     if (!t.is_contiguous()) {
         PyErr_SetString(kernel_error ? kernel_error : PyExc_RuntimeError, "kernels take contiguous tensors");
@@ -52,13 +55,9 @@ bool address_of(PyObject* obj, W& out) {
                         "kernels take tensors on the device; a host tensor's address means nothing there");
         return false;
     }
-    try {
-        out = reinterpret_cast<W>(t.data_ptr());
-    } catch (const std::exception& e) {    // tensors without storage
-        PyErr_SetString(PyExc_RuntimeError, e.what());
-        return false;
-    }
+    out = reinterpret_cast<W>(t.data_ptr());
     return true;
+    END_HANDLE_TH_ERRORS_RET(false)
 }
 
 bool pointer_of(PyObject* obj, W& out) {

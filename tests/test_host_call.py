@@ -1,7 +1,9 @@
 """The extension that calls the launchers (csrc/host_call.cpp): what it takes for a parameter, what it refuses, and that every parameter
 arrives where the launcher looks for it - integers beyond the registers, floats between them, whole 64-bit numbers."""
 import ctypes
+import os
 import subprocess
+import sys
 
 import pytest
 import torch
@@ -64,3 +66,37 @@ def test_tensors_that_a_launcher_cannot_take(calls, library):
         calls.Call(1, "p" * 41, "too many")
     with pytest.raises(ValueError):
         calls.Call(1, "x", "unknown")
+
+
+class _AnswersInPython(torch.Tensor):
+    """A tensor whose questions are answered in Python, by an exception."""
+    @staticmethod
+    def __new__(cls):
+        return torch.Tensor._make_wrapper_subclass(cls, (4,), dispatch_sizes_strides_policy="strides")
+
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        raise ValueError("not to be asked")
+
+
+QUESTIONS = """
+import torch, warnings
+warnings.simplefilter("ignore")
+from kvcache_b200.kernels import api
+from test_host_call import _AnswersInPython
+call = api._host_calls().Call(1, "p", "never called")
+for make, error in ((lambda: torch.eye(4).to_sparse_csr(), RuntimeError), (_AnswersInPython, ValueError)):
+    for ask in (api._ptr, call):
+        try:
+            ask(make())
+        except error:
+            print("raised")
+"""
+
+
+def test_tensors_whose_questions_throw():
+    """An exception in Python for each, not the end of the process (a child, since an exception that leaves C code ends it)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", QUESTIONS], capture_output=True, text=True,
+                          env=dict(os.environ, PYTHONPATH=os.pathsep.join([root, os.path.dirname(os.path.abspath(__file__))])))
+    assert done.returncode == 0 and done.stdout.split() == ["raised"] * 4, done.stderr[-500:]

@@ -36,7 +36,16 @@ def _host_flags() -> List[str]:
             "-ltorch_python", "-ltorch_cpu", "-lc10"]
 
 
-# module name -> (source file, headers it includes, extra flags or a function that returns them, extra link libraries)
+def _host_headers() -> List[str]:
+    """Headers of Python and torch that such a source needs, which an installation may leave out."""
+    import sysconfig
+    import torch
+    return [os.path.join(sysconfig.get_paths()["include"], "Python.h"),
+            os.path.join(os.path.dirname(torch.__file__), "include", "torch", "csrc", "autograd", "python_variable.h")]
+
+
+# module name -> (source file, headers it includes, extra flags or a function that returns them, extra link libraries, a function that
+# names headers of others)
 MODULES: Dict[str, dict] = {
     "elementwise": {"src": "elementwise.cu", "deps": ["common.cuh"]},
     "rope_append": {"src": "rope_append.cu", "deps": ["common.cuh"]},
@@ -60,7 +69,7 @@ MODULES: Dict[str, dict] = {
     # What barrier waits, votes, MMA issue and page copies cost on this GPU (python -m kvcache_b200.kernels.primitive_costs).
     "primitive_costs": {"src": "primitive_costs.cu", "deps": ["common.cuh", "tc_common.cuh"]},
     # Calls of all these from Python (a CPython extension; see `host_call`).
-    "host_call": {"src": "host_call.cpp", "flags": _host_flags},
+    "host_call": {"src": "host_call.cpp", "flags": _host_flags, "needs": _host_headers},
     # One wait that cannot end, with a short poll limit: shows that a stalled wait reaches the host as an error bit.
     "wait_probe": {"src": "wait_probe.cu", "deps": ["common.cuh", "tc_common.cuh"], "flags": ["-DKVB_SPIN_LIMIT=4096"]},
 }
@@ -174,6 +183,9 @@ def compile_module(module: str, variant: str = "", extra_flags: Sequence[str] = 
         if found:
             return found
     info = MODULES[module]
+    for header in info.get("needs", list)():
+        if not os.path.isfile(header):
+            raise BuildError(f"{info['src']} needs {header}, which is not installed (Python's development headers, or those that come with torch)")
     out = library_path(module, variant, extra_flags)
     tmp = f"{out}.{os.getpid()}.tmp"
     cmd = [find_nvcc(), *ARCH_FLAGS, *BASE_FLAGS, *extra_flags,

@@ -100,3 +100,12 @@ def test_tensors_whose_questions_throw():
     done = subprocess.run([sys.executable, "-c", QUESTIONS], capture_output=True, text=True,
                           env=dict(os.environ, PYTHONPATH=os.pathsep.join([root, os.path.dirname(os.path.abspath(__file__))])))
     assert done.returncode == 0 and done.stdout.split() == ["raised"] * 4, done.stderr[-500:]
+
+
+def test_a_missing_header_is_named(monkeypatch, tmp_path):
+    import sysconfig
+    from kvcache_b200.kernels import build
+    paths = dict(sysconfig.get_paths(), include=str(tmp_path))
+    monkeypatch.setattr(sysconfig, "get_paths", lambda: paths)
+    with pytest.raises(build.BuildError, match="Python.h"):
+        build.compile_module("host_call", force=True)

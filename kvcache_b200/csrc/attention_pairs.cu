@@ -30,7 +30,7 @@
 // Work is shared out by key tiles: the streams' tiles, laid end to end, are cut into as many equal runs as there are blocks
 // (one an SM), so that all finish together whatever the lengths.  A stream that a cut divides leaves (m, l, O) of its
 // pieces in scratch, two places a block, and the last piece to finish adds them in order (a ticket per stream and tile).
-// Every mbarrier wait is bounded; on a timeout the error word is set and the block winds down.
+// Every mbarrier wait is bounded; on a timeout the error word is set and the block winds down, the warps of a softmax group together.
 #include "tc_common.cuh"
 
 #ifndef KVB_HEAD_DIM
@@ -124,6 +124,13 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 // lo += v's lower bfloat16, hi += its upper one, in float32.
 __device__ __forceinline__ void add_bf16x2(float& lo, float& hi, uint32_t v) {
     asm("{.reg .b16 x, y; mov.b32 {x, y}, %2; add.rn.f32.bf16 %0, x, %0; add.rn.f32.bf16 %1, y, %1;}" : "+f"(lo), "+f"(hi) : "r"(v));
+}
+// Whether all threads of a tile's four softmax warps say so: named barrier `id`.
+__device__ __forceinline__ bool all_of_tile(int id, bool mine) {
+    uint32_t all;
+    __syncwarp();
+    asm volatile("{.reg .pred p, q; setp.ne.u32 p, %2, 0; bar.red.and.pred q, %1, 128, p; selp.u32 %0, 1, 0, q;}" : "=r"(all) : "r"(id), "r"((uint32_t)mine) : "memory");
+    return all != 0;
 }
 // The lowest `count` bits (none below 0, all from 32).
 __device__ __forceinline__ uint32_t below(int count) { return count >= 32 ? 0xffffffffu : count <= 0 ? 0u : (1u << count) - 1u; }
@@ -624,7 +631,6 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 if (lane == 0) mbar_arrive(&sh.p_ready[wg]);
                 if (!ok) break;
             }
-            if (!ok) break;
             // The blocks whose runs hold a part of what these rows see of the stream.
             const int block0 = x.first / share, block1 = (x.first + hf.limit - 1) / share;
             int* ticket = p.tickets + ((size_t)t * p.Hq + x.index) * 2 + wg;
@@ -632,12 +638,15 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 const bf16* g = p.gate + (size_t)(p.seg_q_start[c.seg] + hf.row0 + row) * p.gate_stride + p.gate_col + (p.gate_per_head ? h : h * D);
                 for (int d = 0; d < (p.gate_per_head ? 1 : D); d += 64) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(g + d));
             }
-            ok = mbar_wait(&sh.o_full[wg], (OWN_P ? s_count - 1 : pieces) & 1);
+            ok = ok && mbar_wait(&sh.o_full[wg], (OWN_P ? s_count - 1 : pieces) & 1);
+            // All four warps have handed over P of this piece, so none still looks at the word of the piece before.
+            if (ok && block0 != block1 && row == 0) sh.ticket[wg] = *reinterpret_cast<volatile int*>(ticket);
+            // The tile's warps give up together: one whose wait ran out comes here as well, and only here do they leave the line of work, so
+            // that none is left alone at one of the barriers below, which have no limit.
+            ok = all_of_tile(1 + wg, ok);
             if (!ok) break;
             ++pieces;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            // All four warps have handed over P of this piece, so none still looks at the word of the piece before.
-            if (block0 != block1 && row == 0) sh.ticket[wg] = *reinterpret_cast<volatile int*>(ticket);
 
             const int q_row0 = p.seg_q_start[c.seg] + hf.row0, q_row = q_row0 + row;
             unsigned char* stage = STAGE_IN_Q ? q_s + wg * Q_BYTES + (warp & 3) * STAGE_BYTES : smem_raw + STAGE_AT + warp * STAGE_BYTES;
@@ -694,7 +703,6 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             } else {
                 auto place_of = [&](int b) -> size_t { return (size_t)(2 * b + (b * share > x.first ? 0 : 1)) * 2 + wg; };
                 // Whether all other pieces have left their sums already: then this one's need not be written down.
-                asm volatile("bar.sync %0, 128;\n" ::"r"(1 + wg) : "memory");       // the tile's four warps
                 bool last = sh.ticket[wg] == block1 - block0;
                 if (!last) {
                     // Leave this piece's (m, l, O), [D / 4][128 rows] of float4, so that a warp's rows make one contiguous store.

@@ -173,6 +173,7 @@ struct Shared {
     uint64_t q_full[2], q_free[2], k_full[KST], k_free[KST], v_full[VST], v_free[VST], s_full[2], s_read[2], p_ready[2], o_full[2], turn[2], top_known[2];
     uint32_t tmem_base;
     int failed;
+    int k_copies, v_copies, q_copies[2];   // tiles asked for, as the copying warp leaves them
     int ticket[2];
     float corr[2][BQ];         // what a row's O is multiplied by before the next P V
     int first[MAX_TILES + 1];  // the line of work - every stream's cost and key tiles, one after the other - before this pair of row tiles
@@ -317,7 +318,7 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // ---- copies: Q of the two tiles of rows, key and value tiles, page by page; lane i copies page i ----
         const int pages = EXPANDED ? 1 : BK >> p.page_shift;
         bool ok = true, waited = false;
-        int count = 0, q_count[2] = {0, 0};
+        int count = 0, k_copies = 0, v_copies = 0, q_count[2] = {0, 0};
         for (int w = w_begin; w < w_end && ok;) {
             while (sh.first[t + 1] <= w) ++t;
             const Tile c = make_tile(p, t);
@@ -349,6 +350,7 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 const int row = EXPANDED ? p.seg_key_row[c.seg] + key_of(j) : page >= 0 ? (page * p.Hkv + x.hk) * p.page_size : -p.page_size;
                 if (count >= KST) ok = mbar_wait(&sh.k_free[ks], ((count / KST) - 1) & 1);
                 if (!ok) break;
+                ++k_copies;
                 if (lane == 0) mbar_expect_tx(&sh.k_full[ks], K_BYTES);
                 __syncwarp();
                 if constexpr (EXPANDED) {
@@ -376,6 +378,7 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 }
                 if (count >= VST) ok = mbar_wait(&sh.v_free[vs], ((count / VST) - 1) & 1);
                 if (!ok) break;
+                ++v_copies;
                 if (lane == 0) mbar_expect_tx(&sh.v_full[vs], V_BYTES);
                 __syncwarp();
                 if constexpr (EXPANDED) {
@@ -388,6 +391,7 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
         }
         if (!ok && lane == 0) { atomicOr(p.err, KVB_DEV_TIMEOUT); sh.failed = 1; }
+        if (lane == 0) { sh.k_copies = k_copies; sh.v_copies = v_copies; sh.q_copies[0] = q_count[0]; sh.q_copies[1] = q_count[1]; }
         __syncwarp();
     } else if (warp == 12 || warp == 14) {
         // ---- products, a warp for each tile of rows.  Every lane waits on the barriers (a wait by one lane and a broadcast
@@ -790,10 +794,11 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
-    if (sh.failed && tid == 0) {      // give copies that may still be in flight a bounded chance to land
-        for (int h = 0; h < 2; ++h) mbar_wait(&sh.q_full[h], 0);
-        for (int s = 0; s < KST; ++s) mbar_wait(&sh.k_full[s], 0);
-        for (int s = 0; s < VST; ++s) mbar_wait(&sh.v_full[s], 0);
+    if (sh.failed && tid == 0) {      // give copies that may still be in flight a bounded chance to land: the last ones into every place
+        for (int h = 0; h < 2; ++h)
+            if (sh.q_copies[h] > 0) mbar_wait(&sh.q_full[h], (sh.q_copies[h] - 1) & 1);
+        for (int c = max(0, sh.k_copies - KST); c < sh.k_copies; ++c) mbar_wait(&sh.k_full[c % KST], (c / KST) & 1);
+        for (int c = max(0, sh.v_copies - VST); c < sh.v_copies; ++c) mbar_wait(&sh.v_full[c % VST], (c / VST) & 1);
     }
     __syncthreads();
     if (warp == 12) {

@@ -437,11 +437,10 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) latent_rows16_kernel(
 #pragma unroll
     for (int nv = 0; nv < NV; ++nv) o[nv][0] = o[nv][1] = o[nv][2] = o[nv][3] = 0.f;
 
-    bool ok = true;
     for (int tile = 0; tile < ntiles; ++tile) {
         const int par = tile & 1;
         const bf16* Kt = Ks + (size_t)(tile % STAGES) * BN * rs;
-        ok = ok && tc::mbar_wait(&full[tile % STAGES], (tile / STAGES) & 1);
+        const bool ok = tc::mbar_wait(&full[tile % STAGES], (tile / STAGES) & 1);
         float s[4][4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) s[c][0] = s[c][1] = s[c][2] = s[c][3] = 0.f;
@@ -468,7 +467,16 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) latent_rows16_kernel(
             top[i] = fmaxf(top[i], __shfl_xor_sync(0xffffffffu, top[i], 2));
             if (t4 == 0) tops[par][g + 8 * i][warp] = top[i];
         }
-        __syncthreads();                                    // ... and all are done with the tile before: its stage may be filled
+        // ... and all are done with the tile before: its stage may be filled.  If anyone's wait has run out nothing more is asked for, and the
+        // copies that are still on their way are waited for, as long again.
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) {
+                atomicOr(err, tc::KVB_DEV_TIMEOUT);
+                for (int c = tile; c < ntiles && c < max(LEAD, tile + STAGES - 1); ++c) tc::mbar_wait(&full[c % STAGES], (c / STAGES) & 1);
+            }
+            __syncthreads();
+            break;
+        }
         const int next = tile + STAGES - 1;
         if (next >= LEAD && next < ntiles) {
             fetch(next, page_next);
@@ -506,8 +514,6 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) latent_rows16_kernel(
             for (int nv = 0; nv < NV; ++nv) mma_bf16(o[nv], p, b[nv][0], b[nv][1]);
         }
     }
-    if (!ok) atomicOr(err, tc::KVB_DEV_TIMEOUT);            // copies that are still asked for have been waited for as long as that
-
     // The rows' sums: over the four lanes of a row, then over the warps in their order.
     __syncthreads();
 #pragma unroll

@@ -42,9 +42,9 @@ struct Call {
 };
 
 // The address of a contiguous tensor on the device; false with an exception set.  Every question to the tensor may throw (a layout
-// without strides, a subclass that answers in Python, a tensor without storage).
-bool address_of(PyObject* obj, W& out) {
-    HANDLE_TH_ERRORS
+// without strides, a subclass that answers in Python, a tensor without storage); torch's own frame for that, HANDLE_TH_ERRORS, also
+// collects warnings, which cost a layer of four launches 3 us.
+bool address_of(PyObject* obj, W& out) try {
     const at::Tensor& t = THPVariable_Unpack(obj);
     if (!t.is_contiguous()) {
         PyErr_SetString(kernel_error ? kernel_error : PyExc_RuntimeError, "kernels take contiguous tensors");
@@ -57,7 +57,9 @@ bool address_of(PyObject* obj, W& out) {
     }
     out = reinterpret_cast<W>(t.data_ptr());
     return true;
-    END_HANDLE_TH_ERRORS_RET(false)
+} catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
+    return false;
 }
 
 bool pointer_of(PyObject* obj, W& out) {

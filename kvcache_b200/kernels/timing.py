@@ -48,6 +48,7 @@ def _attention_bytes(batch, kv, num_heads: int, reach=None) -> int:
 class KernelTiming:
     OPERATORS = ("embed", "add_rmsnorm", "silu_mul", "gate_up_act", "linear", "linear_act", "qkv_rope_append", "rope_append_attention",
                  "paged_attention", "sample", "norm_add_rmsnorm", "latent_norm_rope_append", "head_linear", "latent_attention",
+                 "latent_expanded_attention",
                  "route_top", "route_sigmoid", "routed_experts", "bigram_embed", "head_gate", "head_norm_gate", "gated_linear_scan",
                  "matrix_memory_scan", "token_shift", "activation_", "activation_into", "delta_rule_scan", "lightning_scan",
                  "gated_delta_inputs", "gated_delta_scan", "state_space_inputs", "state_space_scan", "gate_part_norm")
@@ -101,13 +102,17 @@ class KernelTiming:
             return f"head_linear {w.shape[0]}x{w.shape[1]}x{w.shape[2]}", _numel_bytes(w) + _numel_bytes(x) + _numel_bytes(out)
         if name == "latent_attention":
             q, batch, kv, out = args[0], args[1], args[2], args[3]
-            host = batch.host
             window = kwargs.get("window", -1)
-            window = kv.spec.window if window == -1 else window
-            keys = int((host["starts"] + host["counts"]).sum()) if "starts" in host else batch.max_kv_len * batch.num_segments
-            if window and "starts" in host:
-                keys = int(sum(min(int(s + c), window + int(c) - 1) for s, c in zip(host["starts"], host["counts"])))
+            keys = KernelTiming._cached_keys(batch, kv.spec.window if window == -1 else window)
             return name, keys * kv.spec.head_dim * kv.k_pages.element_size() + _numel_bytes(q) + _numel_bytes(out)
+        if name == "latent_expanded_attention":
+            # The cached rows that the step sees, the expansion's weights, queries and gates in, gated heads out; what is expanded on the way is
+            # the operator's own.
+            q, w_ukv, batch, kv, out, H, dim = args[:7]
+            gate_per_head, window = args[12], args[13]
+            rows = q.shape[0] * H * (dim + kv.spec.head_dim - w_ukv.shape[1] + (1 if gate_per_head else dim)) * q.element_size()
+            keys = KernelTiming._cached_keys(batch, window)
+            return name, keys * kv.spec.head_dim * kv.k_pages.element_size() + _numel_bytes(w_ukv) + rows + _numel_bytes(out)
         if name in ("route_top", "route_sigmoid"):
             return name, _numel_bytes(args[0])
         if name == "routed_experts":
@@ -164,6 +169,14 @@ class KernelTiming:
         return name, 0
 
     @staticmethod
+    def _cached_keys(batch, window) -> int:
+        """Keys that any row of the step sees, every request's counted once."""
+        host = batch.host
+        if "starts" not in host:
+            return batch.max_kv_len * batch.num_segments
+        return int(sum(min(int(s + c), window + int(c) - 1) if window else int(s + c) for s, c in zip(host["starts"], host["counts"])))
+
+    @staticmethod
     def _keys_seen(batch, reach: int = 0, keep: int = 0) -> int:
         """Sum over the step's rows of the keys a row sees (its own included): all up to its position, or those of its window
         (and the kept first ones behind it) or chunk."""
@@ -193,6 +206,11 @@ class KernelTiming:
             batch, kv, heads, value_dim = args[1], args[2], args[4], args[5]
             window = kwargs.get("window", -1)
             return 2 * heads * (kv.spec.head_dim + value_dim) * cls._keys_seen(batch, (kv.spec.window if window == -1 else window) or 0)
+        if name == "latent_expanded_attention":
+            w_ukv, batch, kv, heads, dim, window = args[1], args[2], args[3], args[5], args[6], args[13]
+            rot_dim = kv.spec.head_dim - w_ukv.shape[1]
+            return (2 * cls._cached_keys(batch, window) * w_ukv.shape[0] * w_ukv.shape[1]
+                    + 2 * heads * (2 * dim + rot_dim) * cls._keys_seen(batch, window or 0))
         if name == "paged_attention":
             batch, kv, heads = args[1], args[2], args[4]
             reach = kwargs.get("reach")
@@ -245,8 +263,8 @@ class KernelTiming:
             finally:
                 self._depth -= 1
             end.record()
-            if name == "rope_append_attention" and result is False:
-                return result                            # nothing ran: the caller makes the two calls
+            if name in ("rope_append_attention", "latent_expanded_attention") and result is False:
+                return result                            # nothing ran: the caller makes other calls
             self.records.append((label, nbytes, begin, end, self.kernels.launches - launches, flops))
             return result
         return timed

@@ -89,3 +89,30 @@ def test_generation_with_and_without_graphs(tmp_path, kernels, name):
                 rows = plain_kakipel.logits_of(config, weights, prompt + out[:-1])[len(prompt) - 1:]
                 best = rows.max(dim=1).values
                 assert (rows[torch.arange(10), torch.tensor(out)] >= best - 2 * 3e-2 * rows.abs().max(dim=1).values).all()
+
+
+@pytest.mark.parametrize("name", ["karorax", "kakipel"])
+def test_timing_names_the_expanded_attention(tmp_path, kernels, name):
+    """With timing on, a portion's report holds the operator with its launches, bytes and multiply-adds, and a decoded token's does not."""
+    from kvcache_b200.engine.runner import StepEntry
+    runner = make_runner(_folder(tmp_path, name), kernels, dtype="bfloat16", device=DEV, page_size=16, num_pages=96, max_tokens_per_step=256)
+    slot = runner.cache.admit()
+    tokens = random_tokens(211, 201, 4)
+    reports = []
+    for part in (tokens[:200], tokens[200:]):
+        kernels.start_timing(hold_ms=0.0)
+        runner.step([StepEntry(slot, part, [len(part) - 1])])
+        reports.append(kernels.stop_timing())
+    runner.cache.release(slot)
+    kernels.check_errors()
+    layers = KARORAX["layers"] if name == "karorax" else KAKIPEL["layers"]
+    entry = reports[0]["latent_expanded_attention"]
+    assert entry["calls"] == len(layers) and entry["launches"] == 3 * len(layers) and "latent_attention" not in reports[0]
+    assert reports[1]["latent_attention"]["calls"] == len(layers) and "latent_expanded_attention" not in reports[1]
+    flops = nbytes = 0
+    for m in (layer["mixer"] for layer in layers):
+        window, H, dim, rot, rank = m.get("mask", {}).get("size"), m["heads"], m["dim"], m["rot_dim"], m["kv_rank"]
+        seen = sum(min(p + 1, window or p + 1) for p in range(200))
+        flops += 2 * 200 * 2 * H * dim * rank + 2 * H * (2 * dim + rot) * seen
+        nbytes += 2 * (200 * (rank + rot) + 2 * H * dim * rank + 200 * H * (dim + rot + (1 if name == "karorax" else dim)) + 200 * H * dim)
+    assert entry["flops"] == flops and entry["bytes"] == nbytes

@@ -398,16 +398,19 @@ class CudaKernels(KernelSet):
         self.error_word = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.launches = 0
         self.launch_counts: Counter = Counter()      # launches by kernel, as issued from the host (a replayed graph adds none)
+        self.launch_forms: Counter = Counter()       # where one of those names stands for several kernels: launches by kernel
         self._pinned_stream: Optional[int] = None
         self._tma_cluster_capacity: Dict[tuple, int] = {}
         self._timing = None
         self._attention_planner: Optional[PagedAttentionPlanner] = None
 
     # ---- helpers -----------------------------------------------------------
-    def _count(self, kernel: str) -> None:
-        """One launch of `kernel` (while a graph is being recorded: one launch of every later replay)."""
+    def _count(self, kernel: str, form: Optional[str] = None) -> None:
+        """One launch of `kernel` (while a graph is being recorded: one launch of every later replay), which is `form` of it."""
         self.launches += 1
         self.launch_counts[kernel] += 1
+        if form is not None:
+            self.launch_forms[form] += 1
 
     def _stream(self) -> int:
         if self._pinned_stream is not None:
@@ -978,7 +981,7 @@ class CudaKernels(KernelSet):
                 # the kernel leaves zero.
                 scratch = workspace.buffer("attn.pairs_scratch", (4 * self.sm_count * 128 * (D + 2),), torch.float32)
                 tickets = workspace.zeros("attn.pairs_tickets", (2 * pairs * num_heads,), torch.int32)
-                self._count("attention_tc")                   # both tensor-memory kernels go by this name
+                self._count("attention_tc", "attention_pairs")      # both tensor-memory kernels go by the first name
                 _check(pairs_lib.kvb_attention_pairs(
                     _ptr(q), _ptr(out), _ptr(kv.k_pages), _ptr(kv.v_pages), kv.k_pages.shape[0], _ptr(kv.block_table),
                     kv.block_table.shape[1], _ptr(lists["tc_pairs"]), pairs, _ptr(scratch), _ptr(tickets), self.sm_count,
@@ -994,7 +997,7 @@ class CudaKernels(KernelSet):
                 scratch = workspace.buffer("attn.tc_scratch", (units * num_heads * 128 * (D + 2),), torch.float32)
                 # Two counters of the kernel's work queue, then a ticket per (tile, head); the kernel leaves all of them zero.
                 tickets = workspace.zeros("attn.tc_tickets", (2 + max(counts["tc_tiles"], 1) * num_heads,), torch.int32)
-                self._count("attention_tc")
+                self._count("attention_tc", "attention_units")
                 _check(tc.kvb_attention_tc(
                     _ptr(q), _ptr(out), _ptr(kv.k_pages), _ptr(kv.v_pages), kv.k_pages.shape[0], _ptr(kv.block_table),
                     kv.block_table.shape[1], _ptr(lists["tc_units"]), units, _ptr(scratch), _ptr(tickets),

@@ -99,3 +99,15 @@ def test_a_row_whose_maximum_grows_with_every_tile(kernels, request):
         kernels.paged_attention(q.to(DEV), batch_to(batch, DEV), clone_kv(kv, DEV), out, 2, 1.0, Workspace(DEV))
         kernels.check_errors()
         assert_close(out, ref, TOL)
+
+
+def test_launches_of_the_two_kernels_can_be_told_apart(kernels):
+    from kvcache_b200.engine.workspace import Workspace
+    for segments, form in (([(0, 400)], "attention_units"), ([(2048, 1024)], "attention_pairs")):
+        batch, kv = paged_scenario(segments, num_kv_heads=2, head_dim=64, page_size=16, dtype=torch.bfloat16, device=DEV, seed=3)
+        q = torch.randn(batch.num_tokens, 14 * 64, device=DEV).to(torch.bfloat16)
+        before, names = dict(kernels.launch_forms), kernels.launch_counts["attention_tc"]
+        kernels.paged_attention(q, batch, kv, torch.empty_like(q), 14, 0.125, Workspace(DEV))
+        kernels.check_errors()
+        assert {f for f, n in kernels.launch_forms.items() if n > before.get(f, 0)} == {form}
+        assert kernels.launch_counts["attention_tc"] == names + 1

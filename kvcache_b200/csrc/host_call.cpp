@@ -38,6 +38,7 @@ struct Call {
     vectorcallfunc vectorcall;
     Launcher launcher;
     std::string* types;                    // one letter a parameter: p(ointer), i(nt), l(ong long), f(loat)
+    Py_ssize_t required;                   // of so many; those after them are zero where they are left out
     PyObject* name;
 };
 
@@ -82,7 +83,8 @@ PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* k
     Call* c = reinterpret_cast<Call*>(self);
     const Py_ssize_t n = PyVectorcall_NARGS(nargsf);
     if (kwnames && PyTuple_GET_SIZE(kwnames)) return PyErr_Format(PyExc_TypeError, "%U takes no keyword arguments", c->name);
-    if (n != (Py_ssize_t)c->types->size()) return PyErr_Format(PyExc_TypeError, "%U takes %zd arguments, got %zd", c->name, (Py_ssize_t)c->types->size(), n);
+    if (n < c->required || n > (Py_ssize_t)c->types->size())
+        return PyErr_Format(PyExc_TypeError, "%U takes %zd arguments, got %zd", c->name, (Py_ssize_t)c->types->size(), n);
     float f[MAX_FLOATS] = {};
     W w[MAX_OTHERS] = {};
     int nf = 0, nw = 0;
@@ -123,7 +125,12 @@ PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
     void* at = PyLong_AsVoidPtr(address);
     if (!at) return PyErr_Occurred() ? nullptr : PyErr_Format(PyExc_ValueError, "no address for %U", name);
     int floats = 0, others = 0;
+    Py_ssize_t required = -1;              // a '|' stands before the first parameter that may be left out
     for (const char* t = types; *t; ++t) {
+        if (*t == '|' && required < 0) {
+            required = t - types;
+            continue;
+        }
         if (!strchr("pilf", *t)) return PyErr_Format(PyExc_ValueError, "%U: unknown parameter type '%c'", name, *t);
         ++(*t == 'f' ? floats : others);
     }
@@ -133,6 +140,8 @@ PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
     c->vectorcall = call;
     c->launcher = reinterpret_cast<Launcher>(at);
     c->types = new std::string(types);
+    c->required = required < 0 ? (Py_ssize_t)c->types->size() : required;
+    if (required >= 0) c->types->erase(required, 1);
     Py_INCREF(name);
     c->name = name;
     return reinterpret_cast<PyObject*>(c);

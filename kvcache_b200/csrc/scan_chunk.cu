@@ -30,11 +30,13 @@
 // decays 2,048 x 64 x 128 x 64: 278 -> 262.  Level or up to 5 % behind: 2,048 x 14 x 64 under the delta rule (297 -> 311), 48 tokens beside 63
 // single ones under the gated one (46 -> 48), 512 x 28 x 128 x 64 head decays (53 -> 54).  Registers for four blocks an SM: with more, steps of
 // several segments take up to 40 % longer, with the compiler's own choice single ones 5 %.
-// Where heads are few, runs of a segment's chunks are walked at once (modes without Z, further down): 2,048 rows of 7 heads of 64 x 128, records
-// and walk 135 -> 56 us; a layer of 28 heads of 128 x 64 under head decays 277 -> 205 us.  From 256 blocks on the walk has warps enough (64 heads: 431 -> 455).
+// Where heads are few, runs of a long segment's chunks are walked at once (modes without Z, further down): 2,048 rows of 7 heads of 64 x 128, records
+// and walk 147 -> 53 us; of 28 heads of 128 x 64 under head decays 193 -> 133.  From 256 blocks a segment on the walk has warps enough (16 heads of
+// 128 x 256: 280 -> 288), and so have steps of many long segments, which pay a third for it (eight of 1,024 rows of the 7 heads: 160 -> 219).
 // A weight above a diagonal is zero and is multiplied like any other; only in a chunk whose values are not all finite (a vote) are
 // later tokens left out one by one, which takes 15 to 35 % longer where it is done always.
-// A segment's result does not depend on what else the step holds, and a token's not on later ones, whatever they hold (an infinite or undefined
+// A segment's result does not depend on what else the step holds (unless their records are more than is held at once: then no segment is cut
+// into runs), and a token's not on later ones, whatever they hold (an infinite or undefined
 // number of one reaches those after it, as in a walk over tokens).
 // State layout: [slot, head, key channel, value channel].
 #include "common.cuh"
@@ -478,18 +480,43 @@ __device__ __forceinline__ void copy_bulk(float* smem, const float* gmem, uint32
                  ::"r"(tc::smem_u32(smem)), "l"(gmem), "r"(bytes), "r"(tc::smem_u32(bar)) : "memory");
 }
 
-// What a segment's chunks are cut into where several runs of them are walked at once (`chunks` of them each, see launches (2) below).
+// What a segment's chunks are cut into where several runs of them are walked at once (see launches (2) below).  By the segment's own
+// length: what else the step holds changes nothing.
 struct Runs {
-    int chunks;                  // 0: a segment is one run
-    float* starts;               // [runs, H, D, Dv]: the states that runs start from
-    float* decays;               // [runs, H, 64 NI or 1]: the product of a run's decays
+    int wanted;                  // runs a segment is cut into at most (0: every segment is one run)
+    int least, from;             // chunks a run has at least; chunks from which a segment is cut
+    float* starts;               // [runs of segments with several, H, D, Dv]: the states that runs start from
+    float* decays;               // [those runs, H, 64 NI or 1]: the product of a run's decays
 };
-// Run `id` of the step: its segment, its number within it and the segment's count of runs; false beyond the last.
-__device__ __forceinline__ bool find_run(int id, const Segments& seg, const Runs& runs, int& sg, int& k, int& count) {
-    for (sg = 0; sg < seg.count; ++sg) {
-        count = ((seg.q_len[sg] + C - 1) / C + runs.chunks - 1) / runs.chunks;
-        if (id < count) { k = id; return true; }
-        id -= count;
+struct Run {
+    int seg, number, count;      // the run's segment, its number within it and the segment's count of runs
+    int chunks;                  // chunks of each of them but the last
+    int place;                   // among the runs of segments that have several
+};
+__device__ __forceinline__ Run runs_of(int n, const Runs& runs) {
+    const int chunks = (n + C - 1) / C;
+    Run r = {0, 0, chunks > 0, chunks, 0};
+    if (chunks >= runs.from && chunks > 0 && runs.wanted > 1) {
+        r.chunks = max(runs.least, (chunks - 1) / runs.wanted + 1);
+        r.count = (chunks - 1) / r.chunks + 1;
+    }
+    return r;
+}
+// Run `id` of the step, or, with `SEVERAL`, of the segments that have several; false beyond the last.
+template <bool SEVERAL>
+__device__ __forceinline__ bool find_run(int id, const Segments& seg, const Runs& runs, Run& r) {
+    int place = 0;
+    for (int s = 0; s < seg.count; ++s) {
+        r = runs_of(seg.q_len[s], runs);
+        const int mine = SEVERAL && r.count == 1 ? 0 : r.count;
+        if (id < mine) {
+            r.seg = s;
+            r.number = id;
+            r.place = place + id;
+            return true;
+        }
+        id -= mine;
+        place += r.count > 1 ? r.count : 0;
     }
     return false;
 }
@@ -513,23 +540,24 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_walk_kernel
     __shared__ __align__(8) uint64_t full[STAGES];
     const int tid = threadIdx.x, lane = tid & 31, wd = tid >> 5, cg = lane % CG, dg = lane / CG;
     const int h = blockIdx.y;
-    int sg = blockIdx.z, run = 0, run_count = 1;
-    if (runs.chunks > 0 && !find_run(blockIdx.z, seg, runs, sg, run, run_count)) return;
+    Run run = {(int)blockIdx.z, 0, 1, 0, 0};
+    if (runs.wanted > 0 && !find_run<false>(blockIdx.z, seg, runs, run)) return;
+    const int sg = run.seg;
     int n = seg.q_len[sg], r0 = seg.q_start[sg], chunk0 = 0;
     const int slot = seg.slot[sg];
     if (n <= 0) return;
     for (int i = 0; i < sg; ++i) chunk0 += (seg.q_len[i] + C - 1) / C;
     // The segment's chunks from `begin` on that are among the `held` whose records are there.
-    const int begin = max(run * runs.chunks, first - chunk0), d0 = (wd * DG + dg) * TD;
+    const int begin = max(run.number * run.chunks, first - chunk0), d0 = (wd * DG + dg) * TD;
     int chunks = min((n + C - 1) / C, first + held - chunk0) - begin;
-    if (runs.chunks > 0) chunks = min(chunks, runs.chunks);
+    if (run.count > 1) chunks = min(chunks, run.chunks);
     if (chunks <= 0) return;
     n -= begin * C;
     r0 += begin * C;
     chunk0 += begin - first;
 
     float* mem = memory + ((size_t)slot * H + h) * D * Dv;
-    const float* start = runs.chunks > 0 ? runs.starts + ((size_t)blockIdx.z * H + h) * D * Dv : mem;
+    const float* start = run.count > 1 ? runs.starts + ((size_t)run.place * H + h) * D * Dv : mem;
     const int col0 = 16 * blockIdx.x + cg * TC;
     float2 S[TD / 2][TC];                                      // key channels d0 + 2 i and the next
 #pragma unroll
@@ -743,7 +771,7 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_walk_kernel
             for (int i = ci - 1; i < chunks && i < ci + STAGES - 1; ++i) tc::mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
         return;
     }
-    if (run + 1 < run_count) return;                           // the next run has started from this state already
+    if (run.number + 1 < run.count) return;                    // the next run has started from this state already
 #pragma unroll
     for (int i = 0; i < TD / 2; ++i)
 #pragma unroll
@@ -759,7 +787,7 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_walk_kernel
 // A run's end is P S_0 + U, with P the product of its decays and U what its tokens leave of a state of zero.  First U and P of every run but a
 // segment's last (a thread's share of the state as in the walk, no barrier but the one that hands a stage back), then the states that
 // runs start from, one after the other element by element, then the walk with a block for every run.
-// grid (16 value channels, heads, runs).  U of run r goes to place r + 1.
+// grid (16 value channels, heads, runs of segments that have several).  U of run r goes to place r + 1.
 template <int MODE, int NI, int TD, int TC, int STAGES>
 __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_ends_kernel(const Rows in, const Segments seg, const float* __restrict__ records,
                                                                              int held, int H, int D, int Dv, const Runs runs,
@@ -774,12 +802,12 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_ends_kernel
     __shared__ __align__(16) float v_s[2][C][16];
     __shared__ __align__(8) uint64_t full[STAGES];
     const int tid = threadIdx.x, lane = tid & 31, wd = tid >> 5, cg = lane % CG, dg = lane / CG, h = blockIdx.y;
-    int sg, run, run_count;
-    if (!find_run(blockIdx.z, seg, runs, sg, run, run_count) || run + 1 == run_count) return;
-    int r0 = seg.q_start[sg], chunk0 = run * runs.chunks;
-    for (int i = 0; i < sg; ++i) chunk0 += (seg.q_len[i] + C - 1) / C;
-    r0 += run * runs.chunks * C;
-    const int chunks = runs.chunks, d0 = (wd * DG + dg) * TD, col0 = 16 * blockIdx.x + cg * TC, groups = H / in.qk_div;
+    Run run;
+    if (!find_run<true>(blockIdx.z, seg, runs, run) || run.number + 1 == run.count) return;
+    int r0 = seg.q_start[run.seg], chunk0 = run.number * run.chunks;
+    for (int i = 0; i < run.seg; ++i) chunk0 += (seg.q_len[i] + C - 1) / C;
+    r0 += run.number * run.chunks * C;
+    const int chunks = run.chunks, d0 = (wd * DG + dg) * TD, col0 = 16 * blockIdx.x + cg * TC, groups = H / in.qk_div;
     if (tid == 0) {
         for (int i = 0; i < STAGES; ++i) tc::mbar_init(&full[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -888,7 +916,7 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_ends_kernel
             for (int i = ci - 1; i < chunks && i < ci + STAGES - 1; ++i) tc::mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
         return;
     }
-    const size_t place = (size_t)blockIdx.z * H + h;
+    const size_t place = (size_t)run.place * H + h;
     float* end = runs.starts + (place + H) * D * Dv;
 #pragma unroll
     for (int i = 0; i < TD / 2; ++i)
@@ -914,11 +942,13 @@ __global__ void __launch_bounds__(16 * 64 * NI / (TD * TC), 4) chunk_ends_kernel
 template <bool HEAD, int DP>
 __global__ void __launch_bounds__(256) run_starts_kernel(const Segments seg, const float* __restrict__ memory, int H, int D, int Dv, const Runs runs) {
     const int e = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y, sg = blockIdx.z;
-    if (e >= D * Dv || seg.q_len[sg] <= 0) return;
-    auto count_of = [&](int s) { return ((seg.q_len[s] + C - 1) / C + runs.chunks - 1) / runs.chunks; };
+    const int count = runs_of(seg.q_len[sg], runs).count, d = e / Dv;
+    if (e >= D * Dv || count <= 1) return;
     int first = 0;
-    for (int s = 0; s < sg; ++s) first += count_of(s);
-    const int count = count_of(sg), d = e / Dv;
+    for (int s = 0; s < sg; ++s) {
+        const int earlier = runs_of(seg.q_len[s], runs).count;
+        first += earlier > 1 ? earlier : 0;
+    }
     float S = memory[((size_t)seg.slot[sg] * H + h) * D * Dv + e];
     for (int k = 0; k < count; ++k) {
         const size_t place = (size_t)(first + k) * H + h;
@@ -943,7 +973,7 @@ static int launch_walk(const Rows& in, const Segments& seg, const float* records
     return kvb_launch_status();
 }
 
-// The runs' starts: `count` runs at most.
+// The runs' starts: at most `count` runs of segments that have several.
 template <int MODE, int NI, int TD, int TC, int STAGES>
 static int launch_starts(const Rows& in, const Segments& seg, const float* records, int held, const float* memory, int H, int D, int Dv,
                          const Runs& runs, int count, int* err, cudaStream_t stream) {
@@ -977,12 +1007,12 @@ static int run(const Rows& in, const Segments& seg, float* records, int total, i
         // Key and value channels a thread holds: 4 x 2 of 64 (four warps), 8 x 2 of 128 (four warps).  Half of the warps with 4 x 4 or 8 x 2 of 64
         // take 16 to 35 % longer, 4 x 4 and 8 x 4 of 128 8 to 40 %, 8 x 1 30 to 50 %.
         if constexpr (!has_z(MODE))
-            if (runs.chunks > 0) {                             // one run of all chunks then (kvb_chunk_scan)
+            if (runs.wanted > 0) {                             // all chunks are held then (kvb_chunk_scan)
                 rc = launch_starts<MODE, NI, 4 * NI, 2, 2>(in, seg, records, held, memory, H, D, Dv, runs, run_count, err, stream);
                 if (rc != KVB_OK) return rc;
             }
         rc = launch_walk<MODE, NI, 4 * NI, 2, 2>(in, seg, records, first, held, q_scale, memory, out, H, D, Dv, runs,
-                                                 runs.chunks > 0 ? run_count : seg.count, err, stream);
+                                                 runs.wanted > 0 ? run_count + seg.count : seg.count, err, stream);
         if (rc != KVB_OK) return rc;
     }
     return KVB_OK;
@@ -1001,7 +1031,7 @@ static bool rows_fit(int mode, const Rows& in, int H, int G, int D, int Dv) {
 
 template <int MODE>
 static int run(const Rows& in, const Segments& seg, float* records, int held, float q_scale, float* memory, float* out, int T, int H,
-               int G, int D, int Dv, int run_chunks, float* starts, int* err, cudaStream_t stream) {
+               int G, int D, int Dv, Runs runs, int run_count, int* err, cudaStream_t stream) {
     if (H < 1 || G < 1 || H % G || D < 1 || Dv < 1 || !rows_fit(MODE, in, H, G, D, Dv)) return KVB_ERR_SHAPE;
     if (seg.count <= 0 || T <= 0) return KVB_OK;
     if (records == nullptr) return KVB_ERR_SHAPE;
@@ -1010,12 +1040,12 @@ static int run(const Rows& in, const Segments& seg, float* records, int held, fl
     if (MODE == CHUNK_CHANNEL_DECAY && Dv > 512) return KVB_ERR_LIMIT;      // as the other forms of this scan
     const int total = T / C + seg.count;                       // no step has more chunks than this
     held = min(held, total);
-    if (run_chunks < 0 || (run_chunks > 0 && (has_z(MODE) || held < total || !starts))) return KVB_ERR_SHAPE;
-    const int count = run_chunks > 0 ? T / (C * run_chunks) + seg.count : 0;   // no step has more runs than this
-    if (count > 65535) return KVB_ERR_LIMIT;
-    const Runs runs = {run_chunks, starts, starts + (size_t)count * H * D * Dv};
-    return D <= 64 ? run<MODE, 1>(in, seg, records, total, held, q_scale, memory, out, H, D, Dv, runs, count, err, stream)
-                   : run<MODE, 2>(in, seg, records, total, held, q_scale, memory, out, H, D, Dv, runs, count, err, stream);
+    if (runs.wanted < 0 || (runs.wanted > 0 && (has_z(MODE) || held < total || !runs.starts || runs.least < 1 || runs.from < 0 || run_count < 1)))
+        return KVB_ERR_SHAPE;
+    if (runs.wanted > 0 && run_count > 65535 - seg.count) return KVB_ERR_LIMIT;
+    runs.decays = runs.starts + (size_t)run_count * H * D * Dv;
+    return D <= 64 ? run<MODE, 1>(in, seg, records, total, held, q_scale, memory, out, H, D, Dv, runs, run_count, err, stream)
+                   : run<MODE, 2>(in, seg, records, total, held, q_scale, memory, out, H, D, Dv, runs, run_count, err, stream);
 }
 
 }  // namespace sc
@@ -1031,21 +1061,21 @@ KVB_API int kvb_chunk_shared_floats(int mode, int D) { return mode < 0 || mode >
 // number h of Dv for v; H a multiple of G), `gates` [T, gate_stride] the mode's own numbers (sc::Rows); `records`: scratch of `held` times
 // the floats above for all H heads and G groups, on 16 bytes: a step of more chunks (at most T / 16 + S) goes through it `held` chunks at a
 // time, with the same results.  D up to 128.
-// `held` + (r << 20) (modes 2 and 3, all chunks held): a segment's chunks are walked in runs of r of them at once; behind the records
-// `records` then has (T / (16 r) + S) H (D Dv + D rounded up to 64) floats more.
+// `wanted` runs a segment (0: one; modes 2 and 3, all chunks held): a segment of at least `run_from` chunks is cut into runs of
+// max(run_least, ceil(its chunks / wanted)) of them, which are walked at once; `run_count`: no step of this kind has more runs of segments that have
+// several; `starts`: scratch of run_count H (D Dv + D rounded up to 64) floats.
 KVB_API int kvb_chunk_scan(int mode, const float* rows, int stride, int q_col, int k_col, int v_col, int G, const float* gates,
                            int gate_stride, float q_scale, const int* seg_q_start, const int* seg_q_len, const int* seg_slot, float* memory,
-                           float* out, int T, int S, int H, int D, int Dv, int held, float* records, int* err, cudaStream_t stream) {
-    const int run_chunks = held < 0 ? 0 : held >> 20;
-    if (held > 0) held &= (1 << 20) - 1;
-    float* starts = nullptr;
-    if (run_chunks > 0 && records && D >= 1 && H >= 1 && G >= 1)
-        starts = records + (size_t)held * ((size_t)H * kvb_chunk_record_floats(mode, D) + (size_t)G * kvb_chunk_shared_floats(mode, D));
+                           float* out, int T, int S, int H, int D, int Dv, int held, float* records, int* err, cudaStream_t stream, int wanted,
+                           int run_least, int run_from, int run_count, float* starts) {
     const sc::Rows in = {rows, gates, stride, gate_stride, q_col, k_col, v_col, G > 0 ? H / G : 0};
     const sc::Segments seg = {seg_q_start, seg_q_len, seg_slot, S};
-    if (mode == sc::CHUNK_GATED_DELTA) return sc::run<sc::CHUNK_GATED_DELTA>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, run_chunks, starts, err, stream);
-    if (mode == sc::CHUNK_DELTA_RULE) return sc::run<sc::CHUNK_DELTA_RULE>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, run_chunks, starts, err, stream);
-    if (mode == sc::CHUNK_CHANNEL_DECAY) return sc::run<sc::CHUNK_CHANNEL_DECAY>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, run_chunks, starts, err, stream);
-    if (mode == sc::CHUNK_HEAD_DECAY) return sc::run<sc::CHUNK_HEAD_DECAY>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, run_chunks, starts, err, stream);
+    const sc::Runs runs = {wanted, run_least, run_from, starts, nullptr};
+#define KVB_SCAN(MODE) if (mode == MODE) return sc::run<MODE>(in, seg, records, held, q_scale, memory, out, T, H, G, D, Dv, runs, run_count, err, stream)
+    KVB_SCAN(sc::CHUNK_GATED_DELTA);
+    KVB_SCAN(sc::CHUNK_DELTA_RULE);
+    KVB_SCAN(sc::CHUNK_CHANNEL_DECAY);
+    KVB_SCAN(sc::CHUNK_HEAD_DECAY);
+#undef KVB_SCAN
     return KVB_ERR_SHAPE;
 }

@@ -11,7 +11,7 @@ from __future__ import annotations
 import contextlib
 import ctypes
 from collections import Counter
-from typing import Dict, Optional, Sequence
+from typing import Dict, Optional, Sequence, Tuple
 
 import torch
 
@@ -150,7 +150,7 @@ _SIGNATURES = {
         "kvb_chunk_shared_floats": [_c_int, _c_int],
         "kvb_chunk_scan": [_c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p,
                            _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p,
-                           _c_void_p],
+                           _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     },
     "scan_wide": {
         "kvb_gated_delta_scan_wide": [_c_void_p, _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int,
@@ -280,6 +280,8 @@ _SIGNATURES = {
 
 
 # Only in some variants of a module: attention_flash for head sizes 64 and 128, attention_pairs over pages or over expanded rows.
+# Launchers whose parameters from this one on may be left out (they are zero then).
+_REQUIRED = {"kvb_chunk_scan": 24}
 _OPTIONAL = {"kvb_flash_decode_tma", "kvb_flash_decode_tma_max_clusters", "kvb_attention_pairs", "kvb_attention_pairs_expanded"}
 
 
@@ -301,7 +303,10 @@ class _Library:
                         continue              # a variant compiled for a size that has no such entry point
                     raise
                 address = ctypes.cast(fn, _c_void_p).value
-                setattr(self, fname, calls.Call(address, "".join(_TYPE_LETTERS[t] for t in argtypes), fname))
+                letters = "".join(_TYPE_LETTERS[t] for t in argtypes)
+                if fname in _REQUIRED:
+                    letters = letters[:_REQUIRED[fname]] + "|" + letters[_REQUIRED[fname]:]
+                setattr(self, fname, calls.Call(address, letters, fname))
             self._lib = lib
             return getattr(self, name)
         raise AttributeError(f"module '{self.module}' has no entry point '{name}'")
@@ -1482,27 +1487,34 @@ class CudaKernels(KernelSet):
             return False
         if D > 64 or batch.max_q_len <= 1024:
             return True
-        walkers = H * -(-Dv // 16)
-        return walkers >= self.CHUNK_RUN_MIN_WALKERS and self._chunk_runs("channel_decay", batch.num_tokens, batch.num_segments, walkers) > 1
+        return H * -(-Dv // 16) >= self.CHUNK_RUN_MIN_WALKERS and self._chunk_runs("channel_decay", H, Dv)[0] > 1
 
     # Portions go sixteen tokens at a time (csrc/scan_chunk.cu) where a head has at most CHUNK_SCAN_MAX_DIM key channels.
     CHUNK_SCAN_MAX_DIM = 128
     # Scratch of a scan for portions: longer steps go through it in runs of as many chunks as it holds (16 heads of 128 channels under the delta
     # rule: 39 KB a head and chunk, 6,800 tokens a run; the whole of a step of 30,000 would take 1.2 GB).
     CHUNK_SCRATCH_BYTES = 256 << 20
-    # Where a walk of the decays alone has at most so many blocks and its segments on average so many chunks, they are walked in runs of at
-    # least CHUNK_RUN_MIN, as many as bring it to about CHUNK_RUN_BLOCKS blocks (four an SM).  Whole layers, in us, without and with: decays per
-    # channel, 7 heads of 64 x 128, 2,048 rows 220 and 117, 512 81 and 68, 300 (not taken) 62 and 60; 8 heads of 128 x 256, 2,048 rows 339 and
-    # 280, two requests (256 blocks) 312 and 277, three (384; not taken) 255 and 256, 300 rows (not taken) 85 and 91; decays per head, 28 heads of 128 x
-    # 64, 2,048 rows 277 and 205, two requests (224) 262 and 212, four (448; not taken) 175 and 214; 64 heads (256; not taken) 431 and 455.
+    # Segments of decays alone are walked in several runs of chunks at once, where a walk has at most CHUNK_RUN_MAX_BLOCKS blocks a segment: in as
+    # many as bring one segment to CHUNK_RUN_BLOCKS blocks (four an SM), of at least CHUNK_RUN_MIN chunks.  Whether and how is a matter of
+    # the heads and of the segment alone, so that a request's results are the same bits beside any others.  The ends of runs cost a third of the
+    # walk, which is lost where segments fill the GPU by themselves: so the segments have to be so long that a step of 2,048 rows of nothing
+    # else would be walked by at most 256 blocks (CHUNK_RUN_STEP), and at least CHUNK_RUN_MIN_CHUNKS chunks.  Records and walk in us, without runs and with:
+    # decays per channel, 7 heads of 64 x 128 (56 blocks a segment): 400 rows (25 chunks; not cut) 33 and 22, 512 40 and 25, 1,024 75 and 35, 2,048 147 and
+    # 53, two of 1,024 78 and 55, four of 512 51 and 63, eight of 1,024 160 and 219; 8 heads of 128 x 256 (128 blocks): 768 (not cut) 70 and 62, 1,024
+    # 91 and 76, 2,048 182 and 141, two of 1,024 121 and 135, four of 512 (not cut) 105 and 149; 16 such heads (256; not taken) 2,048 280 and 288, 512 62 and 77;
+    # decays per head, 28 heads of 128 x 64 (112): 768 (not cut) 77 and 61, 1,024 100 and 74, 2,048 193 and 135, two of 1,024 130 and 128, four of 512 (not
+    # cut) 106 and 143; 48 heads (192): 2,048 251 and 198, two of 1,024 (not cut) 165 and 196.
     CHUNK_RUN_BLOCKS, CHUNK_RUN_MIN, CHUNK_RUN_MIN_CHUNKS, CHUNK_RUN_MIN_WALKERS = 592, 4, 24, 16
-    CHUNK_RUN_MAX_BLOCKS = {"channel_decay": 256, "head_decay": 224}
+    CHUNK_RUN_STEP = 296             # 128 chunks: CHUNK_RUN_BLOCKS / 256 of them
+    CHUNK_RUN_MAX_BLOCKS = {"channel_decay": 192, "head_decay": 224}
     CHUNK_MODES = {"gated_delta": 0, "delta_rule": 1, "channel_decay": 2, "head_decay": 3}
 
-    def _chunk_runs(self, mode: str, T: int, S: int, walkers: int) -> int:
-        """Runs to cut a step's chunks into, where a walk has `walkers` blocks a segment (0: none)."""
-        few = walkers * S <= self.CHUNK_RUN_MAX_BLOCKS.get(mode, 0) and T >= 16 * self.CHUNK_RUN_MIN_CHUNKS * S
-        return self.CHUNK_RUN_BLOCKS // walkers if few else 0
+    def _chunk_runs(self, mode: str, H: int, Dv: int) -> Tuple[int, int]:
+        """Runs that a long segment is cut into (0 or 1: none), and the chunks from which one is long."""
+        walkers = H * -(-Dv // 16)
+        if walkers > self.CHUNK_RUN_MAX_BLOCKS.get(mode, 0):
+            return 0, 0
+        return self.CHUNK_RUN_BLOCKS // walkers, max(self.CHUNK_RUN_MIN_CHUNKS, self.CHUNK_RUN_STEP * walkers // self.CHUNK_RUN_BLOCKS)
 
     def _chunk_scan(self, mode: str, rows, cols, G: int, gates, q_scale: float, batch: StepBatch, memory, out, H: int, D: int, Dv: int,
                     workspace) -> None:
@@ -1516,19 +1528,21 @@ class CudaKernels(KernelSet):
         held = min(chunks, max(1, self.CHUNK_SCRATCH_BYTES // (4 * size)))
         # Per run: the records (and their triangular systems) and the walk, one of which has been counted.
         self.launches += -(-chunks // held) * (3 if mode == "delta_rule" else 2) - 1
-        # Decays alone: a run's end is its decays times its start, plus what its tokens leave, so that runs of chunks can be walked at once.
-        run_chunks, floats, walkers = 0, held * size, H * -(-Dv // 16)
-        if held == chunks < 1 << 20 and workspace is not None:
-            runs = self._chunk_runs(mode, T, S, walkers)
-            if runs > S:
-                run_chunks = min(2047, max(self.CHUNK_RUN_MIN, -(-(T // 16) // runs)))      # what the bits above `held` hold
-                floats += (T // (16 * run_chunks) + S) * H * (D * Dv + -(-D // 64) * 64)
-                self.launches += 2
+        # Decays alone: a run's end is its decays times its start, plus what its tokens leave, so that runs of chunks can be walked at once
+        # (not where the records of the step's chunks go through their scratch in parts).
+        runs, floats = (), held * size
+        wanted, long = self._chunk_runs(mode, H, Dv) if held == chunks and workspace is not None else (0, 0)
+        if wanted > 1 and -(-batch.max_q_len // 16) >= long:
+            # Segments that can be long enough, times the runs of each; and no run is shorter than CHUNK_RUN_MIN but a segment's last.
+            count = min(min(S, T // (16 * max(long - 1, 0) + 1)) * wanted, T // (16 * self.CHUNK_RUN_MIN) + S)
+            starts = workspace.buffer("recurrent.chunk_starts", (count * H * (D * Dv + -(-D // 64) * 64),), torch.float32)
+            runs = (wanted, self.CHUNK_RUN_MIN, long, count, _ptr(starts))
+            self.launches += 2
         records = (torch.empty(floats, dtype=torch.float32, device=rows.device) if workspace is None else
                    workspace.buffer("recurrent.chunk_records", (floats,), torch.float32))
         _check(lib.kvb_chunk_scan(code, _ptr(rows), rows.shape[1], *cols, G, _ptr(gates), gates.shape[1], float(q_scale),
                                   _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_slot), _ptr(memory), _ptr(out), T, S, H, D,
-                                  Dv, held + (run_chunks << 20), _ptr(records), _ptr(self.error_word), self._stream()), f"{mode} (chunks)")
+                                  Dv, held, _ptr(records), _ptr(self.error_word), self._stream(), *runs), f"{mode} (chunks)")
 
     def gated_linear_scan(self, proj: torch.Tensor, cols, z: torch.Tensor, tau: float, q_scale: float, batch: StepBatch,
                           memory: torch.Tensor, out: torch.Tensor, H: int, D: int, Dv: int, workspace=None) -> None:

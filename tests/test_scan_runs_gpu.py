@@ -93,3 +93,37 @@ def test_an_infinite_or_undefined_number_goes_where_it_goes_in_one_run(kernels, 
                 assert torch.equal(torch.isfinite(a), torch.isfinite(b)) and torch.equal(torch.isnan(a), torch.isnan(b))
                 ok = torch.isfinite(a)
                 assert (a[ok] - b[ok]).abs().max() <= 2e-5 * a[ok].abs().max()
+
+
+@pytest.mark.parametrize("mode,H,G,D,Dv", [("channel_decay", 7, 7, 64, 128), ("channel_decay", 2, 2, 100, 40), ("head_decay", 28, 1, 128, 64), ("head_decay", 3, 3, 64, 64)])
+def test_a_segment_is_the_same_bits_beside_any_others(kernels, mode, H, G, D, Dv):
+    """With the rule as it is: segments that are cut into runs and ones that are not, alone and in steps with others of any length, also
+    more of them than would be cut if their number counted."""
+    from kvcache_b200.engine.workspace import Workspace
+    g = torch.Generator().manual_seed(9)
+    counts = [1000, 383, 1, 900, 640, 385, 1000]
+    starts, T, ws = [sum(counts[:i]) for i in range(len(counts))], sum(counts), Workspace(DEV)
+    rows = torch.randn(T, 2 * G * D + H * Dv, generator=g).to(DEV)
+    decay = 0.8 + 0.2 * torch.rand(T, H * D if mode == "channel_decay" else H, generator=g)
+    gates = (decay if mode == "channel_decay" else torch.cat([decay, torch.rand(T, H, generator=g)], dim=1)).contiguous().to(DEV)
+    memory = torch.randn(len(counts), H, D, Dv, generator=g).to(DEV)
+
+    def scan(which):
+        part = torch.cat([torch.arange(starts[i], starts[i] + counts[i]) for i in which]).to(DEV)
+        mine = [counts[i] for i in which]
+        batch = SimpleNamespace(seg_q_start=_int32([sum(mine[:i]) for i in range(len(mine))]), seg_q_len=_int32(mine), seg_slot=_int32(list(range(len(mine)))),
+                                num_segments=len(mine), num_tokens=sum(mine), max_q_len=max(mine))
+        state, out, before = memory[list(which)].contiguous(), torch.full((sum(mine), H * Dv), float("nan"), device=DEV), kernels.launches
+        kernels._chunk_scan(mode, rows[part].contiguous(), (0, G * D, 2 * G * D), G, gates[part].contiguous(), 0.5, batch, state, out, H, D, Dv, ws)
+        kernels.check_errors()
+        return dict(zip(which, zip(out.split(mine), state))), kernels.launches - before
+
+    want, cut = {}, set()
+    for i in range(len(counts)):
+        one, launches = scan([i])
+        want.update(one)
+        cut.add(launches == 3)
+    assert cut == {True, False}
+    for which in ([0, 6], [0, 3, 4, 5, 6], list(range(len(counts))), [2, 1, 3]):
+        for i, (out, state) in scan(which)[0].items():
+            assert torch.equal(out, want[i][0]) and torch.equal(state, want[i][1]), (which, i)

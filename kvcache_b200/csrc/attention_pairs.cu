@@ -27,6 +27,13 @@
 // O rescaled by the softmax warps only when a maximum had grown by 2^8 (475, but errors against 64 bits up to a fifth larger: P of
 // the key with the maximum is then not 1 exactly).
 //
+// Errors against 64 bits (2-norms, results rounded to bfloat16; this kernel, that of units, mma.sync): 14 heads of 64 without a history 2.030e-3,
+// 2.039e-3, 2.021e-3; behind 2,048 tokens 2.256, 2.222, 2.188; behind 16,000 2.322, 2.258, 2.258.  The weights' rounding makes them: of every piece of a
+// stream the key with the maximum has the weight 1 exactly, and the other kernels cut long histories into more pieces (that of units with none cut: 2.261
+// behind 2,048 and 2.314 behind 16,000).  (Sums in tensor
+// memory cut off at 2^-24 a step: 1.9e-5 of a result after 16,384 keys, 5.6e-5 where all terms have one sign.)  Whole layers of attention: 1.0004 to
+// 1.0013 times what they were before this kernel on average; of latent attention, expanded and not: 0.995 to 0.999 times.
+//
 // Work is shared out by key tiles: the streams' tiles, laid end to end, are cut into as many equal runs as there are blocks
 // (one an SM), so that all finish together whatever the lengths.  A stream that a cut divides leaves (m, l, O) of its
 // pieces in scratch, two places a block, and the last piece to finish adds them in order (a ticket per stream and tile).
@@ -85,7 +92,8 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// 1 / (1 + e^-x), to about 2^-21 of itself.
+// 1 / (1 + e^-x), to about 2^-21 of itself; the gated result is rounded to 2^-9.  With expf and a division errors of latent layers against 64 bits are
+// the same to 3e-5 of themselves either way (26 steps of 64 to 2,048 rows), and 2,048 rows take 161 us instead of 131 (code that is met cold).
 __device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.f, 1.f + ex2(-1.4426950408889634f * x)); }
 // Two float32 numbers in one 64-bit register, and the multiply-add of such pairs (one instruction for two results).
 __device__ __forceinline__ uint64_t pair(float x, float y) {

@@ -14,7 +14,7 @@
 // expert by reading the experts' matrices.  Storing a tile must stay below that: eight warps store (four before), a row's
 // 16 results by one 32-byte store, and the gated activation takes one reciprocal instruction instead of an IEEE division,
 // which alone held 16 divisions for every 32 columns of a row; the reciprocal is within 1 ulp and the result is rounded to
-// 8 bits.  2,048 rows to 2 of 16 experts (L2 flushed, launch included): up 2432 x 896 52.2 -> 37.6 us, down 896 x 1216
+// 8 bits (28 layers against 64 bits: errors the same to 1e-5 of themselves, either way).  2,048 rows to 2 of 16 experts (L2 flushed, launch included): up 2432 x 896 52.2 -> 37.6 us, down 896 x 1216
 // 31.3 -> 25.6 us; to 4 of 32 experts, up 2752 x 2048 113.6 -> 105.3 us, down 2048 x 1376 71.7 -> 69.6 us.
 #include "tc_common.cuh"
 

@@ -637,10 +637,15 @@ static int launch(const bf16* q, bf16* out, const bf16* k_pages, const int* bloc
 }
 
 // Whether an instance of the kernel for tiles of 16 rows takes these sizes: every row on 16 bytes, Q's sixteens in registers, and as many
-// value columns as the instance of that key size has accumulators for.  Other sizes go to the kernel above.
+// value columns as the instance of that key size has accumulators for.  Other sizes go to the kernel above, and so do those that it is
+// ahead at, since an instance multiplies as many columns whatever the key size and the largest one fills an SM.  Layers of 16 heads in a graph, in us, the kernel
+// above and this one, one token with 300 keys / 8 with 600 / 32 with 4,096: keys of 40 numbers (not taken) 20.3 and 21.1 / 22.6 and 24.6 / 41.7 and 44.9;
+// 96 (not taken) 21.5 and 21.7 / 23.8 and 24.8 / 44.0 and 44.1; 112 22.4 and 22.1 / 24.6 and 24.8 / 47.9 and 45.0; 336 with values of 256 (not taken)
+// 25.9 and 26.7 / 31.9 and 36.5 / 67.4 and 72.0; 336 with 272 26.1 and 27.3 / 29.3 and 31.8 / 87.9 and 71.8; 576 29.6 and 29.6 / 33.5 and 33.4 / 106 and 81.
 static bool rows16_fits(int Dk, int Dv, const void* k_pages) {
     const int most = Dk <= 160 ? 128 : Dk <= 320 ? 256 : 512;
-    return Dk <= 576 && Dv <= Dk && Dv <= most && !((uintptr_t)k_pages & 15);
+    const bool two_blocks_above = Dk > 320 && Dk <= 352 && Dv <= 256;       // two blocks an SM of the kernel above, one of the largest instance
+    return Dk >= 104 && Dk <= 576 && Dv <= Dk && Dv <= most && !two_blocks_above && !((uintptr_t)k_pages & 15);
 }
 
 template <int NV, int KS, int STAGES, int BLOCKS>

@@ -503,8 +503,9 @@ class CudaKernels(KernelSet):
         return self._latent_blocks_wanted(key_dim, value_dim), tile
 
     def _latent_blocks_wanted(self, key_dim: int, value_dim: int) -> int:
-        """As many blocks as the GPU holds at once of the kernel's form for decoded tokens (tiles of 16 rows, two key stages):
-        two an SM while their shared memory allows (csrc/latent_flash.cu, make_layout), else one - a second wave of blocks
+        """As many blocks as the GPU holds at once of the kernels for decoded tokens (tiles of 16 rows): two an SM while the shared memory of the
+        general one with two key stages allows (csrc/latent_flash.cu, make_layout; of the sizes that go to the other, its instances for keys of up to
+        320 numbers have two, the larger one one), else one - a second wave of blocks
         costs more than longer runs of keys per block (8 requests of 4,096 tokens, rows of 576: 20.0 us with 144 blocks, 22.9 with 256)."""
         dk_pad = -(-key_dim // 32) * 32
         row = max(dk_pad, 64 * (1 if value_dim <= 64 else 2 if value_dim <= 128 else 4 if value_dim <= 256 else 8)) + 8

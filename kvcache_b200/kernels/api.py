@@ -362,16 +362,22 @@ class CudaKernels(KernelSet):
         # (bfloat16, head size 64 or 128, pages of 8..64 tokens); None turns it off.  Measured on 24 layers of the
         # 0.5B shape: the mma.sync kernel is ahead at 128 and 256 rows (1.09 / 1.24 ms a step against 1.14 / 1.28),
         # the tensor-memory kernel from 512 rows on (1.56 against 1.69 ms).
-        # Behind a longer history (the plan cuts the portion's tiles into this many units) it is ahead from 128 rows on: 128 rows
-        # behind 2,000 tokens 29.7 against 39.9 us (16 heads of 128), 25.6 and 25.6 (14 heads of 64); 200 behind 8,000 60 against 137, 40 and 69.
+        # Behind a longer history (the plan cuts the portion's tiles into this many units) it is ahead from 128 rows on - heads of 64 with at least
+        # a tile of work an SM (`_portion_line`) or a short window -: 128 rows behind 2,000 tokens 29.7 against 39.9 us (16 heads of 128), 25.6 and 25.6 (14 heads of
+        # 64); 200 behind 8,000 60 against 137, 40 and 69; two heads of 64 (not taken) 26.5 against 20.8, four 26.7 against 28.7, eight
+        # with a window of 256 12.0 against 14.2.
         self.tc_attention_min_rows: Optional[int] = 384
         self.tc_history_min_rows, self.tc_history_min_units = 128, 3
-        # Steps that the plan cuts into at least this many units - heads of 64: also two a tile, which they are behind some history -
-        # go through the kernel for pairs of row tiles (csrc/attention_pairs.cu), whose set-up and merge cost more and whose tiles
-        # cost less.  On both sides of the lines, in us, this kernel and that, 16 heads of 128 and 14 of 64: 800 rows (7 units in 7
-        # tiles) 25.5 and 29.7, 23.6 and 23.6; 1,024 rows (8 in 8) 29.5 and 29.7, 23.5 and 21.5; 800 behind 500 (10 in 7) 37.8 and
-        # 35.8, 25.5 and 27.5; 512 behind 2,000 (12 in 4) 48 and 37.9, 29.7 and 27.6; 2,048 (24 in 16) 61 and 43, 32.8 and 33.6 (24
-        # layers of a step of the latter: 2,490 and 2,565); 2,048 behind 2,048 150 and 76, 71 and 53.
+        # Steps that the plan cuts into at least this many units (0: all) - heads of 64: also two a tile, which they are behind some history -
+        # and that bring every SM enough work go through the kernel for pairs of row tiles (csrc/attention_pairs.cu), whose set-up and
+        # merge cost more and whose tiles cost less.  What an SM has to get, in tiles of 256 rows x 128 keys of one head: four with
+        # heads of 128, eight with heads of 64, or where no tile of rows is cut into units (these are short, and the line overestimates them).
+        # This kernel and that of units, in us, each launch by itself (heads x line an SM): 2,048 rows behind 2,048: heads of 128, one (1.5) 40 and 29,
+        # two (3.0) 34 and 30, four (6.1) 37 and 47, sixteen (24) 72 and 143; heads of 64, four (6.1) 28 and 27, eight (12) 37 and 44, sixteen 55 and 74.
+        # 200 behind 8,000: heads of 128, four (1.8) 70 and 32, eight (3.7) 52 and 33, sixteen (7.3) 50 and 55.  2,048 behind none: heads of
+        # 128, four (2.6) 28 and 28, eight (5.2) 30 and 34; four requests of 512 behind none (no tile cut): sixteen (6.9) 25.1 and 22.5, 32 (14)
+        # 37 and 40.  Windows: 2,048 behind 2,048 with 256 keys, heads of 128: eight (2.2) 24 and 19, sixteen (4.3) 20 and 31; heads of 64 want tiles
+        # with at least eleven tiles of keys: 32 heads (8.6) 37 and 32, with a window of 1,024 (19) 60 and 69.
         self.tc_pairs_min_units: Optional[int] = 8
         self.tc_pairs_units_a_tile = {64: 2, 128: 1}
         self.tc_pairs_min_tiles = TC_PAIR_MIN_KEY_TILES
@@ -907,6 +913,29 @@ class CudaKernels(KernelSet):
     # figures on both sides of the lines: csrc/attention_generic.cu.
     ROWS32_MIN, ROWS32_MIN_SHARED = 64, 32
 
+    @staticmethod
+    def _portion_line(counts, heads: int, reach: int) -> Tuple[int, int]:
+        """About how many tiles of 256 rows x 128 keys, all heads together, a step's portions are, and the most that one pair of row
+        tiles has (a plan's unit is 128 rows x 1,024 keys at most; it does not know the layer's window or chunk, `reach`)."""
+        most = (abs(reach) + 255) // 128 + 2 if reach else 1 << 30
+        return heads * min(4 * counts["tc_units"], counts["tc_pairs"] * most), most
+
+    def _history_ahead(self, counts, heads: int, reach: int) -> bool:
+        """Whether portions of few rows and heads of 64 behind a history leave the mma.sync kernel."""
+        line, most = self._portion_line(counts, heads, reach)
+        return line >= self.sm_count or most < 11
+
+    def _pairs_ahead(self, counts, heads: int, D: int, reach: int) -> bool:
+        """Whether a step's portions go through the kernel for pairs of row tiles rather than the one for units."""
+        units, tiles = counts["tc_units"], counts["tc_tiles"]
+        if self.tc_pairs_min_units is None or not 0 < counts["tc_pairs"] <= TC_MAX_PAIRS or units < self.tc_pairs_units_a_tile[D] * tiles:
+            return False
+        if self.tc_pairs_min_units == 0:
+            return True
+        line, most = self._portion_line(counts, heads, reach)
+        return (units >= self.tc_pairs_min_units and line >= self.sm_count * (4 if D == 128 and units > tiles else 8)
+                and (D == 128 or most >= 11))
+
     def paged_attention(self, q: torch.Tensor, batch: StepBatch, kv: PagedKVView, out: torch.Tensor,
                         num_heads: int, scale: float, workspace=None, sink: Optional[torch.Tensor] = None,
                         score_cap: Optional[float] = None, slopes: Optional[torch.Tensor] = None, reach: Optional[int] = None) -> None:
@@ -975,10 +1004,10 @@ class CudaKernels(KernelSet):
             lib = self._flash_library(D)
             counts, lists = plan.counts, plan.arrays
             long_portion = (self.tc_attention_min_rows is not None and D in (64, 128) and 8 <= kv.page_size <= 64
-                            and (batch.max_q_len >= self.tc_attention_min_rows or (batch.max_q_len >= self.tc_history_min_rows
-                                                                                   and counts["tc_units"] >= self.tc_history_min_units)))
-            if (long_portion and self.tc_pairs_min_units is not None and 0 < counts["tc_pairs"] <= TC_MAX_PAIRS
-                    and counts["tc_units"] >= max(self.tc_pairs_min_units, self.tc_pairs_units_a_tile[D] * counts["tc_tiles"])):
+                            and (batch.max_q_len >= self.tc_attention_min_rows
+                                 or (batch.max_q_len >= self.tc_history_min_rows and counts["tc_units"] >= self.tc_history_min_units
+                                     and (D == 128 or self._history_ahead(counts, num_heads, reach)))))
+            if long_portion and self._pairs_ahead(counts, num_heads, D, reach):
                 pairs_lib = self._attn_pairs.get(D)
                 if pairs_lib is None:
                     pairs_lib = self._attn_pairs[D] = _Library("attention_pairs", f"d{D}", [f"-DKVB_HEAD_DIM={D}"])

@@ -101,13 +101,23 @@ def test_a_row_whose_maximum_grows_with_every_tile(kernels, request):
         assert_close(out, ref, TOL)
 
 
-def test_launches_of_the_two_kernels_can_be_told_apart(kernels):
+# (heads of, heads, segments, window, kernel): both sides of every line of the rule
+ROUTES = [(64, 14, [(0, 400)], None, "attention_units"), (64, 14, [(2048, 1024)], None, "attention_pairs"), (64, 4, [(2048, 2048)], None, "attention_units"),
+          (64, 14, [(0, 2048)], None, "attention_units"), (64, 28, [(2048, 2048)], 256, "attention_units"), (64, 28, [(2048, 2048)], 1024, "attention_pairs"),
+          (64, 14, [(2048, 130)], None, "attention_units"), (64, 2, [(8000, 200)], None, None), (64, 2, [(2048, 200)], 256, "attention_units"),
+          (128, 16, [(0, 800)], None, "attention_units"), (128, 16, [(2048, 512)], None, "attention_pairs"), (128, 2, [(2048, 512)], None, "attention_units"),
+          (128, 16, [(0, 512)] * 4, None, "attention_units"), (128, 32, [(0, 512)] * 4, None, "attention_pairs"), (128, 8, [(2048, 2048)], 256, "attention_units"),
+          (128, 2, [(2048, 130)], None, "attention_units")]
+
+
+@pytest.mark.parametrize("route", ROUTES)
+def test_which_kernel_a_portion_takes(kernels, route):
     from kvcache_b200.engine.workspace import Workspace
-    for segments, form in (([(0, 400)], "attention_units"), ([(2048, 1024)], "attention_pairs")):
-        batch, kv = paged_scenario(segments, num_kv_heads=2, head_dim=64, page_size=16, dtype=torch.bfloat16, device=DEV, seed=3)
-        q = torch.randn(batch.num_tokens, 14 * 64, device=DEV).to(torch.bfloat16)
-        before, names = dict(kernels.launch_forms), kernels.launch_counts["attention_tc"]
-        kernels.paged_attention(q, batch, kv, torch.empty_like(q), 14, 0.125, Workspace(DEV))
-        kernels.check_errors()
-        assert {f for f, n in kernels.launch_forms.items() if n > before.get(f, 0)} == {form}
-        assert kernels.launch_counts["attention_tc"] == names + 1
+    D, H, segments, window, form = route
+    batch, kv = paged_scenario(segments, num_kv_heads=2, head_dim=D, page_size=16, dtype=torch.bfloat16, device=DEV, seed=3, window=window)
+    q = torch.randn(batch.num_tokens, H * D, device=DEV).to(torch.bfloat16)
+    before, names = dict(kernels.launch_forms), kernels.launch_counts["attention_tc"]
+    kernels.paged_attention(q, batch, kv, torch.empty_like(q), H, D ** -0.5, Workspace(DEV))
+    kernels.check_errors()
+    assert {f for f, n in kernels.launch_forms.items() if n > before.get(f, 0)} == ({form} if form else set())
+    assert kernels.launch_counts["attention_tc"] == names + (form is not None)

@@ -43,9 +43,9 @@ struct Call {
 };
 
 // The address of a contiguous tensor on the device; false with an exception set.  Every question to the tensor may throw (a layout
-// without strides, a subclass that answers in Python, a tensor without storage); torch's own frame for that, HANDLE_TH_ERRORS, also
-// collects warnings, which cost a layer of four launches 3 us.
-bool address_of(PyObject* obj, W& out) try {
+// without strides, a subclass that answers in Python, a tensor without storage): the functions that Python calls catch that, by
+// `translated` - torch's own frame, HANDLE_TH_ERRORS, also collects warnings, which cost a layer of four launches 3 us.
+bool address_of(PyObject* obj, W& out) {
     const at::Tensor& t = THPVariable_Unpack(obj);
     if (!t.is_contiguous()) {
         PyErr_SetString(kernel_error ? kernel_error : PyExc_RuntimeError, "kernels take contiguous tensors");
@@ -58,9 +58,11 @@ bool address_of(PyObject* obj, W& out) try {
     }
     out = reinterpret_cast<W>(t.data_ptr());
     return true;
-} catch (...) {
+}
+
+PyObject* translated() {
     torch::translate_exception_to_python(std::current_exception());
-    return false;
+    return nullptr;
 }
 
 bool pointer_of(PyObject* obj, W& out) {
@@ -88,25 +90,29 @@ PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* k
     float f[MAX_FLOATS] = {};
     W w[MAX_OTHERS] = {};
     int nf = 0, nw = 0;
-    for (Py_ssize_t i = 0; i < n; ++i) {
-        switch ((*c->types)[i]) {
-            case 'p':
-                if (!pointer_of(args[i], w[nw++])) return nullptr;
-                break;
-            case 'f': {
-                const double v = PyFloat_AsDouble(args[i]);
-                if (v == -1.0 && PyErr_Occurred()) return nullptr;
-                f[nf++] = (float)v;
-                break;
-            }
-            default: {
-                const long long v = PyLong_AsLongLong(args[i]);
-                if (v == -1 && PyErr_Occurred()) return nullptr;
-                if ((*c->types)[i] == 'i' && (v < INT_MIN || v > INT_MAX))
-                    return PyErr_Format(PyExc_OverflowError, "argument %zd of %U does not fit an int", i + 1, c->name);
-                w[nw++] = v;
+    try {
+        for (Py_ssize_t i = 0; i < n; ++i) {
+            switch ((*c->types)[i]) {
+                case 'p':
+                    if (!pointer_of(args[i], w[nw++])) return nullptr;
+                    break;
+                case 'f': {
+                    const double v = PyFloat_AsDouble(args[i]);
+                    if (v == -1.0 && PyErr_Occurred()) return nullptr;
+                    f[nf++] = (float)v;
+                    break;
+                }
+                default: {
+                    const long long v = PyLong_AsLongLong(args[i]);
+                    if (v == -1 && PyErr_Occurred()) return nullptr;
+                    if ((*c->types)[i] == 'i' && (v < INT_MIN || v > INT_MAX))
+                        return PyErr_Format(PyExc_OverflowError, "argument %zd of %U does not fit an int", i + 1, c->name);
+                    w[nw++] = v;
+                }
             }
         }
+    } catch (...) {
+        return translated();
     }
     int code;
     Py_BEGIN_ALLOW_THREADS
@@ -161,7 +167,11 @@ PyObject* ptr(PyObject*, PyObject* obj) {
     W at = 0;
     if (obj == Py_None) return PyLong_FromLong(0);
     if (!THPVariable_Check(obj)) return PyErr_Format(PyExc_TypeError, "expected a tensor or None, got %R", (PyObject*)Py_TYPE(obj));
-    if (!address_of(obj, at)) return nullptr;
+    try {
+        if (!address_of(obj, at)) return nullptr;
+    } catch (...) {
+        return translated();
+    }
     return PyLong_FromVoidPtr(reinterpret_cast<void*>(at));
 }
 

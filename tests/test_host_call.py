@@ -52,6 +52,18 @@ def test_every_parameter_arrives(calls, library):
             many(*args[:place], wrong, *args[place + 1:])
 
 
+def test_parameters_that_may_be_left_out(calls, library):
+    many = calls.Call(ctypes.cast(library.many, ctypes.c_void_p).value, "ipfilpifiipfiliip|iii", "many")
+    args = [4, None, 0.5, 1, 2, None, 5, 1.5, 6, 7, None, 3.0, 8, 9, 10, 11, ctypes.c_void_p(12), 13, 14, 15]
+    library.look.restype = ctypes.c_int64
+    for given in (20, 18, 17):
+        assert many(*args[:given]) == 1
+        assert [library.look(i) for i in (13, 14, 15, 16)] == [12] + [v if 17 + i < given else 0 for i, v in enumerate((13, 14, 15))]
+    for wrong in (args[:16], args + [1]):
+        with pytest.raises(TypeError):
+            many(*wrong)
+
+
 def test_tensors_that_a_launcher_cannot_take(calls, library):
     from kvcache_b200.kernels.api import KernelError, _ptr
     many = calls.Call(ctypes.cast(library.many, ctypes.c_void_p).value, "ipfilpifiipfiliipiii", "many")

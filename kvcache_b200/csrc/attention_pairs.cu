@@ -74,24 +74,7 @@ constexpr float NEG_INF = -INFINITY;
 // the results), in tiles.
 constexpr int STREAM_COST = 1;
 constexpr int TURN_AT = D == 64 ? 64 : 96;            // the thirty-two keys after whose exponentials a group lets the other go on with its own
-// Shared-memory descriptor of an MN-major operand with 128-byte swizzle: rows of 64 elements (128 bytes) along
-// MN, 8 rows along K form a 1024-byte swizzle atom (stride-dimension offset), the next 64 elements along MN lie
-// `lbo_bytes` further (leading-dimension offset).
-__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lbo_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr & 0x3FFFF) >> 4);
-    d |= (uint64_t)(lbo_bytes >> 4) << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 // 1 / (1 + e^-x), to about 2^-21 of itself; the gated result is rounded to 2^-9.  With expf and a division errors of latent layers against 64 bits are
 // the same to 3e-5 of themselves either way (26 steps of 64 to 2,048 rows), and 2,048 rows take 161 us instead of 131 (code that is met cold).
 __device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.f, 1.f + ex2(-1.4426950408889634f * x)); }

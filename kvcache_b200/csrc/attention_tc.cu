@@ -54,25 +54,6 @@ constexpr int TMEM_COLS = D == 64 ? 256 : 512;       // S: 2 x 64 columns, O_t: 
 constexpr int THREADS = 192;                         // warps 0-3: softmax rows; warp 4: keys and Q K^T; warp 5: values and P V
 constexpr float NEG_INF = -INFINITY;
 
-// Shared-memory descriptor of an MN-major operand with 128-byte swizzle: rows of 64 elements (128 bytes) along
-// MN, 8 rows along K form a 1024-byte swizzle atom (stride-dimension offset), the next 64 elements along MN lie
-// `lbo_bytes` further (leading-dimension offset).
-__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lbo_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr & 0x3FFFF) >> 4);
-    d |= (uint64_t)(lbo_bytes >> 4) << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 struct Params {
     bf16* out;                 // [T, Hq * D]
     const int* block_table;    // [segments, table_stride]

@@ -133,15 +133,12 @@ class LatentAttention(Mixer):
             self.sink_logits = tensors[f"{p}sink"].to(torch.float32).to(device).contiguous()
         # [H, kv_rank, dim]: the transposed key expansion, which takes a head's unrotated query to the latent's space.
         self.w_uk_t = place(tensors[f"{p}uk"].view(H, self.dim, self.kv_rank).transpose(1, 2))
-        if self.dtype == torch.bfloat16 and self.dim == self.vdim:
-            # Both expansions as they are, one product for portions of prompts; the values' half also serves the other order.
-            self.w_ukv = place(torch.cat([tensors[f"{p}uk"], tensors[f"{p}uv"]], dim=0))
-            self.w_uv = self.w_ukv[H * self.dim:].view(H, self.vdim, self.kv_rank)
-        else:
-            self.w_uv = place(tensors[f"{p}uv"].view(H, self.vdim, self.kv_rank))
+        self.w_uv = place(tensors[f"{p}uv"].view(H, self.vdim, self.kv_rank))
+        self.w_ukv = None
         self.w_o = place(tensors[f"{p}o"])
 
     def weight_bytes(self) -> int:
+        # What a step of decoded tokens reads: not `w_ukv`, which portions read in the place of `w_uk_t` and `w_uv`.
         mats = [m for m in (self.w_in, self.w_uq, self.w_uk_t, self.w_uv, self.w_o) if m is not None]
         return sum(m.numel() * m.element_size() for m in mats) + 4 * ((self.q_rank or 0) + self.kv_rank)
 
@@ -156,7 +153,15 @@ class LatentAttention(Mixer):
                  planner(self.num_heads, self.key_dim, self.kv_rank),)
         expand = getattr(kernels, "latent_expand_planner", None)
         more = expand(self.dim, self.vdim, self.rot_dim, self.kv_rank, self.window) if expand and self.dtype == torch.bfloat16 else None
-        return plans + (more,) if more is not None else plans
+        if more is None:
+            return plans
+        if self.w_ukv is None and self.w_uk_t is not None:
+            # Both expansions as they are, one product for portions of prompts, where the kernel set has one for these sizes; the values'
+            # half also serves the other order.
+            rows = self.num_heads * self.dim
+            self.w_ukv = torch.cat([self.w_uk_t.transpose(1, 2).reshape(rows, self.kv_rank), self.w_uv.reshape(-1, self.kv_rank)])
+            self.w_uv = self.w_ukv[rows:].view(self.w_uv.shape)
+        return plans + (more,)
 
     def forward(self, x: torch.Tensor, ctx: LayerContext) -> torch.Tensor:
         T, H = x.shape[0], self.num_heads

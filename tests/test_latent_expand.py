@@ -32,6 +32,31 @@ def test_lists_cover_every_key_that_a_row_sees(segments, window):
     assert planner.plan(np.asarray([40000]), np.asarray([100]))[1]["blocks"] == (0 if not window else 2 + (window > 1) + (window > 200))
 
 
+def test_weights_of_the_expansion_are_held_where_a_kernel_set_takes_the_sizes():
+    from kvcache_b200.kernels.latent_plan import LatentAttentionPlanner, LatentExpandPlanner
+    from kvcache_b200.parts.latent_attention import LatentAttention
+    from kvcache_b200.parts.position import RotaryHalf
+
+    class Kernels:
+        def latent_attention_planner(self, *sizes): return LatentAttentionPlanner(sizes[0], 148)
+        def latent_expand_planner(self, dim, vdim, rot_dim, kv_rank, window=None): return LatentExpandPlanner(0) if dim == 64 else None
+
+    for dim, dtype in ((64, "bfloat16"), (48, "bfloat16"), (64, "float32")):
+        part = LatentAttention(96, 3, dim, 16, dim, 40, 24, scale=0.1, eps=1e-6, position=RotaryHalf(16, 10000.0, 64), prefix="l.", dtype=dtype)
+        g = torch.Generator().manual_seed(1)
+        tensors = {name: torch.randn(*spec.shape, generator=g).to(getattr(torch, dtype)) for name, spec in part.tensor_specs().items()}
+        for _ in range(2):                                     # also after weights have been bound anew
+            part.bind(tensors, torch.device("cpu"))
+            read, uv = part.weight_bytes(), part.w_uv.clone()
+            assert part.w_ukv is None
+            expands = dim == 64 and dtype == "bfloat16"
+            for _ in range(2):
+                assert len(part.step_planners(Kernels())) == 1 + expands
+            assert (part.w_ukv is not None) == expands and part.weight_bytes() == read and torch.equal(part.w_uv, uv)
+            if expands:
+                assert torch.equal(part.w_ukv, torch.cat([tensors["l.uk"], tensors["l.uv"]])) and part.w_uv.data_ptr() == part.w_ukv[3 * dim:].data_ptr()
+
+
 CASES = [
     # (segments, heads, dim, rot, rank, page, extra columns of q's rows, window, sink, one gate a head)
     ([(0, 64)], 3, 64, 16, 64, 16, 0, None, False, False),

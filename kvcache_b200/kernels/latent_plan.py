@@ -74,9 +74,10 @@ class LatentAttentionPlanner(StepPlanner):
 EXPAND_BLOCK = 128               # keys of a block of expanded rows: the key tile of csrc/attention_pairs.cu
 EXPAND_MAX_BLOCKS = 256          # blocks a step may bring
 EXPAND_MAX_PAIRS = 128           # pairs of row tiles (csrc/attention_pairs.cu, MAX_TILES)
-# Rows that every request of the step brings: an expanded key has to serve many.  A whole layer on both sides, in us, keys as they are
-# and expanded, 16 heads of 128 (rank 512) and 14 of 64 (rank 256): 64 rows 73 and 61, 52 and 45; 64 behind 2,000 93 and 89, 62.5 and 63;
-# four requests of 50 behind 2,000 208 and 206, 97 and 98; 128 behind 2,000 140 and 93, 80 and 63; 2,048 536 and 168, 269 and 90.
+# Rows that every request of the step brings: an expanded key has to serve many.  A whole layer launched from Python on both sides, in us, keys
+# as they are and expanded, 16 heads of 128 (rank 512) and 14 of 64 (rank 256): 64 rows 80 and 60, 70 and 61; 64 behind 2,000 87 and 78, 70 and 61;
+# 128 behind 2,000 129 and 83, 77 and 61; 2,048 528 and 132, 261 and 80; four requests of 50 behind 2,000 (not taken) 189 and 126, 91 and 77: the line
+# could lie lower.
 EXPAND_MIN_ROWS = 64
 
 
